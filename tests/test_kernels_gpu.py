@@ -266,6 +266,22 @@ def test_gemm_simple_float32(M, N, K):
     assert (x.double() - want).abs().max().item() <= tol
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 129, 33), (9, 257, 36), (16, 130, 63), (17, 65, 31), (65, 63, 100), (1153, 8390, 37), (1153, 8390, 40)])
+def test_gemm_simple_tiles(M, N, K):
+    """Sizes at the edges of every tile and of the 16-byte loads: a row's bits do not depend on the tile its call's sizes pick."""
+    from sprout_lm_b200 import kernels
+    a, w = rand(M, K), rand(N, K, seed=1)
+    out = torch.empty(M, N, device=DEV)
+    kernels.gemm_simple(a, w, out)
+    want = a.double() @ w.double().T
+    tol = 4 * 6e-8 * math.sqrt(K) * want.abs().max().item() + 1e-6      # sequential float32 accumulation
+    assert (out.double() - want).abs().max().item() <= tol
+    for first, rows in ((M - 1, 1), (0, min(M, 16)), (0, min(M, 17))):
+        part = torch.empty(rows, N, device=DEV)
+        kernels.gemm_simple(a[first:first + rows], w, part)
+        assert torch.equal(part, out[first:first + rows])
+
+
 @pytest.mark.parametrize("orientation", [0, 1, 2, 3, 4])
 @pytest.mark.parametrize("M,N,K", SHAPES)
 def test_gemm_bf16_tensor_cores(status, M, N, K, orientation):
