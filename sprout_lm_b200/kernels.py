@@ -36,6 +36,7 @@ _SIGNATURES = {
     "sprout_rope_append": [_P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_gemm_simple": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "sprout_attention_simple": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "sprout_attention_tile": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_sample": [_P, _I, _P, _P, _P, _P, _I, _I, _P, _P],
     "sprout_advance_decode": [_P, _P, _P, _P, _P, _P, _I, _I, _P],
     "sprout_feed_tokens": [_P, _P, _P, _I, _I, _I, _P],
@@ -348,6 +349,33 @@ def attention_simple(q, k_cache, v_cache, block_table, seq_of_token, positions, 
          _ptr(seq_of_token, "seq_of_token", torch.int32), _ptr(positions, "positions", torch.int32),
          _ptr(out, "out"), out.stride(0), _dtype_code(q.dtype), T, heads, kv_heads, head_dim, k_cache.shape[2],
          k_cache.shape[0], _ptr(status, "status", torch.int32), _stream())
+
+
+# float32 attention by tiles of 32 tokens: from this many tokens of one request in the step on (a single token leaves 31 of a
+# tile's 32 rows idle, and the kernel of one block per token and head then has more blocks)
+ATTENTION_TILE_TOKENS = 16
+
+
+def attention_tile(q, k_cache, v_cache, block_table, q_start, positions, out, heads, kv_heads, head_dim, longest, status):
+    """``attention_simple`` for float32 steps with prompt portions, bit for bit, 32 tokens of a request at a time; ``q_start``: int32
+    [requests + 1], ``longest``: the most tokens that one request has.  head_dim 64 or 128."""
+    _rows_contiguous(q, "q")
+    _rows_contiguous(out, "out")
+    _rows_contiguous(block_table, "block_table")
+    T, requests = q.shape[0], q_start.numel() - 1
+    if q.shape[1] != heads * head_dim or tuple(out.shape) != (T, heads * head_dim):
+        raise KernelError("attention_tile: q and out must be [tokens, heads * head_dim]")
+    if k_cache.shape != v_cache.shape or tuple(k_cache.shape[1:]) != (kv_heads, k_cache.shape[2], head_dim) \
+            or not k_cache.is_contiguous() or not v_cache.is_contiguous():
+        raise KernelError("attention_tile: caches must be contiguous [pages, kv_heads, page_tokens, head_dim]")
+    if not (q.dtype == out.dtype == k_cache.dtype == v_cache.dtype == torch.float32):
+        raise KernelError("attention_tile: q, out and the caches must be float32")
+    if block_table.shape[0] < requests or positions.numel() != T:
+        raise KernelError("attention_tile: a block table row per request and a position per token")
+    _run("sprout_attention_tile", _ptr(q, "q"), q.stride(0), _ptr(k_cache, "k_cache"), _ptr(v_cache, "v_cache"),
+         _ptr(block_table, "block_table", torch.int32), block_table.stride(0), _ptr(q_start, "q_start", torch.int32),
+         _ptr(positions, "positions", torch.int32), _ptr(out, "out"), out.stride(0), requests, longest, heads, kv_heads, head_dim,
+         k_cache.shape[2], k_cache.shape[0], _ptr(status, "status", torch.int32), _stream())
 
 
 def gemm_bf16(a, weight, out, status, bias=None, residual=None, orientation=0, split_k=1, swiglu=False, gate_activation="silu",
@@ -891,6 +919,9 @@ def paged_attention(q, cache, ctx, out, heads, kv_heads, head_dim, status):
                 variant = "mma_sync"
             return attention_prefill(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out,
                                      heads, kv_heads, head_dim, status, variant=variant)
+    elif head_dim in (64, 128) and ctx.max_q_len >= ATTENTION_TILE_TOKENS and cache.k.data_ptr() % 16 == 0 and cache.v.data_ptr() % 16 == 0:
+        return attention_tile(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out, heads, kv_heads, head_dim,
+                              ctx.max_q_len, status)
     attention_simple(q, cache.k, cache.v, cache.block_table, ctx.seq_of_token, ctx.positions, out,
                      heads, kv_heads, head_dim, status)
 
@@ -1880,5 +1911,5 @@ def describe_status(word: int) -> str:
 
 
 __all__ = ["KernelError", "BuildError", "load_library", "library_file", "embed", "rmsnorm", "swiglu",
-           "rope_append", "gemm_simple", "gemm_bf16", "attention_simple", "attention_decode", "attention_decode_fused", "attention_decode_resident", "decode_attention_plan", "decode_fusable", "attention_prefill",
+           "rope_append", "gemm_simple", "gemm_bf16", "attention_simple", "attention_tile", "attention_decode", "attention_decode_fused", "attention_decode_resident", "decode_attention_plan", "decode_fusable", "attention_prefill",
            "paged_attention", "sample", "advance_decode", "feed_tokens", "describe_status"]

@@ -558,6 +558,26 @@ def test_attention_simple(status, dtype, heads, kv_heads, head_dim, page, length
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page,lengths,q_counts", [
+    (14, 2, 64, 16, [300, 129, 16], [300, 1, 15]), (4, 4, 64, 8, [31, 32, 33], [31, 32, 33]), (2, 1, 128, 16, [128, 257, 1], [1, 130, 1]),
+    (6, 2, 128, 4, [129], [127])])
+def test_attention_tile(status, heads, kv_heads, head_dim, page, lengths, q_counts):
+    """Edges of the 32-token tiles and the 128-key chunks, portions behind cached tokens: bit for bit the kernel of one token and
+    head a block, also beside a value that only a later token sees and that is infinite."""
+    from sprout_lm_b200 import kernels
+    case = build_paged_case(torch.float32, heads, kv_heads, head_dim, page, lengths, q_counts)
+    last = lengths[0] - 1                                         # the first request's last position
+    case["v_cache"][case["table"][0, last // page].item(), :, last % page] = float("inf")
+    one, tiled = torch.empty(case["T"], heads * head_dim, device=DEV), torch.empty(case["T"], heads * head_dim, device=DEV)
+    kernels.attention_simple(case["q"], case["k_cache"], case["v_cache"], case["table"], case["seq_of_token"],
+                             case["positions"], one, heads, kv_heads, head_dim, status)
+    kernels.attention_tile(case["q"], case["k_cache"], case["v_cache"], case["table"], case["q_start"], case["positions"], tiled,
+                           heads, kv_heads, head_dim, max(q_counts), status)
+    assert torch.equal(one, tiled)
+    assert torch.isfinite(tiled[:q_counts[0] - 1]).all() and torch.isinf(tiled[q_counts[0] - 1]).all()
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("where", [0, 15, 16, 255, 256, 383, 500])
 def test_attention_finds_one_far_key_among_hundreds(status, dtype, where):
