@@ -29,8 +29,10 @@
 //                               the head and the scale happen on the accumulators.  Prompt portions and single
 //                               tokens of a mixed batch in one launch.
 #include "attention_bf16.cuh"
+#include "maps_attention.cuh"
 
 using namespace sprout_attn;
+using namespace sprout_maps;
 
 namespace {
 
@@ -175,27 +177,6 @@ rope_maps_append_kernel(T* __restrict__ rows, int row_stride, const int* __restr
     v_cache[(((size_t)page * kv_heads + g) * page_tokens + pos % page_tokens) * vdim + e] = vrow[i];
   }
 }
-
-// The first position that a query at `pos` sees: 0 (causal), pos - size + 1 (a window of `size` positions, itself
-// included) or the start of its chunk of `size` positions counted from position 0.
-// `keep` (a window only): the first `keep` positions stay visible to every later query, at their own positions.
-enum MaskKind : int { MASK_CAUSAL = 0, MASK_WINDOW = 1, MASK_CHUNK = 2 };
-// cap * tanh(s / cap) for the bfloat16 kernel: through one exponential, absolute error about cap * 2e-7
-__device__ __forceinline__ float soft_cap_fast(float s, float cap, float inv_cap) {
-  const float e = __expf(2.0f * s * inv_cap);
-  return cap * (1.0f - __fdividef(2.0f, e + 1.0f));
-}
-__device__ __forceinline__ int first_visible(int kind, int size, int pos) {
-  if (kind == MASK_WINDOW) return max(0, pos - size + 1);
-  if (kind == MASK_CHUNK) return pos < 0 ? 0 : (pos / size) * size;
-  return 0;
-}
-
-// Turns a head's output back by the query's position (values that were turned by theirs): tables float32
-// [positions, vdim / 2]; null: no turn.  Pair m is (m, m + vdim / 2), or (2m, 2m + 1) when `interleaved`.
-struct OutputTurn {
-  const float* cos; const float* sin; int positions, interleaved;
-};
 
 template <typename T, int MAPS>
 __global__ void __launch_bounds__(CHUNK)
@@ -345,35 +326,6 @@ multimap_attention_simple_kernel(const T* __restrict__ q, int q_stride, const T*
 
 // ------------------------------------------------------------------------------------------ tensor cores
 constexpr int MM_ROWS = 64, MM_KEYS = 64, MM_THREADS = 128;
-
-struct MultiMapParams {
-  const __nv_bfloat16* q; int q_stride;
-  const __nv_bfloat16* k_cache; const __nv_bfloat16* v_cache;
-  const int* block_table; int table_stride;
-  const int* q_start; const int* positions;
-  __nv_bfloat16* out; int out_stride;
-  int requests, heads, kv_heads, page_tokens, num_pages;
-  float scale, lambda, norm_eps, out_scale;
-  int* status;
-  // single-token steps may divide a request's tiles among `ksplit` CTAs (blockIdx.z); each then leaves its maxima, sums
-  // and unnormalised accumulators in `partial` [requests, kv_heads, ksplit, 16 rows, maps, 2 + vdim] for the merge kernel
-  int ksplit; float* partial;
-  // what a query sees (MaskKind and its size), an optional term exp(sink[head]) in every softmax denominator, and an
-  // optional gate: the head's output times sigmoid(gate[token * gate_stride + head])
-  int mask_kind, mask_size; const float* sink; const __nv_bfloat16* gate; int gate_stride;
-  // a window's kept first positions, and the cap on the scaled scores (0: none)
-  int mask_keep; float softcap;
-  // the gate row holds a number per element of the output instead of one per head; the turn back of the output
-  int gate_elements; OutputTurn turn;
-};
-
-// A gate per element: sigmoid of the gate row's number for column `col` of the head's output.
-__device__ __forceinline__ float element_gate(const MultiMapParams& p, int token, int head, int vdim, int col) {
-  return 1.0f / (1.0f + __expf(-__bfloat162float(p.gate[(size_t)token * p.gate_stride + (size_t)head * vdim + col])));
-}
-
-// What the running maxima are multiplied by on their way into the exponentials: capped scores are already scaled.
-__device__ __forceinline__ float score_scale(const MultiMapParams& p) { return p.softcap > 0.f ? 1.0f : p.scale; }
 
 template <int DIM, int VDIM, int MAPS, bool SPLIT>
 __global__ void __launch_bounds__(MM_THREADS)
@@ -870,7 +822,8 @@ SPROUT_API long long sprout_multimap_partial_floats(int requests, int kv_heads, 
   return (long long)requests * kv_heads * ksplit * 16 * maps * (2 + vdim);
 }
 
-// bfloat16 only.  `tiles` bounds the (request, 64 rows) tiles of the batch: sum over requests of
+// bfloat16 only.  `tokens` > 0: the tcgen05 kernel, for a step of that many tokens, with `partial` its scratch and `counters` its
+// counters (both may be null); else the mma.sync kernel.  `tiles` bounds the (request, 64 rows) tiles of the batch: sum over requests of
 // ceil(tokens * heads / kv_heads / 64), or any larger number; `max_q_len` is the most tokens any request brings.
 SPROUT_API int sprout_multimap_attention_mma(const void* q, int q_stride, const void* k_cache, const void* v_cache,
                                              const int* block_table, int table_stride, const int* q_start,
@@ -880,7 +833,7 @@ SPROUT_API int sprout_multimap_attention_mma(const void* q, int q_stride, const 
                                              int ksplit, float* partial, int mask_kind, int mask_size, const float* sink,
                                              const void* gate, int gate_stride, int mask_keep, float softcap, int gate_elements,
                                              const float* turn_cos, const float* turn_sin, int turn_positions, int turn_interleaved,
-                                             int* status, cudaStream_t stream) {
+                                             int tokens, int* counters, int* status, cudaStream_t stream) {
   SPROUT_REQUIRE(q && k_cache && v_cache && block_table && q_start && positions && out && status, "multimap_attention_mma: null pointer");
   SPROUT_REQUIRE(requests > 0 && tiles > 0 && max_q_len > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && page_tokens > 0 &&
                  num_pages > 0, "multimap_attention_mma: bad sizes");
@@ -902,6 +855,7 @@ SPROUT_API int sprout_multimap_attention_mma(const void* q, int q_stride, const 
   SPROUT_REQUIRE(!gate || gate_stride >= (gate_elements ? heads * vdim : heads), "multimap_attention_mma: gate rows hold a number per head or element");
   SPROUT_REQUIRE(ksplit >= 1 && ksplit <= 64 && (ksplit == 1 || (partial && max_q_len * (heads / kv_heads) <= 16)),
                  "multimap_attention_mma: keys are divided among CTAs in single-token steps only, with scratch for the shares");
+  if (tokens > 0) return sprout_maps_attention_tc(p, tokens, maps, dim, vdim, partial, counters, stream);
   const bool split = max_q_len * (heads / kv_heads) <= 16;
 #define PICK(D, V)                                                                                              \
   if (dim == D && vdim == V) {                                                                                  \

@@ -73,7 +73,7 @@ _SIGNATURES = {
     "sprout_multimap_attention_simple": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _I, _I, _P, _P, _I, _I, _F,
                                          _I, _P, _P, _I, _I, _P, _P],
     "sprout_multimap_attention_mma": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _F, _F, _I, _P, _I, _I, _P, _P, _I, _I, _F,
-                                      _I, _P, _P, _I, _I, _P, _P],
+                                      _I, _P, _P, _I, _I, _I, _P, _P, _P],
     "sprout_multimap_attention_mma_supported": [_I, _I, _I],
     "sprout_decay_chunks": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_decay_chunks_supported": [_I, _I, _I],
@@ -121,6 +121,10 @@ def load_library(verbose: bool = True):
             lib.sprout_sample_scratch_bytes.restype = ctypes.c_longlong
             lib.sprout_sample_scratch_bytes.argtypes = [c_int]
             lib.sprout_delta_scratch_floats.restype = ctypes.c_longlong
+            lib.sprout_maps_attention_tc_scratch_floats.restype = ctypes.c_longlong
+            lib.sprout_maps_attention_tc_scratch_floats.argtypes = [c_int] * 6
+            lib.sprout_maps_attention_tc_supported.restype = c_int
+            lib.sprout_maps_attention_tc_supported.argtypes = [c_int] * 5
             lib.sprout_delta_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
             lib.sprout_attention_decode_scratch_floats.restype = ctypes.c_longlong
             lib.sprout_attention_decode_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
@@ -1476,10 +1480,13 @@ def visible_keys(mask, context: int) -> int:
 
 def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int, dim: int, vdim: int, scale: float, lam: float,
                        norm_eps: float, out_scale: float, status, mask=None, sink=None, gate=None, softcap: float = 0.0, turn=None,
-                       interleaved: bool = False):
-    """Attention with one or two maps per head: the tensor-core kernel in bfloat16 for the sizes it is built for
-    (``SPROUT_MULTIMAP_ATTENTION=simple`` keeps the float32-arithmetic kernel), else the float32-arithmetic kernel."""
-    if q.dtype == torch.bfloat16 and os.environ.get("SPROUT_MULTIMAP_ATTENTION", "mma") != "simple" \
+                       interleaved: bool = False, counters=None):
+    """Attention with one or two maps per head: the tensor-core kernels in bfloat16 for the sizes they are built for
+    (``SPROUT_MULTIMAP_ATTENTION=simple`` keeps the float32-arithmetic kernel, ``=mma_sync`` the mma.sync kernel for prompt portions),
+    else the float32-arithmetic kernel.  ``counters``: zeroed int32 [2 * SMs] that no launch on another stream uses, left zeroed; with
+    them the tcgen05 kernel may divide a piece's keys among CTAs."""
+    choice = os.environ.get("SPROUT_MULTIMAP_ATTENTION", "auto")
+    if q.dtype == torch.bfloat16 and choice != "simple" \
             and (_lib or load_library()).sprout_multimap_attention_mma_supported(maps, dim, vdim) \
             and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.stride(0) % 2 == 0:
         global LAUNCHES
@@ -1503,6 +1510,14 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
         if sink is not None and (sink.dtype != torch.float32 or sink.numel() != heads):
             raise KernelError("multimap_attention: one float32 sink per head")
         partial = None
+        # tcgen05 for steps whose requests bring 128 (token, head) rows each on average: a CTA of it takes 256, of the mma.sync kernel 64
+        tensor = 0
+        if choice != "mma_sync" and ksplit == 1 and max_q_len * group > 16 and q.shape[0] * group >= 128 * requests and out.data_ptr() % 16 == 0 \
+                and _lib.sprout_maps_attention_tc_supported(maps, dim, vdim, cache.page_tokens, out.stride(0)):
+            tensor = q.shape[0]
+            floats = 0 if counters is None else _lib.sprout_maps_attention_tc_scratch_floats(tensor, requests, heads, kv_heads, maps, vdim)
+            if floats:
+                partial = torch.empty(floats, dtype=torch.float32, device=q.device)
         if ksplit > 1:
             partial = torch.empty(requests * kv_heads * ksplit * 16 * maps * (2 + vdim), dtype=torch.float32, device=q.device)
             LAUNCHES += 1           # the merge kernel behind the same call
@@ -1513,7 +1528,8 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
              cache.page_tokens, k_cache.shape[0], float(scale),
              float(lam), float(norm_eps), float(out_scale), ksplit, _ptr(partial, "partial", torch.float32, True),
              mask_kind, mask_size, _ptr(sink, "sink", torch.float32, True), gate_ptr, gate_stride, mask_keep, float(softcap),
-             gate_elements, turn_cos, turn_sin, turned, 1 if interleaved else 0, _ptr(status, "status", torch.int32), _stream())
+             gate_elements, turn_cos, turn_sin, turned, 1 if interleaved else 0, tensor, _ptr(counters, "counters", torch.int32, True),
+             _ptr(status, "status", torch.int32), _stream())
         return
     multimap_attention_simple(q, cache, ctx, out, heads, kv_heads, maps, dim, vdim, scale, lam, norm_eps, out_scale, status,
                               mask=mask, sink=sink, gate=gate, softcap=softcap, turn=turn, interleaved=interleaved)

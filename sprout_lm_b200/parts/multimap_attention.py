@@ -221,5 +221,6 @@ class MultiMapAttention(Part):
         kernels.multimap_attention(rows[:, :self.q_width], cache, ctx, attended, self.heads, self.kv_heads, self.maps, self.dim,
                                    self.value_dim, self.scale, self.lam, self.norm_eps, self.out_scale, status, mask=self.mask,
                                    sink=self.sink, softcap=self.softcap, turn=self.turn, interleaved=self.interleaved,
+                                   counters=self.runtime.workspace(("maps_attention_counters",), (2 * self.runtime.sm_count,), torch.int32),
                                    gate=projected[:, self.gate_at:self.gate_at + self.gate_width] if self.has_gate else None)
         self.out.forward(attended, residual=x)

@@ -1011,3 +1011,84 @@ def test_sampling(status, vocab):
     kernels.sample(logits, out, status)
     assert out[2].item() == -1 and int(status.item()) & 4
     status.zero_()
+
+
+# ------------------------------------------------------------------------------- attention with one or two maps on tcgen05
+MAPS_CASES = [
+    # maps, dim, vdim, heads, kv_heads, page, held, new, options
+    (2, 64, 128, 8, 2, 16, [0], [300], dict(norm_eps=1e-5, lam=0.4)),
+    (2, 64, 128, 4, 4, 16, [0, 513, 77], [129, 128, 385], dict(norm_eps=1e-5, lam=0.4, out_scale=0.5)),
+    (2, 64, 64, 6, 2, 8, [40, 0], [100, 257], dict(lam=0.3, sink=True)),
+    (1, 64, 128, 8, 2, 16, [700, 700, 0], [65, 200, 331], dict(mask=("window", 256), gate="head")),
+    (1, 64, 128, 16, 4, 32, [1000, 37], [97, 640], dict(mask=("window", 300, 5), softcap=30.0)),
+    (1, 64, 64, 14, 2, 16, [0, 0], [256, 1], dict()),
+    (1, 64, 64, 7, 1, 64, [127, 128, 129], [128, 128, 255], dict(mask=("chunk", 200), sink=True)),
+    (1, 128, 128, 4, 4, 16, [0, 300], [128, 700], dict(sink=True, softcap=20.0, gate="head")),
+    (1, 128, 128, 8, 2, 128, [0], [1025], dict(mask=("chunk", 512), gate="element", turn="half")),
+    (1, 64, 128, 4, 1, 16, [0], [2100], dict(mask=("window", 100), gate="element", turn="pairs", sink=True)),
+    (1, 128, 128, 2, 1, 16, [5000], [130], dict()),
+]
+
+
+@pytest.mark.parametrize("divided", [False, True])
+@pytest.mark.parametrize("maps,dim,vdim,heads,kv_heads,page,held,new,options", MAPS_CASES)
+def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, heads, kv_heads, page, held, new, options):
+    """The tcgen05 kernel against the float32-arithmetic kernel on the same bfloat16 inputs, with NaN in every cache slot that no
+    query of the step sees and pages before a window given back; with and without a piece's keys divided among CTAs."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(dim + vdim + sum(new))
+    total = [h + n for h, n in zip(held, new)]
+    mask = options.get("mask")
+    counts = [-(-t // page) for t in total]
+    table = torch.full((len(new), max(counts) + 3), -1, dtype=torch.int32)
+    order, at = torch.randperm(sum(counts), generator=g).to(torch.int32), 0
+    k = torch.full((sum(counts), kv_heads, page, maps * dim), float("nan"))
+    v = torch.full((sum(counts), kv_heads, page, vdim), float("nan"))
+    for r, t in enumerate(total):
+        table[r, :counts[r]] = order[at:at + counts[r]]
+        at += counts[r]
+        first = 0 if mask is None else max(0, held[r] - mask[1] + 1) if mask[0] == "window" else held[r] // mask[1] * mask[1]
+        keep = mask[2] if mask is not None and len(mask) > 2 else 0
+        for pos in [*range(min(keep, first)), *range(first, t)]:
+            k[table[r, pos // page], :, pos % page] = torch.randn(kv_heads, maps * dim, generator=g)
+            v[table[r, pos // page], :, pos % page] = torch.randn(kv_heads, vdim, generator=g)
+        for j in range(first // page):
+            if j * page >= keep:
+                table[r, j] = -1
+    T = sum(new)
+    dev = lambda x, dt=None: x.to(dt or x.dtype).to(DEV)
+    starts = np.cumsum([0] + list(new))
+    ctx = SimpleNamespace(
+        seq_of_token=dev(torch.tensor([r for r, n in enumerate(new) for _ in range(n)], dtype=torch.int32)),
+        positions=dev(torch.tensor([h + j for h, n in zip(held, new) for j in range(n)], dtype=torch.int32)),
+        q_start=dev(torch.tensor(starts, dtype=torch.int32)), max_q_len=max(new), max_context=max(total), planned_context=0)
+    cache = SimpleNamespace(k=dev(k, torch.bfloat16), v=dev(v, torch.bfloat16), block_table=dev(table), page_tokens=page)
+    q = dev(torch.randn(T, heads * maps * dim, generator=g), torch.bfloat16)
+    more = dict(mask=mask, softcap=options.get("softcap", 0.0))
+    if options.get("sink"):
+        more["sink"] = dev(torch.randn(heads, generator=g))
+    if options.get("gate"):
+        more["gate"] = dev(torch.randn(T, heads * (vdim if options["gate"] == "element" else 1), generator=g), torch.bfloat16)
+    if options.get("turn"):
+        angle = torch.rand(max(total), vdim // 2, generator=g) * 6.28
+        more.update(turn=(dev(torch.cos(angle)), dev(torch.sin(angle))), interleaved=options["turn"] == "pairs")
+    sizes = (heads, kv_heads, maps, dim, vdim, dim ** -0.5, options.get("lam", 0.0), options.get("norm_eps", 0.0), options.get("out_scale", 1.0), status)
+    counters = torch.zeros(2 * kernels.sm_count(torch.device(DEV)), dtype=torch.int32, device=DEV) if divided else None
+    got = torch.full((T, heads * vdim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.multimap_attention(q, cache, ctx, got, *sizes, counters=counters, **more)
+    assert int(status.item()) == 0
+    assert counters is None or not counters.any()
+    want = torch.empty(T, heads * vdim, dtype=torch.bfloat16, device=DEV)
+    kernels.multimap_attention_simple(q, cache, ctx, want, *sizes, **more)
+    status.zero_()                                 # the plain kernel flags the pages that were given back
+    # probabilities rounded to 8 bits (2^-9 of each, of a sum whose terms are about as large as the result), the result rounded once
+    # more on both sides; a norm over the head brings results to about one
+    error = (got.float() - want.float())
+    assert torch.isfinite(got).all()
+    assert error.norm() <= 6e-3 * want.float().norm()
+    assert error.abs().max() <= 4e-2 * want.float().abs().max()
+    if divided:
+        again = torch.empty_like(got)
+        kernels.multimap_attention(q, cache, ctx, again, *sizes, counters=counters, **more)
+        assert torch.equal(got, again) and not counters.any()
