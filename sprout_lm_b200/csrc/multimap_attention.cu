@@ -178,6 +178,164 @@ rope_maps_append_kernel(T* __restrict__ rows, int row_stride, const int* __restr
   }
 }
 
+// The same for bfloat16 rows in 16-byte accesses: a thread takes 16 elements of a vector, the two 8-element runs whose pairs turn
+// together (i and i + half, or 16 neighbours with interleaved pairs) or, beyond the rotated width, 16 neighbours; dim / 16
+// neighbouring lanes have a vector between them, so its norms are a few shuffles.  Bound by memory latency: a block takes a
+// token, whose loads are all in flight together.  2,048 tokens of 32 query vectors, 8 key vectors of 64 and 4 values of 128: 69 us
+// with 2-byte accesses and a warp per vector in turn, 10 us so.
+struct AppendParams {
+  __nv_bfloat16* rows; int row_stride;
+  const int* positions; const int* seq_of_token; const int* block_table; int table_stride;
+  const float* cos_table; const float* sin_table; int max_positions;
+  __nv_bfloat16* k_cache; __nv_bfloat16* v_cache;
+  int q_vectors, kv_heads, maps, rot, vdim, page_tokens, num_pages, write;
+  float unit_eps; int value_from_key;
+  const float* q_weight; const float* k_weight; float weight_eps;
+  int interleaved; const float* v_cos; const float* v_sin;
+  float growth_coef; int growth_every; int* status;
+};
+
+__device__ __forceinline__ void unpack8(uint4 raw, float (&v)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+  const float4 a = *(const float4*)p, b = *(const float4*)(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// a, b: the runs that turn together; angles `at` on (8 of them): pairs (a[i], b[i]), or with `interleaved` neighbours of a, then of b.
+__device__ __forceinline__ void turn16(float (&a)[8], float (&b)[8], const float* cos_at, const float* sin_at, bool interleaved) {
+  float c[8], s[8];
+  load8(cos_at, c);
+  load8(sin_at, s);
+  if (interleaved) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float x = a[2 * i], y = a[2 * i + 1], z = b[2 * i], w = b[2 * i + 1];
+      a[2 * i] = x * c[i] - y * s[i]; a[2 * i + 1] = y * c[i] + x * s[i];
+      b[2 * i] = z * c[4 + i] - w * s[4 + i]; b[2 * i + 1] = w * c[4 + i] + z * s[4 + i];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const float x = a[i], y = b[i];
+      a[i] = x * c[i] - y * s[i];
+      b[i] = y * c[i] + x * s[i];
+    }
+  }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128)
+rope_maps_append_vec_kernel(const AppendParams p) {
+  constexpr int LANES = DIM / 16;                     // lanes that have a vector between them
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const int pos = p.positions[t];
+  __nv_bfloat16* row = p.rows + (size_t)t * p.row_stride;
+  const int half = p.rot / 2;
+  const bool turn = p.rot > 0 && pos >= 0 && pos < p.max_positions;
+  if (p.rot > 0 && !turn && threadIdx.x == 0) atomicOr(p.status, SPROUT_STATUS_BAD_POSITION);
+  int page = -1;
+  if (p.write) {
+    page = pos >= 0 ? p.block_table[(size_t)p.seq_of_token[t] * p.table_stride + pos / p.page_tokens] : -1;
+    if (page < 0 || page >= p.num_pages) {
+      if (threadIdx.x == 0) atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
+      page = -1;
+    }
+  }
+  const int kw = p.maps * DIM;
+  const float growth = p.growth_every > 0 ? 1.0f + p.growth_coef * logf((float)((pos + 1) / p.growth_every + 1)) : 1.0f;
+  // queries that nothing is done to are left alone
+  const int first = !turn && p.unit_eps <= 0.f && p.q_weight == nullptr && p.growth_every <= 0 ? p.q_vectors : 0;
+  const int vectors = p.q_vectors + (page >= 0 ? p.kv_heads * p.maps : 0);
+  const int items = (vectors - first) * LANES;
+  for (int base = 0; base < items; base += 128) {     // the lanes of a vector stay together in the last round too
+    const int item = base + threadIdx.x;
+    const bool active = item < items;
+    const int vec = first + (active ? item / LANES : 0), i = item % LANES;
+    const bool is_key = vec >= p.q_vectors, turns = turn && i < p.rot / 16;
+    const int e0 = i < p.rot / 16 ? (p.interleaved ? 16 * i : 8 * i) : 16 * i, e1 = i < p.rot / 16 && !p.interleaved ? half + 8 * i : e0 + 8;
+    __nv_bfloat16* src = row + (size_t)vec * DIM;
+    const float* weight = is_key ? p.k_weight : p.q_weight;
+    uint4 raw0 = make_uint4(0, 0, 0, 0), raw1 = raw0;
+    if (active) { raw0 = *(const uint4*)(src + e0); raw1 = *(const uint4*)(src + e1); }
+    float a[8], b[8];
+    unpack8(raw0, a);
+    unpack8(raw1, b);
+    auto root = [&](float eps) {                       // 1 / root mean square of the vector
+      float sq = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; k++) sq = fmaf(a[k], a[k], fmaf(b[k], b[k], sq));
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      return 1.0f / sqrtf(sq / (float)DIM + eps);
+    };
+    if (p.q_weight != nullptr || p.k_weight != nullptr) {          // the same for all lanes: the shuffles meet
+      const float before = root(p.weight_eps);
+      if (weight != nullptr && active) {
+        float w0[8], w1[8];
+        load8(weight + e0, w0);
+        load8(weight + e1, w1);
+#pragma unroll
+        for (int k = 0; k < 8; k++) { a[k] = a[k] * before * w0[k]; b[k] = b[k] * before * w1[k]; }
+      }
+    }
+    if (turns && active) turn16(a, b, p.cos_table + (size_t)pos * half + 8 * i, p.sin_table + (size_t)pos * half + 8 * i, p.interleaved);
+    float factor = p.unit_eps > 0.f ? root(p.unit_eps) : 1.0f;
+    if (!active) continue;
+    if (!is_key) factor *= growth;
+#pragma unroll
+    for (int k = 0; k < 8; k++) { a[k] *= factor; b[k] *= factor; }
+    if (!is_key) {
+      *(uint4*)(src + e0) = pack8(a);
+      *(uint4*)(src + e1) = pack8(b);
+    } else {
+      const int g = (vec - p.q_vectors) / p.maps, m = (vec - p.q_vectors) % p.maps;
+      const size_t at = ((size_t)page * p.kv_heads + g) * p.page_tokens + pos % p.page_tokens;
+      *(uint4*)(p.k_cache + at * kw + m * DIM + e0) = pack8(a);
+      *(uint4*)(p.k_cache + at * kw + m * DIM + e1) = pack8(b);
+      if (p.value_from_key) {
+        *(uint4*)(p.v_cache + at * p.vdim + m * DIM + e0) = raw0;
+        *(uint4*)(p.v_cache + at * p.vdim + m * DIM + e1) = raw1;
+      }
+    }
+  }
+  if (page < 0 || p.value_from_key) return;
+  const __nv_bfloat16* vrow = row + (size_t)p.q_vectors * DIM + (size_t)p.kv_heads * kw;
+  if (p.v_cos != nullptr) {
+    if (pos >= p.max_positions) {
+      if (threadIdx.x == 0) atomicOr(p.status, SPROUT_STATUS_BAD_POSITION);
+      return;
+    }
+    const int per = p.vdim / 16, vhalf = p.vdim / 2;
+    for (int item = threadIdx.x; item < p.kv_heads * per; item += 128) {
+      const int g = item / per, i = item % per, e0 = p.interleaved ? 16 * i : 8 * i, e1 = p.interleaved ? e0 + 8 : vhalf + 8 * i;
+      float a[8], b[8];
+      unpack8(*(const uint4*)(vrow + g * p.vdim + e0), a);
+      unpack8(*(const uint4*)(vrow + g * p.vdim + e1), b);
+      turn16(a, b, p.v_cos + (size_t)pos * vhalf + 8 * i, p.v_sin + (size_t)pos * vhalf + 8 * i, p.interleaved);
+      __nv_bfloat16* dst = p.v_cache + (((size_t)page * p.kv_heads + g) * p.page_tokens + pos % p.page_tokens) * p.vdim;
+      *(uint4*)(dst + e0) = pack8(a);
+      *(uint4*)(dst + e1) = pack8(b);
+    }
+    return;
+  }
+  const int per = p.vdim / 8;
+  for (int item = threadIdx.x; item < p.kv_heads * per; item += 128) {
+    const int g = item / per, e = 8 * (item % per);
+    *(uint4*)(p.v_cache + (((size_t)page * p.kv_heads + g) * p.page_tokens + pos % p.page_tokens) * p.vdim + e) = *(const uint4*)(vrow + g * p.vdim + e);
+  }
+}
+
 template <typename T, int MAPS>
 __global__ void __launch_bounds__(CHUNK)
 multimap_attention_simple_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_cache,
@@ -892,12 +1050,28 @@ SPROUT_API int sprout_rope_maps_append(void* rows, int row_stride, int dtype, co
   SPROUT_REQUIRE(!v_cos || (v_sin && max_positions > 0 && vdim % 2 == 0 && !value_from_key), "rope_maps_append: values turn in pairs, with tables of their own");
   const int need = q_vectors * dim + (write ? kv_heads * (maps * dim + (value_from_key ? 0 : vdim)) : 0);
   SPROUT_REQUIRE(row_stride >= need, "rope_maps_append: rows of %d elements, %d needed", row_stride, need);
+  // 16-byte accesses: a vector is a power of two of 16-element shares, runs that turn together start on 8 elements, and every row,
+  // table and weight starts on a 16-byte boundary; a norm over the whole projection keeps the general kernel
+  auto on16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
+  const bool vec = (dim == 16 || dim == 32 || dim == 64 || dim == 128) && rot % 16 == 0 && !weight_whole && row_stride % 8 == 0 &&
+                   (!write || vdim % (v_cos ? 16 : 8) == 0) && on16(rows) && on16(k_cache) && on16(v_cache) && on16(cos_table) && on16(sin_table) &&
+                   on16(q_weight) && on16(k_weight) && on16(v_cos) && on16(v_sin);
   if (dtype == SPROUT_F32)
     sprout_launch(rope_maps_append_kernel<float>, dim3(tokens), dim3(128), 0, stream, (float*)rows, row_stride, positions,
                   seq_of_token, block_table, table_stride, cos_table, sin_table, max_positions, (float*)k_cache,
                   (float*)v_cache, q_vectors, kv_heads, maps, dim, rot, vdim, page_tokens, num_pages, write, unit_eps,
                   value_from_key, q_weight, k_weight, weight_eps, weight_whole, interleaved, v_cos, v_sin, growth_coef, growth_every, status);
-  else if (dtype == SPROUT_BF16)
+  else if (dtype == SPROUT_BF16 && vec) {
+    const AppendParams p{(__nv_bfloat16*)rows, row_stride, positions, seq_of_token, block_table, table_stride, cos_table, sin_table, max_positions,
+                         (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, q_vectors, kv_heads, maps, rot, vdim, page_tokens, num_pages, write,
+                         unit_eps, value_from_key, q_weight, k_weight, weight_eps, interleaved, v_cos, v_sin, growth_coef, growth_every, status};
+    switch (dim) {
+      case 16: sprout_launch(rope_maps_append_vec_kernel<16>, dim3(tokens), dim3(128), 0, stream, p); break;
+      case 32: sprout_launch(rope_maps_append_vec_kernel<32>, dim3(tokens), dim3(128), 0, stream, p); break;
+      case 64: sprout_launch(rope_maps_append_vec_kernel<64>, dim3(tokens), dim3(128), 0, stream, p); break;
+      default: sprout_launch(rope_maps_append_vec_kernel<128>, dim3(tokens), dim3(128), 0, stream, p); break;
+    }
+  } else if (dtype == SPROUT_BF16)
     sprout_launch(rope_maps_append_kernel<__nv_bfloat16>, dim3(tokens), dim3(128), 0, stream, (__nv_bfloat16*)rows, row_stride,
                   positions, seq_of_token, block_table, table_stride, cos_table, sin_table, max_positions,
                   (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, q_vectors, kv_heads, maps, dim, rot, vdim, page_tokens,

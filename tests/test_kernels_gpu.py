@@ -1092,3 +1092,46 @@ def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, h
         again = torch.empty_like(got)
         kernels.multimap_attention(q, cache, ctx, again, *sizes, counters=counters, **more)
         assert torch.equal(got, again) and not counters.any()
+
+
+@pytest.mark.parametrize("maps,dim,vdim,rot,options", [
+    (2, 64, 128, 64, {}), (1, 128, 128, 32, dict(weights=True)), (1, 64, 128, 64, dict(unit=True, turn=True)), (1, 32, 64, 16, dict(growth=True)),
+    (2, 16, 32, 0, dict(growth=True, unit=True)), (1, 128, 128, 128, dict(interleaved=True, turn=True, weights=True)), (1, 128, 128, 64, dict(from_key=True, unit=True)),
+    (1, 64, 64, 64, dict(read_only=True)), (1, 64, 24, 0, {})])
+def test_rope_maps_append_in_16_byte_accesses(status, maps, dim, vdim, rot, options):
+    """The 16-byte form against the general one (rows that do not start on 16 bytes take that one), with a page that is missing."""
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(dim + vdim + rot)
+    heads, kv_heads, page, T = 6, 2, 4, 37
+    write = not options.get("read_only")
+    widths = [heads * maps * dim, kv_heads * maps * dim if write else 0, 0 if options.get("from_key") or not write else kv_heads * vdim]
+    dev = lambda x, dt=None: x.to(dt or x.dtype).to(DEV)
+    plain = torch.randn(T, sum(widths), generator=g).to(torch.bfloat16)
+    positions, seqs = dev(torch.arange(T, dtype=torch.int32)), dev(torch.zeros(T, dtype=torch.int32))
+    table = torch.randperm(12, generator=g).to(torch.int32)[None]
+    table[0, 5] = -1
+    table = dev(table)
+    angle = torch.rand(64, max(rot, 2) // 2, generator=g) * 6.28
+    cos, sin = (dev(torch.cos(angle)), dev(torch.sin(angle))) if rot else (None, None)
+    more = dict(unit_eps=1e-5 if options.get("unit") else 0.0, value_from_key=bool(options.get("from_key")), interleaved=bool(options.get("interleaved")))
+    if options.get("weights"):
+        more.update(q_weight=dev(torch.randn(dim, generator=g)), k_weight=dev(torch.randn(dim, generator=g)), weight_eps=1e-5)
+    if options.get("growth"):
+        more["growth"] = (0.3, 7)
+    if options.get("turn"):
+        angle = torch.rand(64, vdim // 2, generator=g) * 6.28
+        more["value_turn"] = (dev(torch.cos(angle)), dev(torch.sin(angle)))
+    results = []
+    for extra in (0, 1):                                    # rows of 8 elements and more, or of an odd number
+        rows = torch.zeros(T, -(-sum(widths) // 8) * 8 + extra, dtype=torch.bfloat16, device=DEV)
+        rows[:, :sum(widths)] = plain.to(DEV)
+        k = torch.zeros(12, kv_heads, page, maps * dim, dtype=torch.bfloat16, device=DEV)
+        v = torch.zeros(12, kv_heads, page, vdim, dtype=torch.bfloat16, device=DEV)
+        status.zero_()
+        kernels.rope_maps_append(rows, positions, seqs, table, cos, sin, k if write else None, v if write else None, heads * maps, kv_heads, maps, dim, vdim, page,
+                                 write, status, **more)
+        results.append((rows[:, :sum(widths)].float(), k.float(), v.float(), int(status.item())))
+    assert results[0][3] == results[1][3] == (1 if write else 0)
+    for fast, general in zip(results[0][:3], results[1][:3]):
+        # one rounding to bfloat16 of float32 results whose sums are added in another order
+        assert ((fast - general).abs() <= 2 ** -7 * general.abs() + 1e-6).all()
