@@ -27,6 +27,7 @@
 
 
 #include "common.cuh"
+#include "experts.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -36,7 +37,7 @@ constexpr int BLOCK_K = 64;         // bf16 elements per stage row: 128 bytes, o
 constexpr int NUM_THREADS = 320;      // TMA warp, MMA warp, 8 epilogue warps
 constexpr int SMEM_BUDGET = 196 * 1024;    // for the operand stages; the staging tiles and barriers come on top
 
-enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RESIDUAL_ATOMIC = 2, EPI_SWIGLU = 3, EPI_RESIDUAL_TMA = 4 };
+enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RESIDUAL_ATOMIC = 2, EPI_SWIGLU = 3, EPI_RESIDUAL_TMA = 4, EPI_EXPERT_GLU = 5, EPI_EXPERT_GELU = 6 };
 constexpr int STAGING_BYTES = 2 * 128 * 128;    // two [128 rows, 32 float32] tiles for the TMA reduction of the residual epilogue
 
 // SwiGLU epilogue: the weight rows interleave gate and up in blocks of 8 (rows 16b..16b+7 gate,
@@ -65,6 +66,10 @@ struct Params {
   // weights on M only: the tokens' operand made in the kernel instead of copied: bfloat16(x * gain) of the
   // float32 rows x [M, K] (row stride ldx), written by the epilogue warps into the stages' token tiles
   const float* x32; const float* gain; int ldx;
+  // experts' products (GROUPED): the rows of expert e are offsets[e] .. offsets[e + 1] - 1, its matrix has `expert_rows` rows; what the
+  // gated epilogues need: see sprout_experts_product_tc
+  const int* offsets; const int* order; int experts, expert_rows, unit;
+  const float* row_weights; float limit, alpha;
 };
 
 // PAIR: two CTAs share a 256 x BN tile; each holds its own 128 rows of A and half of B's rows.
@@ -81,7 +86,7 @@ struct Layout {
 };
 
 // One unit of work: a 128 x BN tile of D over a range of K blocks.
-struct Work { int row0, col0, kb_begin, num_kb, split; };
+struct Work { int row0, col0, kb_begin, num_kb, split; int row_end, weight_row; };   // the last two: experts' products only
 
 // SWAP == false: map_rows is the activation map (rows = tokens), map_cols the weight map.
 // SWAP == true:  map_rows is the weight map (rows = output features), map_cols the activation map.
@@ -97,11 +102,16 @@ struct Work { int row0, col0, kb_begin, num_kb, split; };
 // its own tensor memory.  The copies of both CTAs count on the first CTA's "full" barriers; the
 // commits arrive on the "empty" and "accumulator full" barriers of both CTAs; the second CTA's
 // epilogue warps arrive on the first CTA's "accumulator empty" barriers.
-template <int BN, bool SWAP, bool PAIR = false>
+//
+// GROUPED (pairs): the tiles are those of every expert's rows over its own matrix, found from the experts' offsets on the device;
+// a tile's rows beyond the expert's last are computed and not stored.  With a gate the first CTA's half of B is gate rows and
+// the second's the up rows that go with them, so a row's thread has both in its accumulators.
+template <int BN, bool SWAP, bool PAIR = false, bool GROUPED = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols,
                     const __grid_constant__ CUtensorMap map_out, const Params p) {
   static_assert(!(PAIR && SWAP), "pairs work on token tiles");
+  static_assert(!GROUPED || PAIR, "experts' products run in pairs");
   using L = Layout<BN, PAIR>;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0;                       // 0 issues the MMAs
   const int first_work = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;     // this CTA's (pair's) first item and stride
@@ -123,11 +133,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   const int row_tiles = ((SWAP ? p.N : p.M) + TILE_M - 1) / TILE_M;
   const int col_tiles = ((SWAP ? p.M : p.N) + BN - 1) / BN;
   const int splits = (total_kb + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
-  const int total_work = row_tiles * col_tiles * splits;
+  // experts' products: 256-row tiles before expert e, and its first row, in the room that the residual epilogue's tiles would have
+  int* tile_prefix = (int*)staging;
+  int* row_prefix = tile_prefix + p.experts + 1;
+  const bool glu_tiles = GROUPED && p.epilogue == EPI_EXPERT_GLU;
+  const int expert_cols = glu_tiles ? (p.N + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;     // tiles across an expert's outputs
+  int total_work = row_tiles * col_tiles * splits;
   // consecutive work items share the weight tile where they can (tokens on M: same columns,
   // next rows), so that it is served from L2
   auto work_at = [&](int w) {
     Work k;
+    if (GROUPED) {
+      const int tile = w / expert_cols, ct = w % expert_cols;
+      int e = 0, hi = p.experts;                       // the last e with tile_prefix[e] <= tile: it has rows
+      while (hi - e > 1) {
+        const int mid = (e + hi) / 2;
+        if (tile_prefix[mid] <= tile) e = mid; else hi = mid;
+      }
+      k.row0 = row_prefix[e] + (tile - tile_prefix[e]) * TILE_M + (int)rank * BLOCK_M;
+      k.row_end = row_prefix[e + 1];
+      k.col0 = ct * (glu_tiles ? BN / 2 : BN);
+      k.weight_row = e * p.expert_rows + k.col0 + (int)rank * (glu_tiles ? p.N : BN / 2);
+      k.split = 0; k.kb_begin = 0; k.num_kb = total_kb;
+      return k;
+    }
     k.split = w % splits;
     const int tile = w / splits;
     if (SWAP) { k.row0 = (tile / col_tiles) * BLOCK_M; k.col0 = (tile % col_tiles) * BN; }   // token tiles of one weight tile side by side
@@ -151,10 +180,33 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, L::TMEM_COLS);
+  if (GROUPED) {
+    pdl_wait();                                        // the offsets are an earlier kernel's
+    if (warp == 0) {
+      int before = 0;
+      for (int e0 = 0; e0 < p.experts; e0 += 32) {
+        const int e = e0 + lane, begin = e < p.experts ? p.offsets[e] : 0, end = e < p.experts ? p.offsets[e + 1] : 0;
+        int sum = (end - begin + TILE_M - 1) / TILE_M;
+        const int own = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int other = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += other;
+        }
+        if (e < p.experts) {
+          tile_prefix[e] = before + sum - own;
+          row_prefix[e] = begin;
+          if (e == p.experts - 1) { tile_prefix[p.experts] = before + sum; row_prefix[p.experts] = end; }
+        }
+        before += __shfl_sync(0xffffffffu, sum, 31);
+      }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (GROUPED) total_work = tile_prefix[p.experts] * expert_cols;
   if (PAIR) {
     // The pair's MMAs write both CTAs' tensor memory at one address.  Each CTA has its SM to
     // itself (its shared memory leaves no room for another) and has allocated from an empty tensor
@@ -190,7 +242,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     };
     for (int w = first_work; w < total_work && ok; w += work_stride) {
       const Work k = work_at(w);
-      const int weight_row = SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0), act_row = SWAP ? k.col0 : k.row0;
+      const int weight_row = GROUPED ? k.weight_row : SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0), act_row = SWAP ? k.col0 : k.row0;
       int early = 0;
       if (w == first_work) {
         early = min(k.num_kb, L::STAGES);
@@ -384,7 +436,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         continue;
       }
 #pragma unroll 1
-      for (int c = half * 16; c < BN; c += 32) {
+      for (int c = half * 16; c < (glu_tiles ? BN / 2 : BN); c += 32) {
         uint32_t raw[16];
         tmem_load16(taddr + c, raw);
         if (SWAP) {
@@ -416,7 +468,34 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           }
         } else {
           // row = token, columns = output features: each lane writes a contiguous run of its row
-          if (row < p.M) {
+          if (GROUPED && p.epilogue != EPI_STORE) {
+            const int n_base = col0 + c;
+            float v[16];
+            uint32_t up[16];
+            if (p.epilogue == EPI_EXPERT_GLU) tmem_load16(taddr + BN / 2 + c, up);      // warp-wide: also lanes without a row
+            if (row < k.row_end && n_base < p.N) {
+              const float weight = p.row_weights ? p.row_weights[p.order[row]] : 1.0f;
+#pragma unroll
+              for (int j = 0; j < 16; j++) {
+                // rounded to bfloat16 before the activation, as separate products would leave them
+                const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j]) * weight));
+                const float u = p.epilogue == EPI_EXPERT_GLU ? __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j]) * weight)) : 0.f;
+                v[j] = sprout_experts::glu(p.unit, g, u, p.limit, p.alpha);
+              }
+              __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n_base;    // N and ldo are multiples of 8
+#pragma unroll
+              for (int j = 0; j < 16; j += 8) {
+                if (n_base + j >= p.N) break;
+                uint32_t packed[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                  __nv_bfloat162 h = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
+                  packed[i] = *(uint32_t*)&h;
+                }
+                *(uint4*)(o + j) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+              }
+            }
+          } else if (row < (GROUPED ? k.row_end : p.M)) {
             const int n_base = col0 + c;
             float v[16];
 #pragma unroll
@@ -498,13 +577,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 // ------------------------------------------------------------------ host side
 // `work` = tiles x K splits; the grid is one CTA per SM at most, each walking the work list.
 // Pairs: `work` counts 256 x BN tiles; the grid is one cluster of two CTAs per two SMs at most.
-template <int BN>
+template <int BN, bool GROUPED = false>
 int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const Params& p, int work,
                 cudaStream_t stream) {
   using L = Layout<BN, true>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
+    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false, true, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
     if (err != cudaSuccess) return sprout_fail("gemm_bf16: cannot reserve %d bytes of shared memory: %s", L::SMEM_BYTES, cudaGetErrorString(err));
     configured = true;
   }
@@ -523,7 +602,7 @@ int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const 
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = sprout_pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&config, gemm_tcgen05_kernel<BN, false, true>, rows_map, cols_map, out_map, p);
+  cudaLaunchKernelEx(&config, gemm_tcgen05_kernel<BN, false, true, GROUPED>, rows_map, cols_map, out_map, p);
   return sprout_check_launch("gemm_bf16 (pairs)");
 }
 
@@ -543,6 +622,27 @@ int launch(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUten
 }
 
 }  // namespace
+
+int sprout_experts_product_tc(const void* rows, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
+                              int K, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream) {
+  const bool gated = unit == sprout_experts::UNIT_CLAMPED || unit == sprout_experts::UNIT_SILU;
+  SPROUT_REQUIRE(rows && offsets && order && w && out && status && entries > 0 && experts > 0, "experts_product: bad arguments");
+  SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= 2048, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
+  Params p{};
+  p.out = out; p.out_is_f32 = unit < 0; p.epilogue = unit < 0 ? EPI_STORE : gated ? EPI_EXPERT_GLU : EPI_EXPERT_GELU;
+  p.M = entries; p.N = N; p.K = K; p.ldo = N; p.status = status; p.groups = 1;
+  p.k_blocks_per_split = (K + BLOCK_K - 1) / BLOCK_K;
+  p.offsets = offsets; p.order = order; p.experts = experts; p.expert_rows = gated ? 2 * N : N; p.unit = unit;
+  p.row_weights = row_weights; p.limit = limit; p.alpha = alpha;
+  constexpr int BN = 256;
+  const long long matrix_rows = (long long)experts * p.expert_rows;
+  const long long work = ((long long)entries / (2 * BLOCK_M) + experts) * ((N + (gated ? BN / 2 : BN) - 1) / (gated ? BN / 2 : BN));
+  SPROUT_REQUIRE(matrix_rows <= 0x7fffffffLL && work <= 0x7fffffffLL, "experts_product: too many rows");
+  CUtensorMap map_a, map_w;
+  if (tensor_map(rows, entries, K, K, BLOCK_M, &map_a)) return 1;
+  if (tensor_map(w, (int)matrix_rows, K, K, BN / 2, &map_w)) return 1;
+  return launch_pair<BN, true>(map_a, map_w, map_a, p, (int)work, stream);
+}
 
 // A [M, K] bf16 row stride lda; W [N, K] bf16 contiguous; out [M, N] row stride ldo, bf16 or
 // float32.  residual != 0: out is float32 and the product is added to it.  orientation: 0 picks
@@ -591,7 +691,7 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
   SPROUT_REQUIRE(split_k == 1 || (swap && residual && M <= 256), "gemm_bf16: split_k needs weights-on-M with a residual output and at most 256 tokens "
                  "(with tokens on M the kernel splits K by itself where that pays)");
 
-  Params p;
+  Params p{};
   p.gate_gelu = gate_gelu;
   p.bias = bias; p.out = out; p.out_is_f32 = out_dtype == SPROUT_F32;
   p.epilogue = swiglu ? EPI_SWIGLU : residual ? (split_k > 1 ? EPI_RESIDUAL_ATOMIC : EPI_RESIDUAL) : EPI_STORE;
@@ -684,7 +784,7 @@ SPROUT_API int sprout_gemm_bf16_unscaled(const float* x, int ldx, const float* g
   SPROUT_REQUIRE(x && gain && W && out && status, "gemm_bf16_unscaled: null pointer");
   SPROUT_REQUIRE(K % 8 == 0 && ldx % 4 == 0 && ldx >= K && ldo >= N, "gemm_bf16_unscaled: K (%d) must be a multiple of 8, the rows of x (%d) of 4", K, ldx);
   SPROUT_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)gain & 15) == 0 && ((uintptr_t)W & 15) == 0, "gemm_bf16_unscaled: operands must be 16-byte aligned");
-  Params p;
+  Params p{};
   p.gate_gelu = 0;
   p.bias = nullptr; p.out = out; p.out_is_f32 = 1; p.epilogue = EPI_RESIDUAL_ATOMIC;
   p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.status = status;

@@ -22,13 +22,17 @@
 //                  through a three-stage cp.async ring; the tile list follows the experts' row counts on the
 //                  device.  In the up product a tile holds 64 gate columns and the 64 up columns that go with
 //                  them, so the activation is applied to the accumulators.
+//  * moe_gather:   the arranged rows side by side, and the two products in CTA pairs on tcgen05 (gemm_tcgen05.cu) for experts of a
+//                  real layer's size.
 //  * moe_few:      the same two products for steps of at most 8 tokens (bfloat16): a CTA per (expert, 32 output columns)
 //                  keeps the expert's few rows in shared memory and streams every weight row once for all of them.
 //  * moe_combine:  y[t] += sum over the token's places of weight * (identity ? h[t] : its row), or one factor times the
 //                  sum of the rows when the weights went into the experts' inputs.
 #include "attention_bf16.cuh"
+#include "experts.cuh"
 
 using namespace sprout_attn;
+using namespace sprout_experts;
 
 namespace {
 
@@ -222,17 +226,6 @@ __device__ __forceinline__ int expert_of(const int* offsets, int experts, int ro
     if (offsets[mid] <= row) lo = mid; else hi = mid;
   }
   return lo;
-}
-
-// What an expert does with its first products: the clamped gated unit, the exact gelu of one product (an expert without a
-// gate), silu(g) u.
-enum ExpertUnit : int { UNIT_CLAMPED = 0, UNIT_PLAIN = 1, UNIT_SILU = 2 };
-__device__ __forceinline__ float glu(int unit, float g, float u, float limit, float alpha) {
-  if (unit == UNIT_PLAIN) return 0.5f * g * (1.0f + erff(g * 0.7071067811865476f));
-  if (unit == UNIT_SILU) return g / (1.0f + expf(-g)) * u;
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return g * (1.0f / (1.0f + expf(-alpha * g))) * (u + 1.0f);
 }
 
 // grid (rows, column blocks); 8 warps, a warp per output column at a time.  w_gate_up [experts, 2 ff, width] with
@@ -524,6 +517,18 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ a, int a_stride, const int* __r
   }
 }
 
+// rows[at] = h[order[at] / top] for the arranged rows, 16 bytes a thread.
+__global__ void __launch_bounds__(256)
+moe_gather_kernel(const __nv_bfloat16* __restrict__ h, int h_stride, const int* __restrict__ order, const int* __restrict__ offsets, int experts,
+                  int top, int width, __nv_bfloat16* __restrict__ rows) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x;
+  if (row >= offsets[experts]) return;
+  const __nv_bfloat16* src = h + (size_t)(order[row] / top) * h_stride;
+  for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) *(uint4*)(rows + (size_t)row * width + c) = *(const uint4*)(src + c);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(float* __restrict__ y, const T* __restrict__ h, int h_stride, const int* __restrict__ ids,
@@ -666,6 +671,31 @@ SPROUT_API int sprout_moe_down_plain(const void* act, int dtype, const int* offs
 // Whether the tensor-core products take these sizes: rows of 16-byte multiples, pairs of outputs.
 SPROUT_API int sprout_moe_mma_supported(int width, int ff, int h_stride) {
   return width % 8 == 0 && ff % 8 == 0 && h_stride % 8 == 0;
+}
+
+// Whether a step of these sizes takes the tcgen05 products: experts of at least a tile's width (a pair of CTAs makes 256 rows x 256
+// columns, or 128 gated ones), and more tokens than the few-token kernel's.  32 experts of 1,024 over 2,048 wide rows: 2,048 tokens x
+// top 4 374 us (both) on mma.sync, 181 us with the gather here; 64 tokens 175 and 108 us.
+SPROUT_API int sprout_moe_tc_supported(int entries, int experts, int top, int width, int ff, int h_stride) {
+  return sprout_moe_mma_supported(width, ff, h_stride) && width >= 512 && ff >= 256 && experts <= 2048 && entries > FEW * top;
+}
+
+// The same as below through sprout_experts_product_tc; `gathered` bfloat16 [entries, width] is scratch.
+SPROUT_API int sprout_moe_experts_tc(const void* h, int h_stride, const int* order, const int* offsets, const void* w_gate_up,
+                                     const void* w_down, void* gathered, void* act, float* rows_out, int entries, int experts, int top,
+                                     int width, int ff, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream) {
+  SPROUT_REQUIRE(h && order && offsets && w_gate_up && w_down && gathered && act && rows_out && status, "moe_experts_tc: null pointer");
+  SPROUT_REQUIRE(unit >= UNIT_CLAMPED && unit <= UNIT_SILU, "moe_experts_tc: unknown kind of expert %d", unit);
+  SPROUT_REQUIRE(entries > 0 && experts > 0 && top > 0 && sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride),
+                 "moe_experts_tc: sizes not taken (entries %d, width %d, ff %d, row stride %d)", entries, width, ff, h_stride);
+  SPROUT_REQUIRE((((uintptr_t)h | (uintptr_t)w_gate_up | (uintptr_t)w_down | (uintptr_t)gathered | (uintptr_t)act | (uintptr_t)rows_out) & 15) == 0,
+                 "moe_experts_tc: buffers must start on 16-byte boundaries");
+  sprout_launch(moe_gather_kernel, dim3(entries), dim3(256), 0, stream, (const __nv_bfloat16*)h, h_stride, order, offsets, experts, top, width,
+                (__nv_bfloat16*)gathered);
+  if (int code = sprout_check_launch("moe_gather")) return code;
+  if (int code = sprout_experts_product_tc(gathered, offsets, order, w_gate_up, act, entries, experts, ff, width, unit, row_weights, limit, alpha, status, stream))
+    return code;
+  return sprout_experts_product_tc(act, offsets, order, w_down, rows_out, entries, experts, width, ff, -1, nullptr, 0.f, 0.f, status, stream);
 }
 
 // act [entries, ff] bfloat16 = glu(W_gate a, W_up a); rows_out [entries, width] float32 = W_down act, over the arranged rows.

@@ -102,6 +102,8 @@ _SIGNATURES = {
     "sprout_moe_combine": [_P, _P, _I, _I, _P, _P, _F, _P, _P, _I, _I, _I, _P],
     "sprout_moe_mma_supported": [_I, _I, _I],
     "sprout_moe_experts_mma": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _F, _F, _P],
+    "sprout_moe_experts_tc": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _F, _F, _P, _P],
+    "sprout_moe_tc_supported": [_I, _I, _I, _I, _I, _I],
 }
 
 _lock = threading.Lock()
@@ -1573,14 +1575,24 @@ def decay_attention(rows, ctx, state, decay, out, heads: int, dim: int, vdim: in
 
 
 def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: int, top: int, limit: float, alpha: float, unit=None,
-                row_weights=None):
+                row_weights=None, status=None):
     """The routed experts' two products over the arranged rows (``unit``, ``row_weights``: see ``moe_up_plain``): on tensor cores in bfloat16 when the sizes are
-    multiples of 8 (``SPROUT_MOE=plain`` keeps the CUDA-core products), else on CUDA cores."""
+    multiples of 8 (``SPROUT_MOE=plain`` keeps the CUDA-core products, ``=mma_sync`` the mma.sync ones), else on CUDA cores.  With the device
+    ``status`` word experts of a real layer's size run on tcgen05."""
     global LAUNCHES
     width, ff = h.shape[1], act.shape[1]
     if h.dtype == torch.bfloat16 and h.stride(1) == 1 and os.environ.get("SPROUT_MOE", "mma") != "plain" \
             and (_lib or load_library()).sprout_moe_mma_supported(width, ff, h.stride(0)) \
             and all(t.data_ptr() % 16 == 0 for t in (h, w_gate_up, w_down, act, rows_out)):
+        if status is not None and os.environ.get("SPROUT_MOE", "mma") != "mma_sync" \
+                and _lib.sprout_moe_tc_supported(act.shape[0], experts, top, width, ff, h.stride(0)):
+            gathered = torch.empty((act.shape[0], width), dtype=torch.bfloat16, device=h.device)
+            _run("sprout_moe_experts_tc", _ptr(h, "h"), h.stride(0), _ptr(order, "order", torch.int32), _ptr(offsets, "offsets", torch.int32),
+                 _ptr(w_gate_up, "w_gate_up", torch.bfloat16), _ptr(w_down, "w_down", torch.bfloat16), _ptr(gathered, "gathered"),
+                 _ptr(act, "act", torch.bfloat16), _ptr(rows_out, "rows_out", torch.float32), act.shape[0], experts, top, width, ff,
+                 _unit_code(unit, limit), _row_weights_ptr(row_weights, act.shape[0]), float(limit), float(alpha), _ptr(status, "status", torch.int32), _stream())
+            LAUNCHES += 2           # three kernels behind one call
+            return
         _run("sprout_moe_experts_mma", _ptr(h, "h"), h.stride(0), _ptr(order, "order", torch.int32),
              _ptr(offsets, "offsets", torch.int32), _ptr(w_gate_up, "w_gate_up", torch.bfloat16),
              _ptr(w_down, "w_down", torch.bfloat16), _ptr(act, "act", torch.bfloat16), _ptr(rows_out, "rows_out", torch.float32),

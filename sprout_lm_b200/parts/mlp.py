@@ -365,7 +365,7 @@ class RoutedExperts(Part):
             act = torch.empty((entries, self.expert_ff), dtype=h.dtype, device=device)
             rows = torch.empty((entries, self.hidden_size), dtype=torch.float32, device=device)
             kernels.moe_experts(h, order, self.offsets, self.w_gate_up, self.w_down, act, rows, self.experts, self.top,
-                                self.expert_limit, self.alpha, unit=self.expert_kind, row_weights=weights if self.weight_on_input else None)
+                                self.expert_limit, self.alpha, unit=self.expert_kind, row_weights=weights if self.weight_on_input else None, status=self.runtime.status)
         else:
             place_of.fill_(-1)
         if self.shared is not None and self.shared_gate and self.plain:

@@ -1135,3 +1135,33 @@ def test_rope_maps_append_in_16_byte_accesses(status, maps, dim, vdim, rot, opti
     for fast, general in zip(results[0][:3], results[1][:3]):
         # one rounding to bfloat16 of float32 results whose sums are added in another order
         assert ((fast - general).abs() <= 2 ** -7 * general.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("unit", ["clamped_glu", "plain", "silu_glu"])
+@pytest.mark.parametrize("counts,width,ff,weighted", [([256, 0, 257, 1, 30], 512, 256, False), ([0, 700, 0, 3], 520, 264, True), ([17] * 40, 640, 384, True)])
+def test_experts_on_tcgen05(status, monkeypatch, unit, counts, width, ff, weighted):
+    """Experts without rows, with one, at the edges of the 256-row tiles, sizes that no tile divides: against the CUDA-core products."""
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(width + ff)
+    experts, entries, top = len(counts), sum(counts), 1
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(entries, generator=g)].to(torch.int32)[:, None].to(DEV)
+    offsets, order = torch.zeros(experts + 1, dtype=torch.int32, device=DEV), torch.zeros(entries, dtype=torch.int32, device=DEV)
+    place = torch.zeros(entries, dtype=torch.int32, device=DEV)
+    kernels.moe_arrange(ids, torch.tensor(counts, dtype=torch.int32, device=DEV), offsets, order, place, experts)
+    make = lambda *shape, scale=1.0: (torch.randn(*shape, generator=g) * scale).to(torch.bfloat16).to(DEV)
+    h = make(entries, width)
+    w_up, w_down = make(experts, (1 if unit == "plain" else 2) * ff, width, scale=width ** -0.5), make(experts, width, ff, scale=ff ** -0.5)
+    weights = torch.rand(entries, 1, generator=g).to(DEV) if weighted else None
+    limit = 7.0 if unit == "clamped_glu" else 0.0
+    results = []
+    for choice in ("mma", "plain"):
+        monkeypatch.setenv("SPROUT_MOE", choice)
+        act = torch.zeros(entries, ff, dtype=torch.bfloat16, device=DEV)
+        rows = torch.zeros(entries, width, device=DEV)
+        kernels.moe_experts(h, order, offsets, w_up, w_down, act, rows, experts, top, limit, 1.702, unit=unit, row_weights=weights, status=status)
+        results.append((act.float(), rows))
+    assert kernels.load_library().sprout_moe_tc_supported(entries, experts, top, width, ff, width) and int(status.item()) == 0
+    # float32 sums in another order; a product on the edge of a bfloat16 rounding moves its activation by 2^-8 of itself
+    for tc, plain in zip(*results):
+        assert (tc - plain).norm() <= 2 ** -9 * plain.norm()
+        assert (tc - plain).abs().max() <= 2 ** -6 * plain.abs().max()
