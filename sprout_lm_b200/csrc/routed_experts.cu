@@ -38,6 +38,8 @@ namespace {
 
 // threads of a router block: 32 warps, so that the router's rows are walked by as many warps as the SM holds (a block's time is
 // the latency of its rounds over the outputs: 33 outputs are 2 rounds of 32 warps, 5 of 8)
+// Steps of many tokens: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four products (2,048 tokens of
+// 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so).
 constexpr int ROUTE_THREADS = 1024;
 
 // A block takes ROUTE_TOKENS tokens (8 in steps of many tokens, 1 in steps of few, where blocks are scarce; a token's
@@ -46,11 +48,12 @@ constexpr int ROUTE_THREADS = 1024;
 // are multiples of four, else every 32nd), the lanes are added in a fixed order, so a token's
 // scores do not depend on the tokens beside it.  Warp t then takes token t's softmax and choices.
 template <typename T, int ROUTE_TOKENS>
-__global__ void __launch_bounds__(ROUTE_THREADS)
+__global__ void __launch_bounds__(ROUTE_TOKENS > 1 ? 512 : ROUTE_THREADS)
 moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ router, const float* __restrict__ correction,
                  int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int tokens, int width,
                  int softmax_outputs, int experts, int top, float scale, int extra, float* __restrict__ extra_out,
                  int group_count, int group_keep, int renormalize, int sigmoid_scores) {
+  constexpr int ROUTE_OUTPUTS = ROUTE_TOKENS > 1 ? 4 : 1;
   extern __shared__ float smem[];
   int outputs = softmax_outputs + extra;              // rows of the router matrix
   float* zs = smem;                                   // ROUTE_TOKENS x outputs: scores
@@ -60,12 +63,66 @@ moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict_
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * ROUTE_TOKENS;
   const int here = min(ROUTE_TOKENS, tokens - t0);
-  for (int i = threadIdx.x; i < ROUTE_TOKENS * width; i += ROUTE_THREADS) {
-    const int r = i / width, k = i % width;
-    rows[i] = r < here ? to_float(h[(size_t)(t0 + r) * h_stride + k]) : 0.f;
+  if (sizeof(T) == 2 && (width & 7) == 0 && (h_stride & 7) == 0 && ((uintptr_t)h & 15) == 0) {
+    for (int i = threadIdx.x * 8; i < ROUTE_TOKENS * width; i += blockDim.x * 8) {
+      const int r = i / width, k = i % width;
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (r < here) raw = *(const uint4*)(h + (size_t)(t0 + r) * h_stride + k);
+      *(float4*)(rows + i) = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                                         __uint_as_float(raw.y & 0xffff0000u));
+      *(float4*)(rows + i + 4) = make_float4(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u), __uint_as_float(raw.w << 16),
+                                             __uint_as_float(raw.w & 0xffff0000u));
+    }
+  } else {
+    for (int i = threadIdx.x; i < ROUTE_TOKENS * width; i += blockDim.x) {
+      const int r = i / width, k = i % width;
+      rows[i] = r < here ? to_float(h[(size_t)(t0 + r) * h_stride + k]) : 0.f;
+    }
   }
   __syncthreads();
-  for (int e = warp; e < outputs; e += ROUTE_THREADS / 32) {
+  if (ROUTE_OUTPUTS > 1 && (width & 3) == 0) {
+    // a warp takes ROUTE_OUTPUTS neighbouring outputs, so that a token's values are read from shared memory once for all of them
+    for (int e0 = warp * ROUTE_OUTPUTS; e0 < outputs; e0 += blockDim.x / 32 * ROUTE_OUTPUTS) {
+      const float* w[ROUTE_OUTPUTS];
+      float dot[ROUTE_OUTPUTS][ROUTE_TOKENS];
+#pragma unroll
+      for (int u = 0; u < ROUTE_OUTPUTS; u++) {
+        w[u] = router + (size_t)min(e0 + u, outputs - 1) * width;
+#pragma unroll
+        for (int r = 0; r < ROUTE_TOKENS; r++) dot[u][r] = 0.f;
+      }
+      float4 next[ROUTE_OUTPUTS];
+#pragma unroll
+      for (int u = 0; u < ROUTE_OUTPUTS; u++) next[u] = lane * 4 < width ? *reinterpret_cast<const float4*>(w[u] + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = lane * 4; k < width; k += 128) {
+        float4 wk[ROUTE_OUTPUTS];
+#pragma unroll
+        for (int u = 0; u < ROUTE_OUTPUTS; u++) {
+          wk[u] = next[u];
+          if (k + 128 < width) next[u] = *reinterpret_cast<const float4*>(w[u] + k + 128);
+        }
+#pragma unroll
+        for (int r = 0; r < ROUTE_TOKENS; r++) {
+          const float4 xv = *reinterpret_cast<const float4*>(rows + r * width + k);
+#pragma unroll
+          for (int u = 0; u < ROUTE_OUTPUTS; u++) {
+            dot[u][r] = fmaf(xv.x, wk[u].x, dot[u][r]);
+            dot[u][r] = fmaf(xv.y, wk[u].y, dot[u][r]);
+            dot[u][r] = fmaf(xv.z, wk[u].z, dot[u][r]);
+            dot[u][r] = fmaf(xv.w, wk[u].w, dot[u][r]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < ROUTE_OUTPUTS; u++)
+#pragma unroll
+        for (int r = 0; r < ROUTE_TOKENS; r++) {
+          const float sum = warp_sum(dot[u][r]);
+          if (lane == 0 && e0 + u < outputs) zs[r * outputs + e0 + u] = sum;
+        }
+    }
+  } else
+  for (int e = warp; e < outputs; e += blockDim.x / 32) {
     const float* w = router + (size_t)e * width;
     float dot[ROUTE_TOKENS];
 #pragma unroll
@@ -606,8 +663,10 @@ SPROUT_API int sprout_moe_route(const void* h, int h_stride, int dtype, const fl
     prepared = true;
   }
   dim3 grid((tokens + per_block - 1) / per_block);
+  const int warps = (rows_of_router + 3) / 4;                // with four outputs each; a warp per token at least
+  const dim3 threads(per_block == 1 ? ROUTE_THREADS : 32 * (warps < 8 ? 8 : warps > 16 ? 16 : warps));
 #define ROUTE(T, N)                                                                                                    \
-  sprout_launch(moe_route_kernel<T, N>, grid, dim3(ROUTE_THREADS), smem, stream, (const T*)h, h_stride, router, correction, ids, \
+  sprout_launch(moe_route_kernel<T, N>, grid, threads, smem, stream, (const T*)h, h_stride, router, correction, ids, \
                 weights, counts, tokens, width, outputs, experts, top, scale, extra, extra_out, group_count, group_keep, renormalize, sigmoid_scores)
   if (dtype == SPROUT_F32) {
     if (per_block == 1) ROUTE(float, 1); else ROUTE(float, 8);
