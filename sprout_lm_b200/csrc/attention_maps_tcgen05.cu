@@ -125,9 +125,13 @@ struct Params {
   int box_rows;                        // cache rows of a TMA box
   int shares;                          // CTAs that a piece's key tiles may be divided among
   float* scratch; int* counters;       // [pieces][shares] shares; [pieces][2], zero between launches
+  // PACKED: the requests' keys and values lie side by side instead of in pages, each request's from its first visible tile on
+  // (`packed_base`): a head's key is `key_atoms` times 64 columns of its own in map_k's rows and then the columns from `tail_col` of
+  // map_v's rows, which the heads share; its values start at column `value_col` of map_k's rows
+  int key_atoms, tail_col, value_col;
 };
 
-template <int DIM, int VDIM, int MAPS>
+template <int DIM, int VDIM, int MAPS, bool PACKED>
 __global__ void __launch_bounds__(THREADS, 1)
 maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Params tc) {
   using L = Layout<DIM, VDIM, MAPS>;
@@ -189,6 +193,12 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const int n_tiles = (all_tiles - rank + shares - 1) / shares;
   const int tiles_a = MAPS == 2 ? n_tiles : max(0, (all_tiles_a - rank + shares - 1) / shares);
   auto key_of = [&](int j) { return tile_of(rank + shares * j) * KEYS; };
+  int packed_at = 0;                                  // the packed row of the request's position 0, if it were there
+  if (PACKED) {
+    for (int i = 0; i < r; i++)
+      packed_at += p.positions[p.q_start[i + 1] - 1] + 1 - packed_base(p.mask_kind, p.mask_size, p.positions[p.q_start[i]]);
+    packed_at -= packed_base(p.mask_kind, p.mask_size, p.positions[q0]);
+  }
 
   // rows of a stage that no copy fills must hold finite numbers: their probabilities are zero, and zero times a NaN is not
   for (int i = tid; i < NS * L::V_BYTES / 16; i += THREADS) ((uint4*)sV)[i] = make_uint4(0, 0, 0, 0);
@@ -229,21 +239,21 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       uint64_t* full = keys ? k_full : v_full;
       uint64_t* empty = keys ? k_empty : v_empty;
       const uint32_t stages = smem_u32(keys ? sK : sV), stage_bytes = keys ? L::K_BYTES : L::V_BYTES;
-      const int atoms = keys ? KW / 64 : VDIM / 64, boxes = KEYS / tc.box_rows;
+      const int atoms = keys ? KW / 64 : VDIM / 64, boxes = PACKED ? 1 : KEYS / tc.box_rows;
       auto box_key = [&](int j) {                     // the first key of this lane's box of tile j, -1 if no row sees any of it
         if (lane >= boxes || j >= n_tiles) return -1;
         const int key = key_of(j) + lane * tc.box_rows;
         return key > max_limit || (key + tc.box_rows <= min_lo && key >= p.mask_keep) ? -1 : key;
       };
       int key = box_key(0);
-      int page = key >= 0 ? table[key / p.page_tokens] : 0;
+      int page = !PACKED && key >= 0 ? table[key / p.page_tokens] : 0;
       for (int j = 0; j < n_tiles; j++) {
         const int s = j % NS;
-        const bool bad = key >= 0 && (page < 0 || page >= p.num_pages);
+        const bool bad = !PACKED && key >= 0 && (page < 0 || page >= p.num_pages);
         if (bad) atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
-        const int row_at = key >= 0 && !bad ? (page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens : -1;
+        const int row_at = key < 0 || bad ? -1 : PACKED ? packed_at + key : (page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens;
         key = box_key(j + 1);
-        if (key >= 0) page = table[key / p.page_tokens];
+        if (!PACKED && key >= 0) page = table[key / p.page_tokens];
         const uint32_t bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, row_at >= 0)) * tc.box_rows * 128 * atoms;
         bool ok = true;
         if (lane == 0) {
@@ -253,8 +263,13 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         }
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
         if (row_at >= 0)
-          for (int a = 0; a < atoms; a++)
-            tma_load_2d_addr(stages + s * stage_bytes + a * KV_ATOM + lane * tc.box_rows * 128, map, smem_u32(&full[s]), a * 64, row_at);
+          for (int a = 0; a < atoms; a++) {
+            const uint32_t to = stages + s * stage_bytes + a * KV_ATOM + lane * tc.box_rows * 128;
+            if (!PACKED) tma_load_2d_addr(to, map, smem_u32(&full[s]), a * 64, row_at);
+            else if (!keys) tma_load_2d_addr(to, &map_k, smem_u32(&full[s]), tc.value_col + g * VDIM + a * 64, row_at);
+            else if (a < tc.key_atoms) tma_load_2d_addr(to, &map_k, smem_u32(&full[s]), (g * tc.key_atoms + a) * 64, row_at);
+            else tma_load_2d_addr(to, &map_v, smem_u32(&full[s]), tc.tail_col + (a - tc.key_atoms) * 64, row_at);
+          }
         issued = j + 1;
       }
     } else if (warp == 1) {
@@ -636,16 +651,16 @@ long long pieces_bound(int tokens, int requests, int heads, int kv_heads, int ma
   return (((long long)tokens * (heads / kv_heads) + cta_rows(maps) - 1) / cta_rows(maps) + requests) * kv_heads;
 }
 
-template <int DIM, int VDIM, int MAPS>
+template <int DIM, int VDIM, int MAPS, bool PACKED = false>
 int launch(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params& p, int ctas, cudaStream_t stream) {
   using L = Layout<DIM, VDIM, MAPS>;
   static bool configured = false;
   if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(maps_attention_tc_kernel<DIM, VDIM, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+    const cudaError_t err = cudaFuncSetAttribute(maps_attention_tc_kernel<DIM, VDIM, MAPS, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (err != cudaSuccess) return sprout_fail("maps_attention (tcgen05): cannot reserve %d bytes of shared memory: %s", L::SMEM, cudaGetErrorString(err));
     configured = true;
   }
-  sprout_launch(maps_attention_tc_kernel<DIM, VDIM, MAPS>, dim3(ctas), dim3(THREADS), L::SMEM, stream, map_k, map_v, p);
+  sprout_launch(maps_attention_tc_kernel<DIM, VDIM, MAPS, PACKED>, dim3(ctas), dim3(THREADS), L::SMEM, stream, map_k, map_v, p);
   return sprout_check_launch("maps_attention (tcgen05)");
 }
 
@@ -679,7 +694,7 @@ int sprout_maps_attention_tc(const MultiMapParams& m, int tokens, int maps, int 
                  "maps_attention (tcgen05): %d maps of %d with values of %d, page size %d or the output's alignment is not taken", maps, dim, vdim, m.page_tokens);
   const long long cache_rows = (long long)m.num_pages * m.kv_heads * m.page_tokens;
   SPROUT_REQUIRE(cache_rows <= 0x7fffffffLL, "maps_attention (tcgen05): the cache has too many rows for a tensor map coordinate");
-  Params p;
+  Params p{};
   p.m = m;
   p.box_rows = m.page_tokens < KEYS ? m.page_tokens : KEYS;
   p.shares = scratch && counters ? sprout_maps_attention_tc_shares(tokens, m.requests, m.heads, m.kv_heads, maps) : 1;
@@ -692,4 +707,36 @@ int sprout_maps_attention_tc(const MultiMapParams& m, int tokens, int maps, int 
   if (maps == 2) return vdim == 64 ? launch<64, 64, 2>(map_k, map_v, p, (int)ctas, stream) : launch<64, 128, 2>(map_k, map_v, p, (int)ctas, stream);
   if (dim == 64) return vdim == 64 ? launch<64, 64, 1>(map_k, map_v, p, (int)ctas, stream) : launch<64, 128, 1>(map_k, map_v, p, (int)ctas, stream);
   return launch<128, 128, 1>(map_k, map_v, p, (int)ctas, stream);
+}
+
+// Attention of queries [tokens, heads * (dim + tail)] over packed rows: `unfolded` bfloat16 [rows, heads * dim + heads * vdim] (every
+// head's own key part, then every head's values) and `latent` [rows, latent_width], whose columns from tail_col on are the key part that
+// the heads share.  Rows of a request lie in the order of its positions from packed_base on, the requests' one behind the other.
+SPROUT_API int sprout_latent_unfolded_attention(const void* q, int q_stride, const void* unfolded, const void* latent, int rows, int latent_width,
+                                                int tail_col, const int* q_start, const int* positions, const float* sink, void* out, int out_stride,
+                                                int tokens, int requests, int heads, int dim, int tail, int vdim, float scale, int window,
+                                                float* scratch, int* counters, int* status, cudaStream_t stream) {
+  SPROUT_REQUIRE(q && unfolded && latent && q_start && positions && out && status, "latent_unfolded_attention: null pointer");
+  SPROUT_REQUIRE(rows > 0 && tokens > 0 && requests > 0 && heads > 0 && dim > 0 && tail >= 0 && dim % 64 == 0 && tail % 64 == 0 && tc_sizes(1, dim + tail, vdim),
+                 "latent_unfolded_attention: bad sizes (keys of %d + %d, values of %d)", dim, tail, vdim);
+  SPROUT_REQUIRE(q_stride % 8 == 0 && out_stride % 8 == 0 && latent_width % 8 == 0 && tail_col % 8 == 0 && tail_col + tail <= latent_width &&
+                 (((uintptr_t)q | (uintptr_t)unfolded | (uintptr_t)latent | (uintptr_t)out) & 15) == 0, "latent_unfolded_attention: rows must start on 16-byte boundaries");
+  Params p{};
+  p.m.q = (const __nv_bfloat16*)q; p.m.q_stride = q_stride; p.m.q_start = q_start; p.m.positions = positions;
+  p.m.block_table = q_start; p.m.page_tokens = KEYS; p.m.num_pages = 1;                     // not read
+  p.m.out = (__nv_bfloat16*)out; p.m.out_stride = out_stride; p.m.requests = requests; p.m.heads = p.m.kv_heads = heads;
+  p.m.scale = scale; p.m.out_scale = 1.0f; p.m.status = status; p.m.ksplit = 1; p.m.sink = sink;
+  p.m.mask_kind = window > 0 ? MASK_WINDOW : MASK_CAUSAL; p.m.mask_size = window;
+  p.box_rows = KEYS;
+  p.shares = scratch && counters ? sprout_maps_attention_tc_shares(tokens, requests, heads, heads, 1) : 1;
+  p.scratch = scratch; p.counters = counters;
+  p.key_atoms = dim / 64; p.tail_col = tail_col; p.value_col = heads * dim;
+  const int width = heads * (dim + vdim);
+  CUtensorMap map_k, map_v;
+  if (tensor_map(unfolded, rows, width, width, KEYS, &map_k)) return 1;
+  if (tensor_map(latent, rows, latent_width, latent_width, KEYS, &map_v)) return 1;
+  const long long ctas = pieces_bound(tokens, requests, heads, heads, 1) * p.shares;
+  SPROUT_REQUIRE(ctas <= 0x7fffffffLL, "latent_unfolded_attention: too many tokens");
+  if (dim + tail == 64) return vdim == 64 ? launch<64, 64, 1, true>(map_k, map_v, p, (int)ctas, stream) : launch<64, 128, 1, true>(map_k, map_v, p, (int)ctas, stream);
+  return launch<128, 128, 1, true>(map_k, map_v, p, (int)ctas, stream);
 }

@@ -9,6 +9,8 @@
 //  * latent_kv_append:  per token a row [latent (rank) | shared rotary key part]: the latent is
 //                       RMS-normed with a learned weight, the key part rotated by the token's
 //                       position, and both are stored as one row of a paged cache with one head.
+//  * latent_pack:       the cached rows that a step's queries see, request by request side by side (what the unfolded form's product
+//                       reads); latent_rotate: the rotated part of every query head, in place.
 //  * latent_query_tail: the rotated part of every query head, copied behind the head's latent
 //                       query (the row a latent attention kernel multiplies with a cache row).
 //  * headwise_gemm:     out[t, h, :] = W[h] a[t, h, :], one small matrix per head.
@@ -19,8 +21,11 @@
 //                       sum of the history so far.
 //  * softcap:           x = cap * tanh(x / cap), in place, x multiplied by a factor first.
 #include "attention_bf16.cuh"
+#include "maps_attention.cuh"
+#include "row_vectors.cuh"
 
 using namespace sprout_attn;
+using namespace sprout_maps;
 
 namespace {
 
@@ -270,6 +275,59 @@ __global__ void latent_query_tail_kernel(const T* __restrict__ q, T* __restrict_
       dst[d] = src[d];
     }
   }
+}
+
+// ---------------------------------------------------------------- the unfolded form
+// A warp per packed row, 16 bytes a lane.  Rows beyond the requests' are left as they are.
+__global__ void __launch_bounds__(256)
+latent_pack_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int table_stride, const int* __restrict__ q_start,
+                   const int* __restrict__ positions, __nv_bfloat16* __restrict__ packed, int rows, int requests, int width, int page_tokens,
+                   int num_pages, int window, int* status) {
+  pdl_launch_dependents();
+  pdl_wait();
+  int row = blockIdx.x * 8 + (threadIdx.x >> 5), r = 0;
+  __nv_bfloat16* dst = packed + (size_t)row * width;
+  if (row >= rows) return;
+  const int kind = window > 0 ? MASK_WINDOW : MASK_CAUSAL;
+  int key = 0, first = 0;
+  for (; r < requests; r++) {
+    first = positions[q_start[r]];
+    const int base = packed_base(kind, window, first), count = positions[q_start[r + 1] - 1] + 1 - base;
+    if (row < count) { key = base + row; break; }
+    row -= count;
+  }
+  if (r == requests) return;
+  const int lane = threadIdx.x & 31, page = block_table[(size_t)r * table_stride + key / page_tokens];
+  const bool there = page >= 0 && page < num_pages;
+  if (!there && key >= first_visible(kind, window, first) && lane == 0) atomicOr(status, SPROUT_STATUS_BAD_PAGE);
+  const __nv_bfloat16* src = cache + ((size_t)(there ? page : 0) * page_tokens + key % page_tokens) * width;
+  for (int c = lane * 8; c < width; c += 256) *(uint4*)(dst + c) = there ? *(const uint4*)(src + c) : make_uint4(0, 0, 0, 0);
+}
+
+// q [tokens, heads * (dim + tail)]: the first `rot` elements (a multiple of 16) of every head's tail turn by the token's position.
+__global__ void __launch_bounds__(256)
+latent_rotate_kernel(__nv_bfloat16* __restrict__ q, const int* __restrict__ positions, const float* __restrict__ cos_table,
+                     const float* __restrict__ sin_table, int table_positions, int rot, int interleaved, int tokens, int heads, int dim, int tail,
+                     int* status) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int per = rot / 16, half = rot / 2;
+  const long long item = blockIdx.x * 256LL + threadIdx.x;
+  if (item >= (long long)tokens * heads * per) return;
+  const int i = (int)(item % per), h = (int)(item / per % heads), t = (int)(item / per / heads);
+  int pos = positions[t];
+  if (pos < 0 || pos >= table_positions) {
+    atomicOr(status, SPROUT_STATUS_BAD_POSITION);
+    pos = 0;
+  }
+  __nv_bfloat16* at = q + ((size_t)t * heads + h) * (dim + tail) + dim;
+  const int e0 = interleaved ? 16 * i : 8 * i, e1 = interleaved ? e0 + 8 : half + 8 * i;
+  float a[8], b[8];
+  unpack8(*(const uint4*)(at + e0), a);
+  unpack8(*(const uint4*)(at + e1), b);
+  turn16(a, b, cos_table + (size_t)pos * half + 8 * i, sin_table + (size_t)pos * half + 8 * i, interleaved);
+  *(uint4*)(at + e0) = pack8(a);
+  *(uint4*)(at + e1) = pack8(b);
 }
 
 // ---------------------------------------------------------------- headwise_gemm
@@ -705,4 +763,26 @@ SPROUT_API int sprout_softcap(float* x, float cap, float factor, long long count
   SPROUT_REQUIRE(x && count > 0 && cap >= 0.f, "softcap: null pointer, no elements or a negative cap");
   sprout_launch(softcap_kernel, dim3(flat_grid(count, 256)), dim3(256), 0, stream, x, cap, factor, count);
   return sprout_check_launch("softcap");
+}
+
+SPROUT_API int sprout_latent_pack(const void* cache, const int* block_table, int table_stride, const int* q_start, const int* positions, void* packed,
+                                  int rows, int requests, int width, int page_tokens, int num_pages, int window, int* status, cudaStream_t stream) {
+  SPROUT_REQUIRE(cache && block_table && q_start && positions && packed && status && rows > 0 && requests > 0 && page_tokens > 0 && num_pages > 0,
+                 "latent_pack: bad arguments");
+  SPROUT_REQUIRE(width > 0 && width % 8 == 0 && (((uintptr_t)cache | (uintptr_t)packed) & 15) == 0, "latent_pack: rows must start on 16-byte boundaries");
+  sprout_launch(latent_pack_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)cache, block_table, table_stride, q_start,
+                positions, (__nv_bfloat16*)packed, rows, requests, width, page_tokens, num_pages, window, status);
+  return sprout_check_launch("latent_pack");
+}
+
+SPROUT_API int sprout_latent_rotate(void* q, const int* positions, const float* cos_table, const float* sin_table, int table_positions, int rot,
+                                    int interleaved, int tokens, int heads, int dim, int tail, int* status, cudaStream_t stream) {
+  SPROUT_REQUIRE(q && positions && cos_table && sin_table && status && tokens > 0 && heads > 0 && table_positions > 0, "latent_rotate: bad arguments");
+  SPROUT_REQUIRE(rot > 0 && rot % 16 == 0 && rot <= tail && dim % 8 == 0 && tail % 8 == 0 &&
+                 (((uintptr_t)q | (uintptr_t)cos_table | (uintptr_t)sin_table) & 15) == 0, "latent_rotate: sizes in multiples of 8, 16-byte rows");
+  const long long items = (long long)tokens * heads * (rot / 16);
+  SPROUT_REQUIRE(items <= 0x7fffffffLL * 128, "latent_rotate: too many tokens");
+  sprout_launch(latent_rotate_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, (__nv_bfloat16*)q, positions, cos_table, sin_table,
+                table_positions, rot, interleaved, tokens, heads, dim, tail, status);
+  return sprout_check_launch("latent_rotate");
 }

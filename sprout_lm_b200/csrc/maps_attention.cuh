@@ -22,6 +22,10 @@ __device__ __forceinline__ int first_visible(int kind, int size, int pos) {
   return 0;
 }
 
+// Where the packed rows of a request begin whose first query of the step stands at `first`: at the 64-position boundary at or before
+// the first position that any of its queries sees.
+__device__ __forceinline__ int packed_base(int kind, int size, int first) { return first_visible(kind, size, first) & ~63; }
+
 // Turns a head's output back by the query's position (values that were turned by theirs): tables float32
 // [positions, vdim / 2]; null: no turn.  Pair m is (m, m + vdim / 2), or (2m, 2m + 1) when `interleaved`.
 struct OutputTurn {

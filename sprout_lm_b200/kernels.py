@@ -103,6 +103,9 @@ _SIGNATURES = {
     "sprout_moe_mma_supported": [_I, _I, _I],
     "sprout_moe_experts_mma": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _F, _F, _P],
     "sprout_moe_experts_tc": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _F, _F, _P, _P],
+    "sprout_latent_pack": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+    "sprout_latent_rotate": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "sprout_latent_unfolded_attention": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P],
     "sprout_moe_tc_supported": [_I, _I, _I, _I, _I, _I],
 }
 
@@ -1154,6 +1157,64 @@ def latent_attention(qlat, cache, ctx, sink, out, heads: int, rank: int, scale: 
         splits, split_keys = latent_split_plan(ctx.num_seqs, heads, rank, min(planned, window) if window else planned, width)
     latent_attention_mma(qlat, cache.k, cache.block_table, ctx.q_start, ctx.positions, ctx.context_lens, sink, out, heads, rank,
                          scale, status, ctx.num_seqs, splits, split_keys, window=window)
+
+
+# The unfolded form: keys and values of every head are made once per cached row that the step's queries see, and the attention itself
+# multiplies dim + tail + vdim elements a (query, key) pair instead of 2 rank + tail.  Making them pays from some 75 new tokens a
+# request on (2,048 tokens of 16 heads over a latent of 512: 412 us folded with 47 us of products per head, 64 us with 8 us of packing and rotation and 15 us of product unfolded); the
+# rows it is made for are bounded by the block tables' width, and scratch by UNFOLD_ROWS of them.
+UNFOLD_TOKENS, UNFOLD_ROWS = 128, 16384
+
+
+def latent_unfold_rows(ctx, cache, tokens: int, heads: int, dim: int, tail: int, vdim: int, rank: int, rot: int, window: int = 0) -> int:
+    """Rows of scratch for the unfolded form of a step's latent attention, 0 where the folded form runs (few new tokens a request, sizes
+    that the tcgen05 kernel does not take, more rows than UNFOLD_ROWS)."""
+    if LATENT_ATTENTION != "auto" or cache.k.dtype != torch.bfloat16 or dim <= 0 or dim % 64 or tail % 64 or (dim + tail, vdim) not in ((64, 64), (64, 128), (128, 128)) \
+            or rank % 8 or rot % 16 or tokens < UNFOLD_TOKENS * ctx.num_seqs:
+        return 0
+    keys = cache.block_table.shape[1] * cache.page_tokens
+    if window:
+        keys = min(keys, window + ctx.max_q_len + 64)
+    rows = ctx.num_seqs * keys
+    return rows if rows <= UNFOLD_ROWS else 0
+
+
+def latent_pack(cache, ctx, packed, status, window: int = 0):
+    """packed [rows, width] = the cached rows that the step's queries see, request by request in the order of their positions."""
+    k = cache.k
+    if k.dim() != 4 or k.shape[1] != 1 or not k.is_contiguous() or not packed.is_contiguous() or packed.shape[1] != k.shape[3] or packed.dtype != k.dtype:
+        raise KernelError("latent_pack: shapes or dtypes do not fit")
+    _rows_contiguous(cache.block_table, "block_table")
+    _run("sprout_latent_pack", _ptr(k, "cache", torch.bfloat16), _ptr(cache.block_table, "block_table", torch.int32), cache.block_table.stride(0),
+         _ptr(ctx.q_start, "q_start", torch.int32), _ptr(ctx.positions, "positions", torch.int32), _ptr(packed, "packed"), packed.shape[0],
+         ctx.q_start.numel() - 1, k.shape[3], k.shape[2], k.shape[0], int(window), _ptr(status, "status", torch.int32), _stream())
+
+
+def latent_rotate(q, positions, cos, sin, interleaved: bool, heads: int, dim: int, tail: int, status):
+    """The first 2 * table width elements of every head's tail in q [tokens, heads * (dim + tail)] (bfloat16) turn by the position, in place."""
+    if not q.is_contiguous() or q.dtype != torch.bfloat16 or q.shape[1] != heads * (dim + tail) or positions.numel() != q.shape[0]:
+        raise KernelError("latent_rotate: shapes or dtypes do not fit")
+    _run("sprout_latent_rotate", _ptr(q, "q"), _ptr(positions, "positions", torch.int32), _ptr(cos, "cos", torch.float32), _ptr(sin, "sin", torch.float32),
+         cos.shape[0], 2 * cos.shape[1], 1 if interleaved else 0, q.shape[0], heads, dim, tail, _ptr(status, "status", torch.int32), _stream())
+
+
+def latent_unfolded_attention(q, unfolded, packed, ctx, sink, out, heads: int, dim: int, tail: int, vdim: int, rank: int, scale: float, status,
+                              counters, window: int = 0):
+    """Attention of q [tokens, heads * (dim + tail)] over packed rows: head h's key is columns [h dim, (h + 1) dim) of ``unfolded`` [rows,
+    heads * (dim + vdim)] and columns [rank, rank + tail) of ``packed``, its value columns [heads dim + h vdim, ...) of ``unfolded``.
+    ``counters``: zeroed int32 [2 * SMs] that no launch on another stream uses, left zeroed."""
+    T, requests, rows = q.shape[0], ctx.q_start.numel() - 1, packed.shape[0]
+    if not q.is_contiguous() or not unfolded.is_contiguous() or not packed.is_contiguous() or not q.dtype == unfolded.dtype == packed.dtype == out.dtype == torch.bfloat16 \
+            or q.shape[1] != heads * (dim + tail) or tuple(unfolded.shape) != (rows, heads * (dim + vdim)) or tuple(out.shape) != (T, heads * vdim) \
+            or packed.shape[1] < rank + tail or (sink is not None and sink.numel() != heads):
+        raise KernelError("latent_unfolded_attention: shapes or dtypes do not fit")
+    _rows_contiguous(out, "out")
+    floats = (_lib or load_library()).sprout_maps_attention_tc_scratch_floats(T, requests, heads, heads, 1, vdim)
+    scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
+    _run("sprout_latent_unfolded_attention", _ptr(q, "q"), q.stride(0), _ptr(unfolded, "unfolded"), _ptr(packed, "packed"), rows, packed.shape[1], rank,
+         _ptr(ctx.q_start, "q_start", torch.int32), _ptr(ctx.positions, "positions", torch.int32), _ptr(sink, "sink", torch.float32, True), _ptr(out, "out"),
+         out.stride(0), T, requests, heads, dim, tail, vdim, float(scale), int(window), _ptr(scratch, "scratch", torch.float32, True),
+         _ptr(counters, "counters", torch.int32, True), _ptr(status, "status", torch.int32), _stream())
 
 
 def depth_average(history, x, weights, n: int):

@@ -8,8 +8,9 @@ can see are given back.
 
 The up-projections are folded to the query's side, so that nothing per head is ever made of the cache:
 q_lat,n = W_uk,n^T q_n (rank wide), score = scale * ([q_lat,n | q_rot,n] . [c | k_rot]), the weighted sum of
-the rows' c parts is taken once per head (rank wide) and W_uv,n is applied to that sum.  Prefill and
-decode, whole prompts and portions all run this one form over the same rows.
+the rows' c parts is taken once per head (rank wide) and W_uv,n is applied to that sum.  Steps whose requests
+bring many tokens (``kernels.latent_unfold_rows``) unfold instead: W_uk,n c and W_uv,n c are made once per row that the step's
+queries see, in scratch, and the attention runs on heads of their own.  Both read the same cached rows.
 
 Queries come from a latent of their own (``q_rank``: q = W_uq RMSNorm(W_dq h) * w) or straight from h.
 A layer may read the rows another layer cached (its run-order entry has ``writes_cache=False``): it
@@ -102,6 +103,9 @@ class LatentAttention(Part):
         uk = source.raw(n["uk"]).reshape(self.heads, self.dim, self.kv_rank).transpose(1, 2)
         self.uk_t = source.to_device_matrix(uk.contiguous()) if self.dim else None
         self.uv = source.matrix(n["uv"]).reshape(self.heads, self.value_dim, self.kv_rank)
+        # the unfolded form makes every head's key part and values in one product
+        self.unfold = Linear(source.to_device_matrix(torch.cat([source.raw(n["uk"]), source.raw(n["uv"])], dim=0)), None, status, any_inner_size=True) \
+            if self.dim else None
         self.sink = source.vector(n["sink"]) if self.has_sink else None
         self.out = linear(n["o"])
         self.tables = self.position.rotary_tables(source.runtime) if self.rot_dim else None
@@ -127,6 +131,22 @@ class LatentAttention(Part):
             cq = torch.empty((tokens, self.q_rank), dtype=h.dtype, device=h.device)
             kernels.rmsnorm(self.dq.forward_float32(h), self.dq_gain, cq, self.eps)
             q = self.uq.forward(cq)
+        rot = 2 * cos.shape[1] if cos is not None else 0
+        rows = kernels.latent_unfold_rows(ctx, cache, tokens, self.heads, self.dim, self.rot_dim, self.value_dim, self.kv_rank, rot,
+                                          self.window or 0) if self.unfold is not None else 0
+        if rows:
+            # many new tokens a request: keys and values per head, made once per visible row, then ordinary attention
+            if rot:
+                kernels.latent_rotate(q, ctx.positions, cos, sin, self.interleaved, self.heads, self.dim, self.rot_dim, status)
+            packed = torch.empty((rows, self.width), dtype=h.dtype, device=h.device)
+            kernels.latent_pack(cache, ctx, packed, status, window=self.window or 0)
+            attended = torch.empty((tokens, self.heads * self.value_dim), dtype=h.dtype, device=h.device)
+            kernels.latent_unfolded_attention(q, self.unfold.forward(packed[:, :self.kv_rank]), packed, ctx, self.sink, attended, self.heads, self.dim,
+                                              self.rot_dim, self.value_dim, self.kv_rank, self.scale, status,
+                                              self.runtime.workspace(("maps_attention_counters",), (2 * self.runtime.sm_count,), torch.int32),
+                                              window=self.window or 0)
+            self.out.forward(attended, residual=x)
+            return
         q_lat = (torch.empty if self.dim else torch.zeros)((tokens, self.heads * self.width), dtype=h.dtype, device=h.device)
         if self.dim:
             kernels.headwise_gemm(q, self.uk_t, q_lat, self.heads, self.dim + self.rot_dim, self.width)

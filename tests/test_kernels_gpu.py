@@ -1165,3 +1165,50 @@ def test_experts_on_tcgen05(status, monkeypatch, unit, counts, width, ff, weight
     for tc, plain in zip(*results):
         assert (tc - plain).norm() <= 2 ** -9 * plain.norm()
         assert (tc - plain).abs().max() <= 2 ** -6 * plain.abs().max()
+
+
+@pytest.mark.parametrize("window,sink,interleaved,dim,tail,vdim", [(None, True, True, 64, 64, 128), (100, False, False, 64, 64, 128), (64, True, True, 64, 0, 64), (None, True, False, 64, 64, 128)])
+@pytest.mark.parametrize("held,new", [([0], [129]), ([0, 300, 65], [400, 129, 190])])
+def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, tail, vdim, held, new):
+    """A latent attention layer's unfolded form against its folded form, portions behind cached rows, pages before a window given back."""
+    from sprout_lm_b200 import kernels
+    from sprout_lm_b200.config.specs import PartSpec
+    from sprout_lm_b200.engine.batch import StepContext
+    from sprout_lm_b200.parts import CacheView, Runtime, WeightSource, build_part
+    g = torch.Generator().manual_seed(sum(new) + dim + tail)
+    heads, rank, width, page = 4, 128, 256, 16
+    position = PartSpec("none", {}) if not tail else PartSpec("rope_interleaved" if interleaved else "rope_yarn", {"dims": tail, "theta": 1e4, "max_positions": 1024})
+    part = build_part("mixer", PartSpec("latent_attention", dict(hidden_size=width, heads=heads, dim=dim, rot_dim=tail, value_dim=vdim, kv_rank=rank, q_rank=64,
+                                                                 scale=0.1, eps=1e-5, position=position, sink=sink, window=window)))
+    decls = {d.name: d for d in part.tensor_decls()}
+    weights = {name: torch.randn(d.shape, generator=g) * d.shape[-1] ** -0.5 + (d.init == "gain") for name, d in decls.items()}
+    part.load(WeightSource(lambda name: weights[name], Runtime(DEV, torch.bfloat16)))
+    total = [h + n for h, n in zip(held, new)]
+    counts = [-(-t // page) for t in total]
+    pages = torch.randperm(sum(counts), generator=g).to(torch.int32)
+    table, at = torch.full((len(new), 64), -1, dtype=torch.int32), 0
+    cache = torch.randn(sum(counts), 1, page, rank + tail, generator=g)
+    for r in range(len(new)):
+        table[r, :counts[r]] = pages[at:at + counts[r]]
+        at += counts[r]
+        for j in range(max(0, held[r] - (window or 10 ** 6) + 1) // page):
+            cache[table[r, j]] = float("nan")
+            table[r, j] = -1
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    starts = np.cumsum([0] + new).tolist()
+    T = sum(new)
+    ctx = StepContext(num_tokens=T, num_seqs=len(new), max_q_len=max(new), max_context=max(total), token_ids=ints([0] * T),
+                      positions=ints([h + j for h, n in zip(held, new) for j in range(n)]), seq_of_token=ints([i for i, n in enumerate(new) for _ in range(n)]),
+                      q_start=ints(starts), context_lens=ints(total), state_slots=ints([0] * len(new)), logits_rows=ints([0]), block_tables=[table.to(DEV)], page_tokens=page)
+    h = torch.randn(T, width, generator=g).to(torch.bfloat16).to(DEV)
+    results = []
+    for rows in (kernels.UNFOLD_ROWS, 0):
+        monkeypatch.setattr(kernels, "UNFOLD_ROWS", rows)
+        view = CacheView(cache.to(torch.bfloat16).to(DEV), None, ctx.block_tables[0], page, True)
+        assert bool(kernels.latent_unfold_rows(ctx, view, T, heads, dim, tail, vdim, rank, tail, window or 0)) == bool(rows)
+        x = torch.zeros(T, width, device=DEV)
+        part.forward(h, x, ctx, view)
+        assert int(part.runtime.status.item()) == 0 and torch.isfinite(x).all()
+        results.append(x)
+    # two forms of the same sums with the intermediate results rounded to bfloat16 at other places
+    assert (results[0] - results[1]).norm() <= 1.5e-2 * results[1].norm()
