@@ -81,6 +81,24 @@ __device__ __forceinline__ bool find_chunk(const int* q_start, int requests, int
   return false;
 }
 
+// Two float32 in a register pair: sm_100a multiplies, adds and fuses them pairwise in one instruction.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 enum ScanPhase : int { SCAN_WHOLE = 0, SCAN_CHUNK_SUMS = 1, SCAN_CHUNK_OUT = 2 };
 
 constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
@@ -92,7 +110,9 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // Tokens come `batch` at a time: while the threads walk a batch's tokens over their registers, the next batch's q, k,
 // decay inputs and values are on their way from memory into registers; at the batch's end they are turned into
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
-// shuffles.  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
+// shuffles.  Tiles of 8 x 4 (PAIRS) are walked two rows at a time in packed arithmetic: a thread's rows are neighbours, and q, c k and a
+// lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us
+// for the two walks with a number at a time and (q, c k, a) triples, SUMS and OUTS us so).  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
 // depend on the cutting or on the batch.
 //
 // Long portions are cut into chunks of `p.chunk` tokens so that more blocks than (request, head, columns) have work, in
@@ -116,8 +136,12 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   const int rows_log2 = slices_log2 + ROWS_LOG2, rows_pad = 1 << rows_log2;
   const int cb_log2 = 7 - slices_log2 + (COLS == 4 ? 2 : 0), cb = 1 << cb_log2;
   static_assert(COLS == 1 || COLS == 4, "columns of a thread's tile");
+  constexpr bool PAIRS = ROWS == 8 && COLS == 4;
   float4* tok = scan_smem;                                             // [batch][rows_pad]: (q, k, a, -)
-  float* vt = reinterpret_cast<float*>(tok + (size_t)batch * rows_pad);  // [batch][cb]
+  // PAIRS: [batch][4 planes: q, k, a, -][2 halves of every 8 rows][slices][4], a half padded so that the two halves' banks differ
+  const int half_stride = rows_pad / 2 + 16, plane = 2 * half_stride;
+  float* tok2 = reinterpret_cast<float*>(scan_smem);
+  float* vt = PAIRS ? tok2 + (size_t)batch * 4 * plane : reinterpret_cast<float*>(tok + (size_t)batch * rows_pad);  // [batch][cb]
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, tid = threadIdx.x;
@@ -143,9 +167,10 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   const float* from = (PHASE == SCAN_WHOLE || chunk_count == 1) ? mine : held;
   const bool vectors = (p.vdim & 3) == 0;             // rows of the state start on 16-byte boundaries
   float S[ROWS][COLS], P[PHASE == SCAN_CHUNK_SUMS ? ROWS : 1];
+  auto row_of = [&](int j) { return PAIRS ? slice * ROWS + j : j * slices + slice; };
 #pragma unroll
   for (int j = 0; j < ROWS; j++) {
-    const int row = j * slices + slice;
+    const int row = row_of(j);
     if (COLS == 4 && vectors) {                       // four columns of a row in one access
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
       if (PHASE != SCAN_CHUNK_SUMS && col < p.vdim && row < dim) x = *reinterpret_cast<const float4*>(from + (size_t)row * p.vdim + col);
@@ -156,6 +181,15 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
         S[j][c] = (PHASE != SCAN_CHUNK_SUMS && col + c < p.vdim && row < dim) ? from[(size_t)row * p.vdim + col + c] : 0.f;
     }
     if (PHASE == SCAN_CHUNK_SUMS) P[j] = 1.f;
+  }
+  unsigned long long S2[PAIRS ? ROWS / 2 : 1][COLS], P2[PAIRS ? ROWS / 2 : 1];      // PAIRS: rows 2 j and 2 j + 1
+  if (PAIRS) {
+#pragma unroll
+    for (int j = 0; j < ROWS / 2; j++) {
+      P2[j] = pack2(1.f, 1.f);
+#pragma unroll
+      for (int c = 0; c < COLS; c++) S2[j][c] = pack2(S[2 * j][c], S[2 * j + 1][c]);
+    }
   }
   const float skip = p.skip ? p.skip[h] : 0.f;
   const float rate = p.mode == DECAY_PER_HEAD ? expf(p.a_log[h]) : 0.f;
@@ -225,7 +259,15 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
         x.z = floored ? 1.0f - decay : decay;
         if (bonus && PHASE != SCAN_CHUNK_SUMS) x.w = x.x * p.bonus[(size_t)h * dim + i] * x.y;
       }
-      tok[e] = x;
+      if (PAIRS) {
+        float* to = tok2 + (size_t)tt * 4 * plane + ((i & 7) >> 2) * half_stride + (i >> 3) * 4 + (i & 3);
+        if (PHASE != SCAN_CHUNK_SUMS) to[0] = x.x;
+        to[plane] = x.y;
+        to[2 * plane] = x.z;
+        if (bonus && PHASE != SCAN_CHUNK_SUMS) to[3 * plane] = x.w;
+      } else {
+        tok[e] = x;
+      }
     }
 #pragma unroll
     for (int u = 0; u < VPT; u++) {
@@ -248,6 +290,41 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
       for (int c = 0; c < COLS; c++) o[c] = 0.f;
       const float4* cur = tok + ((size_t)tt << rows_log2) + slice;
       float own = 0.f;                                 // the weight of the token's own value
+      if (PAIRS) {
+        const float* at = tok2 + (size_t)tt * 4 * plane + slice * 4;
+        unsigned long long q2[4], k2[4], a2[4], v2[COLS], o2[COLS];
+        auto four = [&](int which, unsigned long long (&to)[4]) {
+          const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(at + which * plane), hi = *reinterpret_cast<const ulonglong2*>(at + which * plane + half_stride);
+          to[0] = lo.x; to[1] = lo.y; to[2] = hi.x; to[3] = hi.y;
+        };
+        four(1, k2);
+        four(2, a2);
+        if (PHASE != SCAN_CHUNK_SUMS) four(0, q2);
+#pragma unroll
+        for (int c = 0; c < COLS; c++) { v2[c] = pack2(v[c], v[c]); o2[c] = 0ull; }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+#pragma unroll
+          for (int c = 0; c < COLS; c++) {
+            const unsigned long long s = fma2(a2[j], S2[PAIRS ? j : 0][c], mul2(k2[j], v2[c]));
+            if (PHASE != SCAN_CHUNK_SUMS) o2[c] = fma2(bonus ? S2[PAIRS ? j : 0][c] : s, q2[j], o2[c]);
+            S2[PAIRS ? j : 0][c] = s;
+          }
+          if (PHASE == SCAN_CHUNK_SUMS) P2[PAIRS ? j : 0] = mul2(P2[PAIRS ? j : 0], a2[j]);
+        }
+        if (PHASE != SCAN_CHUNK_SUMS) {
+#pragma unroll
+          for (int c = 0; c < COLS; c++) {
+            float lo, hi;
+            unpack2(o2[c], lo, hi);
+            o[c] = lo + hi;
+          }
+          if (bonus) {
+            const float4 w0 = *reinterpret_cast<const float4*>(at + 3 * plane), w1 = *reinterpret_cast<const float4*>(at + 3 * plane + half_stride);
+            own = ((w0.x + w0.y) + (w0.z + w0.w)) + ((w1.x + w1.y) + (w1.z + w1.w));
+          }
+        }
+      } else
 #pragma unroll
       for (int j = 0; j < ROWS; j++) {
         const float4 x = cur[j << slices_log2];
@@ -291,9 +368,17 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   }
   if (PHASE == SCAN_CHUNK_OUT && !last_chunk) return;
   float* to = PHASE == SCAN_CHUNK_SUMS ? held : mine;
+  if (PAIRS) {
+#pragma unroll
+    for (int j = 0; j < ROWS / 2; j++) {
+#pragma unroll
+      for (int c = 0; c < COLS; c++) unpack2(S2[PAIRS ? j : 0][c], S[2 * j][c], S[2 * j + 1][c]);
+      if (PHASE == SCAN_CHUNK_SUMS) unpack2(P2[PAIRS ? j : 0], P[(2 * j) % (PHASE == SCAN_CHUNK_SUMS ? ROWS : 1)], P[(2 * j + 1) % (PHASE == SCAN_CHUNK_SUMS ? ROWS : 1)]);
+    }
+  }
 #pragma unroll
   for (int j = 0; j < ROWS; j++) {
-    const int row = j * slices + slice;
+    const int row = row_of(j);
     if (COLS == 4 && vectors) {
       if (col < p.vdim && row < dim)
         *reinterpret_cast<float4*>(to + (size_t)row * p.vdim + col) = make_float4(S[j][0], S[j][1 % COLS], S[j][2 % COLS], S[j][3 % COLS]);
@@ -678,7 +763,8 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
   const int by_rows = (ROWS == 8 ? 128 : 64) / slices, by_values = SCAN_MAX_TOKENS * slices / COLS;
   if (batch > by_rows) batch = by_rows;
   if (batch > by_values) batch = by_values;
-  const size_t smem = (size_t)batch * ((size_t)ROWS * slices * sizeof(float4) + (size_t)cb * sizeof(float));
+  const size_t vectors = ROWS == 8 && COLS == 4 ? (size_t)4 * 2 * (ROWS * slices / 2 + 16) * sizeof(float) : (size_t)ROWS * slices * sizeof(float4);
+  const size_t smem = (size_t)batch * (vectors + (size_t)cb * sizeof(float));
   const dim3 grid(requests, p.heads, (p.vdim + cb - 1) / cb);
   SPROUT_REQUIRE(grid.z <= 65535, "gated_scan: too many value columns");
   if (p.sums == nullptr && p.mode == DECAY_GIVEN) {
