@@ -68,7 +68,23 @@ struct ScanParams {
   int chunk, requests;
   int q_silu;                          // silu on the query rows (with a floor only)
   int v_cols, ones_col;                // columns the value rows really have (<= vdim); column v_cols of the state is fed 1
+  int wide;                            // q, k and decay rows are fetched 8 neighbours at a time (walks over ready-made decays)
 };
+
+// Eight neighbouring elements of a row that start on a 16-byte boundary.
+__device__ __forceinline__ void fetch8(const float* p, float (&v)[8]) {
+  const float4 a = *(const float4*)p, b = *(const float4*)(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void fetch8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 raw = *(const uint4*)p;
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
 
 // The chunks of all requests are numbered in the requests' order, ceil(tokens / chunk) each.  Finds chunk `index`:
 // its request, its place among the request's chunks and how many the request has; false beyond the last chunk.
@@ -112,7 +128,8 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
 // shuffles.  Tiles of 8 x 4 (PAIRS) are walked two rows at a time in packed arithmetic: a thread's rows are neighbours, and q, c k and a
 // lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us
-// for the two walks with a number at a time and (q, c k, a) triples, SUMS and OUTS us so).  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
+// for the two walks with a number at a time, (q, c k, a) triples and 2-byte fetches, 106 and 237 us so, the rows fetched 16 bytes at a
+// time where they start on 16-byte boundaries and fill the slices).  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
 // depend on the cutting or on the batch.
 //
 // Long portions are cut into chunks of `p.chunk` tokens so that more blocks than (request, head, columns) have work, in
@@ -198,8 +215,47 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   auto z_at = [&](size_t index) { return p.z_f32 ? ((const float*)p.z)[index] : to_float(((const T*)p.z)[index]); };
 
   float rq[EPT], rk[EPT], rz[EPT], rc[PHASE == SCAN_WHOLE ? 1 : EPT], rv[VPT];
+  // wide: a thread's eight elements are the rows 8 (tid % slices) on of token tid / slices of the batch, its values neighbours too
+  const bool wide = PAIRS && PHASE != SCAN_WHOLE && p.wide;
+  const int wide_token = tid >> slices_log2, wide_values = (batch << cb_log2) / SCAN_THREADS;
   auto fetch = [&](int t0) {                          // loads only: nothing waits for them here
     const int n = min(batch, last - t0);
+    if (wide) {
+      if (wide_token < n) {
+        const size_t t = (size_t)t0 + wide_token;
+        const int i = slice * 8;
+        float x[8];
+        if (PHASE != SCAN_CHUNK_SUMS) {
+          fetch8(p.q + t * p.q_stride + (size_t)g * dim + i, x);
+#pragma unroll
+          for (int u = 0; u < 8; u++) rq[u % EPT] = x[u];
+        }
+        if (!floored) {
+          fetch8(p.k + t * p.k_stride + (size_t)g * dim + i, x);
+#pragma unroll
+          for (int u = 0; u < 8; u++) rk[u % EPT] = x[u];
+        }
+        if (per_head) {
+          const float a = p.da[t * p.heads + h];
+#pragma unroll
+          for (int u = 0; u < 8; u++) rz[u % EPT] = a;
+          rc[0] = p.dc[t * p.heads + h];
+        } else {
+          fetch8(p.da + (t * p.heads + h) * dim + i, x);
+#pragma unroll
+          for (int u = 0; u < 8; u++) rz[u % EPT] = x[u];
+          rc[0] = 1.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < VPT; u++) {
+        if (u >= wide_values) break;
+        const int e = tid * wide_values + u, tt = e >> cb_log2, column = blockIdx.z * cb + (e & (cb - 1));
+        rv[u] = (tt < n && column < p.v_cols) ? to_float(p.v[(size_t)(t0 + tt) * p.v_stride + (size_t)h * p.v_cols + column])
+                                              : (p.ones_col && tt < n && column == p.v_cols) ? 1.f : 0.f;
+      }
+      return;
+    }
     // the batch's first rows once in 64-bit; within the batch 32-bit offsets do (at most SCAN_MAX_TOKENS rows further)
     const size_t tb = (size_t)t0;
     const T* qrow = p.q + tb * p.q_stride + (size_t)g * dim;
@@ -234,6 +290,32 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   for (int t0 = first; t0 < last; t0 += batch) {
     const int n = min(batch, last - t0);
     __syncthreads();                                   // the batch before has been read by everyone
+    if (wide) {
+      if (wide_token < n) {
+        float4* to = reinterpret_cast<float4*>(tok2 + (size_t)wide_token * 4 * plane + slice * 4);
+        const int half4 = half_stride / 4, plane4 = plane / 4;
+        float x[4][8];                                 // q, k, a, -
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const float decay = rz[u % EPT];
+          x[0][u] = PHASE == SCAN_CHUNK_SUMS ? 0.f : (floored && p.q_silu ? silu_g(rq[u % EPT]) : rq[u % EPT]) * p.q_scale;
+          x[1][u] = floored ? decay : rk[u % EPT] * rc[0];
+          x[2][u] = floored ? 1.0f - decay : decay;
+          if (bonus && PHASE != SCAN_CHUNK_SUMS) x[3][u] = x[0][u] * p.bonus[(size_t)h * dim + slice * 8 + u] * x[1][u];
+        }
+#pragma unroll
+        for (int which = 0; which < 4; which++) {
+          if ((which == 0 && PHASE == SCAN_CHUNK_SUMS) || (which == 3 && (!bonus || PHASE == SCAN_CHUNK_SUMS))) continue;
+          to[which * plane4] = make_float4(x[which][0], x[which][1], x[which][2], x[which][3]);
+          to[which * plane4 + half4] = make_float4(x[which][4], x[which][5], x[which][6], x[which][7]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < VPT; u++) {
+        if (u >= wide_values) break;
+        vt[tid * wide_values + u] = rv[u];
+      }
+    } else {
 #pragma unroll
     for (int u = 0; u < EPT; u++) {
       const int e = tid + u * SCAN_THREADS, tt = e >> rows_log2, i = e & (rows_pad - 1);
@@ -273,6 +355,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
     for (int u = 0; u < VPT; u++) {
       const int e = tid + u * SCAN_THREADS;
       if (e < (n << cb_log2)) vt[e] = rv[u];
+    }
     }
     __syncthreads();
     if (t0 + batch < last) fetch(t0 + batch);          // in flight while this batch is applied
@@ -788,7 +871,12 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
 }
 
 template <typename T>
-int launch_scan(const ScanParams<T>& p, int requests, int max_chunks, cudaStream_t stream) {
+int launch_scan(ScanParams<T> p, int requests, int max_chunks, cudaStream_t stream) {
+  // 16-byte fetches: the rows fill the tile's slices, and every row starts on a 16-byte boundary
+  constexpr int per16 = 16 / (int)sizeof(T);
+  auto on16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
+  p.wide = (p.dim == 8 || p.dim == 16 || p.dim == 32 || p.dim == 64 || p.dim == 128 || p.dim == 256) && p.q_stride % per16 == 0 &&
+           (!p.k || p.k_stride % per16 == 0) && on16(p.q) && on16(p.k) && on16(p.da);
   // a thread's tile of the state: 8 rows x 4 columns up to 256 key channels, 32 rows of one column up to 1024
   const bool narrow = p.dim <= 8 * 32;
   if (p.mode == DECAY_FLOOR)
