@@ -740,3 +740,17 @@ SPROUT_API int sprout_latent_unfolded_attention(const void* q, int q_stride, con
   if (dim + tail == 64) return vdim == 64 ? launch<64, 64, 1, true>(map_k, map_v, p, (int)ctas, stream) : launch<64, 128, 1, true>(map_k, map_v, p, (int)ctas, stream);
   return launch<128, 128, 1, true>(map_k, map_v, p, (int)ctas, stream);
 }
+
+// The arguments of sprout_attention_prefill, checked there; scratch and counters may be null.
+int sprout_attention_prefill_maps(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table, int table_stride,
+                                  const int* q_start, const int* positions, void* out, int out_stride, int num_tokens, int requests, int heads,
+                                  int kv_heads, int head_dim, int page_tokens, int num_pages, float* scratch, long long scratch_floats, int* counters,
+                                  int* status, cudaStream_t stream) {
+  MultiMapParams m{};
+  m.q = (const __nv_bfloat16*)q; m.q_stride = q_stride; m.k_cache = (const __nv_bfloat16*)k_cache; m.v_cache = (const __nv_bfloat16*)v_cache;
+  m.block_table = block_table; m.table_stride = table_stride; m.q_start = q_start; m.positions = positions;
+  m.out = (__nv_bfloat16*)out; m.out_stride = out_stride; m.requests = requests; m.heads = heads; m.kv_heads = kv_heads;
+  m.page_tokens = page_tokens; m.num_pages = num_pages; m.scale = 1.0f / sqrtf((float)head_dim); m.out_scale = 1.0f; m.status = status; m.ksplit = 1;
+  const bool fits = scratch && counters && sprout_maps_attention_tc_scratch_floats(num_tokens, requests, heads, kv_heads, 1, head_dim) <= scratch_floats;
+  return sprout_maps_attention_tc(m, num_tokens, 1, head_dim, head_dim, fits ? scratch : nullptr, fits ? counters : nullptr, stream);
+}

@@ -24,8 +24,8 @@
 // timeout the CTA sets the status word, waits (bounded) for its copies in flight, frees its
 // tensor memory and returns.
 //
-// Takes head_dim 64 or 128 and page sizes of 8, 16, 32, 64 or a multiple of 128 tokens; the
-// mma.sync kernel in attention_bf16.cu takes everything else.
+// Runs for head_dim 64 in launches of many pieces; the kernel in attention_maps_tcgen05.cu takes head_dim 128 and smaller launches.
+// Page sizes of 8, 16, 32, 64 or a multiple of 128 tokens; the mma.sync kernel in attention_bf16.cu takes everything else.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -563,6 +563,12 @@ SPROUT_API long long sprout_attention_prefill_scratch_floats(int head_dim) {
 }
 SPROUT_API int sprout_attention_prefill_counters() { return SPROUT_PREFILL_SPLIT_MAX * TC_QTILES; }
 
+// attention_maps_tcgen05.cu: the same arguments, head_dim 64 or 128.
+int sprout_attention_prefill_maps(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table, int table_stride,
+                                  const int* q_start, const int* positions, void* out, int out_stride, int num_tokens, int requests, int heads,
+                                  int kv_heads, int head_dim, int page_tokens, int num_pages, float* scratch, long long scratch_floats, int* counters,
+                                  int* status, cudaStream_t stream);
+
 // The arguments of sprout_attention_prefill, checked there; scratch and counters may be null.
 int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache, const void* v_cache,
                                 const int* block_table, int table_stride, const int* q_start, const int* positions,
@@ -571,6 +577,13 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
                                 int* counters, int* status, cudaStream_t stream) {
   SPROUT_REQUIRE(sprout_attention_prefill_tc_supported(head_dim, page_tokens, out_stride) && ((uintptr_t)out & 15) == 0,
                  "attention_prefill (tcgen05): head_dim %d, page size %d or the output's alignment is not taken", head_dim, page_tokens);
+  // Head size 128 runs on the kernel whose O stays in tensor memory (28 heads over 4, one prompt of 4,096 tokens: 180 us against 232 with
+  // O added up in registers), and so do launches of few 256-row pieces, whose keys it divides among up to four CTAs (14 heads of 64 over 2,
+  // 300 tokens: 15.6 against 23.7 us).  Larger launches of head size 64 keep this kernel's 128-key tiles (2,048 tokens: 34.5 against 39.5 us).
+  const long long pieces = (((long long)num_tokens * (heads / kv_heads) + TC_QTILES * TC_ROWS - 1) / (TC_QTILES * TC_ROWS) + requests) * kv_heads;
+  if (head_dim == 128 || 2 * pieces <= sm_count())
+    return sprout_attention_prefill_maps(q, q_stride, k_cache, v_cache, block_table, table_stride, q_start, positions, out, out_stride, num_tokens, requests,
+                                         heads, kv_heads, head_dim, page_tokens, num_pages, scratch, scratch_floats, counters, status, stream);
   const long long cache_rows = (long long)num_pages * kv_heads * page_tokens;
   SPROUT_REQUIRE(cache_rows <= 0x7fffffffLL, "attention_prefill (tcgen05): the cache has too many rows for a tensor map coordinate");
   TcParams p;
@@ -578,7 +591,7 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
   p.block_table = block_table; p.table_stride = table_stride; p.q_start = q_start; p.positions = positions;
   p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
   p.requests = requests; p.heads = heads; p.kv_heads = kv_heads; p.page_tokens = page_tokens; p.num_pages = num_pages;
-  const int keys = head_dim == 64 ? TcLayout<64>::KEYS : TcLayout<128>::KEYS;
+  constexpr int keys = TcLayout<64>::KEYS;
   p.box_rows = page_tokens < keys ? page_tokens : keys;
   p.scale = 1.0f / sqrtf((float)head_dim); p.status = status;
   CUtensorMap map_k, map_v;
@@ -598,6 +611,5 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
     if (n > SPROUT_PREFILL_SPLIT_MAX) n = SPROUT_PREFILL_SPLIT_MAX;
     p.split_pieces = (int)n;
   }
-  if (head_dim == 64) return launch_tc<64>(map_k, map_v, p, (int)bound, stream);
-  return launch_tc<128>(map_k, map_v, p, (int)bound, stream);
+  return launch_tc<64>(map_k, map_v, p, (int)bound, stream);
 }

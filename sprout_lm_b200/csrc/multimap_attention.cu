@@ -542,6 +542,9 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   // SPLIT (a step in which no request has more than 16 rows: single tokens, the heads of one key/value group): a CTA
   // divides every tile's keys among its warps instead of its rows, and the warps' partial results are merged at the end.
   constexpr bool split = SPLIT;
+  // rows 8 to 15 of a tile are the second two numbers of every fragment: where a request has at most 8 rows (4 heads a group, usually)
+  // their scores are not capped, compared or exponentiated (64 requests over 6,000 keys, capped scores: 200 us with them, CAPPED us without)
+  const bool upper = !SPLIT || rows_total > 8;
   const int qrow = split ? 0 : warp * 16;             // the warp's 16 rows
   constexpr int nk = split ? 1 : MM_KEYS / 16;        // blocks of 16 keys of a tile that the warp takes, from key kb on
   const int kb = split ? warp * 16 : 0;
@@ -601,7 +604,10 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
         for (int i = 0; i < MM_KEYS / 8; i++) {
           if (i >= 2 * nk) break;
 #pragma unroll
-          for (int c = 0; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
+          for (int c = 0; c < 2; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
+          if (!upper) continue;
+#pragma unroll
+          for (int c = 2; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
         }
       }
       float t_max0 = -INFINITY, t_max1 = -INFINITY;
@@ -650,8 +656,9 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
       for (int i = 0; i < MM_KEYS / 8; i++) {
         if (i >= 2 * nk) break;
         s[i][0] = exp2f(fmaf(s[i][0], scale_log2, -base0)); s[i][1] = exp2f(fmaf(s[i][1], scale_log2, -base0));
-        s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
         l0[m] += s[i][0] + s[i][1];
+        if (!upper) { s[i][2] = s[i][3] = 0.f; continue; }
+        s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
         l1[m] += s[i][2] + s[i][3];
       }
 #pragma unroll
