@@ -24,7 +24,7 @@
 // timeout the CTA sets the status word, waits (bounded) for its copies in flight, frees its
 // tensor memory and returns.
 //
-// Runs for head_dim 64 in launches of many pieces; the kernel in attention_maps_tcgen05.cu takes head_dim 128 and smaller launches.
+// Runs for head_dim 64; the kernel in attention_maps_tcgen05.cu takes head_dim 128.
 // Page sizes of 8, 16, 32, 64 or a multiple of 128 tokens; the mma.sync kernel in attention_bf16.cu takes everything else.
 #include <cuda_bf16.h>
 
@@ -578,10 +578,8 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
   SPROUT_REQUIRE(sprout_attention_prefill_tc_supported(head_dim, page_tokens, out_stride) && ((uintptr_t)out & 15) == 0,
                  "attention_prefill (tcgen05): head_dim %d, page size %d or the output's alignment is not taken", head_dim, page_tokens);
   // Head size 128 runs on the kernel whose O stays in tensor memory (28 heads over 4, one prompt of 4,096 tokens: 180 us against 232 with
-  // O added up in registers), and so do launches of few 256-row pieces, whose keys it divides among up to four CTAs (14 heads of 64 over 2,
-  // 300 tokens: 15.6 against 23.7 us).  Larger launches of head size 64 keep this kernel's 128-key tiles (2,048 tokens: 34.5 against 39.5 us).
-  const long long pieces = (((long long)num_tokens * (heads / kv_heads) + TC_QTILES * TC_ROWS - 1) / (TC_QTILES * TC_ROWS) + requests) * kv_heads;
-  if (head_dim == 128 || 2 * pieces <= sm_count())
+  // O added up in registers); head size 64 keeps this kernel's 128-key tiles (14 heads over 2, 2,048 tokens: 34.5 against 39.5 us).
+  if (head_dim == 128)
     return sprout_attention_prefill_maps(q, q_stride, k_cache, v_cache, block_table, table_stride, q_start, positions, out, out_stride, num_tokens, requests,
                                          heads, kv_heads, head_dim, page_tokens, num_pages, scratch, scratch_floats, counters, status, stream);
   const long long cache_rows = (long long)num_pages * kv_heads * page_tokens;

@@ -68,7 +68,7 @@ struct ScanParams {
   int chunk, requests;
   int q_silu;                          // silu on the query rows (with a floor only)
   int v_cols, ones_col;                // columns the value rows really have (<= vdim); column v_cols of the state is fed 1
-  int wide;                            // q, k and decay rows are fetched 8 neighbours at a time (walks over ready-made decays)
+  int wide;                            // q, k and decay rows are fetched 8 neighbours at a time (chunks' walks)
 };
 
 // Eight neighbouring elements of a row that start on a 16-byte boundary.
@@ -126,7 +126,7 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // Tokens come `batch` at a time: while the threads walk a batch's tokens over their registers, the next batch's q, k,
 // decay inputs and values are on their way from memory into registers; at the batch's end they are turned into
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
-// shuffles.  Tiles of 8 x 4 (PAIRS) are walked two rows at a time in packed arithmetic: a thread's rows are neighbours, and q, c k and a
+// shuffles.  The chunks' walks over tiles of 8 x 4 (PAIRS) go two rows at a time in packed arithmetic: a thread's rows are neighbours, and q, c k and a
 // lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us
 // for the two walks with a number at a time, (q, c k, a) triples and 2-byte fetches, 106 and 237 us so, the rows fetched 16 bytes at a
 // time where they start on 16-byte boundaries and fill the slices).  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
@@ -141,7 +141,7 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // differs: (a_n ... a_1) S + sums instead of a_n (... (a_1 S)).
 // FORM: FORM_FLOOR is the forget gate with a floor (DECAY_FLOOR), FORM_BONUS the output that reads the state before the token
 // (DECAY_BONUS): the fourth number of a row's vector is then q_scale q u k, whose sum over the rows weighs the token's value.
-template <typename T, int ROWS, int COLS, int PHASE, int FORM>
+template <typename T, int ROWS, int COLS, int PHASE, int FORM, bool PAIRS>
 __global__ void __launch_bounds__(SCAN_THREADS, ROWS == 8 ? 4 : 2)
 gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   constexpr int ROWS_LOG2 = ROWS == 8 ? 3 : 5;
@@ -153,7 +153,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   const int rows_log2 = slices_log2 + ROWS_LOG2, rows_pad = 1 << rows_log2;
   const int cb_log2 = 7 - slices_log2 + (COLS == 4 ? 2 : 0), cb = 1 << cb_log2;
   static_assert(COLS == 1 || COLS == 4, "columns of a thread's tile");
-  constexpr bool PAIRS = ROWS == 8 && COLS == 4;
+  static_assert(!PAIRS || (ROWS == 8 && COLS == 4 && PHASE != SCAN_WHOLE), "pairs of rows in tiles of 8 x 4, over ready-made decays");
   float4* tok = scan_smem;                                             // [batch][rows_pad]: (q, k, a, -)
   // PAIRS: [batch][4 planes: q, k, a, -][2 halves of every 8 rows][slices][4], a half padded so that the two halves' banks differ
   const int half_stride = rows_pad / 2 + 16, plane = 2 * half_stride;
@@ -216,7 +216,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
 
   float rq[EPT], rk[EPT], rz[EPT], rc[PHASE == SCAN_WHOLE ? 1 : EPT], rv[VPT];
   // wide: a thread's eight elements are the rows 8 (tid % slices) on of token tid / slices of the batch, its values neighbours too
-  const bool wide = PAIRS && PHASE != SCAN_WHOLE && p.wide;
+  const bool wide = PAIRS && p.wide;
   const int wide_token = tid >> slices_log2, wide_values = (batch << cb_log2) / SCAN_THREADS;
   auto fetch = [&](int t0) {                          // loads only: nothing waits for them here
     const int n = min(batch, last - t0);
@@ -846,27 +846,30 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
   const int by_rows = (ROWS == 8 ? 128 : 64) / slices, by_values = SCAN_MAX_TOKENS * slices / COLS;
   if (batch > by_rows) batch = by_rows;
   if (batch > by_values) batch = by_values;
-  const size_t vectors = ROWS == 8 && COLS == 4 ? (size_t)4 * 2 * (ROWS * slices / 2 + 16) * sizeof(float) : (size_t)ROWS * slices * sizeof(float4);
-  const size_t smem = (size_t)batch * (vectors + (size_t)cb * sizeof(float));
+  // single walks (few tokens: the state's way in and out is most of their time, and rows dealt in turn read it faster: 64 single tokens
+  // of 16 heads 46 against 52 us) keep a number at a time
+  constexpr bool PAIRED = ROWS == 8 && COLS == 4;
+  const size_t smem = (size_t)batch * ((size_t)ROWS * slices * sizeof(float4) + (size_t)cb * sizeof(float));
+  const size_t smem_chunks = PAIRED ? (size_t)batch * ((size_t)4 * 2 * (ROWS * slices / 2 + 16) + cb) * sizeof(float) : smem;
   const dim3 grid(requests, p.heads, (p.vdim + cb - 1) / cb);
   SPROUT_REQUIRE(grid.z <= 65535, "gated_scan: too many value columns");
   if (p.sums == nullptr && p.mode == DECAY_GIVEN) {
-    sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM>, grid, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
+    sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, false>, grid, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
     return sprout_check_launch("gated_scan");
   }
   if (p.sums == nullptr) {
-    sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_WHOLE, FORM>, grid, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
+    sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_WHOLE, FORM, false>, grid, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
     return sprout_check_launch("gated_scan");
   }
   // `max_chunks` blocks per (head, columns): the chunks of all requests, found by their number
   const dim3 chunks(max_chunks, p.heads, grid.z);
-  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM>, chunks, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
+  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, PAIRED>, chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
   if (int rc = sprout_check_launch("gated_scan (chunk sums)")) return rc;
   SPROUT_REQUIRE(requests <= 65535, "gated_scan: too many requests");
   sprout_launch(scan_carry_kernel, dim3((p.dim * p.vdim + 255) / 256, p.heads, requests), dim3(256), 0, stream, p.sums,
                 (const float*)p.prods, (const float*)p.state, p.q_start, p.state_slots, p.num_slots, p.chunk, p.heads, p.dim, p.vdim);
   if (int rc = sprout_check_launch("gated_scan (carry)")) return rc;
-  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM>, chunks, dim3(SCAN_THREADS), smem, stream, p, slices_log2, batch);
+  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, PAIRED>, chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
   return sprout_check_launch("gated_scan (chunk outputs)");
 }
 

@@ -1162,15 +1162,16 @@ def latent_attention(qlat, cache, ctx, sink, out, heads: int, rank: int, scale: 
 # The unfolded form: keys and values of every head are made once per cached row that the step's queries see, and the attention itself
 # multiplies dim + tail + vdim elements a (query, key) pair instead of 2 rank + tail.  Making them pays from some 75 new tokens a
 # request on (2,048 tokens of 16 heads over a latent of 512: 412 us folded with 47 us of products per head, 64 us with 8 us of packing and rotation and 15 us of product unfolded); the
-# rows it is made for are bounded by the block tables' width, and scratch by UNFOLD_ROWS of them.
-UNFOLD_TOKENS, UNFOLD_ROWS = 128, 16384
+# rows it is made for are bounded by the block tables' width, and scratch by UNFOLD_ROWS of them.  Steps under UNFOLD_STEP tokens are
+# short on both ways, and the folded one allocates less (128 tokens, launched one by one: 144 against 156 us a layer).
+UNFOLD_TOKENS, UNFOLD_STEP, UNFOLD_ROWS = 128, 512, 16384
 
 
 def latent_unfold_rows(ctx, cache, tokens: int, heads: int, dim: int, tail: int, vdim: int, rank: int, rot: int, window: int = 0) -> int:
     """Rows of scratch for the unfolded form of a step's latent attention, 0 where the folded form runs (few new tokens a request, sizes
     that the tcgen05 kernel does not take, more rows than UNFOLD_ROWS)."""
     if LATENT_ATTENTION != "auto" or cache.k.dtype != torch.bfloat16 or dim <= 0 or dim % 64 or tail % 64 or (dim + tail, vdim) not in ((64, 64), (64, 128), (128, 128)) \
-            or rank % 8 or rot % 16 or tokens < UNFOLD_TOKENS * ctx.num_seqs:
+            or rank % 8 or rot % 16 or tokens < UNFOLD_TOKENS * ctx.num_seqs or tokens < UNFOLD_STEP:
         return 0
     keys = cache.block_table.shape[1] * cache.page_tokens
     if window:
@@ -1209,7 +1210,8 @@ def latent_unfolded_attention(q, unfolded, packed, ctx, sink, out, heads: int, d
             or packed.shape[1] < rank + tail or (sink is not None and sink.numel() != heads):
         raise KernelError("latent_unfolded_attention: shapes or dtypes do not fit")
     _rows_contiguous(out, "out")
-    floats = (_lib or load_library()).sprout_maps_attention_tc_scratch_floats(T, requests, heads, heads, 1, vdim)
+    load_library()
+    floats = _maps_tc_scratch(T, requests, heads, heads, 1, vdim)
     scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
     _run("sprout_latent_unfolded_attention", _ptr(q, "q"), q.stride(0), _ptr(unfolded, "unfolded"), _ptr(packed, "packed"), rows, packed.shape[1], rank,
          _ptr(ctx.q_start, "q_start", torch.int32), _ptr(ctx.positions, "positions", torch.int32), _ptr(sink, "sink", torch.float32, True), _ptr(out, "out"),
@@ -1541,6 +1543,22 @@ def visible_keys(mask, context: int) -> int:
     return context if kind == 0 else min(context, size + 63 + (-(-keep // 64) * 64 if keep else 0))
 
 
+# (token, head) rows of a step from which prompt attention with one or two maps runs on tcgen05: below, a layer's launches take the host
+# longer than the device either way, and the mma.sync kernel needs no scratch (60 tokens of 8 heads: 77 against 81 us a layer)
+MAPS_TC_ROWS = 2048
+
+
+@functools.lru_cache(maxsize=256)
+def _maps_tc_takes(maps: int, dim: int, vdim: int, page_tokens: int, out_stride: int) -> bool:
+    return bool(_lib.sprout_maps_attention_tc_supported(maps, dim, vdim, page_tokens, out_stride))
+
+
+@functools.lru_cache(maxsize=4096)
+def _maps_tc_scratch(tokens: int, requests: int, heads: int, kv_heads: int, maps: int, vdim: int) -> int:
+    """Floats of scratch with which the tcgen05 kernel divides a piece's keys among CTAs in a step of these sizes (0: it does not)."""
+    return int(_lib.sprout_maps_attention_tc_scratch_floats(tokens, requests, heads, kv_heads, maps, vdim))
+
+
 def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int, dim: int, vdim: int, scale: float, lam: float,
                        norm_eps: float, out_scale: float, status, mask=None, sink=None, gate=None, softcap: float = 0.0, turn=None,
                        interleaved: bool = False, counters=None):
@@ -1565,20 +1583,23 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
         group = heads // kv_heads
         tiles = (q.shape[0] * group + 63) // 64 + requests
         max_q_len = int(getattr(ctx, "max_q_len", 0) or q.shape[0])
-        planned = int(getattr(ctx, "planned_context", 0) or getattr(ctx, "max_context", 0) or 0)
-        ksplit = multimap_key_split(requests, kv_heads, group, max_q_len, visible_keys(mask, planned)) if planned else 1
+        ksplit = 1
+        if max_q_len * group <= 16:                # single tokens; other steps do not divide a request's keys here
+            planned = int(getattr(ctx, "planned_context", 0) or getattr(ctx, "max_context", 0) or 0)
+            ksplit = multimap_key_split(requests, kv_heads, group, max_q_len, visible_keys(mask, planned)) if planned else 1
         mask_kind, mask_size, mask_keep = _mask_code(mask)
         gate_ptr, gate_stride, gate_elements = _gate_args(gate, q.shape[0], heads, vdim, q.dtype, "multimap_attention")
         turn_cos, turn_sin, turned = _turn_args(turn, vdim, "multimap_attention")
         if sink is not None and (sink.dtype != torch.float32 or sink.numel() != heads):
             raise KernelError("multimap_attention: one float32 sink per head")
         partial = None
-        # tcgen05 for steps whose requests bring 128 (token, head) rows each on average: a CTA of it takes 256, of the mma.sync kernel 64
+        # tcgen05 for steps whose requests bring 128 (token, head) rows of a key/value head each on average (a CTA of it takes 256, of the
+        # mma.sync kernel 64) and MAPS_TC_ROWS in all
         tensor = 0
-        if choice != "mma_sync" and ksplit == 1 and max_q_len * group > 16 and q.shape[0] * group >= 128 * requests and out.data_ptr() % 16 == 0 \
-                and _lib.sprout_maps_attention_tc_supported(maps, dim, vdim, cache.page_tokens, out.stride(0)):
+        if q.shape[0] * heads >= MAPS_TC_ROWS and q.shape[0] * group >= 128 * requests and choice != "mma_sync" and max_q_len * group > 16 and out.data_ptr() % 16 == 0 \
+                and _maps_tc_takes(maps, dim, vdim, cache.page_tokens, out.stride(0)):
             tensor = q.shape[0]
-            floats = 0 if counters is None else _lib.sprout_maps_attention_tc_scratch_floats(tensor, requests, heads, kv_heads, maps, vdim)
+            floats = 0 if counters is None else _maps_tc_scratch(tensor, requests, heads, kv_heads, maps, vdim)
             if floats:
                 partial = torch.empty(floats, dtype=torch.float32, device=q.device)
         if ksplit > 1:

@@ -1076,6 +1076,7 @@ def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, h
     sizes = (heads, kv_heads, maps, dim, vdim, dim ** -0.5, options.get("lam", 0.0), options.get("norm_eps", 0.0), options.get("out_scale", 1.0), status)
     counters = torch.zeros(2 * kernels.sm_count(torch.device(DEV)), dtype=torch.int32, device=DEV) if divided else None
     got = torch.full((T, heads * vdim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    monkeypatch.setattr(kernels, "MAPS_TC_ROWS", 0)
     kernels.multimap_attention(q, cache, ctx, got, *sizes, counters=counters, **more)
     assert int(status.item()) == 0
     assert counters is None or not counters.any()
@@ -1131,6 +1132,7 @@ def test_rope_maps_append_in_16_byte_accesses(status, maps, dim, vdim, rot, opti
         kernels.rope_maps_append(rows, positions, seqs, table, cos, sin, k if write else None, v if write else None, heads * maps, kv_heads, maps, dim, vdim, page,
                                  write, status, **more)
         results.append((rows[:, :sum(widths)].float(), k.float(), v.float(), int(status.item())))
+    status.zero_()
     assert results[0][3] == results[1][3] == (1 if write else 0)
     for fast, general in zip(results[0][:3], results[1][:3]):
         # one rounding to bfloat16 of float32 results whose sums are added in another order
@@ -1138,7 +1140,7 @@ def test_rope_maps_append_in_16_byte_accesses(status, maps, dim, vdim, rot, opti
 
 
 @pytest.mark.parametrize("unit", ["clamped_glu", "plain", "silu_glu"])
-@pytest.mark.parametrize("counts,width,ff,weighted", [([256, 0, 257, 1, 30], 512, 256, False), ([0, 700, 0, 3], 520, 264, True), ([17] * 40, 640, 384, True)])
+@pytest.mark.parametrize("counts,width,ff,weighted", [([256, 0, 257, 1, 1540], 512, 256, False), ([0, 2050, 0, 3], 520, 264, True), ([17] * 40, 1032, 1040, True)])
 def test_experts_on_tcgen05(status, monkeypatch, unit, counts, width, ff, weighted):
     """Experts without rows, with one, at the edges of the 256-row tiles, sizes that no tile divides: against the CUDA-core products."""
     from sprout_lm_b200 import kernels
@@ -1202,6 +1204,7 @@ def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, 
                       q_start=ints(starts), context_lens=ints(total), state_slots=ints([0] * len(new)), logits_rows=ints([0]), block_tables=[table.to(DEV)], page_tokens=page)
     h = torch.randn(T, width, generator=g).to(torch.bfloat16).to(DEV)
     results = []
+    monkeypatch.setattr(kernels, "UNFOLD_STEP", 128)
     for rows in (kernels.UNFOLD_ROWS, 0):
         monkeypatch.setattr(kernels, "UNFOLD_ROWS", rows)
         view = CacheView(cache.to(torch.bfloat16).to(DEV), None, ctx.block_tables[0], page, True)
