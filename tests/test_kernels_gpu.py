@@ -1215,3 +1215,51 @@ def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, 
         results.append(x)
     # two forms of the same sums with the intermediate results rounded to bfloat16 at other places
     assert (results[0] - results[1]).norm() <= 1.5e-2 * results[1].norm()
+
+
+@pytest.mark.parametrize("rows,part,groups,period,gate_dtype,gate_first,silu", [
+    (1, 4, 1, 4, None, False, True), (7, 64, 6, 64, torch.float32, True, True), (33, 100, 3, 300, torch.bfloat16, False, False),
+    (5, 128, 9, 128, torch.bfloat16, True, False), (3, 136, 5, 680, torch.float32, False, True), (70, 256, 2, 256, torch.bfloat16, False, True)])
+def test_gated_group_norm_lanes(rows, part, groups, period, gate_dtype, gate_first, silu):
+    """A part per group of lanes: the smallest and largest parts, lanes without elements, a last warp that is not full, every kind of gate."""
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(rows + part)
+    width = part * groups
+    o = torch.randn(rows, width, generator=g)
+    weight = torch.randn(period, generator=g)
+    wide = torch.randn(rows, width + 16, generator=g)
+    gate = None if gate_dtype is None else wide.to(gate_dtype)
+    out = torch.full((rows, width), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.gated_group_norm(o.to(DEV), None if gate is None else gate.to(DEV)[:, :width], weight.to(DEV), out, 1e-5, groups, gate_first, silu)
+    factor = torch.ones(rows, width, dtype=torch.float64)
+    if gate is not None:
+        z = gate[:, :width].double()
+        factor = torch.sigmoid(z) * (z if silu else 1.0)
+    v = (o.double() * (factor if gate_first else 1.0)).view(rows, groups, part)
+    want = ((v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5)).view(rows, width) * weight.double().repeat(width // period)) * (1.0 if gate_first else factor)
+    # one rounding to bfloat16 (2^-9 of the result) and a few float32 operations
+    assert ((out.double().cpu() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("outputs,extra,width", [(32, 0, 1024), (37, 1, 520)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_router_of_many_tokens(dtype, outputs, extra, width):
+    """A step of many tokens (several outputs a warp) picks and weighs as steps of a few tokens do."""
+    from sprout_lm_b200 import kernels
+    T, top, g = 333, 4, torch.Generator().manual_seed(outputs)
+    h = torch.randn(T, width, generator=g).to(dtype).to(DEV)
+    router = (torch.randn(outputs + extra, width, generator=g) * width ** -0.5).to(DEV)
+    correction = (torch.randn(outputs, generator=g) * 0.1).to(DEV)
+
+    def route(rows):
+        n = rows.shape[0]
+        ids, weights = torch.zeros(n, top, dtype=torch.int32, device=DEV), torch.zeros(n, top, device=DEV)
+        counts, more = torch.zeros(outputs, dtype=torch.int32, device=DEV), torch.zeros(n, extra, device=DEV) if extra else None
+        kernels.moe_route(rows, router, correction, ids, weights, counts, outputs, top, 2.5, extra_out=more)
+        return ids, weights, counts, more
+    whole, parts = route(h), [route(h[i:i + 9].contiguous()) for i in range(0, T, 9)]
+    assert torch.equal(whole[0], torch.cat([p[0] for p in parts])) and torch.equal(whole[2], sum(p[2] for p in parts))
+    # float32 sums of width products in another order
+    assert (whole[1] - torch.cat([p[1] for p in parts])).abs().max() <= width * 2 ** -23
+    if extra:
+        assert (whole[3] - torch.cat([p[3] for p in parts])).abs().max() <= width * 2 ** -23
