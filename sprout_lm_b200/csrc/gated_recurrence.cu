@@ -216,8 +216,9 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
 
   float rq[EPT], rk[EPT], rz[EPT], rc[PHASE == SCAN_WHOLE ? 1 : EPT], rv[VPT];
   // wide: a thread's eight elements are the rows 8 (tid % slices) on of token tid / slices of the batch, its values neighbours too
+  // (32 slices: a batch of 4 tokens over 16 columns has a value for every second thread only)
   const bool wide = PAIRS && p.wide;
-  const int wide_token = tid >> slices_log2, wide_values = (batch << cb_log2) / SCAN_THREADS;
+  const int wide_token = tid >> slices_log2, wide_values = max(1, (batch << cb_log2) / SCAN_THREADS);
   auto fetch = [&](int t0) {                          // loads only: nothing waits for them here
     const int n = min(batch, last - t0);
     if (wide) {
@@ -313,7 +314,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
 #pragma unroll
       for (int u = 0; u < VPT; u++) {
         if (u >= wide_values) break;
-        vt[tid * wide_values + u] = rv[u];
+        if (tid * wide_values + u < (batch << cb_log2)) vt[tid * wide_values + u] = rv[u];
       }
     } else {
 #pragma unroll

@@ -1263,3 +1263,80 @@ def test_router_of_many_tokens(dtype, outputs, extra, width):
     assert (whole[1] - torch.cat([p[1] for p in parts])).abs().max() <= width * 2 ** -23
     if extra:
         assert (whole[3] - torch.cat([p[3] for p in parts])).abs().max() <= width * 2 ** -23
+
+
+def scan_oracle(form, q, k, v, decay, factor, extra, state):
+    """The gated scan of one request in float64, all heads at once: q [n, H, dim], k likewise, v [n, H, vdim], decay [n, H, dim], factor [n, H] on k;
+    ``extra``: the bonus [H, dim].  ``state`` [H, dim, vdim] is brought up to date; returns o [n, H, vdim]."""
+    out = np.zeros(v.shape)
+    for t in range(q.shape[0]):
+        write = (1.0 - decay[t]) if form == "floor" else k[t] * factor[t][:, None]
+        own = write[:, :, None] * v[t][:, None, :]
+        before = state.copy() if form == "bonus" else None
+        state *= decay[t][:, :, None]
+        state += own
+        seen = state if before is None else before + extra[:, :, None] * own
+        out[t] = np.einsum("hdv,hd->hv", seen, q[t])
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("form", ["channel", "head", "floor", "bonus", "given"])
+@pytest.mark.parametrize("dim,vdim", [(8, 600), (16, 24), (32, 130), (64, 37), (128, 33), (256, 16), (256, 21)])
+def test_gated_scan_rows_in_16_byte_fetches(status, dtype, form, dim, vdim):
+    """Chunked walks at every key size that fills the tile's slices (a batch then has 2 to 8 tokens and 16 to 512 columns a block, and at 256
+    fewer values than the block has threads), in every form of decay: outputs and states against the recurrence in float64."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    heads, lengths, slots = 2, [131, 1, 66], [2, 0, 3]
+    g = torch.Generator().manual_seed(dim + vdim)
+    T, v_cols = sum(lengths), vdim - 3 if form == "given" else vdim
+    make = lambda *shape: torch.randn(*shape, generator=g).to(dtype)
+    q, k, v = make(T, heads * dim), make(T, heads * dim), make(T, heads * v_cols)
+    z = 2.0 * torch.randn(T, heads if form in ("head", "given") else heads * dim, generator=g)
+    z = z.to(dtype)
+    bias = torch.linspace(-2.0, 1.0, heads) if form == "head" else torch.linspace(-3.0, 3.0, heads * dim)
+    a_log = torch.linspace(-4.0, 0.3, heads)
+    floor, bonus = torch.linspace(0.05, 0.98, heads * dim), torch.linspace(-1.0, 1.5, heads * dim)
+    tau, scale = 3.0, 0.5
+    f64 = lambda t: t.double().numpy()
+    sigmoid = lambda x: 1.0 / (1.0 + np.exp(-x))
+    factor = np.ones((T, heads))
+    more = {}
+    if form == "given":
+        given = torch.rand(T, heads, generator=g), torch.rand(T, heads, generator=g)
+        decay, factor = np.repeat(f64(given[0])[:, :, None], dim, axis=2), f64(given[1])
+        more = dict(given=tuple(t.to(DEV) for t in given), ones_col=True)
+    elif form == "head":
+        factor = np.logaddexp(0.0, f64(z) + f64(bias))
+        decay = np.repeat(np.exp(-np.exp(f64(a_log)) * factor)[:, :, None], dim, axis=2)
+        more = dict(per_head=True, a_log=a_log.to(DEV))
+    else:
+        x = (f64(z) + f64(bias)).reshape(T, heads, dim)
+        if form == "channel":
+            decay, more = sigmoid(x) ** (1.0 / tau), dict(tau=tau)
+        elif form == "floor":
+            low = f64(floor).reshape(heads, dim)
+            decay, more = low + (1.0 - low) * sigmoid(x), dict(floor=floor.to(DEV))
+        else:
+            decay, more = np.exp(-np.exp(x)), dict(bonus=bonus.to(DEV))
+    start = torch.randn(5, heads, dim, vdim, generator=g)
+    want, want_state, at = np.zeros((T, heads, vdim)), f64(start).copy(), 0
+    rows = lambda t, width: f64(t).reshape(T, heads, width)
+    values = rows(v, v_cols)
+    if form == "given":
+        values = np.concatenate([values, np.ones((T, heads, 1)), np.zeros((T, heads, 2))], axis=2)
+    for n, slot in zip(lengths, slots):
+        part = slice(at, at + n)
+        want[part] = scan_oracle(form, rows(q, dim)[part] * scale, rows(k, dim)[part], values[part], decay[part], factor[part],
+                                 f64(bonus).reshape(heads, dim), want_state[slot])
+        at += n
+    ctx = SimpleNamespace(q_start=torch.tensor(np.cumsum([0] + lengths), dtype=torch.int32, device=DEV), max_q_len=max(lengths))
+    state = SimpleNamespace(buffer=start.to(DEV), slots=torch.tensor(slots, dtype=torch.int32, device=DEV))
+    out = torch.full((T, heads * vdim), float("nan"), device=DEV)
+    kernels.gated_scan(q.to(DEV), None if form == "floor" else k.to(DEV), v.to(DEV), None if form == "given" else z.to(DEV),
+                       None if form == "given" else bias.to(DEV), ctx, state, out, heads, heads, dim, vdim, status, q_scale=scale, **more)
+    assert int(status.item()) == 0
+    # float32 recurrences of up to 131 steps and sums over up to 256 products of terms of both signs: some 400 roundings of 2^-24
+    for got, expected in ((out.double().cpu().numpy().reshape(want.shape), want), (state.buffer.double().cpu().numpy(), want_state)):
+        assert np.abs(got - expected).max() <= 2.5e-5 * max(1.0, np.abs(expected).max())
