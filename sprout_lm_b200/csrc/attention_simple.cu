@@ -104,7 +104,7 @@ template <int HD>
 __global__ void __launch_bounds__(TILE_THREADS)
 attention_tile_kernel(const float* __restrict__ q, int q_stride, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                       const int* __restrict__ block_table, int table_stride, const int* __restrict__ q_start,
-                      const int* __restrict__ positions, float* __restrict__ out, int out_stride, int heads, int kv_heads,
+                      const int* __restrict__ positions, float* __restrict__ out, int out_stride, int requests, int heads, int kv_heads,
                       int page_tokens, int num_pages, int* status) {
   constexpr int K_STRIDE = HD + 4, DIMS = HD / 32;               // elements of the output a lane holds
   extern __shared__ __align__(16) float smem[];
@@ -116,10 +116,16 @@ attention_tile_kernel(const float* __restrict__ q, int q_stride, const float* __
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r = blockIdx.y, h = blockIdx.z, g = h / (heads / kv_heads);
-  const int first = q_start[r] + (gridDim.x - 1 - blockIdx.x) * TILE;      // a request's last tokens see most keys: they start first
-  const int rows = min(TILE, q_start[r + 1] - first);
-  if (rows <= 0) return;
+  const int h = blockIdx.y, g = h / (heads / kv_heads);
+  // the tiles of all requests are numbered in the requests' order, a request's last (whose tokens see most keys) first
+  int r = 0, tile = blockIdx.x;
+  for (; r < requests; r++) {
+    const int tiles = (q_start[r + 1] - q_start[r] + TILE - 1) / TILE;
+    if (tile < tiles) { tile = tiles - 1 - tile; break; }
+    tile -= tiles;
+  }
+  if (r == requests) return;
+  const int first = q_start[r] + tile * TILE, rows = min(TILE, q_start[r + 1] - first);
   const int* table = block_table + (size_t)r * table_stride;
   for (int i = tid; i < TILE * HD; i += TILE_THREADS) {
     const int row = i / HD, d = i % HD;
@@ -245,12 +251,13 @@ attention_tile_kernel(const float* __restrict__ q, int q_stride, const float* __
 
 template <int HD>
 int launch_tile(const float* q, int q_stride, const float* k_cache, const float* v_cache, const int* block_table, int table_stride,
-                const int* q_start, const int* positions, float* out, int out_stride, int requests, int longest, int heads, int kv_heads,
+                const int* q_start, const int* positions, float* out, int out_stride, int tokens, int requests, int heads, int kv_heads,
                 int page_tokens, int num_pages, int* status, cudaStream_t stream) {
   const cudaError_t error = cudaFuncSetAttribute(attention_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem<HD>());
   if (error != cudaSuccess) return sprout_fail("attention_tile: %s", cudaGetErrorString(error));
-  sprout_launch(attention_tile_kernel<HD>, dim3((longest + TILE - 1) / TILE, requests, heads), dim3(TILE_THREADS), tile_smem<HD>(), stream,
-                q, q_stride, k_cache, v_cache, block_table, table_stride, q_start, positions, out, out_stride, heads, kv_heads, page_tokens,
+  // blocks for any cutting of the tokens into the requests: a captured launch is replayed for others than its own
+  sprout_launch(attention_tile_kernel<HD>, dim3(tokens / TILE + requests, heads), dim3(TILE_THREADS), tile_smem<HD>(), stream,
+                q, q_stride, k_cache, v_cache, block_table, table_stride, q_start, positions, out, out_stride, requests, heads, kv_heads, page_tokens,
                 num_pages, status);
   return sprout_check_launch("attention_tile");
 }
@@ -258,22 +265,22 @@ int launch_tile(const float* q, int q_stride, const float* k_cache, const float*
 }  // namespace
 
 // float32, head_dim 64 or 128; the caches' rows start on 16-byte boundaries.  q_start: the requests' first tokens and, last, the
-// number of tokens; `longest`: the most tokens that one request has in the step.
+// number of tokens (`tokens`).
 SPROUT_API int sprout_attention_tile(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
-                                     int table_stride, const int* q_start, const int* positions, void* out, int out_stride, int requests,
-                                     int longest, int heads, int kv_heads, int head_dim, int page_tokens, int num_pages, int* status,
+                                     int table_stride, const int* q_start, const int* positions, void* out, int out_stride, int tokens,
+                                     int requests, int heads, int kv_heads, int head_dim, int page_tokens, int num_pages, int* status,
                                      cudaStream_t stream) {
-  SPROUT_REQUIRE(requests > 0 && longest > 0 && heads > 0 && kv_heads > 0 && page_tokens > 0 && num_pages > 0, "attention_tile: sizes must be positive");
+  SPROUT_REQUIRE(requests > 0 && tokens > 0 && heads > 0 && kv_heads > 0 && page_tokens > 0 && num_pages > 0, "attention_tile: sizes must be positive");
   SPROUT_REQUIRE(heads % kv_heads == 0, "attention_tile: heads (%d) must be a multiple of kv_heads (%d)", heads, kv_heads);
-  SPROUT_REQUIRE(heads <= 65535 && requests <= 65535, "attention_tile: too many heads (%d) or requests (%d)", heads, requests);
+  SPROUT_REQUIRE(heads <= 65535, "attention_tile: too many heads (%d)", heads);
   SPROUT_REQUIRE(q && k_cache && v_cache && block_table && q_start && positions && out && status, "attention_tile: null pointer");
   SPROUT_REQUIRE((uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0, "attention_tile: the caches must start on 16-byte boundaries");
   if (head_dim == 64)
     return launch_tile<64>((const float*)q, q_stride, (const float*)k_cache, (const float*)v_cache, block_table, table_stride, q_start, positions,
-                           (float*)out, out_stride, requests, longest, heads, kv_heads, page_tokens, num_pages, status, stream);
+                           (float*)out, out_stride, tokens, requests, heads, kv_heads, page_tokens, num_pages, status, stream);
   if (head_dim == 128)
     return launch_tile<128>((const float*)q, q_stride, (const float*)k_cache, (const float*)v_cache, block_table, table_stride, q_start, positions,
-                            (float*)out, out_stride, requests, longest, heads, kv_heads, page_tokens, num_pages, status, stream);
+                            (float*)out, out_stride, tokens, requests, heads, kv_heads, page_tokens, num_pages, status, stream);
   return sprout_fail("attention_tile: head_dim must be 64 or 128 (got %d)", head_dim);
 }
 

@@ -367,12 +367,13 @@ ATTENTION_TILE_TOKENS = 16
 
 def attention_tile(q, k_cache, v_cache, block_table, q_start, positions, out, heads, kv_heads, head_dim, longest, status):
     """``attention_simple`` for float32 steps with prompt portions, bit for bit, 32 tokens of a request at a time; ``q_start``: int32
-    [requests + 1], ``longest``: the most tokens that one request has.  head_dim 64 or 128."""
+    [requests + 1], ``longest``: the most tokens that one request has.  head_dim 64 or 128.  The launch follows the numbers of tokens and
+    requests alone, not ``longest``: a captured step is replayed for steps that cut the same tokens into other portions."""
     _rows_contiguous(q, "q")
     _rows_contiguous(out, "out")
     _rows_contiguous(block_table, "block_table")
     T, requests = q.shape[0], q_start.numel() - 1
-    if q.shape[1] != heads * head_dim or tuple(out.shape) != (T, heads * head_dim):
+    if q.shape[1] != heads * head_dim or tuple(out.shape) != (T, heads * head_dim) or not 0 < longest <= T:
         raise KernelError("attention_tile: q and out must be [tokens, heads * head_dim]")
     if k_cache.shape != v_cache.shape or tuple(k_cache.shape[1:]) != (kv_heads, k_cache.shape[2], head_dim) \
             or not k_cache.is_contiguous() or not v_cache.is_contiguous():
@@ -383,7 +384,7 @@ def attention_tile(q, k_cache, v_cache, block_table, q_start, positions, out, he
         raise KernelError("attention_tile: a block table row per request and a position per token")
     _run("sprout_attention_tile", _ptr(q, "q"), q.stride(0), _ptr(k_cache, "k_cache"), _ptr(v_cache, "v_cache"),
          _ptr(block_table, "block_table", torch.int32), block_table.stride(0), _ptr(q_start, "q_start", torch.int32),
-         _ptr(positions, "positions", torch.int32), _ptr(out, "out"), out.stride(0), requests, longest, heads, kv_heads, head_dim,
+         _ptr(positions, "positions", torch.int32), _ptr(out, "out"), out.stride(0), T, requests, heads, kv_heads, head_dim,
          k_cache.shape[2], k_cache.shape[0], _ptr(status, "status", torch.int32), _stream())
 
 

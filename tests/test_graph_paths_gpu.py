@@ -327,3 +327,47 @@ def test_large_batch_decodes_with_resident_contexts(tmp_path):
             err = float(np.abs(row - want[rid][head + step]).max())
             assert err <= 0.02 * scale, f"request {rid} position {head + step} differs by {err:.3e} (scale {scale:.3f})"
     runner.check_status()
+
+
+def steps_of_many_cuttings(model, vocab, rounds, capturing, num_pages=400, page=16, max_requests=8, held=(40, 7, 0, 21)):
+    """The logits of one step per round, a round being the portions of its requests (new requests every round, some of them with cached tokens before
+    the step); with ``capturing`` the rounds of a size are replayed from the capture of the third one, whose portions were others."""
+    from sprout_lm_b200.engine.batch import StepEntry
+    from sprout_lm_b200.engine.step import ModelRunner
+    runner = ModelRunner(model, num_pages=num_pages, page_tokens=page, max_requests=max_requests, prefix_caching=False)
+    runner.step_graphs.enabled = capturing
+    rng, out = np.random.default_rng(29), []
+    for portions in rounds:
+        seqs = [runner.new_sequence() for _ in portions]
+        for i, seq in enumerate(seqs):
+            before = held[i % len(held)]
+            if before:
+                assert runner.reserve(seq, before)
+                runner.step([StepEntry(seq, helpers.random_tokens(rng, before, vocab), [])])
+        entries = []
+        for seq, n in zip(seqs, portions):
+            assert runner.reserve(seq, seq.length + n)
+            entries.append(StepEntry(seq, helpers.random_tokens(rng, n, vocab), [n // 2, n - 1] if n > 1 else [0, 0]))
+        out.append(runner.step(entries).float().cpu().numpy())
+        for seq in seqs:
+            runner.release(seq)
+    runner.check_status()
+    return out, runner.step_graphs.replays
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 2, 64), (2, 1, 128)])
+def test_captured_float32_step_serves_every_cutting(tmp_path, heads, kv_heads, head_dim):
+    """Captured with its tokens cut evenly, replayed with them cut as unevenly as they can be: bit for bit the steps of a runner that never
+    captures (the 32-bit attention by tiles of 32 tokens)."""
+    from sprout_lm_b200 import load_model
+    from sprout_lm_b200.config import parse_config
+    from sprout_lm_b200.weights import write_random_model
+    sizes = dict(hidden_size=heads * head_dim, intermediate_size=96, num_hidden_layers=2, num_attention_heads=heads, num_key_value_heads=kv_heads,
+                 vocab_size=300, max_position_embeddings=1024, rms_norm_eps=1e-6, rope_theta=10000.0, tie_word_embeddings=False, eos_token_id=299)
+    model = load_model(write_random_model(tmp_path / "model", parse_config(helpers.raw_config(sizes)), seed=3), dtype="float32")
+    rounds = [(64, 64), (64, 64), (64, 64), (127, 1), (1, 127), (33, 95), (64, 64)]
+    plain, none = steps_of_many_cuttings(model, 300, rounds, False)
+    replayed, count = steps_of_many_cuttings(model, 300, rounds, True)
+    assert none == 0 and count == len(rounds) - 3
+    for portions, want, got in zip(rounds, plain, replayed):
+        assert np.array_equal(want, got), portions
