@@ -117,15 +117,10 @@ attention_tile_kernel(const float* __restrict__ q, int q_stride, const float* __
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, g = h / (heads / kv_heads);
-  // the tiles of all requests are numbered in the requests' order, a request's last (whose tokens see most keys) first
-  int r = 0, tile = blockIdx.x;
-  for (; r < requests; r++) {
-    const int tiles = (q_start[r + 1] - q_start[r] + TILE - 1) / TILE;
-    if (tile < tiles) { tile = tiles - 1 - tile; break; }
-    tile -= tiles;
-  }
-  if (r == requests) return;
-  const int first = q_start[r] + tile * TILE, rows = min(TILE, q_start[r + 1] - first);
+  int r, tile, tiles;
+  if (!warp_find_piece(q_start, requests, TILE, blockIdx.x, r, tile, tiles)) return;
+  const int first = q_start[r] + (tiles - 1 - tile) * TILE;      // a request's last tokens see most keys: they start first
+  const int rows = min(TILE, q_start[r + 1] - first);
   const int* table = block_table + (size_t)r * table_stride;
   for (int i = tid; i < TILE * HD; i += TILE_THREADS) {
     const int row = i / HD, d = i % HD;

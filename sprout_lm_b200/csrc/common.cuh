@@ -102,6 +102,33 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// Pieces of `size` tokens of one request each, numbered over the requests in order (ceil(tokens / size) of a request's own): a whole
+// warp finds piece `index`, 32 requests at a time: its request, its place among the request's pieces, and how many those are.
+// False beyond the last piece.
+__device__ __forceinline__ bool warp_find_piece(const int* q_start, int requests, int size, int index, int& r, int& piece, int& pieces) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < requests; base += 32) {
+    const int i = base + lane;
+    const int own = i < requests ? (q_start[i + 1] - q_start[i] + size - 1) / size : 0;
+    int sum = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += other;
+    }
+    const unsigned found = __ballot_sync(0xffffffffu, index < sum);
+    if (found) {
+      const int at = __ffs(found) - 1;
+      r = base + at;
+      pieces = __shfl_sync(0xffffffffu, own, at);
+      piece = index - (__shfl_sync(0xffffffffu, sum, at) - pieces);
+      return true;
+    }
+    index -= __shfl_sync(0xffffffffu, sum, 31);
+  }
+  return false;
+}
+
 // Block-wide sum / max for blocks of up to 1024 threads; `scratch` holds 33 floats.
 // Every thread gets the result.  The order of the additions is fixed by the
 // block size alone.

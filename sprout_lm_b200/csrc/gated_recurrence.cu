@@ -544,20 +544,22 @@ __global__ void scan_carry_kernel(float* __restrict__ sums, const float* __restr
 
 constexpr int CONV_MAX_TAPS = 8, CONV_TOKENS = 32;
 
-// grid (request, blocks of 128 channels, blocks of CONV_TOKENS tokens); a thread walks its channel through its tokens
-// with the last taps - 1 inputs in registers.  The block of a request's first tokens reads the state (before anything
-// writes it) and is the one that writes the new state at its end.
+// grid (blocks of CONV_TOKENS tokens of one request, numbered over the requests in order; blocks of 128 channels); a thread walks
+// its channel through its tokens with the last taps - 1 inputs in registers.  As many tokens as requests are one each.  The block of
+// a request's first tokens reads the state (before anything writes it) and is the one that writes the new state at its end.
 template <typename T>
 __global__ void __launch_bounds__(128)
 causal_conv_kernel(const T* __restrict__ in, int in_stride, const float* __restrict__ weight, const float* __restrict__ bias,
                    T* __restrict__ out, int out_stride, const int* __restrict__ q_start, const int* __restrict__ state_slots,
-                   float* __restrict__ state, int num_slots, int channels, int taps, int act, int* status) {
+                   float* __restrict__ state, int num_slots, int tokens, int requests, int channels, int taps, int act, int* status) {
   pdl_launch_dependents();
   pdl_wait();
-  const int r = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
+  int r = blockIdx.x, part = 0, parts;
+  if (tokens != requests && !warp_find_piece(q_start, requests, CONV_TOKENS, blockIdx.x, r, part, parts)) return;
+  const int c = blockIdx.y * blockDim.x + threadIdx.x;
   const int begin = q_start[r], end = q_start[r + 1];
-  const int first = begin + blockIdx.z * CONV_TOKENS;
-  if (first >= end || c >= channels) return;
+  const int first = begin + part * CONV_TOKENS;
+  if (c >= channels) return;
   const int slot = state_slots[r];
   if (slot < 0 || slot >= num_slots) {
     if (threadIdx.x == 0) atomicOr(status, SPROUT_STATUS_BAD_PAGE);
@@ -591,7 +593,7 @@ causal_conv_kernel(const T* __restrict__ in, int in_stride, const float* __restr
 #pragma unroll
     for (int b = CONV_MAX_TAPS - 1; b > 0; b--) hist[b] = hist[b - 1];
   }
-  if (blockIdx.z != 0) return;
+  if (part != 0) return;
   // the new state: the last taps - 1 inputs of what the request has seen, oldest first
 #pragma unroll
   for (int s = 0; s < CONV_MAX_TAPS - 1; s++) {
@@ -939,22 +941,22 @@ SPROUT_API int sprout_gated_scan(const void* q, int q_stride, const void* k, int
   return sprout_fail("gated_scan: unknown dtype %d", dtype);
 }
 
-// `max_q_len` bounds the tokens any request brings (it sizes the grid).
+// The grid follows `tokens` and `requests` alone: a captured launch is replayed for other cuttings of the same tokens.
 SPROUT_API int sprout_causal_conv(const void* in, int in_stride, const float* weight, const float* bias, void* out, int out_stride,
                                   int dtype, const int* q_start, const int* state_slots, float* state, int num_slots, int requests,
-                                  int max_q_len, int channels, int taps, int act, int* status, cudaStream_t stream) {
+                                  int tokens, int channels, int taps, int act, int* status, cudaStream_t stream) {
   SPROUT_REQUIRE(in && weight && out && q_start && state_slots && state && status, "causal_conv: null pointer");
-  SPROUT_REQUIRE(requests > 0 && max_q_len > 0 && channels > 0 && num_slots > 0, "causal_conv: bad sizes");
+  SPROUT_REQUIRE(requests > 0 && tokens > 0 && channels > 0 && num_slots > 0, "causal_conv: bad sizes");
   SPROUT_REQUIRE(taps >= 2 && taps <= CONV_MAX_TAPS, "causal_conv: 2 to %d taps (got %d)", CONV_MAX_TAPS, taps);
   SPROUT_REQUIRE(in_stride >= channels && out_stride >= channels, "causal_conv: rows shorter than the channels");
-  const dim3 grid(requests, (channels + 127) / 128, (max_q_len + CONV_TOKENS - 1) / CONV_TOKENS);
-  SPROUT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "causal_conv: too many channels or tokens");
+  const dim3 grid(tokens == requests ? requests : tokens / CONV_TOKENS + requests, (channels + 127) / 128);
+  SPROUT_REQUIRE(grid.y <= 65535, "causal_conv: too many channels");
   if (dtype == SPROUT_F32)
     sprout_launch(causal_conv_kernel<float>, grid, dim3(128), 0, stream, (const float*)in, in_stride, weight, bias, (float*)out,
-                  out_stride, q_start, state_slots, state, num_slots, channels, taps, act, status);
+                  out_stride, q_start, state_slots, state, num_slots, tokens, requests, channels, taps, act, status);
   else if (dtype == SPROUT_BF16)
     sprout_launch(causal_conv_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)in, in_stride, weight, bias,
-                  (__nv_bfloat16*)out, out_stride, q_start, state_slots, state, num_slots, channels, taps, act, status);
+                  (__nv_bfloat16*)out, out_stride, q_start, state_slots, state, num_slots, tokens, requests, channels, taps, act, status);
   else
     return sprout_fail("causal_conv: unknown dtype %d", dtype);
   return sprout_check_launch("causal_conv");

@@ -1828,7 +1828,7 @@ def causal_conv(rows, weight, bias, out, ctx, state, status, silu: bool = True):
     _run("sprout_causal_conv", rows.data_ptr(), rows.stride(0), _ptr(weight, "weight", torch.float32),
          _ptr(bias, "bias", torch.float32, True), out.data_ptr(), out.stride(0), _dtype_code(rows.dtype),
          _ptr(ctx.q_start, "q_start", torch.int32), _ptr(state.slots, "state_slots", torch.int32),
-         _ptr(buffer, "state", torch.float32), buffer.shape[0], state.slots.numel(), int(ctx.max_q_len), channels, taps,
+         _ptr(buffer, "state", torch.float32), buffer.shape[0], state.slots.numel(), rows.shape[0], channels, taps,
          1 if silu else 0, _ptr(status, "status", torch.int32), _stream())
 
 

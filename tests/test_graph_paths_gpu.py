@@ -347,7 +347,7 @@ def steps_of_many_cuttings(model, vocab, rounds, capturing, num_pages=400, page=
         entries = []
         for seq, n in zip(seqs, portions):
             assert runner.reserve(seq, seq.length + n)
-            entries.append(StepEntry(seq, helpers.random_tokens(rng, n, vocab), [n // 2, n - 1] if n > 1 else [0, 0]))
+            entries.append(StepEntry(seq, helpers.random_tokens(rng, n, vocab), [n // 2, n - 1] if len(portions) <= 32 else [n - 1]))
         out.append(runner.step(entries).float().cpu().numpy())
         for seq in seqs:
             runner.release(seq)
@@ -371,3 +371,29 @@ def test_captured_float32_step_serves_every_cutting(tmp_path, heads, kv_heads, h
     assert none == 0 and count == len(rounds) - 3
     for portions, want, got in zip(rounds, plain, replayed):
         assert np.array_equal(want, got), portions
+
+
+# (architecture, model, portions of the captured step, portions of the steps that it is replayed for)
+OTHER_CUTTINGS = [("rarutar", "A", (64, 64), [(127, 1), (1, 127), (33, 95)]), ("zevedra", "C", (64, 64), [(127, 1), (1, 127), (33, 95)])]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("architecture,name,even,others", OTHER_CUTTINGS)
+def test_captured_step_serves_every_cutting(tmp_path, dtype, architecture, name, even, others):
+    """The same for the other architectures: convolutions along the tokens, recurrent states."""
+    import importlib
+    from sprout_lm_b200 import load_model
+    made = importlib.import_module(f"{architecture}_helpers")
+    config, _, page = made.CONFIGS[name]
+    model = load_model(made.make_model_dir(tmp_path, name), dtype=dtype)
+    rounds = [even] * 3 + others
+    many = len(even) > 8
+    run = lambda capturing: steps_of_many_cuttings(model, config["vocab"], rounds, capturing, page=page, max_requests=max(8, len(even)),
+                                                   held=(40, 7, 0, 21) if not many else (3, 9, 0, 20))
+    plain, none = run(False)
+    replayed, count = run(True)
+    assert none == 0 and count == len(others)
+    for portions, want, got in zip(rounds, plain, replayed):
+        # the two runs may take another form of a sum (the captured step keeps the form of its own portions): the architecture's tolerance
+        spread = want.max(axis=1, keepdims=True) - want.min(axis=1, keepdims=True)
+        assert np.abs(got - want).max() <= (6e-5 if dtype == "float32" else 6e-2) * spread.min(), (portions, np.abs(got - want).max())
