@@ -296,7 +296,8 @@ class StepGraphs:
 
     A prefill step of a small model is two hundred launches that the host enqueues more slowly
     than the device runs them.  A step whose sizes (tokens, requests, wanted rows, block-table
-    width rounded up to ``page_multiple``) have come ``after`` times is captured after it has
+    width rounded up to ``page_multiple``, the longest portion up to ``short_portion``) have come
+    ``after`` times is captured after it has
     run, and later steps of the same sizes replay the capture: the batch's arrays live at fixed
     offsets of the stager's device buffer, so only their contents change.  Chunked prefill of
     long prompts at a fixed chunk size makes such steps; the mixed steps of a busy server rarely
@@ -304,7 +305,14 @@ class StepGraphs:
     must have come three times first, a few captures are kept, and steps that ask for many
     logits rows are not captured.  When the captures are full, a new shape takes the place of the
     least used one only once it has been used twice as often (uses are halved now and then, so
-    the count follows the recent past): shapes that take turns do not capture over one another."""
+    the count follows the recent past): shapes that take turns do not capture over one another.
+
+    How the tokens are cut into the requests is not part of the key: launches follow the numbers of
+    tokens and requests, and find the portions on the device.  The exception are kernels for a few
+    rows a request (mapped attention of up to 16 (token, head) rows a key/value head, chosen by the
+    longest portion), so portions of up to 16 tokens are told apart."""
+
+    short_portion = 17
 
     def __init__(self, runner, limit: int = 4, min_tokens: int = 128, max_rows: int = 64, page_multiple: int = 64,
                  after: int = 3):
@@ -330,7 +338,8 @@ class StepGraphs:
             for table in e.seq.tables:
                 pages = max(pages, len(table))
         width = _round_up(pages, self.page_multiple)
-        return (tokens, len(entries), rows, width, sample), width
+        longest = min(self.short_portion, max(len(e.tokens) for e in entries))
+        return (tokens, len(entries), rows, width, sample, longest), width
 
     def run(self, key, ctx, sample: bool):
         """Run the staged step ``ctx``; (logits or None, sampled tokens or None), both on the

@@ -205,6 +205,22 @@ def test_prefill_step_captures_do_not_take_turns_evicting_one_another(monkeypatc
     assert ("shape", 5) in steps.captured and len(steps.captured) == 4
 
 
+def test_captured_steps_tell_short_portions_apart():
+    """A step whose requests all bring a few tokens may have been captured with kernels for a few rows a request: it does not serve a step of the
+    same tokens and requests with a longer portion.  Among longer portions the cutting does not matter."""
+    from types import SimpleNamespace
+    from sprout_lm_b200.engine import graphs
+    from sprout_lm_b200.engine.batch import StepEntry
+    steps = graphs.StepGraphs(SimpleNamespace(page_tokens=16))
+
+    def key(*portions):
+        return steps.plan([StepEntry(SimpleNamespace(tables=[[0]]), [1] * n, [n - 1]) for n in portions], False)[0]
+    assert key(*[2] * 64) == key(*[2] * 64) is not None
+    assert len({key(*[2] * 64), key(3, 1, *[2] * 62), key(16, *[2] * 49, *[1] * 14), key(65, *[1] * 63)}) == 4
+    assert key(64, 64) == key(127, 1) == key(17, 111) is not None
+    assert key(65, *[1] * 63) == key(*[1] * 62, 30, 36)
+
+
 def test_small_batch_kernels_say_what_they_take():
     """The small-batch kernels' size rules are host arithmetic in the kernel library: up to 16 tokens,
     sizes in steps of 16, and a layer small enough for the SMs' shared memory.  What they refuse
