@@ -126,11 +126,13 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // Tokens come `batch` at a time: while the threads walk a batch's tokens over their registers, the next batch's q, k,
 // decay inputs and values are on their way from memory into registers; at the batch's end they are turned into
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
-// shuffles.  The chunks' walks over tiles of 8 x 4 (PAIRS) go two rows at a time in packed arithmetic: a thread's rows are neighbours, and q, c k and a
-// lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us
-// for the two walks with a number at a time, (q, c k, a) triples and 2-byte fetches, 106 and 237 us so, the rows fetched 16 bytes at a
-// time where they start on 16-byte boundaries and fill the slices).  Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order, so the result does not
-// depend on the cutting or on the batch.
+// shuffles.  The bfloat16 path's walks over chunks in tiles of 8 x 4 (PAIRS) go two rows at a time in packed arithmetic: a thread's
+// rows are then neighbours, and q, c k and a lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500
+// tokens of 16 heads of 128 x 128: 154 and 362 us for the two walks with a number at a time, (q, c k, a) triples and 2-byte fetches,
+// 106 and 237 us so, the rows fetched 16 bytes at a time where they start on 16-byte boundaries and fill the slices).
+// Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order.  An output's sum over the rows has one order in
+// the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn, so a bfloat16 request of one
+// chunk may differ in the last bits of a 32-bit sum by whether another portion of the step is long.
 //
 // Long portions are cut into chunks of `p.chunk` tokens so that more blocks than (request, head, columns) have work, in
 // three launches: SCAN_CHUNK_SUMS walks every chunk but a request's last from a zero state and leaves the chunk's own
@@ -850,8 +852,8 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
   if (batch > by_rows) batch = by_rows;
   if (batch > by_values) batch = by_values;
   // single walks (few tokens: the state's way in and out is most of their time, and rows dealt in turn read it faster: 64 single tokens
-  // of 16 heads 46 against 52 us) keep a number at a time
-  constexpr bool PAIRED = ROWS == 8 && COLS == 4;
+  // of 16 heads 46 against 52 us) keep a number at a time, and so does the 32-bit path, whose sums have one order in both walks
+  constexpr bool PAIRED = ROWS == 8 && COLS == 4 && sizeof(T) == 2;
   const size_t smem = (size_t)batch * ((size_t)ROWS * slices * sizeof(float4) + (size_t)cb * sizeof(float));
   const size_t smem_chunks = PAIRED ? (size_t)batch * ((size_t)4 * 2 * (ROWS * slices / 2 + 16) + cb) * sizeof(float) : smem;
   const dim3 grid(requests, p.heads, (p.vdim + cb - 1) / cb);

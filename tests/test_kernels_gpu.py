@@ -1340,3 +1340,34 @@ def test_gated_scan_rows_in_16_byte_fetches(status, dtype, form, dim, vdim):
     # float32 recurrences of up to 131 steps and sums over up to 256 products of terms of both signs: some 400 roundings of 2^-24
     for got, expected in ((out.double().cpu().numpy().reshape(want.shape), want), (state.buffer.double().cpu().numpy(), want_state)):
         assert np.abs(got - expected).max() <= 2.5e-5 * max(1.0, np.abs(expected).max())
+
+
+@pytest.mark.parametrize("form", ["channel", "head", "floor", "bonus"])
+@pytest.mark.parametrize("dim,vdim", [(16, 24), (64, 40), (128, 64), (256, 20), (40, 12)])
+def test_float32_scan_keeps_its_bits_beside_a_long_portion(status, form, dim, vdim):
+    """The 32-bit path adds in one order: a short request (walked whole alone, as a chunk beside a portion of 300 tokens) has the same bits both ways."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    heads, lengths = 2, [33, 300, 1, 64]
+    g = torch.Generator().manual_seed(dim)
+    T = sum(lengths)
+    starts = np.cumsum([0] + lengths)
+    make = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    q, k, v, z = make(T, heads * dim), make(T, heads * dim), make(T, heads * vdim), make(T, heads if form == "head" else heads * dim)
+    bias, first = make(heads if form == "head" else heads * dim), make(len(lengths), heads, dim, vdim)
+    more = {"channel": dict(tau=2.0), "head": dict(per_head=True, a_log=make(heads)), "floor": dict(floor=torch.rand(heads * dim, generator=g).to(DEV)),
+            "bonus": dict(bonus=make(heads * dim))}[form]
+
+    def scan(requests):
+        rows = torch.cat([torch.arange(starts[r], starts[r + 1]) for r in requests]).to(DEV)
+        ctx = SimpleNamespace(q_start=torch.tensor(np.cumsum([0] + [lengths[r] for r in requests]), dtype=torch.int32, device=DEV),
+                              max_q_len=max(lengths[r] for r in requests))
+        state = SimpleNamespace(buffer=first.clone(), slots=torch.tensor(requests, dtype=torch.int32, device=DEV))
+        out = torch.empty(len(rows), heads * vdim, device=DEV)
+        kernels.gated_scan(q[rows], None if form == "floor" else k[rows], v[rows], z[rows], bias, ctx, state, out, heads, heads, dim, vdim, status, **more)
+        return out, state.buffer
+    together, states = scan([0, 1, 2, 3])
+    for r in (0, 2, 3):
+        alone, state = scan([r])
+        assert torch.equal(alone, together[starts[r]:starts[r + 1]]) and torch.equal(state[r], states[r]), r
+    assert int(status.item()) == 0
