@@ -66,11 +66,18 @@ struct Params {
   // weights on M only: the tokens' operand made in the kernel instead of copied: bfloat16(x * gain) of the
   // float32 rows x [M, K] (row stride ldx), written by the epilogue warps into the stages' token tiles
   const float* x32; const float* gain; int ldx;
-  // experts' products (GROUPED): the rows of expert e are offsets[e] .. offsets[e + 1] - 1, its matrix has `expert_rows` rows; what the
-  // gated epilogues need: see sprout_experts_product_tc
+};
+
+// The experts' products (GROUPED) have arguments and a work item of their own: as fields of the dense forms' they cost the weights-on-M
+// kernels four registers a thread (56 to 60, handed out as 64): a decode step of 64 requests of 1,500 tokens 1,282 us, 1,252 us without.
+// The rows of expert e are offsets[e] .. offsets[e + 1] - 1, its matrix has `expert_rows` rows; what the gated epilogues need: see
+// sprout_experts_product_tc.
+struct GroupedParams : Params {
   const int* offsets; const int* order; int experts, expert_rows, unit;
   const float* row_weights; float limit, alpha;
 };
+template <bool GROUPED> struct ParamsOf { using type = Params; };
+template <> struct ParamsOf<true> { using type = GroupedParams; };
 
 // PAIR: two CTAs share a 256 x BN tile; each holds its own 128 rows of A and half of B's rows.
 template <int BN, bool PAIR = false>
@@ -86,7 +93,10 @@ struct Layout {
 };
 
 // One unit of work: a 128 x BN tile of D over a range of K blocks.
-struct Work { int row0, col0, kb_begin, num_kb, split; int row_end, weight_row; };   // the last two: experts' products only
+struct Work { int row0, col0, kb_begin, num_kb, split; };
+struct GroupedWork : Work { int row_end, weight_row; };
+template <bool GROUPED> struct WorkOf { using type = Work; };
+template <> struct WorkOf<true> { using type = GroupedWork; };
 
 // SWAP == false: map_rows is the activation map (rows = tokens), map_cols the weight map.
 // SWAP == true:  map_rows is the weight map (rows = output features), map_cols the activation map.
@@ -109,7 +119,7 @@ struct Work { int row0, col0, kb_begin, num_kb, split; int row_end, weight_row; 
 template <int BN, bool SWAP, bool PAIR = false, bool GROUPED = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols,
-                    const __grid_constant__ CUtensorMap map_out, const Params p) {
+                    const __grid_constant__ CUtensorMap map_out, const typename ParamsOf<GROUPED>::type p) {
   static_assert(!(PAIR && SWAP), "pairs work on token tiles");
   static_assert(!GROUPED || PAIR, "experts' products run in pairs");
   using L = Layout<BN, PAIR>;
@@ -135,15 +145,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   const int splits = (total_kb + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
   // experts' products: 256-row tiles before expert e, and its first row, in the room that the residual epilogue's tiles would have
   int* tile_prefix = (int*)staging;
-  int* row_prefix = tile_prefix + p.experts + 1;
+  int* row_prefix = nullptr;
   const bool glu_tiles = GROUPED && p.epilogue == EPI_EXPERT_GLU;
-  const int expert_cols = glu_tiles ? (p.N + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;     // tiles across an expert's outputs
+  int expert_cols = 0;                                 // tiles across an expert's outputs
+  if constexpr (GROUPED) {
+    row_prefix = tile_prefix + p.experts + 1;
+    expert_cols = glu_tiles ? (p.N + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;
+  }
   int total_work = row_tiles * col_tiles * splits;
   // consecutive work items share the weight tile where they can (tokens on M: same columns,
   // next rows), so that it is served from L2
   auto work_at = [&](int w) {
-    Work k;
-    if (GROUPED) {
+    typename WorkOf<GROUPED>::type k;
+    if constexpr (GROUPED) {
       const int tile = w / expert_cols, ct = w % expert_cols;
       int e = 0, hi = p.experts;                       // the last e with tile_prefix[e] <= tile: it has rows
       while (hi - e > 1) {
@@ -180,7 +194,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, L::TMEM_COLS);
-  if (GROUPED) {
+  if constexpr (GROUPED) {
     pdl_wait();                                        // the offsets are an earlier kernel's
     if (warp == 0) {
       int before = 0;
@@ -206,7 +220,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (GROUPED) total_work = tile_prefix[p.experts] * expert_cols;
+  if constexpr (GROUPED) total_work = tile_prefix[p.experts] * expert_cols;
   if (PAIR) {
     // The pair's MMAs write both CTAs' tensor memory at one address.  Each CTA has its SM to
     // itself (its shared memory leaves no room for another) and has allocated from an empty tensor
@@ -241,8 +255,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       if (PAIR) tma_load_2d_pair(dst, map, bar, x, y); else tma_load_2d_addr(dst, map, bar, x, y);
     };
     for (int w = first_work; w < total_work && ok; w += work_stride) {
-      const Work k = work_at(w);
-      const int weight_row = GROUPED ? k.weight_row : SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0), act_row = SWAP ? k.col0 : k.row0;
+      const auto k = work_at(w);
+      int weight_row = SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0);
+      if constexpr (GROUPED) weight_row = k.weight_row;
+      const int act_row = SWAP ? k.col0 : k.row0;
       int early = 0;
       if (w == first_work) {
         early = min(k.num_kb, L::STAGES);
@@ -279,7 +295,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     bool ok = true;
     int tiles_done = 0;
     for (int w = first_work; w < total_work && ok; w += work_stride, tiles_done++) {
-      const Work k = work_at(w);
+      const auto k = work_at(w);
       const int acc = tiles_done & 1;
       // the epilogue (of both CTAs) must have read this accumulator's previous tile out
       const bool drained = PAIR ? mbar_wait_cluster(smem_u32(&acc_empty[acc]), ((tiles_done >> 1) & 1) ^ 1, abort_flag)
@@ -377,7 +393,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       else mbar_arrive(&acc_empty[acc]);
     };
     for (int w = first_work; w < total_work; w += work_stride, tiles_done++) {
-      const Work k = work_at(w);
+      const auto k = work_at(w);
       const int acc = tiles_done & 1;
       const int row = k.row0 + quarter * 32 + lane;
       const int col0 = k.col0;
@@ -468,34 +484,40 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           }
         } else {
           // row = token, columns = output features: each lane writes a contiguous run of its row
-          if (GROUPED && p.epilogue != EPI_STORE) {
-            const int n_base = col0 + c;
-            float v[16];
-            uint32_t up[16];
-            if (p.epilogue == EPI_EXPERT_GLU) tmem_load16(taddr + BN / 2 + c, up);      // warp-wide: also lanes without a row
-            if (row < k.row_end && n_base < p.N) {
-              const float weight = p.row_weights ? p.row_weights[p.order[row]] : 1.0f;
+          int row_end = p.M;
+          if constexpr (GROUPED) {
+            row_end = k.row_end;
+            if (p.epilogue != EPI_STORE) {
+              const int n_base = col0 + c;
+              float v[16];
+              uint32_t up[16];
+              if (p.epilogue == EPI_EXPERT_GLU) tmem_load16(taddr + BN / 2 + c, up);      // warp-wide: also lanes without a row
+              if (row < k.row_end && n_base < p.N) {
+                const float weight = p.row_weights ? p.row_weights[p.order[row]] : 1.0f;
 #pragma unroll
-              for (int j = 0; j < 16; j++) {
-                // rounded to bfloat16 before the activation, as separate products would leave them
-                const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j]) * weight));
-                const float u = p.epilogue == EPI_EXPERT_GLU ? __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j]) * weight)) : 0.f;
-                v[j] = sprout_experts::glu(p.unit, g, u, p.limit, p.alpha);
-              }
-              __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n_base;    // N and ldo are multiples of 8
-#pragma unroll
-              for (int j = 0; j < 16; j += 8) {
-                if (n_base + j >= p.N) break;
-                uint32_t packed[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                  __nv_bfloat162 h = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
-                  packed[i] = *(uint32_t*)&h;
+                for (int j = 0; j < 16; j++) {
+                  // rounded to bfloat16 before the activation, as separate products would leave them
+                  const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j]) * weight));
+                  const float u = p.epilogue == EPI_EXPERT_GLU ? __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j]) * weight)) : 0.f;
+                  v[j] = sprout_experts::glu(p.unit, g, u, p.limit, p.alpha);
                 }
-                *(uint4*)(o + j) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n_base;    // N and ldo are multiples of 8
+#pragma unroll
+                for (int j = 0; j < 16; j += 8) {
+                  if (n_base + j >= p.N) break;
+                  uint32_t packed[4];
+#pragma unroll
+                  for (int i = 0; i < 4; i++) {
+                    __nv_bfloat162 h = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
+                    packed[i] = *(uint32_t*)&h;
+                  }
+                  *(uint4*)(o + j) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                }
               }
+              continue;
             }
-          } else if (row < (GROUPED ? k.row_end : p.M)) {
+          }
+          if (row < row_end) {
             const int n_base = col0 + c;
             float v[16];
 #pragma unroll
@@ -578,7 +600,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 // `work` = tiles x K splits; the grid is one CTA per SM at most, each walking the work list.
 // Pairs: `work` counts 256 x BN tiles; the grid is one cluster of two CTAs per two SMs at most.
 template <int BN, bool GROUPED = false>
-int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const Params& p, int work,
+int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const typename ParamsOf<GROUPED>::type& p, int work,
                 cudaStream_t stream) {
   using L = Layout<BN, true>;
   static bool configured = false;
@@ -628,7 +650,7 @@ int sprout_experts_product_tc(const void* rows, const int* offsets, const int* o
   const bool gated = unit == sprout_experts::UNIT_CLAMPED || unit == sprout_experts::UNIT_SILU;
   SPROUT_REQUIRE(rows && offsets && order && w && out && status && entries > 0 && experts > 0, "experts_product: bad arguments");
   SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= 2048, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
-  Params p{};
+  GroupedParams p{};
   p.out = out; p.out_is_f32 = unit < 0; p.epilogue = unit < 0 ? EPI_STORE : gated ? EPI_EXPERT_GLU : EPI_EXPERT_GELU;
   p.M = entries; p.N = N; p.K = K; p.ldo = N; p.status = status; p.groups = 1;
   p.k_blocks_per_split = (K + BLOCK_K - 1) / BLOCK_K;
