@@ -9,15 +9,15 @@
 //                memory, over the first half of S's columns
 //   O += P V     tcgen05.mma with P from tensor memory, V as it lies in the cache (MN-major); O stays in tensor memory
 //
-// S of the next tile is ready when a warpgroup has written P: no product stands in its chain.  (128 keys a tile and one buffer of S:
-// the warpgroups waited 1,800 of 4,500 cycles a tile for P V and S.)  A row's O and sum are brought to a new maximum only
-// when that grew by more than 2^8 since the last time (P stays below 256), so the accumulators are hardly ever read back; the sum is
-// that of the bfloat16 weights that multiply V, in float32, so that a row's weights add up to one whatever the reference.
+// S of the next tile is ready when a warpgroup has written P.  (128 keys a tile and one buffer of S: the warpgroups waited 1,800 of
+// 4,500 cycles a tile for P V and S.)  A row's O and sum follow its maximum, so that the largest weight is 1 and those near it use
+// the bfloat16 they multiply V in best: left behind until the maximum had grown by 2^8, which reads O back hardly ever, weights of up to
+// 2^8 were rounded where the step is twice as wide, and results were 1 to 2 % further from 64-bit ones.  The sum is that of the weights in float32.
 // S of tile j + 2 goes over the columns of P of tile j: one thread issues all products, and the tensor cores take them in order.
 //
 // What bounds it: the exponentials (16 an SM and cycle: 1,024 cycles for a pair of tiles, beside 900 to 1,280 of products).
-// Measured, prompts of 2,048 tokens, 16 heads: two maps of 64 with values of 128, 167 us on mma.sync, 70 us here; one map, a window of
-// 1,024, five prompts of 4,001 tokens together, 163 and 73 us.
+// Measured, prompts of 2,048 tokens, 16 heads, two maps of 64 with values of 128: 167 us on mma.sync, 80 us here; layers: this one 297 and
+// 144 us, one map with a window of 1,024, five prompts of 4,001 tokens together, 319 and 183 us.
 //
 // A piece (the CTA's rows) with many key tiles may be divided among `shares` CTAs, each taking every shares-th tile: partial sums
 // go to scratch memory, and the CTA that finds all the others counted in merges them.  Nobody waits for anybody.
@@ -41,7 +41,6 @@ constexpr int KV_ATOM = KEYS * 128;         // and of [KEYS rows, 64 bf16]
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_SHARES = 4;
 constexpr int MIN_SHARE_TILES = 6;          // a share of fewer key tiles costs more than it saves
-constexpr float RESCALE_LOG2 = 8.0f;
 
 template <int DIM, int VDIM, int MAPS>
 struct Layout {
@@ -411,8 +410,8 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           mx[3] = max3(mx[3], __uint_as_float(sc[c][i + 6]), __uint_as_float(sc[c][i + 7]));
         }
       const float n = max3(m, fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      // the row's first visible keys, or a maximum that grew so far that the probabilities would: bring O and the sum to it
-      const bool moved = n != m && (m == -INFINITY || !((n - m) * scale_log2 <= RESCALE_LOG2));
+      // the maximum moved: bring O and the sum to it
+      const bool moved = n != m;
       if (__any_sync(0xffffffffu, moved)) {
         const float alpha = !moved ? 1.0f : m == -INFINITY ? 0.f : exp2_fast((m - n) * scale_log2);
         if (moved) m = n;
@@ -446,8 +445,8 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           unpair(fma2(pair(sc[c][i], sc[c][i + 1]), scale2, nbase2), x0, x1);
           const float p0 = exp2_fast(x0), p1 = exp2_fast(x1);
           __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          const uint32_t bits = packed[i >> 1] = *(uint32_t*)&h;
-          l2 = add2(l2, pair(bits << 16, bits & 0xffff0000u));
+          packed[i >> 1] = *(uint32_t*)&h;
+          l2 = add2(l2, pair(p0, p1));
         }
         tmem_store16(s_addr + c * 16, packed);
       }

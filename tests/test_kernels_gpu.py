@@ -1095,6 +1095,42 @@ def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, h
         assert torch.equal(got, again) and not counters.any()
 
 
+@pytest.mark.parametrize("maps,dim,vdim,mask,softcap", [(2, 64, 128, None, 0.0), (1, 64, 128, ("window", 700), 0.0), (1, 128, 128, None, 30.0), (1, 64, 64, None, 0.0)])
+def test_maps_attention_tcgen05_is_as_close_to_64_bits(status, monkeypatch, maps, dim, vdim, mask, softcap):
+    """A prompt's attention on tcgen05 is no further from float64 than on mma.sync: weights rounded relative to the row's own maximum, sums of
+    weights in float32."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    heads, kv_heads, T, page, lam = 8, 2, 1536, 16, 0.4 if maps == 2 else 0.0
+    g = torch.Generator(device=DEV).manual_seed(dim + vdim + maps)
+    make = lambda *shape: torch.randn(*shape, generator=g, device=DEV).to(torch.bfloat16)
+    q, k, v = make(T, heads * maps * dim), make(T // page, kv_heads, page, maps * dim), make(T // page, kv_heads, page, vdim)
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(seq_of_token=ints([0] * T), positions=ints(list(range(T))), q_start=ints([0, T]), max_q_len=T, max_context=T, planned_context=0)
+    cache = SimpleNamespace(k=k, v=v, block_table=ints([list(range(T // page))]), page_tokens=page)
+    at = torch.arange(T, device=DEV)
+    hidden = at[None] > at[:, None]
+    if mask is not None:
+        hidden |= at[None] <= at[:, None] - mask[1]
+    want = torch.zeros(T, heads, vdim, dtype=torch.float64, device=DEV)
+    for h in range(heads):
+        kh, vh = (x[:, h // (heads // kv_heads)].reshape(T, -1).double() for x in (k, v))
+        for m in range(maps):
+            part = slice(m * dim, (m + 1) * dim)
+            score = q.view(T, heads, maps * dim)[:, h, part].double() @ kh[:, part].T * dim ** -0.5
+            score = softcap * torch.tanh(score / softcap) if softcap else score
+            want[:, h] += (1.0 if m == 0 else -lam) * (torch.softmax(score.masked_fill(hidden, -math.inf), -1) @ vh)
+    error = {}
+    for choice in ("mma_sync", "auto"):
+        monkeypatch.setenv("SPROUT_MULTIMAP_ATTENTION", choice)
+        out = torch.empty(T, heads * vdim, dtype=torch.bfloat16, device=DEV)
+        kernels.multimap_attention(q, cache, ctx, out, heads, kv_heads, maps, dim, vdim, dim ** -0.5, lam, 0.0, 1.0, status, mask=mask, softcap=softcap)
+        error[choice] = float((out.double().view(want.shape) - want).norm() / want.norm())
+    assert int(status.item()) == 0 and 0 < error["auto"] < 5e-3
+    # the two errors are norms over more than 700,000 roundings each: equal ones differ by a few thousandths
+    assert error["auto"] <= 1.005 * error["mma_sync"], error
+
+
 @pytest.mark.parametrize("maps,dim,vdim,rot,options", [
     (2, 64, 128, 64, {}), (1, 128, 128, 32, dict(weights=True)), (1, 64, 128, 64, dict(unit=True, turn=True)), (1, 32, 64, 16, dict(growth=True)),
     (2, 16, 32, 0, dict(growth=True, unit=True)), (1, 128, 128, 128, dict(interleaved=True, turn=True, weights=True)), (1, 128, 128, 64, dict(from_key=True, unit=True)),
