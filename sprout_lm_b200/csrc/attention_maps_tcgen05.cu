@@ -119,10 +119,22 @@ __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
+// Among how many CTAs a piece's key tiles go when the launch has `pieces` of them, a request's last piece `last` tiles and its first
+// `first`.  As many as leave every CTA an SM; two where all pieces have one but lengths differ so much that the longest would run
+// alone for long (a CTA takes some 9 us and 1.2 us a tile, 4 us more when it is divided, and a second round of CTAs starts late).
+// Head size 128, 512 queries over 900 cached tokens, 64 heads over 8 (128 pieces of 15 to 23 tiles): undivided 41 us, two shares, which two
+// rounds of CTAs take, 61 us; 4,096 tokens, 8 heads over 1 (128 pieces of 1 to 64 tiles): 91 and 71 us (all while O lagged behind the maximum).
+__device__ __forceinline__ int shares_of(int pieces, int last, int first, int sms) {
+  if (pieces > sms) return 1;
+  if (2 * pieces <= sms) return sms / pieces;
+  const float undivided = 9.f + 1.2f * last, divided = fmaxf(pieces * (26.f + 0.6f * (last + first)) / sms + 13.f, 26.f + 1.2f * first);
+  return divided < undivided ? 2 : 1;
+}
+
 struct Params {
   MultiMapParams m;                    // what every kernel of this attention takes
   int box_rows;                        // cache rows of a TMA box
-  int shares;                          // CTAs that a piece's key tiles may be divided among
+  int shares, sms;                     // CTAs that a piece's key tiles may be divided among; SMs of the device
   float* scratch; int* counters;       // [pieces][shares] shares; [pieces][2], zero between launches
   // PACKED: the requests' keys and values lie side by side instead of in pages, each request's from its first visible tile on
   // (`packed_base`): a head's key is `key_atoms` times 64 columns of its own in map_k's rows and then the columns from `tail_col` of
@@ -186,7 +198,20 @@ maps_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   auto tile_of = [&](int i) { return i < keep_tiles ? i : tile_lo + (i - keep_tiles); };
   const int all_tiles = keep_tiles + max(0, max_limit / KEYS + 1 - tile_lo);
   const int all_tiles_a = min(all_tiles, keep_tiles + max(0, limit_a / KEYS + 1 - tile_lo));
-  const int shares = max(1, min(tc.shares, all_tiles / MIN_SHARE_TILES));
+  int shares = 1;
+  if (tc.shares > 1) {
+    // every thread takes the same decision: the launch's pieces, and the tiles of the request's last and first piece
+    int pieces = 0;
+    for (int base = 0; base < p.requests; base += 32) {
+      const int i = base + lane;
+      pieces += i < p.requests ? ((p.q_start[i + 1] - p.q_start[i]) * group + L::CTA_ROWS - 1) / L::CTA_ROWS : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pieces += __shfl_xor_sync(0xffffffffu, pieces, o);
+    const int lo = first_visible(p.mask_kind, p.mask_size, p.positions[q0]), end = p.positions[p.q_start[r + 1] - 1];
+    const int last_tiles = (end - first_visible(p.mask_kind, p.mask_size, end)) / KEYS + 1, first_tiles = (p.positions[q0] - lo) / KEYS + 1;
+    shares = max(1, min(min(tc.shares, shares_of(pieces * p.kv_heads, last_tiles, first_tiles, tc.sms)), all_tiles / MIN_SHARE_TILES));
+  }
   if (rank >= shares) return;
   // below, j counts the CTA's own tiles: rank + shares * j is the index among the piece's
   const int n_tiles = (all_tiles - rank + shares - 1) / shares;
@@ -647,7 +672,7 @@ bool tc_sizes(int maps, int dim, int vdim) {
 }
 int cta_rows(int maps) { return maps == 1 ? 2 * ROWS : ROWS; }
 long long pieces_bound(int tokens, int requests, int heads, int kv_heads, int maps) {
-  return (((long long)tokens * (heads / kv_heads) + cta_rows(maps) - 1) / cta_rows(maps) + requests) * kv_heads;
+  return ((long long)tokens * (heads / kv_heads) + (long long)requests * (cta_rows(maps) - 1)) / cta_rows(maps) * kv_heads;
 }
 
 template <int DIM, int VDIM, int MAPS, bool PACKED = false>
@@ -671,7 +696,7 @@ SPROUT_API int sprout_maps_attention_tc_supported(int maps, int dim, int vdim, i
   return tc_sizes(maps, dim, vdim) && pages_ok && out_stride % 8 == 0;
 }
 
-// How many CTAs a piece's key tiles are divided among in a launch of these sizes, and the floats of scratch and the counters
+// How many CTAs a piece's key tiles are divided among at most in a launch of these sizes (the kernel knows the pieces exactly), and the floats of scratch and the counters
 // that takes (scratch: none for one share).
 SPROUT_API int sprout_maps_attention_tc_shares(int tokens, int requests, int heads, int kv_heads, int maps) {
   const long long pieces = pieces_bound(tokens, requests, heads, kv_heads, maps);
@@ -697,7 +722,7 @@ int sprout_maps_attention_tc(const MultiMapParams& m, int tokens, int maps, int 
   p.m = m;
   p.box_rows = m.page_tokens < KEYS ? m.page_tokens : KEYS;
   p.shares = scratch && counters ? sprout_maps_attention_tc_shares(tokens, m.requests, m.heads, m.kv_heads, maps) : 1;
-  p.scratch = scratch; p.counters = counters;
+  p.scratch = scratch; p.counters = counters; p.sms = sm_count();
   CUtensorMap map_k, map_v;
   if (tensor_map(m.k_cache, (int)cache_rows, maps * dim, maps * dim, p.box_rows, &map_k)) return 1;
   if (tensor_map(m.v_cache, (int)cache_rows, vdim, vdim, p.box_rows, &map_v)) return 1;
@@ -728,7 +753,7 @@ SPROUT_API int sprout_latent_unfolded_attention(const void* q, int q_stride, con
   p.m.mask_kind = window > 0 ? MASK_WINDOW : MASK_CAUSAL; p.m.mask_size = window;
   p.box_rows = KEYS;
   p.shares = scratch && counters ? sprout_maps_attention_tc_shares(tokens, requests, heads, heads, 1) : 1;
-  p.scratch = scratch; p.counters = counters;
+  p.scratch = scratch; p.counters = counters; p.sms = sm_count();
   p.key_atoms = dim / 64; p.tail_col = tail_col; p.value_col = heads * dim;
   const int width = heads * (dim + vdim);
   CUtensorMap map_k, map_v;
