@@ -449,9 +449,14 @@ multimap_attention_simple_kernel(const T* __restrict__ q, int q_stride, const T*
 // ------------------------------------------------------------------------------------------ tensor cores
 constexpr int MM_ROWS = 64, MM_KEYS = 64, MM_THREADS = 128;
 
-template <int DIM, int VDIM, int MAPS, bool SPLIT>
+// How the rows of a step go to the CTAs: tiles of 64 rows; or, where no request has more than 16 rows (usually single tokens, the heads of
+// one key/value group), a CTA's warps share the keys of its request's tile, with the 16 rows of the fragments or the first 8 alone.
+enum RowsForm : int { ROWS_TILES = 0, ROWS_16 = 1, ROWS_8 = 2 };
+
+template <int DIM, int VDIM, int MAPS, int ROWS>
 __global__ void __launch_bounds__(MM_THREADS)
 multimap_attention_mma_kernel(const MultiMapParams p) {
+  constexpr bool SPLIT = ROWS != ROWS_TILES;
   constexpr int KW = MAPS * DIM, KSTRIDE = KW + 8, VSTRIDE = VDIM + 8, KCHUNKS = KW / 8, VCHUNKS = VDIM / 8;
   extern __shared__ __align__(16) unsigned char mm_smem[];
   __nv_bfloat16* sQ = (__nv_bfloat16*)mm_smem;                   // MM_ROWS x KSTRIDE
@@ -542,9 +547,10 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   // SPLIT (a step in which no request has more than 16 rows: single tokens, the heads of one key/value group): a CTA
   // divides every tile's keys among its warps instead of its rows, and the warps' partial results are merged at the end.
   constexpr bool split = SPLIT;
-  // rows 8 to 15 of a tile are the second two numbers of every fragment: where a request has at most 8 rows (4 heads a group, usually)
-  // their scores are not capped, compared or exponentiated (64 requests over 6,000 keys, capped scores: 200 us with them, 193 us without)
-  const bool upper = !SPLIT || rows_total > 8;
+  // rows 8 to 15 of a tile are the second two numbers of every fragment: where no request has more than 8 rows (4 heads a group, usually)
+  // their scores are not capped or exponentiated (64 requests over 6,000 keys, capped scores: 200 us with them, 193 us without; as a
+  // question to every tile instead of a form of its own it cost steps with more rows 4 %)
+  constexpr bool upper = ROWS != ROWS_8;
   const int qrow = split ? 0 : warp * 16;             // the warp's 16 rows
   constexpr int nk = split ? 1 : MM_KEYS / 16;        // blocks of 16 keys of a tile that the warp takes, from key kb on
   const int kb = split ? warp * 16 : 0;
@@ -605,9 +611,10 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
           if (i >= 2 * nk) break;
 #pragma unroll
           for (int c = 0; c < 2; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
-          if (!upper) continue;
+          if (upper) {
 #pragma unroll
-          for (int c = 2; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
+            for (int c = 2; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
+          }
         }
       }
       float t_max0 = -INFINITY, t_max1 = -INFINITY;
@@ -657,9 +664,12 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
         if (i >= 2 * nk) break;
         s[i][0] = exp2f(fmaf(s[i][0], scale_log2, -base0)); s[i][1] = exp2f(fmaf(s[i][1], scale_log2, -base0));
         l0[m] += s[i][0] + s[i][1];
-        if (!upper) { s[i][2] = s[i][3] = 0.f; continue; }
-        s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
-        l1[m] += s[i][2] + s[i][3];
+        if (upper) {
+          s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
+          l1[m] += s[i][2] + s[i][3];
+        } else {
+          s[i][2] = s[i][3] = 0.f;
+        }
       }
 #pragma unroll
       for (int kk = 0; kk < MM_KEYS / 16; kk++) {
@@ -915,18 +925,19 @@ multimap_merge_kernel(const MultiMapParams p, int vdim) {
     if (threadIdx.x + part * 128 < vdim) dst[threadIdx.x + part * 128] = __float2bfloat16_rn(v[part] * factor);
 }
 
-template <int DIM, int VDIM, int MAPS, bool SPLIT>
+template <int DIM, int VDIM, int MAPS, int ROWS>
 int launch_multimap(const MultiMapParams& p, int grid_x, cudaStream_t stream) {
+  constexpr bool SPLIT = ROWS != ROWS_TILES;
   const int tiles_bytes = (3 * MM_ROWS * (MAPS * DIM + 8) + 2 * MM_KEYS * (VDIM + 8)) * 2;
   const int merge_bytes = MM_THREADS * MAPS * (VDIM / 8 * 4 + 4) * 4;         // the warps' partial results of a 16-row CTA
   const int smem = tiles_bytes > merge_bytes ? tiles_bytes : merge_bytes;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(multimap_attention_mma_kernel<DIM, VDIM, MAPS, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t err = cudaFuncSetAttribute(multimap_attention_mma_kernel<DIM, VDIM, MAPS, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return sprout_fail("multimap_attention_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
     configured = true;
   }
-  sprout_launch(multimap_attention_mma_kernel<DIM, VDIM, MAPS, SPLIT>, dim3(grid_x, p.kv_heads, SPLIT ? p.ksplit : 1), dim3(MM_THREADS),
+  sprout_launch(multimap_attention_mma_kernel<DIM, VDIM, MAPS, ROWS>, dim3(grid_x, p.kv_heads, SPLIT ? p.ksplit : 1), dim3(MM_THREADS),
                 smem, stream, p);
   if (int code = sprout_check_launch("multimap_attention_mma")) return code;
   if (SPLIT && p.ksplit > 1) {
@@ -986,18 +997,17 @@ SPROUT_API int sprout_multimap_attention_mma(const void* q, int q_stride, const 
                  "multimap_attention_mma: keys are divided among CTAs in single-token steps only, with scratch for the shares");
   if (tokens > 0) return sprout_maps_attention_tc(p, tokens, maps, dim, vdim, partial, counters, stream);
   const bool split = max_q_len * (heads / kv_heads) <= 16;
-#define PICK(D, V)                                                                                              \
-  if (dim == D && vdim == V) {                                                                                  \
-    if (split) return maps == 2 ? launch_multimap<D, V, 2, true>(p, tiles, stream) : launch_multimap<D, V, 1, true>(p, tiles, stream); \
-    return maps == 2 ? launch_multimap<D, V, 2, false>(p, tiles, stream) : launch_multimap<D, V, 1, false>(p, tiles, stream);         \
-  }
+  const bool eight = max_q_len * (heads / kv_heads) <= 8;
+#define PICK_ROWS(D, V, M)                                                                                      \
+  (!split ? launch_multimap<D, V, M, ROWS_TILES>(p, tiles, stream)                                              \
+          : eight ? launch_multimap<D, V, M, ROWS_8>(p, tiles, stream) : launch_multimap<D, V, M, ROWS_16>(p, tiles, stream))
+#define PICK(D, V) if (dim == D && vdim == V) return maps == 2 ? PICK_ROWS(D, V, 2) : PICK_ROWS(D, V, 1);
   PICK(32, 64) PICK(64, 64) PICK(64, 128) PICK(128, 128) PICK(16, 32) PICK(32, 32)
 #undef PICK
-#define PICK(D, V)                                                                                              \
-  if (dim == D && vdim == V && maps == 1)                                                                       \
-    return split ? launch_multimap<D, V, 1, true>(p, tiles, stream) : launch_multimap<D, V, 1, false>(p, tiles, stream);
+#define PICK(D, V) if (dim == D && vdim == V && maps == 1) return PICK_ROWS(D, V, 1);
   PICK(96, 96) PICK(48, 48) PICK(80, 80)
 #undef PICK
+#undef PICK_ROWS
   return sprout_fail("multimap_attention_mma: no kernel for these sizes");
 }
 
