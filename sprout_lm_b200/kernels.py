@@ -1545,8 +1545,22 @@ def visible_keys(mask, context: int) -> int:
 
 
 # (token, head) rows of a step from which prompt attention with one or two maps runs on tcgen05: below, a layer's launches take the host
-# longer than the device either way, and the mma.sync kernel needs no scratch (60 tokens of 8 heads: 77 against 81 us a layer)
+# longer than the device either way, and the mma.sync kernel needs no scratch (60 tokens of 8 heads: 77 against 81 us a layer).
+# From as many 64-key tiles on as a query of the step sees at most, by (maps, key size, value size, capped scores): a CTA of the tcgen05
+# kernel takes 7 to 13 us before its first and after its last tile, one of the mma.sync kernel 3 to 5, but 1.1 to 1.3 us a tile (2.7 to
+# 3.2 where scores are capped) against 1.7 to 3.4; the numbers are for steps of few tiles of 64 rows (the mma.sync kernel's CTAs), of 1.25
+# an SM and of 2 an SM on, where those come in rounds.  (One map of 128, 16 heads over 4, one prompt: 256 tokens 13.5 us on mma.sync,
+# 18.4 on tcgen05; 777 tokens 38.8 and 27.9; two maps of 64: 128 tokens 11.2 and 14.1, 256 tokens 18.0 and 17.0.)
 MAPS_TC_ROWS = 2048
+MAPS_TC_TILES = {(2, 64, 64, False): (4, 4, 4), (2, 64, 128, False): (4, 4, 4), (2, 64, 64, True): (14, 10, 10), (2, 64, 128, True): (14, 10, 10),
+                 (1, 64, 64, False): (10, 10, 8), (1, 64, 64, True): (14, 10, 10), (1, 64, 128, False): (6, 5, 4), (1, 64, 128, True): (14, 10, 10),
+                 (1, 128, 128, False): (9, 9, 4), (1, 128, 128, True): (12, 12, 5)}
+
+
+def _maps_tc_pays(maps: int, dim: int, vdim: int, capped: bool, keys: int, rows64: int, sms: int) -> bool:
+    """Whether a step's prompt attention is faster on tcgen05: ``keys`` a query sees at most, ``rows64`` tiles of 64 rows over all key/value heads."""
+    tiles = MAPS_TC_TILES.get((maps, dim, vdim, capped), (0, 0, 0))
+    return -(-keys // 64) >= tiles[2 if rows64 >= 2 * sms else 1 if 4 * rows64 >= 5 * sms else 0]
 
 
 @functools.lru_cache(maxsize=256)
@@ -1598,7 +1612,9 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
         # mma.sync kernel 64) and MAPS_TC_ROWS in all
         tensor = 0
         if q.shape[0] * heads >= MAPS_TC_ROWS and q.shape[0] * group >= 128 * requests and choice != "mma_sync" and max_q_len * group > 16 and out.data_ptr() % 16 == 0 \
-                and _maps_tc_takes(maps, dim, vdim, cache.page_tokens, out.stride(0)):
+                and _maps_tc_takes(maps, dim, vdim, cache.page_tokens, out.stride(0)) \
+                and _maps_tc_pays(maps, dim, vdim, softcap > 0.0, visible_keys(mask, int(getattr(ctx, "max_context", 0) or 1 << 30)),
+                                  (tiles - requests) * kv_heads, sm_count(q.device)):
             tensor = q.shape[0]
             floats = 0 if counters is None else _maps_tc_scratch(tensor, requests, heads, kv_heads, maps, vdim)
             if floats:

@@ -221,6 +221,18 @@ def test_captured_steps_tell_short_portions_apart():
     assert key(65, *[1] * 63) == key(*[1] * 62, 30, 36)
 
 
+def test_mapped_prompt_attention_keeps_short_contexts_on_mma_sync():
+    """The tcgen05 kernel of mapped attention pays from some key tiles on, fewer where the step has many rows; sizes without an entry take it always."""
+    pays = lambda keys, rows64, maps=1, dim=128, capped=False: kernels._maps_tc_pays(maps, dim, 128, capped, keys, rows64, 148)
+    assert not pays(256, 64) and not pays(512, 64) and pays(513, 64)              # one prompt of 256 tokens of 16 heads over 4, and of more
+    assert pays(256, 296) and not pays(192, 296)                                  # many prompts of 256 tokens
+    assert not pays(704, 64, capped=True) and pays(705, 64, capped=True)
+    assert not pays(192, 32, maps=2, dim=64) and pays(193, 32, maps=2, dim=64)
+    for maps, dim, vdim, capped in kernels.MAPS_TC_TILES:
+        few, some, many = kernels.MAPS_TC_TILES[maps, dim, vdim, capped]
+        assert few >= some >= many > 0                                            # more rows never raise the bar
+
+
 def test_small_batch_kernels_say_what_they_take():
     """The small-batch kernels' size rules are host arithmetic in the kernel library: up to 16 tokens,
     sizes in steps of 16, and a layer small enough for the SMs' shared memory.  What they refuse

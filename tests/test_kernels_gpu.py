@@ -1077,6 +1077,7 @@ def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, h
     counters = torch.zeros(2 * kernels.sm_count(torch.device(DEV)), dtype=torch.int32, device=DEV) if divided else None
     got = torch.full((T, heads * vdim), float("nan"), dtype=torch.bfloat16, device=DEV)
     monkeypatch.setattr(kernels, "MAPS_TC_ROWS", 0)
+    monkeypatch.setattr(kernels, "MAPS_TC_TILES", {})                # the kernel under test, whether it pays at these sizes or not
     kernels.multimap_attention(q, cache, ctx, got, *sizes, counters=counters, **more)
     assert int(status.item()) == 0
     assert counters is None or not counters.any()
