@@ -24,7 +24,7 @@
 // timeout the CTA sets the status word, waits (bounded) for its copies in flight, frees its
 // tensor memory and returns.
 //
-// Runs for head_dim 64; the kernel in attention_maps_tcgen05.cu takes head_dim 128.
+// Runs for head_dim 64, and for head_dim 128 over short contexts; the kernel in attention_maps_tcgen05.cu takes head_dim 128 otherwise.
 // Page sizes of 8, 16, 32, 64 or a multiple of 128 tokens; the mma.sync kernel in attention_bf16.cu takes everything else.
 #include <cuda_bf16.h>
 
@@ -574,12 +574,13 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
                                 const int* block_table, int table_stride, const int* q_start, const int* positions,
                                 void* out, int out_stride, int num_tokens, int requests, int heads, int kv_heads,
                                 int head_dim, int page_tokens, int num_pages, float* scratch, long long scratch_floats,
-                                int* counters, int* status, cudaStream_t stream) {
+                                int* counters, int in_registers, int* status, cudaStream_t stream) {
   SPROUT_REQUIRE(sprout_attention_prefill_tc_supported(head_dim, page_tokens, out_stride) && ((uintptr_t)out & 15) == 0,
                  "attention_prefill (tcgen05): head_dim %d, page size %d or the output's alignment is not taken", head_dim, page_tokens);
-  // Head size 128 runs on the kernel whose O stays in tensor memory (28 heads over 4, one prompt of 4,096 tokens: 180 us against 232 with
-  // O added up in registers); head size 64 keeps this kernel's 128-key tiles (14 heads over 2, 2,048 tokens: 34.5 against 39.5 us).
-  if (head_dim == 128)
+  // Head size 128 runs on the kernel whose O stays in tensor memory (28 heads over 4, one prompt of 4,096 tokens: 190 us against 227 with
+  // O added up in registers) unless the caller asks for this one; head size 64 keeps this kernel's 128-key tiles (14 heads over 2, 2,048
+  // tokens: 34.5 against 39.5 us).
+  if (head_dim == 128 && !in_registers)
     return sprout_attention_prefill_maps(q, q_stride, k_cache, v_cache, block_table, table_stride, q_start, positions, out, out_stride, num_tokens, requests,
                                          heads, kv_heads, head_dim, page_tokens, num_pages, scratch, scratch_floats, counters, status, stream);
   const long long cache_rows = (long long)num_pages * kv_heads * page_tokens;
@@ -589,7 +590,7 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
   p.block_table = block_table; p.table_stride = table_stride; p.q_start = q_start; p.positions = positions;
   p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
   p.requests = requests; p.heads = heads; p.kv_heads = kv_heads; p.page_tokens = page_tokens; p.num_pages = num_pages;
-  constexpr int keys = TcLayout<64>::KEYS;
+  const int keys = head_dim == 64 ? TcLayout<64>::KEYS : TcLayout<128>::KEYS;
   p.box_rows = page_tokens < keys ? page_tokens : keys;
   p.scale = 1.0f / sqrtf((float)head_dim); p.status = status;
   CUtensorMap map_k, map_v;
@@ -609,5 +610,5 @@ int sprout_attention_prefill_tc(const void* q, int q_stride, const void* k_cache
     if (n > SPROUT_PREFILL_SPLIT_MAX) n = SPROUT_PREFILL_SPLIT_MAX;
     p.split_pieces = (int)n;
   }
-  return launch_tc<64>(map_k, map_v, p, (int)bound, stream);
+  return head_dim == 64 ? launch_tc<64>(map_k, map_v, p, (int)bound, stream) : launch_tc<128>(map_k, map_v, p, (int)bound, stream);
 }

@@ -44,7 +44,7 @@ _SIGNATURES = {
     "sprout_attention_decode_fused": [_P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P],
     "sprout_attention_decode_resident": [_P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P],
     "sprout_attention_decode_resident_cap": [_I, _I, _I, _I],
-    "sprout_attention_prefill": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _P, _P],
+    "sprout_attention_prefill": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P],
     "sprout_attention_prefill_tc_supported": [_I, _I, _I],
     "sprout_gemm_bf16": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_gemm_bf16_unscaled": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
@@ -890,15 +890,29 @@ def _prefill_workspace(device, head_dim):
     return held
 
 
+# Prompt attention of head size 128 on tcgen05: from as many 64-key tiles on the kernel that keeps O in tensor memory, for launches of up to
+# an SM's worth of 256-row pieces and of more; below, the one that adds it up in registers, whose CTAs are set up and leave sooner (28 heads
+# over 4: 64 tokens 13.3 against 15.2 us, 16 x 256 tokens 59.0 and 68.4, but 512 tokens 29.7 and 25.6, 4 x 512 over 300 cached 60.4 and 57.8).
+PREFILL_TILES = (4, 9)
+
+
+def _prefill_in_registers(tokens: int, requests: int, heads: int, kv_heads: int, max_context: int, sms: int) -> bool:
+    """``max_context``: the longest context of the step (0: not known, taken for long)."""
+    pieces = (tokens * (heads // kv_heads) + 255 * requests) // 256 * kv_heads
+    return 0 < max_context <= 64 * (PREFILL_TILES[0 if pieces <= sms else 1] - 1)
+
+
 def attention_prefill(q, k_cache, v_cache, block_table, q_start, positions, out, heads, kv_heads, head_dim, status,
-                      variant="auto"):
+                      variant="auto", max_context=0):
     """Tensor-core flash attention of the step's queries (portions of prompts, single tokens) over
     their requests' pages (bfloat16, float32 softmax).  ``variant``: "tcgen05" (S and P V in tensor
     memory, K and V pages by TMA; head_dim 64 or 128, pages of 8..64 or a multiple of 128 tokens),
     "mma_sync" (every head_dim up to 128 in steps of 16, every page size), or "auto": tcgen05
-    where it takes the sizes and the requests bring 128 (token, head) rows each on average."""
+    where it takes the sizes and the requests bring 128 (token, head) rows each on average.
+    ``max_context``: the step's longest context, where the caller knows it."""
     _check_paged(q, k_cache, v_cache, block_table, out, heads, head_dim, "attention_prefill")
     scratch = counters = None
+    in_registers = head_dim == 128 and _prefill_in_registers(q.shape[0], q_start.numel() - 1, heads, kv_heads, max_context, sm_count(q.device))
     if variant != "mma_sync" and head_dim in (64, 128):
         scratch, counters = _prefill_workspace(q.device, head_dim)
     _run("sprout_attention_prefill", _ptr(q, "q"), q.stride(0), _ptr(k_cache, "k_cache"), _ptr(v_cache, "v_cache"),
@@ -906,7 +920,7 @@ def attention_prefill(q, k_cache, v_cache, block_table, q_start, positions, out,
          _ptr(positions, "positions", torch.int32), _ptr(out, "out"), out.stride(0), q.shape[0], q_start.numel() - 1,
          heads, kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], PREFILL_VARIANTS[variant],
          _ptr(scratch, "scratch", torch.float32, True), scratch.numel() if scratch is not None else 0,
-         _ptr(counters, "counters", torch.int32, True), _ptr(status, "status", torch.int32), _stream())
+         _ptr(counters, "counters", torch.int32, True), 1 if in_registers else 0, _ptr(status, "status", torch.int32), _stream())
 
 
 def paged_attention(q, cache, ctx, out, heads, kv_heads, head_dim, status):
@@ -928,7 +942,7 @@ def paged_attention(q, cache, ctx, out, heads, kv_heads, head_dim, status):
             if variant == "tcgen05" and not load_library().sprout_attention_prefill_tc_supported(head_dim, cache.k.shape[2], out.stride(0)):
                 variant = "mma_sync"
             return attention_prefill(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out,
-                                     heads, kv_heads, head_dim, status, variant=variant)
+                                     heads, kv_heads, head_dim, status, variant=variant, max_context=ctx.max_context)
     elif head_dim in (64, 128) and ctx.max_q_len >= ATTENTION_TILE_TOKENS and cache.k.data_ptr() % 16 == 0 and cache.v.data_ptr() % 16 == 0:
         return attention_tile(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out, heads, kv_heads, head_dim,
                               ctx.max_q_len, status)
