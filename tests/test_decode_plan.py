@@ -233,6 +233,13 @@ def test_mapped_prompt_attention_keeps_short_contexts_on_mma_sync():
         assert few >= some >= many > 0                                            # more rows never raise the bar
 
 
+def test_prompt_attention_of_head_size_128_adds_short_contexts_up_in_registers():
+    pick = lambda tokens, requests, context, heads=28, kv_heads=4: kernels._prefill_in_registers(tokens, requests, heads, kv_heads, context, 148)
+    assert pick(64, 1, 64) and pick(192, 1, 192) and not pick(256, 1, 256)          # a launch that leaves SMs idle
+    assert pick(4096, 16, 256) and pick(4096, 16, 512) and not pick(4096, 16, 513)  # 512 pieces
+    assert not pick(64, 1, 0)                                                       # a caller that does not know its contexts
+
+
 def test_small_batch_kernels_say_what_they_take():
     """The small-batch kernels' size rules are host arithmetic in the kernel library: up to 16 tokens,
     sizes in steps of 16, and a layer small enough for the SMs' shared memory.  What they refuse

@@ -1408,3 +1408,23 @@ def test_float32_scan_keeps_its_bits_beside_a_long_portion(status, form, dim, vd
         alone, state = scan([r])
         assert torch.equal(alone, together[starts[r]:starts[r + 1]]) and torch.equal(state[r], states[r]), r
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,held,new", [(28, 4, [0, 0, 70], [64, 130, 61]), (8, 1, [0], [192]), (16, 16, [5, 0], [128, 177])])
+def test_prompt_attention_of_head_size_128_both_kernels(status, heads, kv_heads, held, new):
+    """Short contexts: the kernel that adds O up in registers (the step's longest context given) and the one in tensor memory (not given) against
+    the float32-arithmetic kernel."""
+    from sprout_lm_b200 import kernels
+    case = build_paged_case(torch.bfloat16, heads, kv_heads, 128, 16, [h + n for h, n in zip(held, new)], new)
+    outs = []
+    for context in (max(h + n for h, n in zip(held, new)), 0):
+        out = torch.full((case["T"], heads * 128), float("nan"), dtype=torch.bfloat16, device=DEV)
+        kernels.attention_prefill(case["q"], case["k_cache"], case["v_cache"], case["table"], case["q_start"], case["positions"], out, heads, kv_heads, 128,
+                                  status, variant="tcgen05", max_context=context)
+        outs.append(out.float())
+    want = torch.empty(case["T"], heads * 128, dtype=torch.bfloat16, device=DEV)
+    kernels.attention_simple(case["q"], case["k_cache"], case["v_cache"], case["table"], case["seq_of_token"], case["positions"], want, heads, kv_heads, 128, status)
+    for out in outs:
+        # probabilities and the result rounded to 8 bits
+        assert (out - want.float()).norm() <= 6e-3 * want.float().norm()
+    assert int(status.item()) == 0
