@@ -68,7 +68,6 @@ struct ScanParams {
   int chunk, requests;
   int q_silu;                          // silu on the query rows (with a floor only)
   int v_cols, ones_col;                // columns the value rows really have (<= vdim); column v_cols of the state is fed 1
-  int wide;                            // q, k and decay rows are fetched 8 neighbours at a time (chunks' walks)
 };
 
 // Eight neighbouring elements of a row that start on a 16-byte boundary.
@@ -126,10 +125,11 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // Tokens come `batch` at a time: while the threads walk a batch's tokens over their registers, the next batch's q, k,
 // decay inputs and values are on their way from memory into registers; at the batch's end they are turned into
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
-// shuffles.  The bfloat16 path's walks over chunks in tiles of 8 x 4 (PAIRS) go two rows at a time in packed arithmetic: a thread's
-// rows are then neighbours, and q, c k and a lie in planes of their own, so that a 16-byte read is two pairs of one of them (2,500
-// tokens of 16 heads of 128 x 128: 154 and 362 us for the two walks with a number at a time, (q, c k, a) triples and 2-byte fetches,
-// 106 and 237 us so, the rows fetched 16 bytes at a time where they start on 16-byte boundaries and fill the slices).
+// shuffles.  The bfloat16 path's walks over chunks of key sizes 64, 128 and 256, whose rows fill the slices (PAIRS), go two rows at a
+// time in packed arithmetic: a thread's rows are then neighbours, fetched 16 bytes at a time, and q, c k and a lie in planes of their
+// own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us for the two walks with
+// a number at a time, (q, c k, a) triples and 2-byte fetches, 106 and 237 us so).  Other sizes and rows off 16-byte boundaries keep a
+// number at a time: pairs without the wide fetches cost 12 % (four heads of 96 x 96), and with two slices or one, 4 % (8 x 512, 16 x 64).
 // Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order.  An output's sum over the rows has one order in
 // the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn, so a bfloat16 request of one
 // chunk may differ in the last bits of a 32-bit sum by whether another portion of the step is long.
@@ -217,13 +217,12 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   auto z_at = [&](size_t index) { return p.z_f32 ? ((const float*)p.z)[index] : to_float(((const T*)p.z)[index]); };
 
   float rq[EPT], rk[EPT], rz[EPT], rc[PHASE == SCAN_WHOLE ? 1 : EPT], rv[VPT];
-  // wide: a thread's eight elements are the rows 8 (tid % slices) on of token tid / slices of the batch, its values neighbours too
+  // PAIRS: a thread's eight elements are the rows 8 (tid % slices) on of token tid / slices of the batch, its values neighbours too
   // (32 slices: a batch of 4 tokens over 16 columns has a value for every second thread only)
-  const bool wide = PAIRS && p.wide;
   const int wide_token = tid >> slices_log2, wide_values = max(1, (batch << cb_log2) / SCAN_THREADS);
   auto fetch = [&](int t0) {                          // loads only: nothing waits for them here
     const int n = min(batch, last - t0);
-    if (wide) {
+    if (PAIRS) {
       if (wide_token < n) {
         const size_t t = (size_t)t0 + wide_token;
         const int i = slice * 8;
@@ -293,7 +292,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
   for (int t0 = first; t0 < last; t0 += batch) {
     const int n = min(batch, last - t0);
     __syncthreads();                                   // the batch before has been read by everyone
-    if (wide) {
+    if (PAIRS) {
       if (wide_token < n) {
         float4* to = reinterpret_cast<float4*>(tok2 + (size_t)wide_token * 4 * plane + slice * 4);
         const int half4 = half_stride / 4, plane4 = plane / 4;
@@ -344,15 +343,7 @@ gated_scan_kernel(const ScanParams<T> p, int slices_log2, int batch) {
         x.z = floored ? 1.0f - decay : decay;
         if (bonus && PHASE != SCAN_CHUNK_SUMS) x.w = x.x * p.bonus[(size_t)h * dim + i] * x.y;
       }
-      if (PAIRS) {
-        float* to = tok2 + (size_t)tt * 4 * plane + ((i & 7) >> 2) * half_stride + (i >> 3) * 4 + (i & 3);
-        if (PHASE != SCAN_CHUNK_SUMS) to[0] = x.x;
-        to[plane] = x.y;
-        to[2 * plane] = x.z;
-        if (bonus && PHASE != SCAN_CHUNK_SUMS) to[3 * plane] = x.w;
-      } else {
-        tok[e] = x;
-      }
+      tok[e] = x;
     }
 #pragma unroll
     for (int u = 0; u < VPT; u++) {
@@ -840,7 +831,7 @@ __global__ void scaled_sum_kernel(float* __restrict__ x, const float* __restrict
 }
 
 template <typename T, int ROWS, int COLS, int FORM>
-int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cudaStream_t stream) {
+int launch_scan_tiles(const ScanParams<T>& p, bool pairs, int requests, int max_chunks, cudaStream_t stream) {
   int slices_log2 = 0;
   while ((ROWS << slices_log2) < p.dim) slices_log2++;
   SPROUT_REQUIRE(slices_log2 <= 5, "gated_scan: key vectors too long (%d)", p.dim);
@@ -854,8 +845,9 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
   // single walks (few tokens: the state's way in and out is most of their time, and rows dealt in turn read it faster: 64 single tokens
   // of 16 heads 46 against 52 us) keep a number at a time, and so does the 32-bit path, whose sums have one order in both walks
   constexpr bool PAIRED = ROWS == 8 && COLS == 4 && sizeof(T) == 2;
+  pairs = pairs && PAIRED;
   const size_t smem = (size_t)batch * ((size_t)ROWS * slices * sizeof(float4) + (size_t)cb * sizeof(float));
-  const size_t smem_chunks = PAIRED ? (size_t)batch * ((size_t)4 * 2 * (ROWS * slices / 2 + 16) + cb) * sizeof(float) : smem;
+  const size_t smem_chunks = pairs ? (size_t)batch * ((size_t)4 * 2 * (ROWS * slices / 2 + 16) + cb) * sizeof(float) : smem;
   const dim3 grid(requests, p.heads, (p.vdim + cb - 1) / cb);
   SPROUT_REQUIRE(grid.z <= 65535, "gated_scan: too many value columns");
   if (p.sums == nullptr && p.mode == DECAY_GIVEN) {
@@ -868,30 +860,32 @@ int launch_scan_tiles(const ScanParams<T>& p, int requests, int max_chunks, cuda
   }
   // `max_chunks` blocks per (head, columns): the chunks of all requests, found by their number
   const dim3 chunks(max_chunks, p.heads, grid.z);
-  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, PAIRED>, chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
+  sprout_launch(pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, false>,
+                chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
   if (int rc = sprout_check_launch("gated_scan (chunk sums)")) return rc;
   SPROUT_REQUIRE(requests <= 65535, "gated_scan: too many requests");
   sprout_launch(scan_carry_kernel, dim3((p.dim * p.vdim + 255) / 256, p.heads, requests), dim3(256), 0, stream, p.sums,
                 (const float*)p.prods, (const float*)p.state, p.q_start, p.state_slots, p.num_slots, p.chunk, p.heads, p.dim, p.vdim);
   if (int rc = sprout_check_launch("gated_scan (carry)")) return rc;
-  sprout_launch(gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, PAIRED>, chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
+  sprout_launch(pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, false>,
+                chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
   return sprout_check_launch("gated_scan (chunk outputs)");
 }
 
 template <typename T>
-int launch_scan(ScanParams<T> p, int requests, int max_chunks, cudaStream_t stream) {
-  // 16-byte fetches: the rows fill the tile's slices, and every row starts on a 16-byte boundary
+int launch_scan(const ScanParams<T>& p, int requests, int max_chunks, cudaStream_t stream) {
+  // pairs of rows: the key's rows fill the tile's slices, and every row starts on a 16-byte boundary
   constexpr int per16 = 16 / (int)sizeof(T);
   auto on16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
-  p.wide = (p.dim == 8 || p.dim == 16 || p.dim == 32 || p.dim == 64 || p.dim == 128 || p.dim == 256) && p.q_stride % per16 == 0 &&
-           (!p.k || p.k_stride % per16 == 0) && on16(p.q) && on16(p.k) && on16(p.da);
+  const bool pairs = (p.dim == 64 || p.dim == 128 || p.dim == 256) && p.q_stride % per16 == 0 && (!p.k || p.k_stride % per16 == 0) && on16(p.q) &&
+                     on16(p.k) && on16(p.da);
   // a thread's tile of the state: 8 rows x 4 columns up to 256 key channels, 32 rows of one column up to 1024
   const bool narrow = p.dim <= 8 * 32;
   if (p.mode == DECAY_FLOOR)
-    return narrow ? launch_scan_tiles<T, 8, 4, FORM_FLOOR>(p, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_FLOOR>(p, requests, max_chunks, stream);
+    return narrow ? launch_scan_tiles<T, 8, 4, FORM_FLOOR>(p, pairs, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_FLOOR>(p, pairs, requests, max_chunks, stream);
   if (p.mode == DECAY_BONUS)
-    return narrow ? launch_scan_tiles<T, 8, 4, FORM_BONUS>(p, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_BONUS>(p, requests, max_chunks, stream);
-  return narrow ? launch_scan_tiles<T, 8, 4, FORM_PLAIN>(p, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_PLAIN>(p, requests, max_chunks, stream);
+    return narrow ? launch_scan_tiles<T, 8, 4, FORM_BONUS>(p, pairs, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_BONUS>(p, pairs, requests, max_chunks, stream);
+  return narrow ? launch_scan_tiles<T, 8, 4, FORM_PLAIN>(p, pairs, requests, max_chunks, stream) : launch_scan_tiles<T, 32, 1, FORM_PLAIN>(p, pairs, requests, max_chunks, stream);
 }
 
 }  // namespace
