@@ -38,22 +38,21 @@ namespace {
 
 // threads of a router block: 32 warps, so that the router's rows are walked by as many warps as the SM holds (a block's time is
 // the latency of its rounds over the outputs: 33 outputs are 2 rounds of 32 warps, 5 of 8)
-// Steps of many tokens: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four products (2,048 tokens of
-// 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so).
+// Steps of many tokens over enough outputs: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four
+// products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so).
 constexpr int ROUTE_THREADS = 1024;
 
 // A block takes ROUTE_TOKENS tokens (8 in steps of many tokens, 1 in steps of few, where blocks are scarce; a token's
-// sums are the same in both): the 32 warps share the router's outputs (warp w takes outputs w, w + 32, ...) and apply every
-// weight they load to all 8 tokens; a lane sums its own elements in ascending order (four neighbours of every 128 where the rows
+// sums are the same in all forms): its warps share the router's outputs (warp w of 32 takes outputs w, w + 32, ...; of 8 to 16 warps four
+// neighbouring outputs at a time) and apply every weight they load to all the block's tokens; a lane sums its own elements in ascending order (four neighbours of every 128 where the rows
 // are multiples of four, else every 32nd), the lanes are added in a fixed order, so a token's
 // scores do not depend on the tokens beside it.  Warp t then takes token t's softmax and choices.
-template <typename T, int ROUTE_TOKENS>
-__global__ void __launch_bounds__(ROUTE_TOKENS > 1 ? 512 : ROUTE_THREADS)
+template <typename T, int ROUTE_TOKENS, int ROUTE_OUTPUTS>
+__global__ void __launch_bounds__(ROUTE_OUTPUTS > 1 ? 512 : ROUTE_THREADS)
 moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ router, const float* __restrict__ correction,
                  int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int tokens, int width,
                  int softmax_outputs, int experts, int top, float scale, int extra, float* __restrict__ extra_out,
                  int group_count, int group_keep, int renormalize, int sigmoid_scores) {
-  constexpr int ROUTE_OUTPUTS = ROUTE_TOKENS > 1 ? 4 : 1;
   extern __shared__ float smem[];
   int outputs = softmax_outputs + extra;              // rows of the router matrix
   float* zs = smem;                                   // ROUTE_TOKENS x outputs: scores
@@ -80,7 +79,7 @@ moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict_
     }
   }
   __syncthreads();
-  if (ROUTE_OUTPUTS > 1 && (width & 3) == 0) {
+  if (ROUTE_OUTPUTS > 1) {
     // a warp takes ROUTE_OUTPUTS neighbouring outputs, so that a token's values are read from shared memory once for all of them
     for (int e0 = warp * ROUTE_OUTPUTS; e0 < outputs; e0 += blockDim.x / 32 * ROUTE_OUTPUTS) {
       const float* w[ROUTE_OUTPUTS];
@@ -656,22 +655,28 @@ SPROUT_API int sprout_moe_route(const void* h, int h_stride, int dtype, const fl
   SPROUT_REQUIRE(smem <= 200 * 1024, "moe_route: too many router outputs (%d) or too wide rows (%d)", outputs, width);
   static bool prepared = false;
   if (!prepared) {
-    cudaFuncSetAttribute(moe_route_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_route_kernel<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<float, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<float, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<float, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     prepared = true;
   }
   dim3 grid((tokens + per_block - 1) / per_block);
-  const int warps = (rows_of_router + 3) / 4;                // with four outputs each; a warp per token at least
-  const dim3 threads(per_block == 1 ? ROUTE_THREADS : 32 * (warps < 8 ? 8 : warps > 16 ? 16 : warps));
-#define ROUTE(T, N)                                                                                                    \
-  sprout_launch(moe_route_kernel<T, N>, grid, threads, smem, stream, (const T*)h, h_stride, router, correction, ids, \
+  // four outputs a warp, a warp per token at least: where their 16-byte weight loads do, from 16 outputs on in bfloat16 and 64 in float32
+  // (1,000 tokens: float32, 18 outputs of 1,024 wide rows 11.0 us with an output a warp, 16.8 us so, 36 of 2,048 26.4 and 28.1; bfloat16, 5 of
+  // 40 4.6 and 5.1, 18 of 1,024 faster so)
+  const bool four = per_block > 1 && width % 4 == 0 && rows_of_router >= (dtype == SPROUT_BF16 ? 16 : 64);
+  const int warps = (rows_of_router + 3) / 4;
+  const dim3 threads(!four ? ROUTE_THREADS : 32 * (warps < 8 ? 8 : warps > 16 ? 16 : warps));
+#define ROUTE(T, N, U)                                                                                                 \
+  sprout_launch(moe_route_kernel<T, N, U>, grid, threads, smem, stream, (const T*)h, h_stride, router, correction, ids, \
                 weights, counts, tokens, width, outputs, experts, top, scale, extra, extra_out, group_count, group_keep, renormalize, sigmoid_scores)
   if (dtype == SPROUT_F32) {
-    if (per_block == 1) ROUTE(float, 1); else ROUTE(float, 8);
+    if (per_block == 1) ROUTE(float, 1, 1); else if (four) ROUTE(float, 8, 4); else ROUTE(float, 8, 1);
   } else if (dtype == SPROUT_BF16) {
-    if (per_block == 1) ROUTE(__nv_bfloat16, 1); else ROUTE(__nv_bfloat16, 8);
+    if (per_block == 1) ROUTE(__nv_bfloat16, 1, 1); else if (four) ROUTE(__nv_bfloat16, 8, 4); else ROUTE(__nv_bfloat16, 8, 1);
   } else {
     return sprout_fail("moe_route: unknown dtype %d", dtype);
   }
