@@ -360,9 +360,12 @@ def attention_simple(q, k_cache, v_cache, block_table, seq_of_token, positions, 
          k_cache.shape[0], _ptr(status, "status", torch.int32), _stream())
 
 
-# float32 attention by tiles of 32 tokens: from this many tokens of one request in the step on (a single token leaves 31 of a
-# tile's 32 rows idle, and the kernel of one block per token and head then has more blocks)
-ATTENTION_TILE_TOKENS = 16
+# float32 attention by tiles of 32 tokens: from this many tokens of one request in the step on (steps of shorter portions leave most of a
+# tile's 32 rows idle, and the kernel of one block per token and head then has more blocks).  Single tokens beside a portion run in
+# tiles of their own (14 heads of 64, 256 tokens beside 32 single ones over 1,000 cached: 128 us, 381 with a block per token and head).
+# A tile costs its 128-key chunk even where a request has fewer: up to ATTENTION_SHORT_CONTEXT keys it pays from ATTENTION_SHORT_ROWS (token,
+# head) rows on (head size 128, 8 heads: 16 tokens 12.7 us against 6.6, 4 x 24 tokens 15.5 and 14.1, 8 x 24 faster by tiles).
+ATTENTION_TILE_TOKENS, ATTENTION_SHORT_CONTEXT, ATTENTION_SHORT_ROWS = 16, 96, 769
 
 
 def attention_tile(q, k_cache, v_cache, block_table, q_start, positions, out, heads, kv_heads, head_dim, longest, status):
@@ -943,7 +946,8 @@ def paged_attention(q, cache, ctx, out, heads, kv_heads, head_dim, status):
                 variant = "mma_sync"
             return attention_prefill(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out,
                                      heads, kv_heads, head_dim, status, variant=variant, max_context=ctx.max_context)
-    elif head_dim in (64, 128) and ctx.max_q_len >= ATTENTION_TILE_TOKENS and cache.k.data_ptr() % 16 == 0 and cache.v.data_ptr() % 16 == 0:
+    elif head_dim in (64, 128) and ctx.max_q_len >= ATTENTION_TILE_TOKENS \
+            and (ctx.max_context > ATTENTION_SHORT_CONTEXT or q.shape[0] * heads >= ATTENTION_SHORT_ROWS) and cache.k.data_ptr() % 16 == 0 and cache.v.data_ptr() % 16 == 0:
         return attention_tile(q, cache.k, cache.v, cache.block_table, ctx.q_start, ctx.positions, out, heads, kv_heads, head_dim,
                               ctx.max_q_len, status)
     attention_simple(q, cache.k, cache.v, cache.block_table, ctx.seq_of_token, ctx.positions, out,
