@@ -1582,6 +1582,11 @@ def _maps_tc_pays(maps: int, dim: int, vdim: int, capped: bool, keys: int, rows6
 
 
 @functools.lru_cache(maxsize=256)
+def _maps_mma_takes(maps: int, dim: int, vdim: int) -> bool:
+    return bool(load_library().sprout_multimap_attention_mma_supported(maps, dim, vdim))
+
+
+@functools.lru_cache(maxsize=256)
 def _maps_tc_takes(maps: int, dim: int, vdim: int, page_tokens: int, out_stride: int) -> bool:
     return bool(_lib.sprout_maps_attention_tc_supported(maps, dim, vdim, page_tokens, out_stride))
 
@@ -1601,7 +1606,7 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
     them the tcgen05 kernel may divide a piece's keys among CTAs."""
     choice = os.environ.get("SPROUT_MULTIMAP_ATTENTION", "auto")
     if q.dtype == torch.bfloat16 and choice != "simple" \
-            and (_lib or load_library()).sprout_multimap_attention_mma_supported(maps, dim, vdim) \
+            and _maps_mma_takes(maps, dim, vdim) \
             and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.stride(0) % 2 == 0:
         global LAUNCHES
         _rows_contiguous(q, "q")
@@ -1691,6 +1696,16 @@ def decay_attention(rows, ctx, state, decay, out, heads: int, dim: int, vdim: in
     decay_scan(rows, ctx.q_start, state.slots, state.buffer, decay, out, heads, dim, vdim, silu, status)
 
 
+@functools.lru_cache(maxsize=4096)
+def _experts_route(entries: int, experts: int, top: int, width: int, ff: int, h_stride: int) -> str:
+    """The kernels that take a step's routed rows of bfloat16: "tcgen05", "mma_sync" or "plain".  Asked once per sizes: a layer of a small step is
+    bound by the host."""
+    lib = load_library()
+    if not lib.sprout_moe_mma_supported(width, ff, h_stride):
+        return "plain"
+    return "tcgen05" if lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
+
+
 def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: int, top: int, limit: float, alpha: float, unit=None,
                 row_weights=None, status=None):
     """The routed experts' two products over the arranged rows (``unit``, ``row_weights``: see ``moe_up_plain``): on tensor cores in bfloat16 when the sizes are
@@ -1698,11 +1713,10 @@ def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: in
     ``status`` word experts of a real layer's size run on tcgen05."""
     global LAUNCHES
     width, ff = h.shape[1], act.shape[1]
-    if h.dtype == torch.bfloat16 and h.stride(1) == 1 and os.environ.get("SPROUT_MOE", "mma") != "plain" \
-            and (_lib or load_library()).sprout_moe_mma_supported(width, ff, h.stride(0)) \
-            and all(t.data_ptr() % 16 == 0 for t in (h, w_gate_up, w_down, act, rows_out)):
-        if status is not None and os.environ.get("SPROUT_MOE", "mma") != "mma_sync" \
-                and _lib.sprout_moe_tc_supported(act.shape[0], experts, top, width, ff, h.stride(0)):
+    choice = os.environ.get("SPROUT_MOE", "mma")
+    route = _experts_route(act.shape[0], experts, top, width, ff, h.stride(0)) if h.dtype == torch.bfloat16 and h.stride(1) == 1 and choice != "plain" else "plain"
+    if route != "plain" and all(t.data_ptr() % 16 == 0 for t in (h, w_gate_up, w_down, act, rows_out)):
+        if route == "tcgen05" and status is not None and choice != "mma_sync":
             gathered = torch.empty((act.shape[0], width), dtype=torch.bfloat16, device=h.device)
             _run("sprout_moe_experts_tc", _ptr(h, "h"), h.stride(0), _ptr(order, "order", torch.int32), _ptr(offsets, "offsets", torch.int32),
                  _ptr(w_gate_up, "w_gate_up", torch.bfloat16), _ptr(w_down, "w_down", torch.bfloat16), _ptr(gathered, "gathered"),

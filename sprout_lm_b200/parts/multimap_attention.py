@@ -183,6 +183,7 @@ class MultiMapAttention(Part):
             self.q_norm, self.k_norm = source.vector(n["q_norm"]), source.vector(n["k_norm"])
         self.qkv = Linear(source.to_device_matrix(fused), bias, status, any_inner_size=True)
         self.out = Linear(source.matrix(n["o"]), None, status, any_inner_size=True)
+        self.counters = source.runtime.workspace(("maps_attention_counters",), (2 * source.runtime.sm_count,), torch.int32)
         if self.maps == 2:
             lq1, lk1, lq2, lk2 = (source.raw(n[key]).to(torch.float32) for key in ("lq1", "lk1", "lq2", "lk2"))
             # one number per layer, in float32 as the other 32-bit quantities
@@ -221,6 +222,6 @@ class MultiMapAttention(Part):
         kernels.multimap_attention(rows[:, :self.q_width], cache, ctx, attended, self.heads, self.kv_heads, self.maps, self.dim,
                                    self.value_dim, self.scale, self.lam, self.norm_eps, self.out_scale, status, mask=self.mask,
                                    sink=self.sink, softcap=self.softcap, turn=self.turn, interleaved=self.interleaved,
-                                   counters=self.runtime.workspace(("maps_attention_counters",), (2 * self.runtime.sm_count,), torch.int32),
+                                   counters=self.counters,
                                    gate=projected[:, self.gate_at:self.gate_at + self.gate_width] if self.has_gate else None)
         self.out.forward(attended, residual=x)
