@@ -1696,14 +1696,19 @@ def decay_attention(rows, ctx, state, decay, out, heads: int, dim: int, vdim: in
     decay_scan(rows, ctx.q_start, state.slots, state.buffer, decay, out, heads, dim, vdim, silu, status)
 
 
+# Elements of an expert's matrix from which its products run on tcgen05 at all: below, many rows do not pay for the gather either (8 experts of
+# 256 over 512, 2,048 rows: 30 us on mma.sync, 34 us on tcgen05; 64 of 512 over 512 71 and 76; 16 of 512 over 1,024 55 and 39)
+EXPERTS_TC_ELEMENTS = 1 << 19
+
+
 @functools.lru_cache(maxsize=4096)
-def _experts_route(entries: int, experts: int, top: int, width: int, ff: int, h_stride: int) -> str:
+def _experts_route(entries: int, experts: int, top: int, width: int, ff: int, h_stride: int, least: int) -> str:
     """The kernels that take a step's routed rows of bfloat16: "tcgen05", "mma_sync" or "plain".  Asked once per sizes: a layer of a small step is
     bound by the host."""
     lib = load_library()
     if not lib.sprout_moe_mma_supported(width, ff, h_stride):
         return "plain"
-    return "tcgen05" if lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
+    return "tcgen05" if width * ff >= least and lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
 
 
 def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: int, top: int, limit: float, alpha: float, unit=None,
@@ -1714,7 +1719,8 @@ def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: in
     global LAUNCHES
     width, ff = h.shape[1], act.shape[1]
     choice = os.environ.get("SPROUT_MOE", "mma")
-    route = _experts_route(act.shape[0], experts, top, width, ff, h.stride(0)) if h.dtype == torch.bfloat16 and h.stride(1) == 1 and choice != "plain" else "plain"
+    route = _experts_route(act.shape[0], experts, top, width, ff, h.stride(0), EXPERTS_TC_ELEMENTS) \
+        if h.dtype == torch.bfloat16 and h.stride(1) == 1 and choice != "plain" else "plain"
     if route != "plain" and all(t.data_ptr() % 16 == 0 for t in (h, w_gate_up, w_down, act, rows_out)):
         if route == "tcgen05" and status is not None and choice != "mma_sync":
             gathered = torch.empty((act.shape[0], width), dtype=torch.bfloat16, device=h.device)
