@@ -1186,11 +1186,16 @@ def latent_attention(qlat, cache, ctx, sink, out, heads: int, rank: int, scale: 
 UNFOLD_TOKENS, UNFOLD_STEP, UNFOLD_ROWS = 128, 512, 16384
 
 
+def latent_unfold_sizes(dtype, dim: int, tail: int, vdim: int, rank: int, rot: int) -> bool:
+    """Whether a layer of these sizes can take the unfolded form in some step: its matrix is kept then only."""
+    return LATENT_ATTENTION == "auto" and dtype == torch.bfloat16 and dim > 0 and dim % 64 == 0 and tail % 64 == 0 \
+        and (dim + tail, vdim) in ((64, 64), (64, 128), (128, 128)) and rank % 8 == 0 and rot % 16 == 0
+
+
 def latent_unfold_rows(ctx, cache, tokens: int, heads: int, dim: int, tail: int, vdim: int, rank: int, rot: int, window: int = 0) -> int:
     """Rows of scratch for the unfolded form of a step's latent attention, 0 where the folded form runs (few new tokens a request, sizes
     that the tcgen05 kernel does not take, more rows than UNFOLD_ROWS)."""
-    if LATENT_ATTENTION != "auto" or cache.k.dtype != torch.bfloat16 or dim <= 0 or dim % 64 or tail % 64 or (dim + tail, vdim) not in ((64, 64), (64, 128), (128, 128)) \
-            or rank % 8 or rot % 16 or tokens < UNFOLD_TOKENS * ctx.num_seqs or tokens < UNFOLD_STEP:
+    if tokens < UNFOLD_STEP or tokens < UNFOLD_TOKENS * ctx.num_seqs or not latent_unfold_sizes(cache.k.dtype, dim, tail, vdim, rank, rot):
         return 0
     keys = cache.block_table.shape[1] * cache.page_tokens
     if window:

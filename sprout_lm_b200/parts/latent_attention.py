@@ -99,16 +99,23 @@ class LatentAttention(Part):
         if self.own_kv:
             self.dkv = linear(n["dkv"])
             self.dkv_gain = source.vector(n["dkv_norm"])
+        self.tables = self.position.rotary_tables(source.runtime) if self.rot_dim else None
         # folded to the query's side: per head W_uk^T [rank, dim]; W_uv stays [value_dim, rank] per head
         uk = source.raw(n["uk"]).reshape(self.heads, self.dim, self.kv_rank).transpose(1, 2)
         self.uk_t = source.to_device_matrix(uk.contiguous()) if self.dim else None
-        self.uv = source.matrix(n["uv"]).reshape(self.heads, self.value_dim, self.kv_rank)
-        # the unfolded form makes every head's key part and values in one product
-        self.unfold = Linear(source.to_device_matrix(torch.cat([source.raw(n["uk"]), source.raw(n["uv"])], dim=0)), None, status, any_inner_size=True) \
-            if self.dim else None
+        # the unfolded form makes every head's key part and values in one product, whose last rows are W_uv: a layer that no step can
+        # unfold keeps W_uv alone
+        self.unfold = None
+        rot = 2 * self.tables[0].shape[1] if self.tables is not None else 0
+        if kernels.latent_unfold_sizes(source.runtime.dtype, self.dim, self.rot_dim, self.value_dim, self.kv_rank, rot):
+            both = source.to_device_matrix(torch.cat([source.raw(n["uk"]), source.raw(n["uv"])], dim=0))
+            self.unfold = Linear(both, None, status)
+            uv = both[self.heads * self.dim:]
+        else:
+            uv = source.matrix(n["uv"])
+        self.uv = uv.reshape(self.heads, self.value_dim, self.kv_rank)
         self.sink = source.vector(n["sink"]) if self.has_sink else None
         self.out = linear(n["o"])
-        self.tables = self.position.rotary_tables(source.runtime) if self.rot_dim else None
         self.interleaved = bool(getattr(self.position, "interleaved", False))
         if self.tables is not None and 2 * self.tables[0].shape[1] > self.rot_dim:
             raise ValueError("latent_attention: the rotation is wider than the rotated part")
