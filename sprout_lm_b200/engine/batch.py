@@ -44,6 +44,7 @@ class StepContext:
     # the longest context that the step's launches should be laid out for: the step's own, or, in a
     # captured graph, that of the steps it is replayed for (0: max_context)
     planned_context: int = 0
+    context_total: int = 0          # the requests' contexts together, as the step was staged (0: not known)
 
     @property
     def all_decode(self) -> bool:
@@ -150,7 +151,7 @@ class BatchStager:
             return v.view(shape) if shape else v
 
         return StepContext(
-            num_tokens=T, num_seqs=R, max_q_len=max(counts), max_context=max(context),
+            num_tokens=T, num_seqs=R, max_q_len=max(counts), max_context=max(context), context_total=sum(context),
             token_ids=view("token_ids"), positions=view("positions"), seq_of_token=view("seq_of_token"),
             q_start=view("q_start"), context_lens=view("context_lens"), state_slots=view("state_slots"),
             logits_rows=view("logits_rows"),

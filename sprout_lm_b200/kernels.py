@@ -1179,11 +1179,14 @@ def latent_attention(qlat, cache, ctx, sink, out, heads: int, rank: int, scale: 
 
 
 # The unfolded form: keys and values of every head are made once per cached row that the step's queries see, and the attention itself
-# multiplies dim + tail + vdim elements a (query, key) pair instead of 2 rank + tail.  Making them pays from some 75 new tokens a
-# request on (2,048 tokens of 16 heads over a latent of 512: 412 us folded with 47 us of products per head, 64 us with 8 us of packing and rotation and 15 us of product unfolded); the
-# rows it is made for are bounded by the block tables' width, and scratch by UNFOLD_ROWS of them.  Steps under UNFOLD_STEP tokens are
-# short on both ways, and the folded one allocates less (128 tokens, launched one by one: 144 against 156 us a layer).
-UNFOLD_TOKENS, UNFOLD_STEP, UNFOLD_ROWS = 128, 512, 16384
+# multiplies dim + tail + vdim elements a (query, key) pair instead of 2 rank + tail (2,048 tokens of 16 heads over a latent of 512: 412 us
+# folded with 47 us of products per head, 64 us with 8 us of packing and rotation and 15 us of product unfolded).  It pays where the pairs'
+# saving is more than UNFOLD_GAIN-th of the rows' product (the product runs on tcgen05 at some six times the rate of the folded scores).
+# The rows are bounded by the block tables' width, so a wide table beside short contexts keeps the folded form (16 heads, four prompts of
+# 128 tokens: 127 us folded; 111 unfolded with tables of 256 positions, 129 with 1,024, 197 with 4,096; one of 512: 162, and 117 to 133 with up to
+# 4,096).  Steps under UNFOLD_STEP tokens are short on both ways, and the folded one allocates less (128 tokens, launched one by one: 144
+# against 156 us a layer).  Scratch is bounded by UNFOLD_ROWS rows and UNFOLD_BYTES.
+UNFOLD_TOKENS, UNFOLD_STEP, UNFOLD_ROWS, UNFOLD_BYTES, UNFOLD_GAIN = 128, 512, 16384, 256 << 20, 6.0
 
 
 def latent_unfold_sizes(dtype, dim: int, tail: int, vdim: int, rank: int, rot: int) -> bool:
@@ -1201,7 +1204,15 @@ def latent_unfold_rows(ctx, cache, tokens: int, heads: int, dim: int, tail: int,
     if window:
         keys = min(keys, window + ctx.max_q_len + 64)
     rows = ctx.num_seqs * keys
-    return rows if rows <= UNFOLD_ROWS else 0
+    if rows > UNFOLD_ROWS or 2 * rows * (heads * (dim + vdim) + rank + tail) > UNFOLD_BYTES:
+        return 0
+    # (query, key) pairs, as far as the host knows the contexts
+    each = tokens / ctx.num_seqs
+    total = getattr(ctx, "context_total", 0) or (ctx.max_context if ctx.num_seqs == 1 else 0)
+    held = total / ctx.num_seqs - each if total else (ctx.max_context - ctx.max_q_len) / ctx.num_seqs
+    seen = held + each / 2
+    pairs = tokens * (min(seen, window) if window else seen)
+    return rows if rows * (dim + vdim) * rank <= UNFOLD_GAIN * pairs * (2 * rank - dim - vdim) else 0
 
 
 def latent_pack(cache, ctx, packed, status, window: int = 0):

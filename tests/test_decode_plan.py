@@ -240,6 +240,28 @@ def test_prompt_attention_of_head_size_128_adds_short_contexts_up_in_registers()
     assert not pick(64, 1, 0)                                                       # a caller that does not know its contexts
 
 
+def test_latent_attention_unfolds_where_the_rows_pay():
+    """The unfolded form is made for every row that the block tables could hold: long prompts and contexts take it, a few tokens beside wide tables, a
+    scratch beyond its bound and sizes that no kernel takes do not."""
+    import torch
+    from types import SimpleNamespace
+
+    def rows(new, held, pages, rank=512, heads=16, dim=64, tail=64, vdim=128, window=0, total=True):
+        context = [h + n for h, n in zip(held, new)]
+        ctx = SimpleNamespace(num_seqs=len(new), max_q_len=max(new), max_context=max(context), context_total=sum(context) if total else 0)
+        cache = SimpleNamespace(k=torch.empty(0, dtype=torch.bfloat16), block_table=torch.empty(len(new), pages), page_tokens=16)
+        return kernels.latent_unfold_rows(ctx, cache, sum(new), heads, dim, tail, vdim, rank, tail, window)
+    assert rows([2048], [0], 128) == 2048 and rows([512], [0], 256) == 4096
+    assert rows([512], [0], 1024) == 0                                   # 16,384 rows for 512 tokens' scores
+    assert rows([512], [3000], 256) == 4096 and rows([512], [3000], 256, total=False) == 4096
+    assert rows([128] * 4, [0] * 4, 16) == 1024 and rows([128] * 4, [0] * 4, 64) == 0
+    assert rows([128] * 4, [3000, 0, 0, 0], 256) == 16384                # one long context: its scores outweigh the rows
+    assert rows([2048], [0], 128, heads=128) == 2048 and rows([2048], [0], 512, heads=128) == 0        # 0.4 GB of scratch
+    assert rows([2048], [0], 128, rank=96) == 0                          # a narrow latent: the folded form multiplies no more
+    assert rows([2048], [0], 128, window=256) == 2048 and rows([256], [0], 16) == 0 and rows([2048], [0], 128, dim=128) == 0
+    assert kernels.latent_unfold_sizes(torch.bfloat16, 64, 64, 128, 512, 64) and not kernels.latent_unfold_sizes(torch.float32, 64, 64, 128, 512, 64)
+
+
 def test_small_batch_kernels_say_what_they_take():
     """The small-batch kernels' size rules are host arithmetic in the kernel library: up to 16 tokens,
     sizes in steps of 16, and a layer small enough for the SMs' shared memory.  What they refuse

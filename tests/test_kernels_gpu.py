@@ -1243,6 +1243,7 @@ def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, 
     h = torch.randn(T, width, generator=g).to(torch.bfloat16).to(DEV)
     results = []
     monkeypatch.setattr(kernels, "UNFOLD_STEP", 128)
+    monkeypatch.setattr(kernels, "UNFOLD_GAIN", 1e9)                 # the form under test, whether it pays at these sizes or not
     for rows in (kernels.UNFOLD_ROWS, 0):
         monkeypatch.setattr(kernels, "UNFOLD_ROWS", rows)
         view = CacheView(cache.to(torch.bfloat16).to(DEV), None, ctx.block_tables[0], page, True)
