@@ -16,7 +16,7 @@
 // S of tile j + 2 goes over the columns of P of tile j: one thread issues all products, and the tensor cores take them in order.
 //
 // What bounds it: the exponentials (16 an SM and cycle: 1,024 cycles for a pair of tiles, beside 900 to 1,280 of products).
-// Measured, prompts of 2,048 tokens, 16 heads, two maps of 64 with values of 128: 167 us on mma.sync, 80 us here; layers: this one 297 and
+// Measured, prompts of 2,048 tokens, 16 heads, two maps of 64 with values of 128: 167 us on mma.sync, 64 us here; layers: this one 297 and
 // 144 us, one map with a window of 1,024, five prompts of 4,001 tokens together, 319 and 183 us.
 //
 // A piece (the CTA's rows) with many key tiles may be divided among `shares` CTAs, each taking every shares-th tile: partial sums
@@ -122,8 +122,8 @@ __device__ __forceinline__ void named_barrier(int id, int threads) { asm volatil
 // Among how many CTAs a piece's key tiles go when the launch has `pieces` of them, a request's last piece `last` tiles and its first
 // `first`.  As many as leave every CTA an SM; two where all pieces have one but lengths differ so much that the longest would run
 // alone for long (a CTA takes some 9 us and 1.2 us a tile, 4 us more when it is divided, and a second round of CTAs starts late).
-// Head size 128, 512 queries over 900 cached tokens, 64 heads over 8 (128 pieces of 15 to 23 tiles): undivided 41 us, two shares, which two
-// rounds of CTAs take, 61 us; 4,096 tokens, 8 heads over 1 (128 pieces of 1 to 64 tiles): 91 and 71 us (all while O lagged behind the maximum).
+// Head size 128, 512 queries over 900 cached tokens, 64 heads over 8 (128 pieces of 15 to 23 tiles): undivided 46 us, two shares, which two
+// rounds of CTAs take, about 65; 4,096 tokens, 8 heads over 1 (128 pieces of 1 to 64 tiles): about 97 and 77 us.
 __device__ __forceinline__ int shares_of(int pieces, int last, int first, int sms) {
   if (pieces > sms) return 1;
   if (2 * pieces <= sms) return sms / pieces;
@@ -696,8 +696,9 @@ SPROUT_API int sprout_maps_attention_tc_supported(int maps, int dim, int vdim, i
   return tc_sizes(maps, dim, vdim) && pages_ok && out_stride % 8 == 0;
 }
 
-// How many CTAs a piece's key tiles are divided among at most in a launch of these sizes (the kernel knows the pieces exactly), and the floats of scratch and the counters
-// that takes (scratch: none for one share).
+// How many CTAs a piece's key tiles are divided among at most in a launch of these sizes (the kernel knows the pieces exactly), and the
+// floats of scratch that takes (none for one share).  A launch that divides has at most as many pieces as there are SMs, and two
+// counters a piece.
 SPROUT_API int sprout_maps_attention_tc_shares(int tokens, int requests, int heads, int kv_heads, int maps) {
   const long long pieces = pieces_bound(tokens, requests, heads, kv_heads, maps);
   const long long want = 2LL * sm_count() / (pieces > 0 ? pieces : 1);
@@ -707,12 +708,9 @@ SPROUT_API long long sprout_maps_attention_tc_scratch_floats(int tokens, int req
   const int shares = sprout_maps_attention_tc_shares(tokens, requests, heads, kv_heads, maps);
   return shares == 1 ? 0 : pieces_bound(tokens, requests, heads, kv_heads, maps) * shares * 2 * ROWS * (vdim + 4);
 }
-SPROUT_API long long sprout_maps_attention_tc_counters(int tokens, int requests, int heads, int kv_heads, int maps) {
-  return 2 * pieces_bound(tokens, requests, heads, kv_heads, maps);
-}
 
-// The arguments of sprout_multimap_attention_mma, checked there.  `scratch` and `counters` (zeroed) hold what the functions above
-// say, or are null: then no piece is divided.
+// The arguments of sprout_multimap_attention_mma, checked there.  `scratch` holds what the function above says, `counters` (zeroed) two
+// numbers an SM, or they are null: then no piece is divided.
 int sprout_maps_attention_tc(const MultiMapParams& m, int tokens, int maps, int dim, int vdim, float* scratch, int* counters, cudaStream_t stream) {
   SPROUT_REQUIRE(sprout_maps_attention_tc_supported(maps, dim, vdim, m.page_tokens, m.out_stride) && ((uintptr_t)m.out & 15) == 0,
                  "maps_attention (tcgen05): %d maps of %d with values of %d, page size %d or the output's alignment is not taken", maps, dim, vdim, m.page_tokens);

@@ -725,10 +725,10 @@ gated_group_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate
 // (32 / LANES of them, LANES = part / VEC rounded up to a power of two), VEC elements a lane in 16-byte accesses, the part in registers
 // between its sum and its scaling, no block-wide barrier.  Bound by memory: 2,500 rows of 16 parts of 128: 45 us as a block of 128
 // threads per part, 19 us so.
-template <typename TG, typename T, int VEC>
+template <typename TG, int VEC>
 __global__ void __launch_bounds__(256)
 gated_group_norm_warp_kernel(const float* __restrict__ o, const TG* __restrict__ gate, int gate_stride, const float* __restrict__ weight,
-                             int period, T* __restrict__ out, int width, int groups, int lanes, long long parts, float eps, int gate_first, int act) {
+                             int period, __nv_bfloat16* __restrict__ out, int width, int groups, int lanes, long long parts, float eps, int gate_first, int act) {
   pdl_launch_dependents();
   pdl_wait();
   const int part = width / groups, lane = threadIdx.x & (lanes - 1);
@@ -776,7 +776,7 @@ gated_group_norm_warp_kernel(const float* __restrict__ o, const TG* __restrict__
   for (int d = lanes >> 1; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
   if (!active) return;
   const float r = 1.0f / sqrtf(q / (float)part + eps);
-  T* dst = out + (size_t)row * width + base;
+  __nv_bfloat16* dst = out + (size_t)row * width + base;
 #pragma unroll
   for (int i = 0; i < VEC; i += 4) {
     float y[4];
@@ -785,12 +785,8 @@ gated_group_norm_warp_kernel(const float* __restrict__ o, const TG* __restrict__
       const float w = weight[(base + i + e) % period];
       y[e] = gate_first ? v[i + e] * r * w : v[i + e] * r * w * factor[i + e];
     }
-    if (sizeof(T) == 4) {
-      *(float4*)((float*)dst + i) = make_float4(y[0], y[1], y[2], y[3]);
-    } else {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
-      *(uint2*)((__nv_bfloat16*)dst + i) = make_uint2(*(uint32_t*)&lo, *(uint32_t*)&hi);
-    }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
+    *(uint2*)(dst + i) = make_uint2(*(uint32_t*)&lo, *(uint32_t*)&hi);
   }
 }
 
@@ -802,7 +798,7 @@ int launch_group_norm(const float* o, const void* gate, int gate_stride, const f
                        ((uintptr_t)gate & 15) == 0;
   // the 32-bit path keeps one order of additions for all its calls: the block kernel's.  Below 1,024 parts either kernel is one short wave
   // and the block kernel's is shorter (256 parts of 256: 2.95 against 3.37 us; 512 of 64: 2.36 and 2.45; 1,024 of 128: 2.87 and 2.52).
-  if (sizeof(T) == 2 && aligned && (long long)rows * groups >= 1024) {
+  if constexpr (sizeof(T) == 2) if (aligned && (long long)rows * groups >= 1024) {
     const int vec = part > 128 ? 8 : 4;
     int lanes = 1;
     while (lanes * vec < part) lanes <<= 1;
@@ -810,10 +806,10 @@ int launch_group_norm(const float* o, const void* gate, int gate_stride, const f
       const long long parts = (long long)rows * groups, blocks = (parts * lanes + 255) / 256;
       SPROUT_REQUIRE(blocks <= 0x7fffffffLL, "gated_group_norm: too many rows");
       if (vec == 8)
-        sprout_launch(gated_group_norm_warp_kernel<TG, T, 8>, dim3((unsigned)blocks), dim3(256), 0, stream, o, (const TG*)gate, gate_stride, weight,
+        sprout_launch(gated_group_norm_warp_kernel<TG, 8>, dim3((unsigned)blocks), dim3(256), 0, stream, o, (const TG*)gate, gate_stride, weight,
                       period, (T*)out, width, groups, lanes, parts, eps, gate_first, act);
       else
-        sprout_launch(gated_group_norm_warp_kernel<TG, T, 4>, dim3((unsigned)blocks), dim3(256), 0, stream, o, (const TG*)gate, gate_stride, weight,
+        sprout_launch(gated_group_norm_warp_kernel<TG, 4>, dim3((unsigned)blocks), dim3(256), 0, stream, o, (const TG*)gate, gate_stride, weight,
                       period, (T*)out, width, groups, lanes, parts, eps, gate_first, act);
       return sprout_check_launch("gated_group_norm");
     }

@@ -1258,7 +1258,11 @@ def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, 
 
 @pytest.mark.parametrize("rows,part,groups,period,gate_dtype,gate_first,silu", [
     (1, 4, 1, 4, None, False, True), (7, 64, 6, 64, torch.float32, True, True), (33, 100, 3, 300, torch.bfloat16, False, False),
-    (5, 128, 9, 128, torch.bfloat16, True, False), (3, 136, 5, 680, torch.float32, False, True), (70, 256, 2, 256, torch.bfloat16, False, True)])
+    (5, 128, 9, 128, torch.bfloat16, True, False), (3, 136, 5, 680, torch.float32, False, True), (70, 256, 2, 256, torch.bfloat16, False, True),
+    # from 1,024 parts on a group of lanes has a part, below a block
+    (1023, 4, 1, 4, None, False, True), (1025, 4, 1, 4, None, False, True), (171, 64, 6, 64, torch.float32, True, True),
+    (343, 100, 3, 300, torch.bfloat16, False, False), (114, 128, 9, 128, torch.bfloat16, True, False), (205, 136, 5, 680, torch.float32, False, True),
+    (513, 256, 2, 256, torch.bfloat16, False, True)])
 def test_gated_group_norm_lanes(rows, part, groups, period, gate_dtype, gate_first, silu):
     """A part per group of lanes: the smallest and largest parts, lanes without elements, a last warp that is not full, every kind of gate."""
     from sprout_lm_b200 import kernels
