@@ -1180,7 +1180,7 @@ def latent_attention(qlat, cache, ctx, sink, out, heads: int, rank: int, scale: 
 
 # The unfolded form: keys and values of every head are made once per cached row that the step's queries see, and the attention itself
 # multiplies dim + tail + vdim elements a (query, key) pair instead of 2 rank + tail (2,048 tokens of 16 heads over a latent of 512: 412 us
-# folded with 47 us of products per head, 64 us with 8 us of packing and rotation and 15 us of product unfolded).  It pays where the pairs'
+# folded with 47 us of products per head, 72 us with 8 us of packing and rotation and 15 us of product unfolded).  It pays where the pairs'
 # saving is more than UNFOLD_GAIN-th of the rows' product (the product runs on tcgen05 at some six times the rate of the folded scores).
 # The rows are bounded by the block tables' width, so a wide table beside short contexts keeps the folded form (16 heads, four prompts of
 # 128 tokens: 127 us folded; 111 unfolded with tables of 256 positions, 129 with 1,024, 197 with 4,096; one of 512: 162, and 117 to 133 with up to
@@ -1581,8 +1581,8 @@ def visible_keys(mask, context: int) -> int:
 # (token, head) rows of a step from which prompt attention with one or two maps runs on tcgen05: below, a layer's launches take the host
 # longer than the device either way, and the mma.sync kernel needs no scratch (60 tokens of 8 heads: 77 against 81 us a layer).
 # From as many 64-key tiles on as a query of the step sees at most, by (maps, key size, value size, capped scores): a CTA of the tcgen05
-# kernel takes 7 to 13 us before its first and after its last tile, one of the mma.sync kernel 3 to 5, but 1.1 to 1.3 us a tile (2.7 to
-# 3.2 where scores are capped) against 1.7 to 3.4; the numbers are for steps of few tiles of 64 rows (the mma.sync kernel's CTAs), of 1.25
+# kernel takes 6 to 13 us before its first and after its last tile, one of the mma.sync kernel 3 to 5, but 1.3 to 1.6 us a tile (2.9 to
+# 3.6 where scores are capped) against 1.7 to 3.4; the numbers are for steps of few tiles of 64 rows (the mma.sync kernel's CTAs), of 1.25
 # an SM and of 2 an SM on, where those come in rounds.  (One map of 128, 16 heads over 4, one prompt: 256 tokens 13.5 us on mma.sync,
 # 18.4 on tcgen05; 777 tokens 38.8 and 27.9; two maps of 64: 128 tokens 11.2 and 14.1, 256 tokens 18.0 and 17.0.)
 MAPS_TC_ROWS = 2048
