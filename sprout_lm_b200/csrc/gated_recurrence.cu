@@ -127,8 +127,8 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // float32 vectors in shared memory ([q_scale q | c k | a] per row).  The slices of a column add their parts of o with
 // shuffles.  The bfloat16 path's walks over chunks of key sizes 64, 128 and 256, whose rows fill the slices (PAIRS), go two rows at a
 // time in packed arithmetic: a thread's rows are then neighbours, fetched 16 bytes at a time, and q, c k and a lie in planes of their
-// own, so that a 16-byte read is two pairs of one of them (2,500 tokens of 16 heads of 128 x 128: 154 and 362 us for the two walks with
-// a number at a time, (q, c k, a) triples and 2-byte fetches, 106 and 237 us so).  Other sizes and rows off 16-byte boundaries keep a
+// own, so that a 16-byte read is two pairs of one of them (2,048 tokens of 16 heads of 128 x 128, with the decays and the carry: 443 us
+// with a number at a time, (q, c k, a) triples and 2-byte fetches, 296 us so).  Other sizes and rows off 16-byte boundaries keep a
 // number at a time: pairs without the wide fetches cost 12 % (four heads of 96 x 96), and with two slices or one, 4 % (8 x 512, 16 x 64).
 // Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order.  An output's sum over the rows has one order in
 // the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn, so a bfloat16 request of one
