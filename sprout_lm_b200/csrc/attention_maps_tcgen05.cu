@@ -103,12 +103,6 @@ __device__ __forceinline__ void umma_bf16_from_tmem_words(uint32_t d_tmem, uint3
       " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
 }
-// One lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t yes;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(yes));
-  return yes != 0;
-}
 __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"

@@ -147,7 +147,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // and positions, the block table) was written before the step's first kernel; the queries and
   // the newest keys and values are read after the wait, below.
   pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const bool paired = SPLIT && (int)blockIdx.x < 2 * p.split_pieces;      // one of the two CTAs of a piece
   const int piece_index = !SPLIT ? (int)blockIdx.x : paired ? (int)blockIdx.x >> 1 : (int)blockIdx.x - p.split_pieces;
   const int rank = paired ? blockIdx.x & 1 : 0;
@@ -258,7 +258,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             tma_load_2d(sV + s * L::KV_BYTES + kb * L::KV_ATOM_BYTES + lane * p.box_rows * 128, &map_v, &v_full[s], kb * 64, row_at);
         v_issued = j + 1;
       }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
       // ---------------- MMA issuer.  Order: S0(0) S1(0), then for every key tile
       //   [P0(j)] P0 V(j), S0(j+1), [P1(j)] P1 V(j), S1(j+1)
       // so that the products of one Q tile run under the softmax of the other.  S of a Q tile has

@@ -21,6 +21,12 @@
 // Groups of output features may read columns of their own of A (several matrices over several inputs in one launch): A is then
 // [M, groups * K], and the features of group g multiply A's columns [g K, (g + 1) K).
 //
+// What bounds the products with tokens on M: the tensor cores and the operands' way from L2 (256 x 256 tiles of CTA pairs), and in
+// small ones the way in and out of a CTA's one tile.  The epilogue must be through a tile before the next one's products are: stored a
+// row a lane, it took longer than they did.  2,048 x 9,728 x 896 with SwiGLU: 43.4 us so, 26.7 through the warps' shared memory (1,340
+// TFLOP/s; 139 and 93.7 us at 8,192 tokens); 2,048 x 2,048 x 2,048 19.6 and 16.1; 2,048 x 896 x 4,864 added to the residual, whose warps
+// no longer meet for every 32 columns, 20.1 and 16.1.  The issuing threads' part in that: see elect_one.
+//
 // Every wait on an mbarrier is bounded; a wait that runs out sets SPROUT_STATUS_WAIT_TIMEOUT,
 // the CTA stops issuing, waits (bounded) for its copies in flight, frees its TMEM and returns.
 #include <cuda.h>
@@ -35,10 +41,12 @@ namespace {
 constexpr int BLOCK_M = 128;        // rows of D per CTA == TMEM lanes
 constexpr int BLOCK_K = 64;         // bf16 elements per stage row: 128 bytes, one swizzle row
 constexpr int NUM_THREADS = 320;      // TMA warp, MMA warp, 8 epilogue warps
-constexpr int SMEM_BUDGET = 196 * 1024;    // for the operand stages; the staging tiles and barriers come on top
+constexpr int SMEM_BUDGET = 193 * 1024;    // for the operand stages; the staging tiles and barriers come on top
 
 enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RESIDUAL_ATOMIC = 2, EPI_SWIGLU = 3, EPI_RESIDUAL_TMA = 4, EPI_EXPERT_GLU = 5, EPI_EXPERT_GELU = 6 };
-constexpr int STAGING_BYTES = 2 * 128 * 128;    // two [128 rows, 32 float32] tiles for the TMA reduction of the residual epilogue
+constexpr int SLOT_BYTES = 32 * 128;            // an epilogue warp's 32 rows of 128 bytes on their way to memory
+constexpr int STAGING_BYTES = 8 * SLOT_BYTES;
+constexpr int MAX_EXPERTS = 2048;
 
 // SwiGLU epilogue: the weight rows interleave gate and up in blocks of 8 (rows 16b..16b+7 gate,
 // 16b+8..16b+15 up), so output feature 8b+j is silu(D[.., 16b+j]) * D[.., 16b+8+j]; the output
@@ -80,16 +88,18 @@ template <bool GROUPED> struct ParamsOf { using type = Params; };
 template <> struct ParamsOf<true> { using type = GroupedParams; };
 
 // PAIR: two CTAs share a 256 x BN tile; each holds its own 128 rows of A and half of B's rows.
-template <int BN, bool PAIR = false>
+// GROUPED: a table of the experts' tiles and rows takes a stage's room.
+template <int BN, bool PAIR = false, bool GROUPED = false>
 struct Layout {
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BLOCK_K * 2;
   static constexpr int B_PADDED = (B_BYTES + 1023) / 1024 * 1024;
   static constexpr int STAGE_BYTES = A_BYTES + B_PADDED;
-  static constexpr int STAGES = (SMEM_BUDGET / STAGE_BYTES) > 12 ? 12 : (SMEM_BUDGET / STAGE_BYTES);
+  static constexpr int TABLE_BYTES = GROUPED ? (2 * (MAX_EXPERTS + 1) * 4 + 15) / 16 * 16 : 0;
+  static constexpr int STAGES = ((SMEM_BUDGET - TABLE_BYTES) / STAGE_BYTES) > 12 ? 12 : ((SMEM_BUDGET - TABLE_BYTES) / STAGE_BYTES);
   // two accumulators; allocations are powers of two from 32 columns
   static constexpr int TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + TABLE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
 // One unit of work: a 128 x BN tile of D over a range of K blocks.
@@ -122,7 +132,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
                     const __grid_constant__ CUtensorMap map_out, const typename ParamsOf<GROUPED>::type p) {
   static_assert(!(PAIR && SWAP), "pairs work on token tiles");
   static_assert(!GROUPED || PAIR, "experts' products run in pairs");
-  using L = Layout<BN, PAIR>;
+  using L = Layout<BN, PAIR, GROUPED>;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0;                       // 0 issues the MMAs
   const int first_work = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;     // this CTA's (pair's) first item and stride
   const int work_stride = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
@@ -130,7 +140,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* staging = smem + L::STAGES * L::STAGE_BYTES;
-  uint64_t* full_bar = (uint64_t*)(staging + STAGING_BYTES);
+  uint64_t* full_bar = (uint64_t*)(staging + STAGING_BYTES + L::TABLE_BYTES);
   uint64_t* empty_bar = full_bar + L::STAGES;
   uint64_t* acc_full = empty_bar + L::STAGES;     // [2] accumulator complete (MMA -> epilogue)
   uint64_t* acc_empty = acc_full + 2;             // [2] accumulator read out (epilogue -> MMA)
@@ -138,13 +148,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   uint32_t* tmem_slot = (uint32_t*)(epi_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int total_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
   const int row_tiles = ((SWAP ? p.N : p.M) + TILE_M - 1) / TILE_M;
   const int col_tiles = ((SWAP ? p.M : p.N) + BN - 1) / BN;
   const int splits = (total_kb + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
-  // experts' products: 256-row tiles before expert e, and its first row, in the room that the residual epilogue's tiles would have
-  int* tile_prefix = (int*)staging;
+  // experts' products: 256-row tiles before expert e, and its first row
+  int* tile_prefix = (int*)(staging + STAGING_BYTES);
   int* row_prefix = nullptr;
   const bool glu_tiles = GROUPED && p.epilogue == EPI_EXPERT_GLU;
   int expert_cols = 0;                                 // tiles across an expert's outputs
@@ -236,7 +246,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   // the abort flag only while a wait is not satisfied at once.
   const uint32_t smem_base = smem_u32(smem), full_base = smem_u32(full_bar), empty_base = smem_u32(empty_bar);
   int issued = 0;
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---------------- producer: TMA loads of the two operand tiles, stage by stage.
     // The weights were written before any kernel of the step ran: their tiles for the first
     // round of stages are requested before waiting for the kernel that produces the activations.
@@ -285,7 +295,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         if (++s == L::STAGES) { s = 0; parity ^= 1; stage_addr = smem_base; } else stage_addr += L::STAGE_BYTES;
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
+  } else if (warp == 1 && rank == 0 && elect_one()) {
     // ---------------- MMA issuer (of a pair: the first CTA's)
     const uint32_t idesc = umma_idesc(TILE_M, BN);
     const uint64_t a_desc0 = umma_smem_desc(smem), b_desc0 = umma_smem_desc(smem + L::A_BYTES);
@@ -332,10 +342,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     // ---------------- epilogue: TMEM -> registers -> global
     pdl_wait();                         // the epilogue reads and writes `out`
     const int quarter = warp & 3;       // a warp reads TMEM lanes 32 * (warp % 4) ..
-    const int half = (warp - 2) >> 2;   // two warps per lane quarter take alternate 16-column chunks
+    const int half = (warp - 2) >> 2;   // two warps per lane quarter take alternate groups of columns
     int tiles_done = 0;
-    uint32_t groups_done = 0, epi_phase = 0;
-    const bool issuer = warp == 2 && lane == 0;   // issues the reductions of the residual epilogue
+    uint32_t epi_phase = 0;
+    const bool issuer = warp == 2 && lane == 0;
+    uint8_t* slot = staging + (warp - 2) * SLOT_BYTES;
     // all 8 warps meet; false when the wait ran out
     auto epi_sync = [&]() {
       bool met = true;
@@ -408,54 +419,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       const bool first_split = k.split == 0;
-      if (!SWAP && p.epilogue == EPI_RESIDUAL_TMA) {
-        // out += D through shared memory: the 8 warps fill a [128 rows, 32 columns] float32 tile
-        // in the swizzled layout of the output's tensor map, one thread hands it to the TMA unit,
-        // which adds it to the output in L2 (rows and columns beyond the matrix are clipped).
-        // Two tiles alternate; a tile is written again once the reduction before last has read it.
-        const int tile_row = quarter * 32 + lane;
-        bool met = true;
-#pragma unroll 1
-        for (int c = half * 16; c < BN && met; c += 32, groups_done++) {
-          uint32_t raw[16];
-          tmem_load16(taddr + c, raw);
-          const int n_base = col0 + c;
-          uint8_t* tile = staging + (groups_done & 1) * (STAGING_BYTES / 2);
-          if (groups_done >= 2) {
-            if (issuer) bulk_wait_group_read<1>();
-            met = epi_sync();
-            if (!met) break;
-          }
-#pragma unroll
-          for (int q4 = 0; q4 < 4; q4++) {
-            float4 v;
-            const bool biased = p.bias && first_split;     // the K splits of a tile all add into the output: one brings the bias
-            v.x = __uint_as_float(raw[4 * q4]) + ((biased && n_base + 4 * q4 < p.N) ? p.bias[n_base + 4 * q4] : 0.f);
-            v.y = __uint_as_float(raw[4 * q4 + 1]) + ((biased && n_base + 4 * q4 + 1 < p.N) ? p.bias[n_base + 4 * q4 + 1] : 0.f);
-            v.z = __uint_as_float(raw[4 * q4 + 2]) + ((biased && n_base + 4 * q4 + 2 < p.N) ? p.bias[n_base + 4 * q4 + 2] : 0.f);
-            v.w = __uint_as_float(raw[4 * q4 + 3]) + ((biased && n_base + 4 * q4 + 3 < p.N) ? p.bias[n_base + 4 * q4 + 3] : 0.f);
-            const int chunk = half * 4 + q4;
-            *(float4*)(tile + tile_row * 128 + ((chunk ^ (tile_row & 7)) << 4)) = v;
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          met = epi_sync();
-          if (!met) break;
-          if (issuer) {
-            tma_reduce_add_2d(&map_out, smem_u32(tile), col0 + (c & ~31), k.row0);
-            bulk_commit_group();
-          }
-        }
-        if (!met) break;
+      // once a warp has read its part of the accumulator out, the MMA issuer may have it back
+      auto hand_back = [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) release_accumulator(acc);
-        continue;
-      }
+      };
+      if constexpr (SWAP) {
 #pragma unroll 1
-      for (int c = half * 16; c < (glu_tiles ? BN / 2 : BN); c += 32) {
-        uint32_t raw[16];
-        tmem_load16(taddr + c, raw);
-        if (SWAP) {
+        for (int c = half * 16; c < BN; c += 32) {
+          uint32_t raw[16];
+          tmem_load16(taddr + c, raw);
           // row = output feature, columns = tokens: lanes hold consecutive features
           if (p.epilogue == EPI_SWIGLU) {
             // lanes l and l ^ 8 hold a gate row and its up row (128-row tiles start on multiples of 16)
@@ -482,107 +456,156 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
               else ((__nv_bfloat16*)p.out)[at] = __float2bfloat16_rn(v);
             }
           }
-        } else {
-          // row = token, columns = output features: each lane writes a contiguous run of its row
-          int row_end = p.M;
-          if constexpr (GROUPED) {
-            row_end = k.row_end;
-            if (p.epilogue != EPI_STORE) {
-              const int n_base = col0 + c;
-              float v[16];
-              uint32_t up[16];
-              if (p.epilogue == EPI_EXPERT_GLU) tmem_load16(taddr + BN / 2 + c, up);      // warp-wide: also lanes without a row
-              if (row < k.row_end && n_base < p.N) {
-                const float weight = p.row_weights ? p.row_weights[p.order[row]] : 1.0f;
+        }
+        hand_back();
+      } else {
+        // Row = token, columns = output features.  A lane has a row: stored by the lane, its 16-byte pieces of 32 rows would be 32
+        // accesses to memory an instruction (a 128 x 256 tile of bfloat16: 15,000 cycles, twice its products at K = 896).  They go
+        // through the warp's own 4 KB of shared memory (16-byte chunk c of row r at chunk c ^ (r & 7)) and leave as rows of 128
+        // bytes, four an instruction, or as one addition by the TMA unit; no warp waits for another.
+        const int warp_row = k.row0 + quarter * 32;              // the warp's first row
+        const bool biased = p.bias != nullptr && first_split;    // the K splits of a tile all add into the output: one brings the bias
+        auto put = [&](int chunk, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+          *(uint4*)(slot + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = make_uint4(a, b, c, d);
+        };
+        auto pack = [](float lo, float hi) {
+          __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+          return *(uint32_t*)&h;
+        };
+        // 32 columns of the accumulator from c on, with their bias
+        auto load = [&](int c, uint32_t (&raw)[32]) {
+          tmem_load32(taddr + c, raw);
+          if (biased) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
+            for (int j = 0; j < 32; j++) {
+              const int n = col0 + c + j;
+              raw[j] = __float_as_uint(__uint_as_float(raw[j]) + (n < p.N ? p.bias[n] : 0.f));
+            }
+          }
+        };
+        if (p.epilogue == EPI_RESIDUAL_TMA) {
+          // out += D: the TMA unit adds [32 rows, 32 columns] of float32 to the output in L2 (rows and columns beyond the
+          // matrix are clipped)
+#pragma unroll 1
+          for (int c = half * 32; c < BN; c += 64) {
+            uint32_t raw[32];
+            load(c, raw);
+            if (c + 64 >= BN) hand_back();
+            if (lane == 0) bulk_wait_group_read<0>();            // the addition before has read the slot
+            __syncwarp();
+#pragma unroll
+            for (int q4 = 0; q4 < 8; q4++) put(q4, raw[4 * q4], raw[4 * q4 + 1], raw[4 * q4 + 2], raw[4 * q4 + 3]);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+              tma_reduce_add_2d(&map_out, smem_u32(slot), col0 + c, warp_row);
+              bulk_commit_group();
+            }
+          }
+          if (half * 32 >= BN) hand_back();
+          continue;
+        }
+        const bool gated = p.epilogue == EPI_SWIGLU;
+        int row_end = p.M, out_cols = gated ? p.N >> 1 : p.N;
+        float weight = 1.0f;
+        if constexpr (GROUPED) {
+          row_end = k.row_end;
+          if (p.row_weights && row < row_end) weight = p.row_weights[p.order[row]];
+        }
+        // columns of the accumulator that a round takes (a gate's up columns beside them): 128 bytes of output, or 64 where the two
+        // warps of a quarter would not both have a round
+        const int step = gated ? (BN >= 256 ? 128 : 64) : p.out_is_f32 ? 32 : 64;
+        const int elem_log2 = p.out_is_f32 ? 2 : 1, per16 = 16 >> elem_log2;
+        const int end = glu_tiles ? BN / 2 : BN;
+        uint8_t* const out = (uint8_t*)p.out;
+        const bool wide = (((uintptr_t)p.out | ((size_t)p.ldo << elem_log2)) & 15) == 0;
+#pragma unroll 1
+        for (int c = half * step; c < end; c += 2 * step) {
+          const int stop = min(c + step, end);
+#pragma unroll 1
+          for (int at = c; at < stop; at += 32) {
+            uint32_t raw[32];
+            if constexpr (GROUPED) {
+              if (p.epilogue != EPI_STORE) {
+                uint32_t up[32];
+                tmem_load32(taddr + at, raw);
+                if (p.epilogue == EPI_EXPERT_GLU) tmem_load32(taddr + BN / 2 + at, up);
+                if (at + 32 >= stop && c + 2 * step >= end) hand_back();
+                float v[32];
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
                   // rounded to bfloat16 before the activation, as separate products would leave them
                   const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j]) * weight));
                   const float u = p.epilogue == EPI_EXPERT_GLU ? __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j]) * weight)) : 0.f;
                   v[j] = sprout_experts::glu(p.unit, g, u, p.limit, p.alpha);
                 }
-                __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + n_base;    // N and ldo are multiples of 8
 #pragma unroll
-                for (int j = 0; j < 16; j += 8) {
-                  if (n_base + j >= p.N) break;
-                  uint32_t packed[4];
-#pragma unroll
-                  for (int i = 0; i < 4; i++) {
-                    __nv_bfloat162 h = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
-                    packed[i] = *(uint32_t*)&h;
-                  }
-                  *(uint4*)(o + j) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                }
+                for (int q4 = 0; q4 < 4; q4++)
+                  put((at - c) / 8 + q4, pack(v[8 * q4], v[8 * q4 + 1]), pack(v[8 * q4 + 2], v[8 * q4 + 3]), pack(v[8 * q4 + 4], v[8 * q4 + 5]),
+                      pack(v[8 * q4 + 6], v[8 * q4 + 7]));
+                continue;
               }
-              continue;
             }
-          }
-          if (row < row_end) {
-            const int n_base = col0 + c;
-            float v[16];
+            load(at, raw);
+            if (at + 32 >= stop && c + 2 * step >= end) hand_back();
+            if (gated) {
+              // columns 16 b .. 16 b + 7 are gates, the next eight the up columns that go with them
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] = __uint_as_float(raw[j]) + ((p.bias && n_base + j < p.N) ? p.bias[n_base + j] : 0.f);
-            const size_t at = (size_t)row * p.ldo + n_base;
-            const bool whole = n_base + 16 <= p.N;
-            if (p.epilogue == EPI_SWIGLU) {
-              if (n_base < p.N) {
-                uint32_t packed[4];
+              for (int b = 0; b < 2; b++) {
+                uint32_t h[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                  __nv_bfloat162 h = __floats2bfloat162_rn(gated_mul(v[2 * j], v[2 * j + 8], p.gate_gelu), gated_mul(v[2 * j + 1], v[2 * j + 9], p.gate_gelu));
-                  packed[j] = *(uint32_t*)&h;
-                }
-                __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)row * p.ldo + (n_base >> 1);
-                if ((((size_t)row * p.ldo + (n_base >> 1)) & 7) == 0) *(uint4*)o = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                else { for (int j = 0; j < 4; j++) ((uint32_t*)o)[j] = packed[j]; }
-              }
-            } else if (p.epilogue == EPI_RESIDUAL) {
-              float* o = (float*)p.out + at;
-              if (whole && (at & 3) == 0) {
-#pragma unroll
-                for (int j = 0; j < 16; j += 4) {
-                  float4 r = *(float4*)(o + j);
-                  r.x += v[j]; r.y += v[j + 1]; r.z += v[j + 2]; r.w += v[j + 3];
-                  *(float4*)(o + j) = r;
-                }
-              } else {
-                for (int j = 0; j < 16 && n_base + j < p.N; j++) o[j] += v[j];
+                for (int j = 0; j < 4; j++)
+                  h[j] = pack(gated_mul(__uint_as_float(raw[16 * b + 2 * j]), __uint_as_float(raw[16 * b + 2 * j + 8]), p.gate_gelu),
+                              gated_mul(__uint_as_float(raw[16 * b + 2 * j + 1]), __uint_as_float(raw[16 * b + 2 * j + 9]), p.gate_gelu));
+                put((at - c) / 16 + b, h[0], h[1], h[2], h[3]);
               }
             } else if (p.out_is_f32) {
-              float* o = (float*)p.out + at;
-              if (whole && (at & 3) == 0) {
 #pragma unroll
-                for (int j = 0; j < 16; j += 4) *(float4*)(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-              } else {
-                for (int j = 0; j < 16 && n_base + j < p.N; j++) o[j] = v[j];
-              }
+              for (int q4 = 0; q4 < 8; q4++) put(q4, raw[4 * q4], raw[4 * q4 + 1], raw[4 * q4 + 2], raw[4 * q4 + 3]);
             } else {
-              __nv_bfloat16* o = (__nv_bfloat16*)p.out + at;
-              if (whole && (at & 7) == 0) {
-                uint32_t packed[8];
+              auto two = [&](int j) { return pack(__uint_as_float(raw[j]), __uint_as_float(raw[j + 1])); };
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                  __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                  packed[j] = *(uint32_t*)&h;
-                }
-                *(uint4*)(o) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                *(uint4*)(o + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+              for (int q4 = 0; q4 < 4; q4++) put((at - c) / 8 + q4, two(8 * q4), two(8 * q4 + 2), two(8 * q4 + 4), two(8 * q4 + 6));
+            }
+          }
+          __syncwarp();
+          const int first_col = gated ? (col0 + c) >> 1 : col0 + c;                     // of the output
+          const int chunk = lane & 7, n = first_col + chunk * per16, limit = min(out_cols, first_col + (gated ? (stop - c) >> 1 : stop - c));
+          if (n < limit) {
+#pragma unroll
+            for (int it = 0; it < 8; it++) {
+              const int r = it * 4 + (lane >> 3);
+              if (warp_row + r >= row_end) break;
+              const uint4 v = *(const uint4*)(slot + r * 128 + ((chunk ^ (r & 7)) << 4));
+              uint8_t* dst = out + (((size_t)(warp_row + r) * p.ldo + n) << elem_log2);
+              const bool whole = wide && n + per16 <= limit;
+              if (p.epilogue == EPI_RESIDUAL) {                  // a residual whose rows allow no tensor map
+                const float add[4] = {__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)};
+#pragma unroll
+                for (int j = 0; j < 4; j++) if (n + j < limit) ((float*)dst)[j] += add[j];
+              } else if (whole) {
+                *(uint4*)dst = v;
+              } else if (p.out_is_f32) {
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) if (n + j < limit) ((uint32_t*)dst)[j] = words[j];
               } else {
-                for (int j = 0; j < 16 && n_base + j < p.N; j++) o[j] = __float2bfloat16_rn(v[j]);
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 8; j++) if (n + j < limit) ((uint16_t*)dst)[j] = (uint16_t)(words[j / 2] >> (16 * (j & 1)));
               }
             }
           }
+          __syncwarp();                                          // the slot has been read
         }
+        if (half * step >= end) hand_back();                     // this warp had no columns
       }
-      // this warp has read the accumulator out: hand it back to the MMA issuer
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) release_accumulator(acc);
     }
   }
-  if (warp == 2 && lane == 0) bulk_wait_group<0>();     // the reductions have been performed
+  if (!SWAP && warp >= 2 && lane == 0) bulk_wait_group<0>();     // the additions have been performed
   tc_fence_before();
   __syncthreads();
+  if (warp == 0) issued = __reduce_max_sync(0xffffffffu, issued);      // the copy thread's count
   if (*abort_flag && warp == 0 && lane == 0) {
     // copies already issued still write shared memory: wait for them (bounded) before leaving
     for (int i = max(0, issued - L::STAGES); i < issued; i++)
@@ -602,7 +625,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 template <int BN, bool GROUPED = false>
 int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const typename ParamsOf<GROUPED>::type& p, int work,
                 cudaStream_t stream) {
-  using L = Layout<BN, true>;
+  using L = Layout<BN, true, GROUPED>;
   static bool configured = false;
   if (!configured) {
     cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false, true, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
@@ -649,7 +672,7 @@ int sprout_experts_product_tc(const void* rows, const int* offsets, const int* o
                               int K, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream) {
   const bool gated = unit == sprout_experts::UNIT_CLAMPED || unit == sprout_experts::UNIT_SILU;
   SPROUT_REQUIRE(rows && offsets && order && w && out && status && entries > 0 && experts > 0, "experts_product: bad arguments");
-  SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= 2048, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
+  SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= MAX_EXPERTS, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
   GroupedParams p{};
   p.out = out; p.out_is_f32 = unit < 0; p.epilogue = unit < 0 ? EPI_STORE : gated ? EPI_EXPERT_GLU : EPI_EXPERT_GELU;
   p.M = entries; p.N = N; p.K = K; p.ldo = N; p.status = status; p.groups = 1;
@@ -759,7 +782,7 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
     const long long row_tiles = (M + BLOCK_M - 1) / BLOCK_M;
     long long best = -1;
     for (int width : widths) {
-      if (width != 128 && (N % width != 0 || (groups > 1 && group_rows % width != 0))) continue;
+      if (width != 128 && (N % width != 0 || (groups > 1 && group_rows % width != 0) || (swiglu && width % 64 != 0))) continue;
       for (int split = 1; split <= (reduce ? 4 : 1); split++) {
         const int kb = (total_kb + split - 1) / split;
         if (split > 1 && kb < 4) break;
@@ -778,7 +801,7 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
   SPROUT_REQUIRE(work <= 0x7fffffffLL, "gemm_bf16: too many tiles");
   CUtensorMap map_out = map_a;
   if (reduce) {
-    if (tensor_map(out, M, N, ldo, BLOCK_M, &map_out, 4)) return 1;
+    if (tensor_map(out, M, N, ldo, 32, &map_out, 4)) return 1;      // a box is a warp's rows
     p.epilogue = EPI_RESIDUAL_TMA;
   }
   if (pair) {

@@ -325,6 +325,36 @@ def test_gemm_bf16_swiglu_epilogue(status, M, inter, K, orientation):
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("kind", ["bfloat16", "float32", "residual", "swiglu"])
+@pytest.mark.parametrize("orientation", [3, 4])
+@pytest.mark.parametrize("M,N,K,lead,extra", [(257, 272, 72, 0, 0), (300, 528, 136, 8, 8), (129, 1344, 200, 1, 3), (513, 224, 264, 0, 5), (260, 96, 64, 2, 2)])
+def test_gemm_bf16_tokens_on_m_stores_rows(status, kind, orientation, M, N, K, lead, extra):
+    """The epilogues with tokens on M go through a warp's shared memory in rows of 128 bytes: outputs that are columns of a wider buffer, on and off
+    16-byte boundaries, ragged last tiles of rows and columns; what lies beside the output stays as it was."""
+    from sprout_lm_b200 import kernels
+    from sprout_lm_b200.parts.mlp import interleave_gate_up
+    a, bias = rand(M, K, dtype=torch.bfloat16), rand(N, seed=2)
+    cols, dtype = (N // 2, torch.bfloat16) if kind == "swiglu" else (N, torch.bfloat16 if kind == "bfloat16" else torch.float32)
+    if kind == "swiglu" and (lead + cols + extra) % 2:
+        extra += 1                                             # that epilogue takes even row strides
+    buffer = torch.full((M, lead + cols + extra), 3.0, dtype=dtype, device=DEV)
+    out = buffer[:, lead:lead + cols]
+    if kind == "swiglu":
+        gate, up = rand(cols, K, dtype=torch.bfloat16, seed=1), rand(cols, K, dtype=torch.bfloat16, seed=4)
+        kernels.gemm_bf16(a, interleave_gate_up(gate, up), out, status, swiglu=True, orientation=orientation)
+        g = a.double() @ gate.double().T
+        want = g / (1 + torch.exp(-g)) * (a.double() @ up.double().T)
+    else:
+        w = rand(N, K, dtype=torch.bfloat16, seed=1)
+        kernels.gemm_bf16(a, w, out, status, bias=bias, residual=out if kind == "residual" else None, orientation=orientation)
+        want = a.double() @ w.double().T + bias.double() + (3.0 if kind == "residual" else 0.0)
+    # float32 sums of exact products; a bfloat16 output is rounded by up to 2^-9 of its value (twice that, and the activation, with a gate)
+    tol = 1e-5 if dtype == torch.float32 else 8e-3
+    assert (out.double() - want).abs().max().item() <= tol * max(1.0, want.abs().max().item())
+    assert (buffer[:, :lead] == 3.0).all() and (buffer[:, lead + cols:] == 3.0).all()
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K,split", [(1, 896, 4864, 16), (8, 896, 896, 14), (64, 130, 1000, 5), (128, 256, 264, 9)])
 def test_gemm_bf16_split_k(status, M, N, K, split):
     from sprout_lm_b200 import kernels
