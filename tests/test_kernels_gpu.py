@@ -282,6 +282,28 @@ def test_gemm_simple_tiles(M, N, K):
         assert torch.equal(part, out[first:first + rows])
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 129, 256), (16, 65, 300), (17, 200, 4099), (130, 4097, 257), (64, 4096, 1000), (1153, 63, 260), (700, 2048, 256)])
+def test_gemm_simple_shares_of_k(M, N, K):
+    """K shared by a cluster's CTAs (in four up to 4,096 columns, in two beyond), at ragged ends of rows, columns and shares, on and off 16-byte rows:
+    a row's bits depend neither on the rows beside it nor on the tile; strided output, bias and residual."""
+    from sprout_lm_b200 import kernels
+    a, w, bias = rand(M, K), rand(N, K, seed=1), rand(N, seed=2)
+    out = torch.empty(M, N, device=DEV)
+    kernels.gemm_simple(a, w, out, bias=bias)
+    want = a.double() @ w.double().T + bias.double()
+    tol = 4 * 6e-8 * math.sqrt(K) * want.abs().max().item() + 1e-6      # sequential float32 accumulation; shares only shorten it
+    assert (out.double() - want).abs().max().item() <= tol
+    for first, rows in ((M - 1, 1), (0, min(M, 16)), (0, min(M, 17)), (0, min(M, 65))):
+        part = torch.empty(rows, N, device=DEV)
+        kernels.gemm_simple(a[first:first + rows], w, part, bias=bias)
+        assert torch.equal(part, out[first:first + rows])
+    for lead in (1, 4):
+        wide = torch.full((M, N + 2 * lead), 2.0, device=DEV)
+        x = wide[:, lead:lead + N]
+        kernels.gemm_simple(a, w, x, bias=bias, residual=x)
+        assert torch.equal(x, out + 2.0) and (wide[:, :lead] == 2.0).all() and (wide[:, lead + N:] == 2.0).all()
+
+
 @pytest.mark.parametrize("orientation", [0, 1, 2, 3, 4])
 @pytest.mark.parametrize("M,N,K", SHAPES)
 def test_gemm_bf16_tensor_cores(status, M, N, K, orientation):
