@@ -28,7 +28,9 @@
 //  * gated_group_norm: rows in `groups` equal parts, each divided by its own root mean square, times a weight that
 //                  repeats every `period` elements, times act(gate) before or after the norm (or without a gate).
 //  * scaled_sum:   x += a y_1 + b y_2.
-#include "common.cuh"
+#include "gated_scan.cuh"
+
+using namespace sprout_scan;
 
 namespace {
 
@@ -36,7 +38,6 @@ __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + lo
 __device__ __forceinline__ float silu_g(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float sigmoid_g(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-enum ScanDecay : int { DECAY_PER_CHANNEL = 0, DECAY_PER_HEAD = 1, DECAY_GIVEN = 2, DECAY_FLOOR = 3, DECAY_BONUS = 4 };
 // Forms of the scan's kernel (the others share FORM_PLAIN), so that each keeps its own registers.
 enum ScanForm : int { FORM_PLAIN = 0, FORM_FLOOR = 1, FORM_BONUS = 2 };
 
@@ -44,31 +45,6 @@ __device__ __forceinline__ float double_exp_decay(float z) { return expf(-expf(z
 
 // What a forget gate with a floor writes: 1 - f for f = floor + (1 - floor) sigmoid(z).
 __device__ __forceinline__ float write_share(float z, float floor) { return (1.0f - floor) * sigmoid_g(-z); }
-
-template <typename T>
-struct ScanParams {
-  const T* q; int q_stride;            // [tokens, groups * dim]
-  const T* k; int k_stride;            // [tokens, groups * dim]
-  const T* v; int v_stride;            // [tokens, heads * vdim]
-  const void* z; int z_stride, z_f32;  // per channel: [tokens, heads * dim]; per head: [tokens, heads]; of T, or float when z_f32
-  const float* bias;                   // added to z: [heads * dim] or [heads]
-  const float* a_log;                  // per head (per-head decay only); with a floor: the floors [heads * dim]
-  const float* skip;                   // per head, or null
-  const float* bonus;                  // [heads * dim] (DECAY_BONUS only)
-  float inv_tau, q_scale;
-  int mode, heads, groups, dim, vdim;
-  const int* q_start; const int* state_slots; float* state; int num_slots;
-  float* out;                          // [tokens, heads * vdim]
-  int* status;
-  // portions cut into chunks (null / 0 when every request's tokens are walked by one block):
-  const float* da;                     // decays made beforehand: [tokens, heads * dim] per channel, [tokens, heads] per head
-  const float* dc;                     // per head: the factor on k, [tokens, heads]
-  float* sums;                         // [max_chunks, heads, dim, vdim]: a chunk's own sums, then the state before the chunk
-  float* prods;                        // [max_chunks, heads, dim]: the product of a chunk's decays
-  int chunk, requests;
-  int q_silu;                          // silu on the query rows (with a floor only)
-  int v_cols, ones_col;                // columns the value rows really have (<= vdim); column v_cols of the state is fed 1
-};
 
 // Eight neighbouring elements of a row that start on a 16-byte boundary.
 __device__ __forceinline__ void fetch8(const float* p, float (&v)[8]) {
@@ -83,17 +59,6 @@ __device__ __forceinline__ void fetch8(const __nv_bfloat16* p, float (&v)[8]) {
     v[2 * i] = __uint_as_float(w[i] << 16);
     v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
-}
-
-// The chunks of all requests are numbered in the requests' order, ceil(tokens / chunk) each.  Finds chunk `index`:
-// its request, its place among the request's chunks and how many the request has; false beyond the last chunk.
-__device__ __forceinline__ bool find_chunk(const int* q_start, int requests, int chunk, int index, int& r, int& c, int& n) {
-  for (int i = 0; i < requests; i++) {
-    n = (q_start[i + 1] - q_start[i] + chunk - 1) / chunk;
-    if (index < n) { r = i; c = index; return true; }
-    index -= n;
-  }
-  return false;
 }
 
 // Two float32 in a register pair: sm_100a multiplies, adds and fuses them pairwise in one instruction.
@@ -114,8 +79,6 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   return d;
 }
 
-enum ScanPhase : int { SCAN_WHOLE = 0, SCAN_CHUNK_SUMS = 1, SCAN_CHUNK_OUT = 2 };
-
 constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 
 // A block of SCAN_THREADS threads owns (request, head, `cb` value columns).  A thread keeps a tile of ROWS x COLS
@@ -128,7 +91,8 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // shuffles.  The bfloat16 path's walks over chunks of key sizes 64, 128 and 256, whose rows fill the slices (PAIRS), go two rows at a
 // time in packed arithmetic: a thread's rows are then neighbours, fetched 16 bytes at a time, and q, c k and a lie in planes of their
 // own, so that a 16-byte read is two pairs of one of them (2,048 tokens of 16 heads of 128 x 128, with the decays and the carry: 443 us
-// with a number at a time, (q, c k, a) triples and 2-byte fetches, 296 us so).  Other sizes and rows off 16-byte boundaries keep a
+// with a number at a time, (q, c k, a) triples and 2-byte fetches, 296 us so).  Decays per channel or per head at key sizes 64 and 128 run in
+// gated_scan_mma.cu where their rows allow it, in the same three launches around the same carry.  Other sizes and rows off 16-byte boundaries keep a
 // number at a time: pairs without the wide fetches cost 12 % (four heads of 96 x 96), and with two slices or one, 4 % (8 x 512, 16 x 64).
 // Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order.  An output's sum over the rows has one order in
 // the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn, so a bfloat16 request of one
@@ -857,16 +821,22 @@ int launch_scan_tiles(const ScanParams<T>& p, bool pairs, int requests, int max_
   }
   // `max_chunks` blocks per (head, columns): the chunks of all requests, found by their number
   const dim3 chunks(max_chunks, p.heads, grid.z);
-  sprout_launch(pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, false>,
-                chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
-  if (int rc = sprout_check_launch("gated_scan (chunk sums)")) return rc;
+  bool mma = false;                                    // 16 tokens at a time on tensor cores
+  if constexpr (sizeof(T) == 2 && FORM == FORM_PLAIN) mma = scan_mma_takes(p);
+  auto walk = [&](int phase) {
+    if constexpr (sizeof(T) == 2 && FORM == FORM_PLAIN)
+      if (mma) return launch_scan_mma(p, phase, max_chunks, stream);
+    auto* kernel = phase == SCAN_CHUNK_SUMS ? (pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_SUMS, FORM, false>)
+                                            : (pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, false>);
+    sprout_launch(kernel, chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
+    return sprout_check_launch(phase == SCAN_CHUNK_SUMS ? "gated_scan (chunk sums)" : "gated_scan (chunk outputs)");
+  };
+  if (int rc = walk(SCAN_CHUNK_SUMS)) return rc;
   SPROUT_REQUIRE(requests <= 65535, "gated_scan: too many requests");
   sprout_launch(scan_carry_kernel, dim3((p.dim * p.vdim + 255) / 256, p.heads, requests), dim3(256), 0, stream, p.sums,
                 (const float*)p.prods, (const float*)p.state, p.q_start, p.state_slots, p.num_slots, p.chunk, p.heads, p.dim, p.vdim);
   if (int rc = sprout_check_launch("gated_scan (carry)")) return rc;
-  sprout_launch(pairs ? gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, PAIRED> : gated_scan_kernel<T, ROWS, COLS, SCAN_CHUNK_OUT, FORM, false>,
-                chunks, dim3(SCAN_THREADS), smem_chunks, stream, p, slices_log2, batch);
-  return sprout_check_launch("gated_scan (chunk outputs)");
+  return walk(SCAN_CHUNK_OUT);
 }
 
 template <typename T>

@@ -1437,6 +1437,57 @@ def test_gated_scan_rows_in_16_byte_fetches(status, dtype, form, dim, vdim):
         assert np.abs(got - expected).max() <= 2.5e-5 * max(1.0, np.abs(expected).max())
 
 
+@pytest.mark.parametrize("form", ["channel", "head", "given"])
+@pytest.mark.parametrize("strength", [0.02, 1.0, 60.0])
+@pytest.mark.parametrize("dim,vdim,ones", [(64, 8, False), (64, 72, False), (128, 64, False), (128, 136, False), (128, 130, True), (64, 65, True)])
+def test_gated_scan_16_tokens_at_a_time(status, form, strength, dim, vdim, ones):
+    """The walk on tensor cores: portions that end within 16 tokens and within a chunk, a single token, value columns short of a block's and beyond one,
+    the column of ones, heads that share their keys, decays from almost none to all at once; outputs and states against the recurrence in float64."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    heads, groups, lengths, slots = 4, 2, [145, 1, 66, 128, 17], [2, 0, 3, 5, 1]
+    g = torch.Generator().manual_seed(dim + vdim)
+    T, v_cols = sum(lengths), vdim // 8 * 8
+    make = lambda *shape: torch.randn(*shape, generator=g).to(torch.bfloat16)
+    q, k, v = make(T, groups * dim), make(T, groups * dim), make(T, heads * v_cols)
+    f64 = lambda t: t.double().numpy()
+    factor, skip = np.ones((T, heads)), torch.linspace(-1.0, 1.0, heads)
+    z = bias = None
+    if form == "given":
+        given = (torch.rand(T, heads, generator=g) ** strength, torch.rand(T, heads, generator=g))
+        decay, factor = np.repeat(f64(given[0])[:, :, None], dim, axis=2), f64(given[1])
+        more = dict(given=tuple(t.to(DEV) for t in given))
+    elif form == "head":
+        z, bias, a_log = torch.randn(T, heads, generator=g), torch.linspace(-2.0, 1.0, heads), torch.full((heads,), math.log(strength))
+        factor = np.logaddexp(0.0, f64(z) + f64(bias))
+        decay = np.repeat(np.exp(-strength * factor)[:, :, None], dim, axis=2)
+        more = dict(per_head=True, a_log=a_log.to(DEV))
+    else:
+        z, bias = 2.0 * torch.randn(T, heads * dim, generator=g), torch.linspace(-3.0, 3.0, heads * dim)
+        x = (f64(z) + f64(bias)).reshape(T, heads, dim)
+        decay, more = (1.0 / (1.0 + np.exp(-x))) ** strength, dict(tau=1.0 / strength)
+    start = torch.randn(7, heads, dim, vdim, generator=g)
+    want, want_state, at = np.zeros((T, heads, vdim)), f64(start).copy(), 0
+    values = f64(v).reshape(T, heads, v_cols)
+    if ones:
+        values = np.concatenate([values, np.ones((T, heads, 1)), np.zeros((T, heads, vdim - v_cols - 1))], axis=2)
+    of_head = lambda t: np.repeat(f64(t).reshape(T, groups, dim), heads // groups, axis=1)
+    for n, slot in zip(lengths, slots):
+        part = slice(at, at + n)
+        want[part] = scan_oracle(form, of_head(q)[part] * 0.5, of_head(k)[part], values[part], decay[part], factor[part], None, want_state[slot])
+        at += n
+    want += f64(skip)[:, None] * values
+    ctx = SimpleNamespace(q_start=torch.tensor(np.cumsum([0] + lengths), dtype=torch.int32, device=DEV), max_q_len=max(lengths))
+    state = SimpleNamespace(buffer=start.to(DEV), slots=torch.tensor(slots, dtype=torch.int32, device=DEV))
+    out = torch.full((T, heads * vdim), float("nan"), device=DEV)
+    kernels.gated_scan(q.to(DEV), k.to(DEV), v.to(DEV), None if z is None else z.to(DEV), None if bias is None else bias.to(DEV), ctx, state, out, heads,
+                       groups, dim, vdim, status, q_scale=0.5, ones_col=ones, skip=skip.to(DEV), **more)
+    assert int(status.item()) == 0
+    # float32 recurrences of up to 145 steps and sums over up to 128 products of terms of both signs: some 300 roundings of 2^-24
+    for got, expected in ((out.double().cpu().numpy().reshape(want.shape), want), (state.buffer.double().cpu().numpy(), want_state)):
+        assert np.abs(got - expected).max() <= 2e-5 * max(1.0, np.abs(expected).max())
+
+
 @pytest.mark.parametrize("form", ["channel", "head", "floor", "bonus"])
 @pytest.mark.parametrize("dim,vdim", [(16, 24), (64, 40), (128, 64), (256, 20), (40, 12)])
 def test_float32_scan_keeps_its_bits_beside_a_long_portion(status, form, dim, vdim):
