@@ -62,6 +62,13 @@ __device__ __forceinline__ float4 fetch(const T* row, bool exists, int k, int K)
                      k + 3 < K ? to_float(row[k + 3]) : 0.f);
 }
 
+// A k's row of an operand in shared memory.  A warp's stores go to several k at one row: whole banks of 32 are swizzled, row r of k at
+// place r ^ (k / 4 << 3) (<< 2 with 32 k: groups of eight or four rows move), other rows are padded.  With 8 x 8 sums a thread the
+// padded rows are the faster ones (2,048 x 9,728 x 896: 744 us, 768 swizzled); with fewer the swizzled (512 x 896 x 4,864: 160 padded, 153
+// swizzled; 64 x 896 x 4,864: 58 and 54; 1 x 151,936 x 896: 180 and 136).
+constexpr bool swizzled(int rows, int TN) { return TN == 4 && rows % 32 == 0; }
+constexpr int row_floats(int rows, int TN) { return swizzled(rows, TN) ? rows : rows + 4; }
+
 // Four neighbouring results of a row into `out`: bias and residual added, in one access where the row allows it.
 template <typename TO>
 __device__ __forceinline__ void put4(float4 sum, const float* bias, const float* residual, TO* out, size_t at, int gn, int N, bool wide) {
@@ -91,7 +98,11 @@ gemm_simple_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const flo
                    const float* residual, TO* out, int M, int N, int whole_K, int k_share, int lda, int ldo, bool wide) {
   constexpr int THREADS = (BM / TM) * (BN / TN), COLS = BN / TN;
   constexpr int A_LOADS = (BM * BK / 4 + THREADS - 1) / THREADS, W_LOADS = (BN * BK / 4 + THREADS - 1) / THREADS;
-  constexpr int A_STRIDE = BM + 4, W_STRIDE = BN + 4;              // floats of a k's row, padded against conflicts of the stores
+  constexpr bool W_SWIZZLED = swizzled(BN, TN), A_SWIZZLED = swizzled(BM, TN);
+  constexpr int A_STRIDE = row_floats(BM, TN), W_STRIDE = row_floats(BN, TN);
+  // r's place in the row of k
+  auto a_place = [](int k, int r) { return A_SWIZZLED ? r ^ ((k / 4) << (BK == 16 ? 3 : 2)) : r; };
+  auto w_place = [](int k, int r) { return W_SWIZZLED ? r ^ ((k / 4) << (BK == 16 ? 3 : 2)) : r; };
   static_assert(TM == 2 || TM == 4 || TM == 8, "a thread's rows are neighbours");
   static_assert(TN == 4 || TN == 8, "a thread's columns are one or two groups of four");
   static_assert(COLS % 8 == 0 && (BM / TM) % 4 == 0, "a warp is 4 x 8 threads");
@@ -137,7 +148,7 @@ gemm_simple_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const flo
       if (BM * BK / 4 % THREADS == 0 || idx < BM * BK / 4) {
         const float v[4] = {a_next[i].x, a_next[i].y, a_next[i].z, a_next[i].w};
 #pragma unroll
-        for (int e = 0; e < 4; e++) a_s[(k + e) * A_STRIDE + row] = v[e];
+        for (int e = 0; e < 4; e++) a_s[(k + e) * A_STRIDE + a_place(k, row)] = v[e];
       }
     }
 #pragma unroll
@@ -146,7 +157,7 @@ gemm_simple_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const flo
       if (BN * BK / 4 % THREADS == 0 || idx < BN * BK / 4) {
         const float v[4] = {w_next[i].x, w_next[i].y, w_next[i].z, w_next[i].w};
 #pragma unroll
-        for (int e = 0; e < 4; e++) w_s[(k + e) * W_STRIDE + row] = v[e];
+        for (int e = 0; e < 4; e++) w_s[(k + e) * W_STRIDE + w_place(k, row)] = v[e];
       }
     }
   };
@@ -163,16 +174,16 @@ gemm_simple_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const flo
       fetch_block(k_begin + (block + 1) * BK);
       fetch_weights(k_begin + (block + 1) * BK);
     }
-    const float* a_s = As + stage * BK * A_STRIDE + ty * TM;
-    const float* w_s = Ws + stage * BK * W_STRIDE + tx * 4;
+    const float* a_s = As + stage * BK * A_STRIDE;
+    const float* w_s = Ws + stage * BK * W_STRIDE;
     unsigned long long a[2][TM / 2];
     float w[2][TN];
     auto read = [&](int k, int slot) {
-      if (TM == 2) a[slot][0] = *(const unsigned long long*)&a_s[k * A_STRIDE];
+      if (TM == 2) a[slot][0] = *(const unsigned long long*)&a_s[k * A_STRIDE + a_place(k, ty * TM)];
 #pragma unroll
-      for (int i = 0; i < TM / 4; i++) *(ulonglong2*)&a[slot][2 * i] = *(const ulonglong2*)&a_s[k * A_STRIDE + 4 * i];
+      for (int i = 0; i < TM / 4; i++) *(ulonglong2*)&a[slot][2 * i] = *(const ulonglong2*)&a_s[k * A_STRIDE + a_place(k, ty * TM + 4 * i)];
 #pragma unroll
-      for (int j = 0; j < TN / 4; j++) *(float4*)&w[slot][4 * j] = *(const float4*)&w_s[k * W_STRIDE + j * (BN / 2)];
+      for (int j = 0; j < TN / 4; j++) *(float4*)&w[slot][4 * j] = *(const float4*)&w_s[k * W_STRIDE + w_place(k, j * (BN / 2) + tx * 4)];
     };
     read(0, 0);
 #pragma unroll
@@ -236,7 +247,7 @@ template <int BM, int BN, int BK, int TM, int TN, int SPLIT, bool VEC, typename 
 int launch_tile(const TA* A, const TW* W, const float* bias, const float* residual, TO* out, int M, int N, int K, int lda, int ldo,
                 cudaStream_t stream) {
   constexpr int THREADS = (BM / TM) * (BN / TN);
-  constexpr size_t operands = (size_t)2 * BK * (BM + 4 + BN + 4) * sizeof(float), sums = SPLIT > 1 ? (size_t)BM * (BN + 4) * sizeof(float) : 0;
+  constexpr size_t operands = (size_t)2 * BK * (row_floats(BM, TN) + row_floats(BN, TN)) * sizeof(float), sums = SPLIT > 1 ? (size_t)BM * (BN + 4) * sizeof(float) : 0;
   constexpr size_t smem = operands > sums ? operands : sums;
   auto* kernel = gemm_simple_kernel<BM, BN, BK, TM, TN, SPLIT, VEC, TA, TW, TO>;
   static_assert(smem <= 48 * 1024, "fits without asking for more");
@@ -280,10 +291,10 @@ int launch_sizes(const TA* A, const TW* W, const float* bias, const float* resid
 }
 
 // How many CTAs (a cluster) share K: by the matrix alone, so that a row's bits do not depend on the rows beside it.  Small matrices
-// have too few tiles for the device (M x 896 x 4864 in one, two, four shares: 1 row 135, 73, 38 us; 64 rows 203, 113, 58; 512 rows 203,
-// 152, 161; 2,048 rows 712, 468, 432; M x 1,152 x 896: 64 rows 39, 24, 14, 2,048 rows 138, 104, 111).  Wide ones fill it by their columns
-// from some hundred rows on (M x 9,728 x 896: 64 rows 60, 48, 36; 512 rows 230, 211, 213; 2,048 rows 752, 745, 804), and a vocabulary's
-// from one (1 x 151,936 x 896: 180, 193, 195).
+// have too few tiles for the device (M x 896 x 4,864 in one, two, four shares: 1 row 135, 73, 33 us; 64 rows 203, 113, 54; 512 rows 203,
+// 152, 153; 2,048 rows 712, 468, 413; M x 1,152 x 896: 64 rows 39, 24, 13, 2,048 rows 138, 104, 106).  Wide ones fill it by their columns
+// from some hundred rows on (M x 9,728 x 896: 64 rows 60, 46, 36; 512 rows 230, 211, 213; 2,048 rows 752, 745, 804), and a vocabulary's
+// from one (1 x 151,936 x 896: 136, 160, 165).
 int split_of(int N, int K) {
   if (K < 256 || N > 65536) return 1;
   return N <= 4096 ? 4 : 2;
