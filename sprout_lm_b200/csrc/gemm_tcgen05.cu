@@ -666,6 +666,38 @@ int launch(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUten
   return sprout_check_launch("gemm_bf16");
 }
 
+// Tiles of a product with tokens on M: single CTAs or pairs, the tile's width, among how many CTAs a tile's k-blocks are divided
+// (where the epilogue adds).  Any N: a last tile may reach beyond it.  The pick is the smallest of
+//   in and out of a tile + rounds x k-blocks x a k-block's time,
+// in ns, measured alone and in products of 2 to 9 rounds (a k-block moves (rows + width) x 128 bytes a CTA, which is what its time
+// follows); a single CTA's k-block is faster while a round leaves the way from L2 to other SMs free, and its tiles' ends are not hidden
+// as a pair's are.  Over 16 shapes (300 to 4,001 tokens, 896 to 9,728 columns, K of 512 to 4,864) it names the fastest of these forms
+// but once (2,048 x 6,144 x 512: 15.7 us, 14.3 with single CTAs).  Widths that divide N only, pairs for every multiple of 256, as
+// before: 4,001 x 3,088 x 2,048 43.3 us and 36.3 now, 2,500 x 8,224 x 2,048 69.7 and 57.2, 300 x 3,072 x 1,024 9.9 and 5.8,
+// 2,048 x 3,072 x 2,048 24.2 and 20.9.
+struct TokenTiles { bool pair; int width, split; };
+TokenTiles pick_token_tiles(long long M, long long N, int total_kb, int group_rows, bool reduce, bool swiglu) {
+  struct Form { bool pair; int width, ends, block; };
+  const Form forms[] = {{false, 128, 3900, 230}, {false, 192, 4500, 327}, {false, 224, 5700, 350}, {false, 256, 5300, 375},
+                        {true, 192, 5900, 277}, {true, 224, 6100, 320}, {true, 256, 6000, 337}};
+  TokenTiles best{false, 128, 1};
+  long long best_cost = -1;
+  for (const Form& f : forms) {
+    if (group_rows && group_rows % f.width) continue;
+    if (swiglu && f.width % 128) continue;               // the two warps of a quarter would not have equal shares
+    const long long rows = f.pair ? 2 * BLOCK_M : BLOCK_M, slots = f.pair ? sm_count() / 2 : sm_count();
+    for (int split = 1; split <= (reduce && !f.pair ? 4 : 1); split++) {
+      const int kb = (total_kb + split - 1) / split;
+      if (split > 1 && kb < 4) break;
+      const long long items = (M + rows - 1) / rows * ((N + f.width - 1) / f.width) * split, rounds = (items + slots - 1) / slots;
+      const long long block = rounds > 1 ? f.block : f.pair ? f.block * 97 / 100 : f.block * 79 / 100;
+      const long long cost = f.ends + rounds * kb * block + (split > 1 ? 700 : 0) + (f.pair ? 0 : 800 * (rounds - 1));
+      if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {f.pair, f.width, split}; }
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 int sprout_experts_product_tc(const void* rows, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
@@ -766,33 +798,15 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
   // Tokens on M.  The residual epilogue goes through the TMA unit where the output's rows allow a
   // tensor map; its additions are atomic in L2, so a tile's K range may then be split among CTAs.
   const bool reduce = p.epilogue == EPI_RESIDUAL && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
-  // Tile width and K split: a k-block of a 128 x bn tile moves (128 + bn) x 128 bytes into shared
-  // memory and out again, which is what its time follows; wider tiles move less per product but
-  // make fewer CTAs.  The pick minimises rounds x k-blocks x (128 + bn) over the widths that
-  // divide N (128 always) and, for the reducing epilogue, splits of at least 4 k-blocks.
-  // N a multiple of 256: 256 x 256 tiles of CTA pairs (measured: gate/up 2048 x 9728 x 896
-  // 41 -> 39 us, 8192 tokens 145 -> 134 us; on narrower tiles single CTAs are as fast).
-  int bn = 128;
-  split_k = 1;
-  const bool pair = orientation == 4 || (orientation != 3 && N % 256 == 0 && (groups == 1 || group_rows % 256 == 0) && !(orientation == 0 && swiglu && M <= 128));
-  if (pair) {
-    bn = N % 256 == 0 && (groups == 1 || group_rows % 256 == 0) ? 256 : 128;
+  TokenTiles tiles{orientation == 4, 128, 1};
+  if (orientation == 4) {
+    if (N % 256 == 0 && (groups == 1 || group_rows % 256 == 0)) tiles.width = 256;
   } else if (orientation != 3) {
-    const int widths[4] = {128, 192, 224, 256};
-    const long long row_tiles = (M + BLOCK_M - 1) / BLOCK_M;
-    long long best = -1;
-    for (int width : widths) {
-      if (width != 128 && (N % width != 0 || (groups > 1 && group_rows % width != 0) || (swiglu && width % 64 != 0))) continue;
-      for (int split = 1; split <= (reduce ? 4 : 1); split++) {
-        const int kb = (total_kb + split - 1) / split;
-        if (split > 1 && kb < 4) break;
-        const long long items = row_tiles * ((N + width - 1) / width) * split;
-        const long long rounds = (items + sm_count() - 1) / sm_count();
-        const long long cost = rounds * (kb + 4 * (split > 1)) * (128 + width);   // a split costs another epilogue and its reduction
-        if (best < 0 || cost < best) { best = cost; bn = width; split_k = split; }
-      }
-    }
+    tiles = pick_token_tiles(M, N, total_kb, groups > 1 ? group_rows : 0, reduce, swiglu);
   }
+  const bool pair = tiles.pair;
+  const int bn = tiles.width;
+  split_k = tiles.split;
   p.k_blocks_per_split = (total_kb + split_k - 1) / split_k;
   split_k = (total_kb + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
   if (tensor_map(A, M, groups * K, lda, BLOCK_M, &map_a)) return 1;
@@ -805,8 +819,12 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
     p.epilogue = EPI_RESIDUAL_TMA;
   }
   if (pair) {
-    if (bn == 256) return launch_pair<256>(map_a, map_w, map_out, p, (int)work, stream);
-    return launch_pair<128>(map_a, map_w, map_out, p, (int)work, stream);
+    switch (bn) {
+      case 256: return launch_pair<256>(map_a, map_w, map_out, p, (int)work, stream);
+      case 224: return launch_pair<224>(map_a, map_w, map_out, p, (int)work, stream);
+      case 192: return launch_pair<192>(map_a, map_w, map_out, p, (int)work, stream);
+      default: return launch_pair<128>(map_a, map_w, map_out, p, (int)work, stream);
+    }
   }
   switch (bn) {
     case 256: return launch<256, false>(map_a, map_w, map_out, p, (int)work, stream);

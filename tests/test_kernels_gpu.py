@@ -377,6 +377,23 @@ def test_gemm_bf16_tokens_on_m_stores_rows(status, kind, orientation, M, N, K, l
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("M,N,K,residual", [(2048, 1152, 896, False), (2048, 1344, 2048, False), (2048, 896, 4864, True), (2048, 2048, 2048, True),
+                                            (2048, 3072, 2048, False), (2500, 8224, 1024, False), (4001, 3088, 1024, False), (600, 896, 4864, True),
+                                            (2049, 900, 4864, True)])
+def test_gemm_bf16_token_tiles_of_every_form(status, M, N, K, residual):
+    """Sizes whose tiles the kernel picks among all forms: single CTAs of 128, 192, 224 and 256 columns, pairs of 192, 224 and 256, K divided where the
+    output is added to, last tiles that reach beyond the matrix."""
+    from sprout_lm_b200 import kernels
+    a, w = rand(M, K, dtype=torch.bfloat16), rand(N, K, dtype=torch.bfloat16, seed=1)
+    buffer = torch.full((M, N + 4), 2.0 if residual else float("nan"), device=DEV)
+    out = buffer[:, :N]
+    kernels.gemm_bf16(a, w, out, status, residual=out if residual else None)
+    want = a.double() @ w.double().T + (2.0 if residual else 0.0)
+    assert (out.double() - want).abs().max().item() <= 1e-5 * want.abs().max().item()       # float32 sums of exact products
+    assert torch.equal(buffer[:, N:], torch.full((M, 4), 2.0, device=DEV)) if residual else bool(buffer[:, N:].isnan().all())
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K,split", [(1, 896, 4864, 16), (8, 896, 896, 14), (64, 130, 1000, 5), (128, 256, 264, 9)])
 def test_gemm_bf16_split_k(status, M, N, K, split):
     from sprout_lm_b200 import kernels
