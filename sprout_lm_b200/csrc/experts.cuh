@@ -18,7 +18,7 @@ __device__ __forceinline__ float glu(int unit, float g, float u, float limit, fl
 
 }  // namespace sprout_experts
 
-// One of the experts' products on tcgen05 in CTA pairs (gemm_tcgen05.cu): rows [entries, K] bfloat16 arranged by expert (`offsets`
+// One of the experts' products on tcgen05 in CTA pairs (experts_tcgen05.cu): rows [entries, K] bfloat16 arranged by expert (`offsets`
 // [experts + 1]), w [experts, matrix rows, K].  GLU or gelu units (`unit` >= 0): out bfloat16 [entries, N], the matrix has 2 N rows
 // (gate rows, then up rows) or for UNIT_PLAIN N; `row_weights` (of entry order[row]) multiply the products before the activation.
 // `unit` -1: out float32 [entries, N], the products as they are.

@@ -33,7 +33,6 @@
 
 
 #include "common.cuh"
-#include "experts.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -43,10 +42,9 @@ constexpr int BLOCK_K = 64;         // bf16 elements per stage row: 128 bytes, o
 constexpr int NUM_THREADS = 320;      // TMA warp, MMA warp, 8 epilogue warps
 constexpr int SMEM_BUDGET = 193 * 1024;    // for the operand stages; the staging tiles and barriers come on top
 
-enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RESIDUAL_ATOMIC = 2, EPI_SWIGLU = 3, EPI_RESIDUAL_TMA = 4, EPI_EXPERT_GLU = 5, EPI_EXPERT_GELU = 6 };
+enum Epilogue : int { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_RESIDUAL_ATOMIC = 2, EPI_SWIGLU = 3, EPI_RESIDUAL_TMA = 4 };
 constexpr int SLOT_BYTES = 32 * 128;            // an epilogue warp's 32 rows of 128 bytes on their way to memory
 constexpr int STAGING_BYTES = 8 * SLOT_BYTES;
-constexpr int MAX_EXPERTS = 2048;
 
 // SwiGLU epilogue: the weight rows interleave gate and up in blocks of 8 (rows 16b..16b+7 gate,
 // 16b+8..16b+15 up), so output feature 8b+j is silu(D[.., 16b+j]) * D[.., 16b+8+j]; the output
@@ -76,37 +74,21 @@ struct Params {
   const float* x32; const float* gain; int ldx;
 };
 
-// The experts' products (GROUPED) have arguments and a work item of their own: as fields of the dense forms' they cost the weights-on-M
-// kernels four registers a thread (56 to 60, handed out as 64): a decode step of 64 requests of 1,500 tokens 1,282 us, 1,252 us without.
-// The rows of expert e are offsets[e] .. offsets[e + 1] - 1, its matrix has `expert_rows` rows; what the gated epilogues need: see
-// sprout_experts_product_tc.
-struct GroupedParams : Params {
-  const int* offsets; const int* order; int experts, expert_rows, unit;
-  const float* row_weights; float limit, alpha;
-};
-template <bool GROUPED> struct ParamsOf { using type = Params; };
-template <> struct ParamsOf<true> { using type = GroupedParams; };
-
 // PAIR: two CTAs share a 256 x BN tile; each holds its own 128 rows of A and half of B's rows.
-// GROUPED: a table of the experts' tiles and rows takes a stage's room.
-template <int BN, bool PAIR = false, bool GROUPED = false>
+template <int BN, bool PAIR = false>
 struct Layout {
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BLOCK_K * 2;
   static constexpr int B_PADDED = (B_BYTES + 1023) / 1024 * 1024;
   static constexpr int STAGE_BYTES = A_BYTES + B_PADDED;
-  static constexpr int TABLE_BYTES = GROUPED ? (2 * (MAX_EXPERTS + 1) * 4 + 15) / 16 * 16 : 0;
-  static constexpr int STAGES = ((SMEM_BUDGET - TABLE_BYTES) / STAGE_BYTES) > 12 ? 12 : ((SMEM_BUDGET - TABLE_BYTES) / STAGE_BYTES);
+  static constexpr int STAGES = (SMEM_BUDGET / STAGE_BYTES) > 12 ? 12 : (SMEM_BUDGET / STAGE_BYTES);
   // two accumulators; allocations are powers of two from 32 columns
   static constexpr int TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + TABLE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
 // One unit of work: a 128 x BN tile of D over a range of K blocks.
 struct Work { int row0, col0, kb_begin, num_kb, split; };
-struct GroupedWork : Work { int row_end, weight_row; };
-template <bool GROUPED> struct WorkOf { using type = Work; };
-template <> struct WorkOf<true> { using type = GroupedWork; };
 
 // SWAP == false: map_rows is the activation map (rows = tokens), map_cols the weight map.
 // SWAP == true:  map_rows is the weight map (rows = output features), map_cols the activation map.
@@ -122,17 +104,12 @@ template <> struct WorkOf<true> { using type = GroupedWork; };
 // its own tensor memory.  The copies of both CTAs count on the first CTA's "full" barriers; the
 // commits arrive on the "empty" and "accumulator full" barriers of both CTAs; the second CTA's
 // epilogue warps arrive on the first CTA's "accumulator empty" barriers.
-//
-// GROUPED (pairs): the tiles are those of every expert's rows over its own matrix, found from the experts' offsets on the device;
-// a tile's rows beyond the expert's last are computed and not stored.  With a gate the first CTA's half of B is gate rows and
-// the second's the up rows that go with them, so a row's thread has both in its accumulators.
-template <int BN, bool SWAP, bool PAIR = false, bool GROUPED = false>
+template <int BN, bool SWAP, bool PAIR = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols,
-                    const __grid_constant__ CUtensorMap map_out, const typename ParamsOf<GROUPED>::type p) {
+                    const __grid_constant__ CUtensorMap map_out, const Params p) {
   static_assert(!(PAIR && SWAP), "pairs work on token tiles");
-  static_assert(!GROUPED || PAIR, "experts' products run in pairs");
-  using L = Layout<BN, PAIR, GROUPED>;
+  using L = Layout<BN, PAIR>;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0;                       // 0 issues the MMAs
   const int first_work = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;     // this CTA's (pair's) first item and stride
   const int work_stride = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
@@ -140,7 +117,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* staging = smem + L::STAGES * L::STAGE_BYTES;
-  uint64_t* full_bar = (uint64_t*)(staging + STAGING_BYTES + L::TABLE_BYTES);
+  uint64_t* full_bar = (uint64_t*)(staging + STAGING_BYTES);
   uint64_t* empty_bar = full_bar + L::STAGES;
   uint64_t* acc_full = empty_bar + L::STAGES;     // [2] accumulator complete (MMA -> epilogue)
   uint64_t* acc_empty = acc_full + 2;             // [2] accumulator read out (epilogue -> MMA)
@@ -153,34 +130,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   const int row_tiles = ((SWAP ? p.N : p.M) + TILE_M - 1) / TILE_M;
   const int col_tiles = ((SWAP ? p.M : p.N) + BN - 1) / BN;
   const int splits = (total_kb + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
-  // experts' products: 256-row tiles before expert e, and its first row
-  int* tile_prefix = (int*)(staging + STAGING_BYTES);
-  int* row_prefix = nullptr;
-  const bool glu_tiles = GROUPED && p.epilogue == EPI_EXPERT_GLU;
-  int expert_cols = 0;                                 // tiles across an expert's outputs
-  if constexpr (GROUPED) {
-    row_prefix = tile_prefix + p.experts + 1;
-    expert_cols = glu_tiles ? (p.N + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;
-  }
-  int total_work = row_tiles * col_tiles * splits;
+  const int total_work = row_tiles * col_tiles * splits;
   // consecutive work items share the weight tile where they can (tokens on M: same columns,
   // next rows), so that it is served from L2
   auto work_at = [&](int w) {
-    typename WorkOf<GROUPED>::type k;
-    if constexpr (GROUPED) {
-      const int tile = w / expert_cols, ct = w % expert_cols;
-      int e = 0, hi = p.experts;                       // the last e with tile_prefix[e] <= tile: it has rows
-      while (hi - e > 1) {
-        const int mid = (e + hi) / 2;
-        if (tile_prefix[mid] <= tile) e = mid; else hi = mid;
-      }
-      k.row0 = row_prefix[e] + (tile - tile_prefix[e]) * TILE_M + (int)rank * BLOCK_M;
-      k.row_end = row_prefix[e + 1];
-      k.col0 = ct * (glu_tiles ? BN / 2 : BN);
-      k.weight_row = e * p.expert_rows + k.col0 + (int)rank * (glu_tiles ? p.N : BN / 2);
-      k.split = 0; k.kb_begin = 0; k.num_kb = total_kb;
-      return k;
-    }
+    Work k;
     k.split = w % splits;
     const int tile = w / splits;
     if (SWAP) { k.row0 = (tile / col_tiles) * BLOCK_M; k.col0 = (tile % col_tiles) * BN; }   // token tiles of one weight tile side by side
@@ -204,33 +158,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, L::TMEM_COLS);
-  if constexpr (GROUPED) {
-    pdl_wait();                                        // the offsets are an earlier kernel's
-    if (warp == 0) {
-      int before = 0;
-      for (int e0 = 0; e0 < p.experts; e0 += 32) {
-        const int e = e0 + lane, begin = e < p.experts ? p.offsets[e] : 0, end = e < p.experts ? p.offsets[e + 1] : 0;
-        int sum = (end - begin + TILE_M - 1) / TILE_M;
-        const int own = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int other = __shfl_up_sync(0xffffffffu, sum, o);
-          if (lane >= o) sum += other;
-        }
-        if (e < p.experts) {
-          tile_prefix[e] = before + sum - own;
-          row_prefix[e] = begin;
-          if (e == p.experts - 1) { tile_prefix[p.experts] = before + sum; row_prefix[p.experts] = end; }
-        }
-        before += __shfl_sync(0xffffffffu, sum, 31);
-      }
-    }
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (GROUPED) total_work = tile_prefix[p.experts] * expert_cols;
   if (PAIR) {
     // The pair's MMAs write both CTAs' tensor memory at one address.  Each CTA has its SM to
     // itself (its shared memory leaves no room for another) and has allocated from an empty tensor
@@ -266,8 +197,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     };
     for (int w = first_work; w < total_work && ok; w += work_stride) {
       const auto k = work_at(w);
-      int weight_row = SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0);
-      if constexpr (GROUPED) weight_row = k.weight_row;
+      const int weight_row = SWAP ? k.row0 : k.col0 + (PAIR ? (int)rank * (BN / 2) : 0);
       const int act_row = SWAP ? k.col0 : k.row0;
       int early = 0;
       if (w == first_work) {
@@ -506,48 +436,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           continue;
         }
         const bool gated = p.epilogue == EPI_SWIGLU;
-        int row_end = p.M, out_cols = gated ? p.N >> 1 : p.N;
-        float weight = 1.0f;
-        if constexpr (GROUPED) {
-          row_end = k.row_end;
-          if (p.row_weights && row < row_end) weight = p.row_weights[p.order[row]];
-        }
+        const int out_cols = gated ? p.N >> 1 : p.N;
         // columns of the accumulator that a round takes (a gate's up columns beside them): 128 bytes of output, or 64 where the two
         // warps of a quarter would not both have a round
         const int step = gated ? (BN >= 256 ? 128 : 64) : p.out_is_f32 ? 32 : 64;
         const int elem_log2 = p.out_is_f32 ? 2 : 1, per16 = 16 >> elem_log2;
-        const int end = glu_tiles ? BN / 2 : BN;
         uint8_t* const out = (uint8_t*)p.out;
         const bool wide = (((uintptr_t)p.out | ((size_t)p.ldo << elem_log2)) & 15) == 0;
 #pragma unroll 1
-        for (int c = half * step; c < end; c += 2 * step) {
-          const int stop = min(c + step, end);
+        for (int c = half * step; c < BN; c += 2 * step) {
+          const int stop = min(c + step, BN);
 #pragma unroll 1
           for (int at = c; at < stop; at += 32) {
             uint32_t raw[32];
-            if constexpr (GROUPED) {
-              if (p.epilogue != EPI_STORE) {
-                uint32_t up[32];
-                tmem_load32(taddr + at, raw);
-                if (p.epilogue == EPI_EXPERT_GLU) tmem_load32(taddr + BN / 2 + at, up);
-                if (at + 32 >= stop && c + 2 * step >= end) hand_back();
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                  // rounded to bfloat16 before the activation, as separate products would leave them
-                  const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j]) * weight));
-                  const float u = p.epilogue == EPI_EXPERT_GLU ? __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j]) * weight)) : 0.f;
-                  v[j] = sprout_experts::glu(p.unit, g, u, p.limit, p.alpha);
-                }
-#pragma unroll
-                for (int q4 = 0; q4 < 4; q4++)
-                  put((at - c) / 8 + q4, pack(v[8 * q4], v[8 * q4 + 1]), pack(v[8 * q4 + 2], v[8 * q4 + 3]), pack(v[8 * q4 + 4], v[8 * q4 + 5]),
-                      pack(v[8 * q4 + 6], v[8 * q4 + 7]));
-                continue;
-              }
-            }
             load(at, raw);
-            if (at + 32 >= stop && c + 2 * step >= end) hand_back();
+            if (at + 32 >= stop && c + 2 * step >= BN) hand_back();
             if (gated) {
               // columns 16 b .. 16 b + 7 are gates, the next eight the up columns that go with them
 #pragma unroll
@@ -575,7 +478,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 #pragma unroll
             for (int it = 0; it < 8; it++) {
               const int r = it * 4 + (lane >> 3);
-              if (warp_row + r >= row_end) break;
+              if (warp_row + r >= p.M) break;
               const uint4 v = *(const uint4*)(slot + r * 128 + ((chunk ^ (r & 7)) << 4));
               uint8_t* dst = out + (((size_t)(warp_row + r) * p.ldo + n) << elem_log2);
               const bool whole = wide && n + per16 <= limit;
@@ -598,7 +501,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           }
           __syncwarp();                                          // the slot has been read
         }
-        if (half * step >= end) hand_back();                     // this warp had no columns
+        if (half * step >= BN) hand_back();                     // this warp had no columns
       }
     }
   }
@@ -622,13 +525,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 // ------------------------------------------------------------------ host side
 // `work` = tiles x K splits; the grid is one CTA per SM at most, each walking the work list.
 // Pairs: `work` counts 256 x BN tiles; the grid is one cluster of two CTAs per two SMs at most.
-template <int BN, bool GROUPED = false>
-int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const typename ParamsOf<GROUPED>::type& p, int work,
-                cudaStream_t stream) {
-  using L = Layout<BN, true, GROUPED>;
+template <int BN>
+int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUtensorMap& out_map, const Params& p, int work, cudaStream_t stream) {
+  using L = Layout<BN, true>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false, true, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
+    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
     if (err != cudaSuccess) return sprout_fail("gemm_bf16: cannot reserve %d bytes of shared memory: %s", L::SMEM_BYTES, cudaGetErrorString(err));
     configured = true;
   }
@@ -647,7 +549,7 @@ int launch_pair(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const 
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = sprout_pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&config, gemm_tcgen05_kernel<BN, false, true, GROUPED>, rows_map, cols_map, out_map, p);
+  cudaLaunchKernelEx(&config, gemm_tcgen05_kernel<BN, false, true>, rows_map, cols_map, out_map, p);
   return sprout_check_launch("gemm_bf16 (pairs)");
 }
 
@@ -699,27 +601,6 @@ TokenTiles pick_token_tiles(long long M, long long N, int total_kb, int group_ro
 }
 
 }  // namespace
-
-int sprout_experts_product_tc(const void* rows, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
-                              int K, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream) {
-  const bool gated = unit == sprout_experts::UNIT_CLAMPED || unit == sprout_experts::UNIT_SILU;
-  SPROUT_REQUIRE(rows && offsets && order && w && out && status && entries > 0 && experts > 0, "experts_product: bad arguments");
-  SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= MAX_EXPERTS, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
-  GroupedParams p{};
-  p.out = out; p.out_is_f32 = unit < 0; p.epilogue = unit < 0 ? EPI_STORE : gated ? EPI_EXPERT_GLU : EPI_EXPERT_GELU;
-  p.M = entries; p.N = N; p.K = K; p.ldo = N; p.status = status; p.groups = 1;
-  p.k_blocks_per_split = (K + BLOCK_K - 1) / BLOCK_K;
-  p.offsets = offsets; p.order = order; p.experts = experts; p.expert_rows = gated ? 2 * N : N; p.unit = unit;
-  p.row_weights = row_weights; p.limit = limit; p.alpha = alpha;
-  constexpr int BN = 256;
-  const long long matrix_rows = (long long)experts * p.expert_rows;
-  const long long work = ((long long)entries / (2 * BLOCK_M) + experts) * ((N + (gated ? BN / 2 : BN) - 1) / (gated ? BN / 2 : BN));
-  SPROUT_REQUIRE(matrix_rows <= 0x7fffffffLL && work <= 0x7fffffffLL, "experts_product: too many rows");
-  CUtensorMap map_a, map_w;
-  if (tensor_map(rows, entries, K, K, BLOCK_M, &map_a)) return 1;
-  if (tensor_map(w, (int)matrix_rows, K, K, BN / 2, &map_w)) return 1;
-  return launch_pair<BN, true>(map_a, map_w, map_a, p, (int)work, stream);
-}
 
 // A [M, K] bf16 row stride lda; W [N, K] bf16 contiguous; out [M, N] row stride ldo, bf16 or
 // float32.  residual != 0: out is float32 and the product is added to it.  orientation: 0 picks

@@ -737,14 +737,12 @@ SPROUT_API int sprout_moe_mma_supported(int width, int ff, int h_stride) {
   return width % 8 == 0 && ff % 8 == 0 && h_stride % 8 == 0;
 }
 
-// Whether a step of these sizes takes the tcgen05 products: experts of at least a tile's width (a pair of CTAs makes 256 rows x 256
-// columns, or 128 gated ones), and more tokens than the few-token kernel's.  Matrices under a million elements need 2,048 rows to pay for
-// the gather's launch (16 experts of 512 over 1,024, 200 tokens x top 4: 102 us a layer on mma.sync, 110 us here, launched one by one).
-// 32 experts of 1,024 over 2,048 wide rows: 2,048 tokens x top 4 374 us (both) on mma.sync, 181 us with the gather here; 64 tokens 175
-// and 108 us.
+// Whether the tcgen05 products take these sizes: experts of at least a tile's width (a pair of CTAs makes 256 features, or 128 gated ones).
+// They pay for any number of tokens (their tiles are as wide as an expert's rows): 32 experts of 1,024 over 2,048, top 4, both products with
+// the gather, on the kernels below and so: 1 token 46 and 34 us, 8 97 and 75, 64 179 and 95, 512 200 and 103, 2,048 425 and 143; 16 of 512
+// over 1,024: 8 tokens 42 and 28, 256 58 and 34; 64 of 512 over 512: 8 tokens 29.7 both.
 SPROUT_API int sprout_moe_tc_supported(int entries, int experts, int top, int width, int ff, int h_stride) {
-  return sprout_moe_mma_supported(width, ff, h_stride) && width >= 512 && ff >= 256 && experts <= 2048 && entries > FEW * top &&
-         ((long long)width * ff >= (1 << 20) || entries >= 2048);
+  return sprout_moe_mma_supported(width, ff, h_stride) && width >= 512 && ff >= 256 && experts <= 2048;
 }
 
 // The same as below through sprout_experts_product_tc; `gathered` bfloat16 [entries, width] is scratch.

@@ -1712,9 +1712,9 @@ def decay_attention(rows, ctx, state, decay, out, heads: int, dim: int, vdim: in
     decay_scan(rows, ctx.q_start, state.slots, state.buffer, decay, out, heads, dim, vdim, silu, status)
 
 
-# Elements of an expert's matrix from which its products run on tcgen05 at all: below, many rows do not pay for the gather either (8 experts of
-# 256 over 512, 2,048 rows: 30 us on mma.sync, 34 us on tcgen05; 64 of 512 over 512 71 and 76; 16 of 512 over 1,024 55 and 39)
-EXPERTS_TC_ELEMENTS = 1 << 19
+# Elements of an expert's matrix from which its products run on tcgen05 (16 experts of 512 over 512, 256 tokens: 38 us on mma.sync, 28 us
+# on tcgen05; 8 of 256 over 512: 28 and 26 us, but 512 tokens 28 and 34)
+EXPERTS_TC_ELEMENTS = 1 << 18
 
 
 @functools.lru_cache(maxsize=4096)

@@ -1276,6 +1276,12 @@ def test_experts_on_tcgen05(status, monkeypatch, unit, counts, width, ff, weight
         assert (tc - plain).abs().max() <= 2 ** -6 * plain.abs().max()
 
 
+@pytest.mark.parametrize("unit", ["clamped_glu", "plain"])
+def test_experts_tiles_of_every_width(status, monkeypatch, unit):
+    """Rows of an expert in one tile of 16 to 256 columns, in two and more of equal size, features and K that no tile divides."""
+    test_experts_on_tcgen05(status, monkeypatch, unit, [15, 16, 31, 33, 240, 241, 255, 513, 0, 783, 4353], 648, 328, False)
+
+
 @pytest.mark.parametrize("window,sink,interleaved,dim,tail,vdim", [(None, True, True, 64, 64, 128), (100, False, False, 64, 64, 128), (64, True, True, 64, 0, 64), (None, True, False, 64, 64, 128)])
 @pytest.mark.parametrize("held,new", [([0], [129]), ([0, 300, 65], [400, 129, 190])])
 def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, tail, vdim, held, new):
