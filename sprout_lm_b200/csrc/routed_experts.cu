@@ -245,34 +245,65 @@ moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict_
   for (int place = lane; place < top; place += 32) weights[(size_t)t * top + place] *= norm;
 }
 
-// One block.  counts -> offsets [experts + 1]; counts are left zeroed for the next call.
+// One block.  counts -> offsets [experts + 1]; counts are left zeroed for the next call.  Bound by latencies in turn: the counts are
+// added up by all threads (by one, a memory access after the other, 32 experts took 12.7 us with 256 entries, 33 with 8,192), the
+// first entries are fetched beside them.
+constexpr int ARRANGE_AHEAD = 8;
 __global__ void __launch_bounds__(1024)
 moe_arrange_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ sorted,
                    int* __restrict__ place_of, int entries, int experts) {
   extern __shared__ int cursor[];       // experts
+  __shared__ int warp_sums[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_launch_dependents();
   pdl_wait();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < experts; e++) {
+  int ahead[ARRANGE_AHEAD];
+#pragma unroll
+  for (int j = 0; j < ARRANGE_AHEAD; j++) {
+    const int i = tid + j * 1024;
+    ahead[j] = i < entries ? ids[i] : 0;
+  }
+  int before = 0;                       // entries of the experts of earlier rounds
+  for (int e0 = 0; e0 < experts; e0 += 1024) {
+    const int e = e0 + tid, own = e < experts ? counts[e] : 0;
+    int sum = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += other;
+    }
+    if (lane == 31) warp_sums[warp] = sum;
+    __syncthreads();
+    int ahead_of_warp = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 32; w++) {
+      const int part = warp_sums[w];
+      if (w < warp) ahead_of_warp += part;
+      all += part;
+    }
+    const int at = before + ahead_of_warp + sum - own;
+    if (e < experts) {
       offsets[e] = at;
       cursor[e] = at;
-      at += counts[e];
       counts[e] = 0;
     }
-    offsets[experts] = at;
+    before += all;
+    __syncthreads();                    // the sums have been read
   }
+  if (tid == 0) offsets[experts] = before;
   __syncthreads();
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-    const int e = ids[i];
+  auto place = [&](int i, int e) {
+    int at = -1;
     if (e < experts) {
-      const int at = atomicAdd(&cursor[e], 1);
+      at = atomicAdd(&cursor[e], 1);
       sorted[at] = i;
-      place_of[i] = at;
-    } else {
-      place_of[i] = -1;
     }
-  }
+    place_of[i] = at;
+  };
+#pragma unroll
+  for (int j = 0; j < ARRANGE_AHEAD; j++)
+    if (tid + j * 1024 < entries) place(tid + j * 1024, ahead[j]);
+  for (int i = tid + ARRANGE_AHEAD * 1024; i < entries; i += 1024) place(i, ids[i]);
 }
 
 __device__ __forceinline__ int expert_of(const int* offsets, int experts, int row) {

@@ -1282,6 +1282,26 @@ def test_experts_tiles_of_every_width(status, monkeypatch, unit):
     test_experts_on_tcgen05(status, monkeypatch, unit, [15, 16, 31, 33, 240, 241, 255, 513, 0, 783, 4353], 648, 328, False)
 
 
+@pytest.mark.parametrize("experts,entries", [(1, 1), (5, 1025), (33, 8193), (1025, 9000), (2048, 700)])
+def test_entries_arranged_by_expert(experts, entries):
+    """Offsets from the counts, every entry once within its expert, identity experts without a place, the counts left zeroed."""
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(experts + entries)
+    ids = torch.randint(0, experts + 2, (entries, 1), generator=g).to(torch.int32)      # the last two: identity experts
+    counts = torch.bincount(ids.flatten().long(), minlength=experts + 2)[:experts]
+    device_counts = counts.to(torch.int32).to(DEV)
+    offsets, order = torch.zeros(experts + 1, dtype=torch.int32, device=DEV), torch.zeros(entries, dtype=torch.int32, device=DEV)
+    place = torch.zeros(entries, dtype=torch.int32, device=DEV)
+    kernels.moe_arrange(ids.to(DEV), device_counts, offsets, order, place, experts)
+    want = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    total = int(want[-1])
+    order, place = order.cpu().long()[:total], place.cpu().long()
+    assert (offsets.cpu().long() == want).all() and (device_counts == 0).all()
+    assert (order.sort().values == torch.nonzero(ids.flatten() < experts).flatten()).all()
+    assert (ids.flatten().long()[order] == torch.repeat_interleave(torch.arange(experts), counts)).all()
+    assert (place[order] == torch.arange(total)).all() and (place[ids.flatten() >= experts] == -1).all()
+
+
 @pytest.mark.parametrize("window,sink,interleaved,dim,tail,vdim", [(None, True, True, 64, 64, 128), (100, False, False, 64, 64, 128), (64, True, True, 64, 0, 64), (None, True, False, 64, 64, 128)])
 @pytest.mark.parametrize("held,new", [([0], [129]), ([0, 300, 65], [400, 129, 190])])
 def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, tail, vdim, held, new):
