@@ -39,7 +39,8 @@ namespace {
 // threads of a router block: 32 warps, so that the router's rows are walked by as many warps as the SM holds (a block's time is
 // the latency of its rounds over the outputs: 33 outputs are 2 rounds of 32 warps, 5 of 8)
 // Steps of many tokens over enough outputs: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four
-// products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so).
+// products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so, 25 us with registers
+// for two blocks of 9 warps an SM).
 constexpr int ROUTE_THREADS = 1024;
 
 // A block takes ROUTE_TOKENS tokens (8 in steps of many tokens, 1 in steps of few, where blocks are scarce; a token's
@@ -48,7 +49,7 @@ constexpr int ROUTE_THREADS = 1024;
 // are multiples of four, else every 32nd), the lanes are added in a fixed order, so a token's
 // scores do not depend on the tokens beside it.  Warp t then takes token t's softmax and choices.
 template <typename T, int ROUTE_TOKENS, int ROUTE_OUTPUTS>
-__global__ void __launch_bounds__(ROUTE_OUTPUTS > 1 ? 512 : ROUTE_THREADS)
+__global__ void __launch_bounds__(ROUTE_OUTPUTS > 1 ? 512 : ROUTE_THREADS) __maxnreg__(ROUTE_OUTPUTS > 1 ? 104 : 64)
 moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ router, const float* __restrict__ correction,
                  int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int tokens, int width,
                  int softmax_outputs, int experts, int top, float scale, int extra, float* __restrict__ extra_out,
