@@ -463,17 +463,18 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     if (SPLIT && split) {
       // this CTA's rows go to scratch memory; the warpgroup then counts itself in for its Q tile,
       // and if the other CTA was there before, it merges that CTA's rows into its own
-      constexpr int ROW_FLOATS = HD + 4;
-      float* mine = p.scratch + ((size_t)(piece_index * 2 + rank) * CTA_ROWS + q * TC_ROWS + row) * ROW_FLOATS;
-      const float* theirs = p.scratch + ((size_t)(piece_index * 2 + (rank ^ 1)) * CTA_ROWS + q * TC_ROWS + row) * ROW_FLOATS;
+      // in planes of 16 bytes a row, so that a warp's accesses are 512 bytes side by side; the last plane holds the maxima and sums
+      constexpr int PLANES = HD / 4 + 1;
+      float4* mine = (float4*)p.scratch + ((size_t)(piece_index * 2 + rank) * TC_QTILES + q) * PLANES * TC_ROWS + row;
+      const float4* theirs = (const float4*)p.scratch + ((size_t)(piece_index * 2 + (rank ^ 1)) * TC_QTILES + q) * PLANES * TC_ROWS + row;
 #pragma unroll
       for (int i = 0; i < HD / 4; i++) {
         float a, b, c, d;
         f2_unpack(o2[2 * i], a, b);
         f2_unpack(o2[2 * i + 1], c, d);
-        ((float4*)mine)[i] = make_float4(a, b, c, d);
+        mine[i * TC_ROWS] = make_float4(a, b, c, d);
       }
-      *(float2*)(mine + HD) = make_float2(ok ? m : -INFINITY, l);
+      mine[HD / 4 * TC_ROWS] = make_float4(ok ? m : -INFINITY, l, 0.f, 0.f);
       __threadfence();
       asm volatile("bar.sync %0, 128;" ::"r"(1 + q) : "memory");          // the warpgroup's rows are written
       int* counter = p.counters + piece_index * TC_QTILES + q;
@@ -483,7 +484,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       if (*seen == 1) {
         __threadfence();
         if ((tid & 127) == 0) *counter = 0;                                // ready for the next launch
-        const float2 ml = __ldcg((const float2*)(theirs + HD));
+        const float4 ml = __ldcg(theirs + HD / 4 * TC_ROWS);
         const float m1 = ml.x, l1 = ml.y;
         const float top = fmaxf(m, m1);
         const float a0 = m == -INFINITY ? 0.f : exp2_fast((m - top) * scale_log2);
@@ -492,27 +493,33 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         const uint64_t a0_2 = f2_pack(a0, a0), a1_2 = f2_pack(a1, a1);
 #pragma unroll
         for (int i = 0; i < HD / 4; i++) {
-          const float4 t = __ldcg((const float4*)theirs + i);
+          const float4 t = __ldcg(theirs + i * TC_ROWS);
           o2[2 * i] = f2_fma(o2[2 * i], a0_2, f2_mul(f2_pack(t.x, t.y), a1_2));
           o2[2 * i + 1] = f2_fma(o2[2 * i + 1], a0_2, f2_mul(f2_pack(t.z, t.w), a1_2));
         }
         writes = true;
       }
     }
-    if (ok && row_valid && writes) {
+    if (ok && writes) {                                // the same for the whole warp
+      // rows leave through the Q tile's own P, whose last product is complete (see warp_rows_out)
       const float inv = 1.0f / l;
-      __nv_bfloat16* dst = p.out + (size_t)token * p.out_stride + (size_t)head * HD;
+      uint8_t* slot = sP + q * L::P_BYTES + quarter * 32 * 128;
+      __nv_bfloat16* dst = row_valid ? p.out + (size_t)token * p.out_stride + (size_t)head * HD : nullptr;
 #pragma unroll
-      for (int i = 0; i < HD; i += 8) {
-        uint32_t packed[4];
+      for (int half = 0; half < HD / 64; half++) {
 #pragma unroll
-        for (int k2 = 0; k2 < 4; k2++) {
-          float lo, hi;
-          f2_unpack(o2[i / 2 + k2], lo, hi);
-          __nv_bfloat162 h = __floats2bfloat162_rn(lo * inv, hi * inv);
-          packed[k2] = *(uint32_t*)&h;
+        for (int c = 0; c < 8; c++) {
+          uint32_t packed[4];
+#pragma unroll
+          for (int k2 = 0; k2 < 4; k2++) {
+            float lo, hi;
+            f2_unpack(o2[half * 32 + c * 4 + k2], lo, hi);
+            __nv_bfloat162 h = __floats2bfloat162_rn(lo * inv, hi * inv);
+            packed[k2] = *(uint32_t*)&h;
+          }
+          *(uint4*)(slot + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
-        *(uint4*)(dst + i) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        warp_rows_out(slot, dst, half * 64);
       }
     }
   }

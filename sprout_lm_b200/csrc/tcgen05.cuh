@@ -241,6 +241,20 @@ __device__ __forceinline__ void tmem_load_wait(uint32_t (&r)[32]) {
         "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
       :: "memory");
 }
+// A warp's 32 rows of 64 bfloat16 from its 4 KB of shared memory (16-byte chunk c of row r at chunk c ^ (r & 7)) to memory, columns `col`
+// on of the row that lane r's `dst` points to (null: none): rows of 128 bytes, four an instruction.  Stored by its own lane, a row's
+// 16-byte pieces are 32 accesses an instruction.
+__device__ __forceinline__ void warp_rows_out(const uint8_t* slot, __nv_bfloat16* dst, int col) {
+  const int lane = threadIdx.x & 31, chunk = lane & 7;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int r = i * 4 + (lane >> 3);
+    __nv_bfloat16* to = (__nv_bfloat16*)__shfl_sync(0xffffffffu, (unsigned long long)dst, r);
+    if (to != nullptr) *(uint4*)(to + col + chunk * 8) = *(const uint4*)(slot + r * 128 + ((chunk ^ (r & 7)) << 4));
+  }
+  __syncwarp();                                        // the slot has been read
+}
 // Registers move between the warpgroups of a CTA: a warpgroup that needs few gives them up, one
 // that needs many takes them (every warp of the warpgroup executes the same instruction).
 template <int REGS> __device__ __forceinline__ void warpgroup_regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
