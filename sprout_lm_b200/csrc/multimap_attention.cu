@@ -450,8 +450,14 @@ multimap_attention_simple_kernel(const T* __restrict__ q, int q_stride, const T*
 constexpr int MM_ROWS = 64, MM_KEYS = 64, MM_THREADS = 128;
 
 // How the rows of a step go to the CTAs: tiles of 64 rows; or, where no request has more than 16 rows (usually single tokens, the heads of
-// one key/value group), a CTA's warps share the keys of its request's tile, with the 16 rows of the fragments or the first 8 alone.
-enum RowsForm : int { ROWS_TILES = 0, ROWS_16 = 1, ROWS_8 = 2 };
+// one key/value group), a CTA's warps share the keys of its request's tile; with up to 8 rows: multimap_rows8_kernel.
+enum RowsForm : int { ROWS_TILES = 0, ROWS_16 = 1 };
+
+// The forms that share keys: each warp takes 16 keys of every 64-key tile and copies them itself, through stages of its own in shared
+// memory, so that no warp waits for another before the end and every warp has two stages on their way while it works on a third.  These
+// launches are bound by the caches' way from memory; a CTA's warps meeting twice a tile, with one tile on its way, read them at 0.45
+// of the copy rate (64 requests over 3,000 to 6,000 keys of 4 heads of 128 + 128).
+constexpr int WARP_KEYS = 16, WARP_STAGES = 3;
 
 template <int DIM, int VDIM, int MAPS, int ROWS>
 __global__ void __launch_bounds__(MM_THREADS)
@@ -460,10 +466,10 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   constexpr int KW = MAPS * DIM, KSTRIDE = KW + 8, VSTRIDE = VDIM + 8, KCHUNKS = KW / 8, VCHUNKS = VDIM / 8;
   extern __shared__ __align__(16) unsigned char mm_smem[];
   __nv_bfloat16* sQ = (__nv_bfloat16*)mm_smem;                   // MM_ROWS x KSTRIDE
-  __nv_bfloat16* sK = sQ + MM_ROWS * KSTRIDE;                    // 2 x MM_KEYS x KSTRIDE
-  __nv_bfloat16* sV = sK + 2 * MM_KEYS * KSTRIDE;                // 2 x MM_KEYS x VSTRIDE
+  __nv_bfloat16* sK = sQ + (SPLIT ? 16 : MM_ROWS) * KSTRIDE;     // 2 x MM_KEYS x KSTRIDE; keys shared: WARP_STAGES x MM_KEYS
+  __nv_bfloat16* sV = sK + (SPLIT ? WARP_STAGES : 2) * MM_KEYS * KSTRIDE;
   __shared__ int s_token[MM_ROWS], s_head[MM_ROWS], s_limit[MM_ROWS], s_lo[MM_ROWS];
-  __shared__ long long s_row[2][MM_KEYS];
+  __shared__ long long s_row[SPLIT ? 1 : 2][SPLIT ? 1 : MM_KEYS];
 
   pdl_launch_dependents();
   pdl_wait();
@@ -504,24 +510,20 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   const int list_tiles = keep_tiles + (kv_tiles - tile_lo);
   auto tile_of = [&](int i) { return i < keep_tiles ? i : tile_lo + (i - keep_tiles); };
 
-  for (int idx = tid; idx < MM_ROWS * KCHUNKS; idx += MM_THREADS) {
+  for (int idx = tid; idx < (SPLIT ? 16 : MM_ROWS) * KCHUNKS; idx += MM_THREADS) {
     const int row = idx / KCHUNKS, c = idx % KCHUNKS;
     __nv_bfloat16* dst = sQ + row * KSTRIDE + c * 8;
     if (s_token[row] >= 0) cp_async16(dst, p.q + (size_t)s_token[row] * p.q_stride + (size_t)s_head[row] * KW + c * 8);
     else *(uint4*)dst = make_uint4(0, 0, 0, 0);
   }
-  auto find_rows = [&](int t, int buf) {
-    if (tid < MM_KEYS) {
-      const int key = t * MM_KEYS + tid;
-      long long row = -1;
-      if ((key >= min_lo || key < p.mask_keep) && key <= max_limit) {
-        const int page = table[key / p.page_tokens];
-        if (page < 0 || page >= p.num_pages) atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
-        else row = ((long long)page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens;
-      }
-      s_row[buf][tid] = row;
-    }
+  auto row_of = [&](int key) -> long long {                         // where a key's rows lie in the caches, -1: no query sees it
+    if ((key < min_lo && key >= p.mask_keep) || key > max_limit) return -1;
+    const int page = table[key / p.page_tokens];
+    if (page >= 0 && page < p.num_pages) return ((long long)page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens;
+    atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
+    return -1;
   };
+  auto find_rows = [&](int t, int buf) { if (tid < MM_KEYS) s_row[buf][tid] = row_of(t * MM_KEYS + tid); };
   auto load_tile = [&](int buf) {
     for (int idx = tid; idx < MM_KEYS * KCHUNKS; idx += MM_THREADS) {
       const int row = idx / KCHUNKS, c = idx % KCHUNKS;
@@ -539,18 +541,49 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
     }
   };
   const int first_tile = SPLIT ? (int)blockIdx.z : 0, tile_step = SPLIT ? p.ksplit : 1;    // this CTA's tiles: every tile_step-th of the list
-  if (first_tile < list_tiles) find_rows(tile_of(first_tile), 0);
-  __syncthreads();
-  if (first_tile < list_tiles) load_tile(0);
-  cp_async_commit();
+  // keys shared: this warp's 16 keys of a tile, from the rows that its lanes 0 to 15 hold, into a stage
+  long long ahead = -1;                                             // of lane l: key l of the next tile to copy
+  auto look_ahead = [&](int i) { ahead = i < list_tiles && lane < WARP_KEYS ? row_of(tile_of(i) * MM_KEYS + warp * WARP_KEYS + lane) : -1; };
+  auto copy_keys = [&](int stage) {
+    const int first = (stage * (MM_THREADS / 32) + warp) * WARP_KEYS;
+#pragma unroll
+    for (int idx = lane; idx < WARP_KEYS * KCHUNKS; idx += 32) {
+      const int row = idx / KCHUNKS, c = idx % KCHUNKS;
+      const long long at = __shfl_sync(0xffffffffu, ahead, row);
+      __nv_bfloat16* dst = sK + (first + row) * KSTRIDE + c * 8;
+      if (at >= 0) cp_async16(dst, p.k_cache + at * KW + c * 8);
+      else *(uint4*)dst = make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int idx = lane; idx < WARP_KEYS * VCHUNKS; idx += 32) {
+      const int row = idx / VCHUNKS, c = idx % VCHUNKS;
+      const long long at = __shfl_sync(0xffffffffu, ahead, row);
+      __nv_bfloat16* dst = sV + (first + row) * VSTRIDE + c * 8;
+      if (at >= 0) cp_async16(dst, p.v_cache + at * VDIM + c * 8);
+      else *(uint4*)dst = make_uint4(0, 0, 0, 0);
+    }
+  };
+  if constexpr (SPLIT) {
+    cp_async_commit();                                              // Q
+    look_ahead(first_tile);
+#pragma unroll
+    for (int d = 0; d < WARP_STAGES - 1; d++) {
+      if (first_tile + d * tile_step < list_tiles) copy_keys(d);
+      cp_async_commit();
+      look_ahead(first_tile + (d + 1) * tile_step);
+    }
+    cp_async_wait<WARP_STAGES - 1>();
+    __syncthreads();                                                // Q has landed, all of it
+  } else {
+    if (first_tile < list_tiles) find_rows(tile_of(first_tile), 0);
+    __syncthreads();
+    if (first_tile < list_tiles) load_tile(0);
+    cp_async_commit();
+  }
 
   // SPLIT (a step in which no request has more than 16 rows: single tokens, the heads of one key/value group): a CTA
   // divides every tile's keys among its warps instead of its rows, and the warps' partial results are merged at the end.
   constexpr bool split = SPLIT;
-  // rows 8 to 15 of a tile are the second two numbers of every fragment: where no request has more than 8 rows (4 heads a group, usually)
-  // their scores are not capped or exponentiated (64 requests over 6,000 keys, capped scores: 200 us with them, 193 us without; as a
-  // question to every tile instead of a form of its own it cost steps with more rows 4 %)
-  constexpr bool upper = ROWS != ROWS_8;
   const int qrow = split ? 0 : warp * 16;             // the warp's 16 rows
   constexpr int nk = split ? 1 : MM_KEYS / 16;        // blocks of 16 keys of a tile that the warp takes, from key kb on
   const int kb = split ? warp * 16 : 0;
@@ -572,16 +605,26 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   const int warp_min_limit = s_limit[min(qrow, last_row)];
   const int warp_min_lo = s_lo[min(qrow, last_row)], warp_max_lo = s_lo[min(qrow + 15, last_row)];
 
-  int buf = 1;
+  int buf = SPLIT ? WARP_STAGES - 1 : 1;
   for (int ti = first_tile; ti < list_tiles; ti += tile_step) {
     const int t = tile_of(ti);
-    buf ^= 1;
-    if (ti + tile_step < list_tiles) find_rows(tile_of(ti + tile_step), buf ^ 1);
-    __syncthreads();                                   // rows visible; everyone is done with buffer buf ^ 1
-    if (ti + tile_step < list_tiles) load_tile(buf ^ 1);
-    cp_async_commit();
-    cp_async_wait<1>();                                // tile t (and Q) have landed
-    __syncthreads();
+    if constexpr (SPLIT) {
+      __syncwarp();                                    // this warp is done with the stage that it read last
+      if (ti + (WARP_STAGES - 1) * tile_step < list_tiles) copy_keys(buf);
+      cp_async_commit();
+      look_ahead(ti + WARP_STAGES * tile_step);
+      buf = buf + 1 == WARP_STAGES ? 0 : buf + 1;
+      cp_async_wait<WARP_STAGES - 1>();                // its keys of tile t have landed
+      __syncwarp();
+    } else {
+      buf ^= 1;
+      if (ti + tile_step < list_tiles) find_rows(tile_of(ti + tile_step), buf ^ 1);
+      __syncthreads();                                 // rows visible; everyone is done with buffer buf ^ 1
+      if (ti + tile_step < list_tiles) load_tile(buf ^ 1);
+      cp_async_commit();
+      cp_async_wait<1>();                              // tile t (and Q) have landed
+      __syncthreads();
+    }
     const __nv_bfloat16* tK = sK + buf * MM_KEYS * KSTRIDE;
     const __nv_bfloat16* tV = sV + buf * MM_KEYS * VSTRIDE;
     const int kv0 = t * MM_KEYS;
@@ -610,11 +653,7 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
         for (int i = 0; i < MM_KEYS / 8; i++) {
           if (i >= 2 * nk) break;
 #pragma unroll
-          for (int c = 0; c < 2; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
-          if (upper) {
-#pragma unroll
-            for (int c = 2; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
-          }
+          for (int c = 0; c < 4; c++) s[i][c] = soft_cap_fast(s[i][c] * pre, cap, inv_cap);
         }
       }
       float t_max0 = -INFINITY, t_max1 = -INFINITY;
@@ -664,12 +703,8 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
         if (i >= 2 * nk) break;
         s[i][0] = exp2f(fmaf(s[i][0], scale_log2, -base0)); s[i][1] = exp2f(fmaf(s[i][1], scale_log2, -base0));
         l0[m] += s[i][0] + s[i][1];
-        if (upper) {
-          s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
-          l1[m] += s[i][2] + s[i][3];
-        } else {
-          s[i][2] = s[i][3] = 0.f;
-        }
+        s[i][2] = exp2f(fmaf(s[i][2], scale_log2, -base1)); s[i][3] = exp2f(fmaf(s[i][3], scale_log2, -base1));
+        l1[m] += s[i][2] + s[i][3];
       }
 #pragma unroll
       for (int kk = 0; kk < MM_KEYS / 16; kk++) {
@@ -851,6 +886,305 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
   }
 }
 
+// Single tokens, up to 8 rows of a request and key/value head.  The keys are the MMA's 16 rows and the rows its 8 columns (S^T = K Q^T,
+// O^T = V^T P^T), so that nothing is done for rows that are not there, and a warp keeps half the accumulators.  Each warp takes 16 keys
+// of every 64-key tile through stages of its own, as above; 16 keys that lie in one page and are all seen are one run of memory, whose
+// copies need one look at the block table and no arithmetic.  The four warps' results meet in shared memory at the end.
+//
+// Bound by the caches' way from memory once a tile's instructions are few: 64 requests over 3,000 to 6,000 keys of 4 heads of 128 + 128,
+// capped scores (590 MB):
+// 199 us with the keys as columns and 64-key tiles that a CTA's warps copy together, 167 with a warp's own copies, 145 so (4.1 TB/s); one
+// map of 64 172 and 115, two maps of 64 268 and 150, 8 requests over 3,000 to 6,000 keys 54 and 42.  A warp alone takes 1.1 us a tile.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+
+template <int DIM, int VDIM, int MAPS>
+__global__ void __launch_bounds__(MM_THREADS)
+multimap_rows8_kernel(const MultiMapParams p) {
+  constexpr int KW = MAPS * DIM, KSTRIDE = KW + 8, VSTRIDE = VDIM + 8, KCHUNKS = KW / 8, VCHUNKS = VDIM / 8, WARPS = MM_THREADS / 32;
+  constexpr int STAGE = WARP_KEYS * (KSTRIDE + VSTRIDE), SHARE = MAPS * (2 + VDIM);    // elements of a warp's stage; floats of a row's results
+  extern __shared__ __align__(16) unsigned char mm_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x, g = blockIdx.y, group = p.heads / p.kv_heads;
+  const int q0 = p.q_start[r], rows_total = (p.q_start[r + 1] - q0) * group;
+  if (rows_total <= 0) return;
+  const int* table = p.block_table + (size_t)r * p.table_stride;
+  __nv_bfloat16* stages = (__nv_bfloat16*)mm_smem + warp * WARP_STAGES * STAGE;
+  const int max_limit = p.positions[q0 + (rows_total - 1) / group];                    // positions grow with the row
+  const int min_lo = first_visible(p.mask_kind, p.mask_size, p.positions[q0]);
+  // this lane's columns of S^T and O^T: rows 2 (lane % 4) and the next
+  const int row0 = (lane & 3) * 2;
+  auto limit_of = [&](int row) { return row < rows_total ? p.positions[q0 + row / group] : -1; };
+  const int limit0 = limit_of(row0), limit1 = limit_of(row0 + 1);
+  const int lo0 = first_visible(p.mask_kind, p.mask_size, limit0), lo1 = first_visible(p.mask_kind, p.mask_size, limit1);
+  const int max_lo = first_visible(p.mask_kind, p.mask_size, max_limit), min_limit = p.positions[q0];
+  const int kv_tiles = max_limit / MM_KEYS + 1, tile_lo = min_lo / MM_KEYS;
+  // the tiles of the kept first positions that lie before the window's, then the window's up to the last query
+  const int keep_tiles = min((p.mask_keep + MM_KEYS - 1) / MM_KEYS, tile_lo), list_tiles = keep_tiles + (kv_tiles - tile_lo);
+  auto key_of = [&](int i) { return (i < keep_tiles ? i : tile_lo + (i - keep_tiles)) * MM_KEYS + warp * WARP_KEYS; };   // the warp's first of tile i
+
+  // Q as the second operand: k = 2 (lane % 4) and the next (and 8 further) of row lane / 4
+  uint32_t qf[MAPS][DIM / 16][2];
+  {
+    const int row = lane >> 2;
+    const __nv_bfloat16* src = p.q + (size_t)(q0 + row / group) * p.q_stride + (size_t)(g * group + row % group) * KW + (lane & 3) * 2;
+#pragma unroll
+    for (int m = 0; m < MAPS; m++)
+#pragma unroll
+      for (int kk = 0; kk < DIM / 16; kk++) {
+        qf[m][kk][0] = row < rows_total ? *(const uint32_t*)(src + m * DIM + kk * 16) : 0u;
+        qf[m][kk][1] = row < rows_total ? *(const uint32_t*)(src + m * DIM + kk * 16 + 8) : 0u;
+      }
+  }
+
+  // The next 16 keys to copy: `ahead` is where the first one's rows lie, of all lanes (`whole`: they follow one another), or lane l holds
+  // where key l's rows lie, -1 if no row sees it.
+  const bool runs = p.page_tokens % WARP_KEYS == 0;
+  long long ahead = -1;
+  bool whole = false;
+  auto row_of = [&](int key) -> long long {
+    const int page = table[key / p.page_tokens];
+    if (page >= 0 && page < p.num_pages) return ((long long)page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens;
+    atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
+    return -1;
+  };
+  auto look_ahead = [&](int i) {
+    ahead = -1;
+    whole = false;
+    if (i >= list_tiles) return;
+    const int key = key_of(i);
+    if (runs && key + WARP_KEYS - 1 <= max_limit && (key >= min_lo || key + WARP_KEYS <= p.mask_keep)) {
+      ahead = row_of(key);
+      whole = true;                                    // a page that is not there: -1 in every lane
+    } else if (lane < WARP_KEYS && key + lane <= max_limit && (key + lane >= min_lo || key + lane < p.mask_keep)) {
+      ahead = row_of(key + lane);
+    }
+  };
+  auto copy_keys = [&](int stage) {
+    __nv_bfloat16* sk = stages + stage * STAGE;
+    __nv_bfloat16* sv = sk + WARP_KEYS * KSTRIDE;
+    if (whole && ahead >= 0) {
+      const __nv_bfloat16* ks = p.k_cache + ahead * KW + lane * 8;
+      const __nv_bfloat16* vs = p.v_cache + ahead * VDIM + lane * 8;
+#pragma unroll
+      for (int it = 0; it < WARP_KEYS * KCHUNKS / 32; it++) {
+        const int idx = it * 32 + lane;
+        cp_async16(sk + idx / KCHUNKS * KSTRIDE + idx % KCHUNKS * 8, ks + it * 256);
+      }
+#pragma unroll
+      for (int it = 0; it < WARP_KEYS * VCHUNKS / 32; it++) {
+        const int idx = it * 32 + lane;
+        cp_async16(sv + idx / VCHUNKS * VSTRIDE + idx % VCHUNKS * 8, vs + it * 256);
+      }
+      return;
+    }
+#pragma unroll 4
+    for (int idx = lane; idx < WARP_KEYS * KCHUNKS; idx += 32) {
+      const long long at = __shfl_sync(0xffffffffu, ahead, idx / KCHUNKS);
+      __nv_bfloat16* dst = sk + idx / KCHUNKS * KSTRIDE + idx % KCHUNKS * 8;
+      if (at >= 0) cp_async16(dst, p.k_cache + at * KW + idx % KCHUNKS * 8);
+      else *(uint4*)dst = make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll 4
+    for (int idx = lane; idx < WARP_KEYS * VCHUNKS; idx += 32) {
+      const long long at = __shfl_sync(0xffffffffu, ahead, idx / VCHUNKS);
+      __nv_bfloat16* dst = sv + idx / VCHUNKS * VSTRIDE + idx % VCHUNKS * 8;
+      if (at >= 0) cp_async16(dst, p.v_cache + at * VDIM + idx % VCHUNKS * 8);
+      else *(uint4*)dst = make_uint4(0, 0, 0, 0);
+    }
+  };
+  const int first_tile = blockIdx.z, tile_step = p.ksplit;
+  look_ahead(first_tile);
+#pragma unroll
+  for (int d = 0; d < WARP_STAGES - 1; d++) {
+    if (first_tile + d * tile_step < list_tiles) copy_keys(d);
+    cp_async_commit();
+    look_ahead(first_tile + (d + 1) * tile_step);
+  }
+
+  float top0[MAPS], top1[MAPS], sum0[MAPS], sum1[MAPS], o[MAPS][VDIM / 16][4];
+#pragma unroll
+  for (int m = 0; m < MAPS; m++) {
+    top0[m] = top1[m] = -INFINITY;
+    sum0[m] = sum1[m] = 0.f;
+#pragma unroll
+    for (int i = 0; i < VDIM / 16; i++) o[m][i][0] = o[m][i][1] = o[m][i][2] = o[m][i][3] = 0.f;
+  }
+  const float scale_log2 = score_scale(p) * 1.4426950408889634f, inv_cap = p.softcap > 0.f ? 1.0f / p.softcap : 0.f;
+  int stage = WARP_STAGES - 1;                         // the one that is free
+  for (int ti = first_tile; ti < list_tiles; ti += tile_step) {
+    __syncwarp();                                      // this warp is done with the stage that it read last
+    if (ti + (WARP_STAGES - 1) * tile_step < list_tiles) copy_keys(stage);
+    cp_async_commit();
+    look_ahead(ti + WARP_STAGES * tile_step);
+    stage = stage + 1 == WARP_STAGES ? 0 : stage + 1;
+    cp_async_wait<WARP_STAGES - 1>();
+    __syncwarp();
+    const int kv0 = key_of(ti);
+    if (kv0 > max_limit || (kv0 + WARP_KEYS <= min_lo && kv0 >= p.mask_keep)) continue;      // no row sees these keys
+    const __nv_bfloat16* sk = stages + stage * STAGE;
+    const __nv_bfloat16* sv = sk + WARP_KEYS * KSTRIDE;
+#pragma unroll
+    for (int m = 0; m < MAPS; m++) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};        // two chains
+#pragma unroll
+      for (int kk = 0; kk < DIM / 16; kk++) {
+        uint32_t a[4];
+        ldmatrix_x4(a, sk + ((lane & 7) + ((lane >> 3) & 1) * 8) * KSTRIDE + m * DIM + kk * 16 + (lane >> 4) * 8);
+        mma_bf16(kk & 1 ? s2 : s, a, qf[m][kk][0], qf[m][kk][1]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) s[c] += s2[c];
+      if (p.softcap > 0.f) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) s[c] = soft_cap_fast(s[c] * p.scale, p.softcap, inv_cap);
+      }
+      // element c: key lane / 4 (+ 8 for c of 2 and 3), row row0 (+ 1 for odd c)
+      if (kv0 + WARP_KEYS - 1 > min_limit) {
+        const int key = kv0 + (lane >> 2);
+        if (key > limit0) s[0] = -INFINITY;
+        if (key > limit1) s[1] = -INFINITY;
+        if (key + 8 > limit0) s[2] = -INFINITY;
+        if (key + 8 > limit1) s[3] = -INFINITY;
+      }
+      if (kv0 < max_lo) {
+        const int key = kv0 + (lane >> 2);
+        if (key < lo0 && key >= p.mask_keep) s[0] = -INFINITY;
+        if (key < lo1 && key >= p.mask_keep) s[1] = -INFINITY;
+        if (key + 8 < lo0 && key + 8 >= p.mask_keep) s[2] = -INFINITY;
+        if (key + 8 < lo1 && key + 8 >= p.mask_keep) s[3] = -INFINITY;
+      }
+      float n0 = fmaxf(top0[m], fmaxf(s[0], s[2])), n1 = fmaxf(top1[m], fmaxf(s[1], s[3]));
+#pragma unroll
+      for (int i = 4; i < 32; i <<= 1) {
+        n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, i));
+        n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, i));
+      }
+      const float base0 = n0 == -INFINITY ? 0.f : n0 * scale_log2, base1 = n1 == -INFINITY ? 0.f : n1 * scale_log2;
+      if (__any_sync(0xffffffffu, n0 != top0[m] || n1 != top1[m])) {                         // a maximum moved: bring the sums to it
+        const float alpha0 = top0[m] == -INFINITY ? 0.f : exp2f(top0[m] * scale_log2 - base0);
+        const float alpha1 = top1[m] == -INFINITY ? 0.f : exp2f(top1[m] * scale_log2 - base1);
+        top0[m] = n0; top1[m] = n1;
+        sum0[m] *= alpha0; sum1[m] *= alpha1;
+#pragma unroll
+        for (int i = 0; i < VDIM / 16; i++) { o[m][i][0] *= alpha0; o[m][i][1] *= alpha1; o[m][i][2] *= alpha0; o[m][i][3] *= alpha1; }
+      }
+      s[0] = exp2f(fmaf(s[0], scale_log2, -base0)); s[1] = exp2f(fmaf(s[1], scale_log2, -base1));
+      s[2] = exp2f(fmaf(s[2], scale_log2, -base0)); s[3] = exp2f(fmaf(s[3], scale_log2, -base1));
+      sum0[m] += s[0] + s[2];
+      sum1[m] += s[1] + s[3];
+      const uint32_t b0 = transpose_8x8(pack_bf16(s[0], s[1])), b1 = transpose_8x8(pack_bf16(s[2], s[3]));
+#pragma unroll
+      for (int d = 0; d < VDIM / 16; d++) {
+        uint32_t a[4];
+        ldmatrix_x4_trans(a, sv + ((lane & 7) + (lane >> 4) * 8) * VSTRIDE + d * 16 + ((lane >> 3) & 1) * 8);
+        mma_bf16(o[m][d], a, b0, b1);
+      }
+    }
+  }
+  cp_async_wait<0>();
+
+  // every warp's maxima, sums and O of its keys: [warp][8 rows][MAPS][2 + VDIM]
+  __syncthreads();
+  float* shares = (float*)mm_smem;
+  float* turned = shares + WARPS * 8 * SHARE + warp * VDIM;
+#pragma unroll
+  for (int m = 0; m < MAPS; m++) {
+#pragma unroll
+    for (int i = 4; i < 32; i <<= 1) {
+      sum0[m] += __shfl_xor_sync(0xffffffffu, sum0[m], i);
+      sum1[m] += __shfl_xor_sync(0xffffffffu, sum1[m], i);
+    }
+    float* at0 = shares + (warp * 8 + row0) * SHARE + m * (2 + VDIM);
+    float* at1 = at0 + SHARE;
+    if (lane < 4) { at0[0] = top0[m]; at0[1] = sum0[m]; at1[0] = top1[m]; at1[1] = sum1[m]; }
+#pragma unroll
+    for (int d = 0; d < VDIM / 16; d++) {
+      const int dim = 2 + d * 16 + (lane >> 2);
+      at0[dim] = o[m][d][0]; at1[dim] = o[m][d][1]; at0[dim + 8] = o[m][d][2]; at1[dim + 8] = o[m][d][3];
+    }
+  }
+  __syncthreads();
+  constexpr int COLS = (VDIM + 31) / 32;               // a warp finishes a row: columns lane, lane + 32, ...
+  for (int row = warp; row < rows_total; row += WARPS) {
+    const int token = q0 + row / group, head = g * group + row % group;
+    float v[COLS];
+#pragma unroll
+    for (int c = 0; c < COLS; c++) v[c] = 0.f;
+#pragma unroll
+    for (int m = 0; m < MAPS; m++) {
+      const float* base = shares + row * SHARE + m * (2 + VDIM);
+      float top = -INFINITY, sum = 0.f, a[COLS];
+#pragma unroll
+      for (int c = 0; c < COLS; c++) a[c] = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; w++) top = fmaxf(top, base[w * 8 * SHARE]);
+      float top_log2 = top == -INFINITY ? -INFINITY : top * scale_log2;
+      if (p.sink != nullptr && p.ksplit == 1) {
+        const float sk = p.sink[head] * 1.4426950408889634f;
+        top_log2 = fmaxf(top_log2, sk);
+        sum = exp2f(sk - top_log2);
+      }
+#pragma unroll
+      for (int w = 0; w < WARPS; w++) {
+        const float* at = base + w * 8 * SHARE;
+        const float f = at[0] == -INFINITY ? 0.f : exp2f(at[0] * scale_log2 - top_log2);
+        sum = fmaf(at[1], f, sum);
+#pragma unroll
+        for (int c = 0; c < COLS; c++)
+          if (lane + c * 32 < VDIM) a[c] = fmaf(at[2 + lane + c * 32], f, a[c]);
+      }
+      if (p.ksplit > 1) {                              // the CTA's share, for the merge kernel
+        float* dst = p.partial + ((((size_t)r * p.kv_heads + g) * p.ksplit + blockIdx.z) * 16 + row) * SHARE + m * (2 + VDIM);
+        if (lane == 0) { dst[0] = top; dst[1] = sum; }
+#pragma unroll
+        for (int c = 0; c < COLS; c++)
+          if (lane + c * 32 < VDIM) dst[2 + lane + c * 32] = a[c];
+        continue;
+      }
+#pragma unroll
+      for (int c = 0; c < COLS; c++) v[c] += (m == 0 ? 1.0f : -p.lambda) * (a[c] / sum);
+    }
+    if (p.ksplit > 1) continue;
+    float factor = p.out_scale;
+    if (p.norm_eps > 0.f) {
+      float squares = 0.f;
+#pragma unroll
+      for (int c = 0; c < COLS; c++) squares = fmaf(v[c], v[c], squares);
+      factor *= 1.0f / sqrtf(warp_sum(squares) / (float)VDIM + p.norm_eps);
+    }
+    if (MAPS == 1 && p.turn.cos != nullptr) {
+#pragma unroll
+      for (int c = 0; c < COLS; c++)
+        if (lane + c * 32 < VDIM) turned[lane + c * 32] = v[c];
+      __syncwarp();
+      const size_t at = (size_t)min(max(p.positions[token], 0), p.turn.positions - 1) * (VDIM / 2);
+#pragma unroll
+      for (int c = 0; c < COLS; c++) {
+        const int e = lane + c * 32;
+        if (e >= VDIM) continue;
+        const bool leads = p.turn.interleaved ? (e & 1) == 0 : e < VDIM / 2;
+        const int pair = p.turn.interleaved ? e >> 1 : leads ? e : e - VDIM / 2;
+        const float other = turned[p.turn.interleaved ? e ^ 1 : leads ? e + VDIM / 2 : e - VDIM / 2], cs = p.turn.cos[at + pair], sn = p.turn.sin[at + pair];
+        v[c] = leads ? v[c] * cs + other * sn : v[c] * cs - other * sn;
+      }
+      __syncwarp();
+    }
+    const bool per_element = MAPS == 1 && p.gate != nullptr && p.gate_elements;
+    if (p.gate != nullptr && !per_element) factor *= 1.0f / (1.0f + expf(-__bfloat162float(p.gate[(size_t)token * p.gate_stride + head])));
+    __nv_bfloat16* dst = p.out + (size_t)token * p.out_stride + (size_t)head * VDIM;
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+      const int e = lane + c * 32;
+      if (e < VDIM) dst[e] = __float2bfloat16_rn(v[c] * factor * (per_element ? element_gate(p, token, head, VDIM, e) : 1.0f));
+    }
+  }
+}
+
 // One block per (request, key/value head, row): the CTAs' shares of a request's keys into the head's output.
 template <int MAPS>
 __global__ void __launch_bounds__(128)
@@ -925,10 +1259,31 @@ multimap_merge_kernel(const MultiMapParams p, int vdim) {
     if (threadIdx.x + part * 128 < vdim) dst[threadIdx.x + part * 128] = __float2bfloat16_rn(v[part] * factor);
 }
 
+template <int DIM, int VDIM, int MAPS>
+int launch_rows8(const MultiMapParams& p, cudaStream_t stream) {
+  const int stage_bytes = (MM_THREADS / 32) * WARP_STAGES * WARP_KEYS * (MAPS * DIM + VDIM + 16) * 2;
+  const int share_bytes = (MM_THREADS / 32) * (8 * MAPS * (2 + VDIM) + VDIM) * 4;
+  const int smem = stage_bytes > share_bytes ? stage_bytes : share_bytes;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t err = cudaFuncSetAttribute(multimap_rows8_kernel<DIM, VDIM, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return sprout_fail("multimap_attention_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
+    configured = true;
+  }
+  sprout_launch(multimap_rows8_kernel<DIM, VDIM, MAPS>, dim3(p.requests, p.kv_heads, p.ksplit), dim3(MM_THREADS), smem, stream, p);
+  if (int code = sprout_check_launch("multimap_attention_mma")) return code;
+  if (p.ksplit > 1) {
+    sprout_launch(multimap_merge_kernel<MAPS>, dim3(p.requests, p.kv_heads, 16), dim3(128), 0, stream, p, VDIM);
+    return sprout_check_launch("multimap_merge");
+  }
+  return 0;
+}
+
 template <int DIM, int VDIM, int MAPS, int ROWS>
 int launch_multimap(const MultiMapParams& p, int grid_x, cudaStream_t stream) {
   constexpr bool SPLIT = ROWS != ROWS_TILES;
-  const int tiles_bytes = (3 * MM_ROWS * (MAPS * DIM + 8) + 2 * MM_KEYS * (VDIM + 8)) * 2;
+  const int tiles_bytes = SPLIT ? ((16 + WARP_STAGES * MM_KEYS) * (MAPS * DIM + 8) + WARP_STAGES * MM_KEYS * (VDIM + 8)) * 2
+                                : (3 * MM_ROWS * (MAPS * DIM + 8) + 2 * MM_KEYS * (VDIM + 8)) * 2;
   const int merge_bytes = MM_THREADS * MAPS * (VDIM / 8 * 4 + 4) * 4;         // the warps' partial results of a 16-row CTA
   const int smem = tiles_bytes > merge_bytes ? tiles_bytes : merge_bytes;
   static bool configured = false;
@@ -1000,7 +1355,7 @@ SPROUT_API int sprout_multimap_attention_mma(const void* q, int q_stride, const 
   const bool eight = max_q_len * (heads / kv_heads) <= 8;
 #define PICK_ROWS(D, V, M)                                                                                      \
   (!split ? launch_multimap<D, V, M, ROWS_TILES>(p, tiles, stream)                                              \
-          : eight ? launch_multimap<D, V, M, ROWS_8>(p, tiles, stream) : launch_multimap<D, V, M, ROWS_16>(p, tiles, stream))
+          : eight ? launch_rows8<D, V, M>(p, stream) : launch_multimap<D, V, M, ROWS_16>(p, tiles, stream))
 #define PICK(D, V) if (dim == D && vdim == V) return maps == 2 ? PICK_ROWS(D, V, 2) : PICK_ROWS(D, V, 1);
   PICK(32, 64) PICK(64, 64) PICK(64, 128) PICK(128, 128) PICK(16, 32) PICK(32, 32)
 #undef PICK

@@ -1165,6 +1165,21 @@ def test_maps_attention_tcgen05(status, monkeypatch, divided, maps, dim, vdim, h
         assert torch.equal(got, again) and not counters.any()
 
 
+@pytest.mark.parametrize("whole", [False, True])
+@pytest.mark.parametrize("maps,dim,vdim,heads,kv_heads,page,options", [
+    (1, 128, 128, 8, 2, 16, dict(softcap=30.0, sink=True, gate="head")), (1, 64, 128, 12, 1, 8, dict(mask=("window", 130, 5))),
+    (1, 64, 64, 14, 2, 16, dict()), (1, 48, 48, 4, 4, 64, dict(mask=("chunk", 100), gate="element")), (1, 96, 96, 6, 2, 16, dict(turn="half")),
+    (2, 64, 128, 8, 2, 16, dict(norm_eps=1e-5, lam=0.4)), (2, 128, 128, 4, 4, 32, dict(lam=0.3, sink=True)), (2, 16, 32, 16, 1, 8, dict(lam=0.3))])
+def test_maps_attention_single_tokens(status, monkeypatch, whole, maps, dim, vdim, heads, kv_heads, page, options):
+    """One token per request, contexts around a warp's 16 keys, a tile's 64 and the tiles that are on their way, with NaN in every slot
+    that no query sees; a request's keys in one CTA or divided."""
+    from sprout_lm_b200 import kernels
+    if whole:
+        monkeypatch.setattr(kernels, "multimap_key_split", lambda *a, **k: 1)
+    held = [0, 1, 15, 16, 47, 63, 64, 127, 128, 191, 192, 255, 1300]
+    test_maps_attention_tcgen05(status, monkeypatch, False, maps, dim, vdim, heads, kv_heads, page, held, [1] * len(held), options)
+
+
 @pytest.mark.parametrize("maps,dim,vdim,mask,softcap", [(2, 64, 128, None, 0.0), (1, 64, 128, ("window", 700), 0.0), (1, 128, 128, None, 30.0), (1, 64, 64, None, 0.0)])
 def test_maps_attention_tcgen05_is_as_close_to_64_bits(status, monkeypatch, maps, dim, vdim, mask, softcap):
     """A prompt's attention on tcgen05 is no further from float64 than on mma.sync: weights rounded relative to the row's own maximum, sums of
