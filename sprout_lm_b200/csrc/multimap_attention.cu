@@ -454,10 +454,11 @@ constexpr int MM_ROWS = 64, MM_KEYS = 64, MM_THREADS = 128;
 enum RowsForm : int { ROWS_TILES = 0, ROWS_16 = 1 };
 
 // The forms that share keys: each warp takes 16 keys of every 64-key tile and copies them itself, through stages of its own in shared
-// memory, so that no warp waits for another before the end and every warp has two stages on their way while it works on a third.  These
-// launches are bound by the caches' way from memory; a CTA's warps meeting twice a tile, with one tile on its way, read them at 0.45
-// of the copy rate (64 requests over 3,000 to 6,000 keys of 4 heads of 128 + 128).
-constexpr int WARP_KEYS = 16, WARP_STAGES = 3;
+// memory, so that no warp waits for another before the end.  These launches are bound by the caches' way from memory; a CTA's warps
+// meeting twice a tile, with one tile on its way, read them at 0.45 of the copy rate (64 requests over 3,000 to 6,000 keys of 4 heads of
+// 128 + 128).  A third stage a warp costs a CTA its place beside two others on an SM (the same in 4 shares: 132 us with three stages, 128
+// with two).
+constexpr int WARP_KEYS = 16, WARP_STAGES = 2;
 
 template <int DIM, int VDIM, int MAPS, int ROWS>
 __global__ void __launch_bounds__(MM_THREADS)
@@ -541,11 +542,20 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
     }
   };
   const int first_tile = SPLIT ? (int)blockIdx.z : 0, tile_step = SPLIT ? p.ksplit : 1;    // this CTA's tiles: every tile_step-th of the list
-  // keys shared: this warp's 16 keys of a tile, from the rows that its lanes 0 to 15 hold, into a stage
-  long long ahead = -1;                                             // of lane l: key l of the next tile to copy
-  auto look_ahead = [&](int i) { ahead = i < list_tiles && lane < WARP_KEYS ? row_of(tile_of(i) * MM_KEYS + warp * WARP_KEYS + lane) : -1; };
+  // keys shared: this warp's 16 keys of a tile, whose pages its lanes 0 to 15 hold, into a stage
+  constexpr int NO_PAGE = -0x7fffffff;
+  int next_key = 0, next_page = NO_PAGE;                            // of lane l: key l of the next tile to copy, looked up a tile ahead
+  auto look_ahead = [&](int i) {
+    next_page = NO_PAGE;
+    if (i >= list_tiles || lane >= WARP_KEYS) return;
+    next_key = tile_of(i) * MM_KEYS + warp * WARP_KEYS + lane;
+    if (next_key <= max_limit && (next_key >= min_lo || next_key < p.mask_keep)) next_page = table[next_key / p.page_tokens];
+  };
   auto copy_keys = [&](int stage) {
     const int first = (stage * (MM_THREADS / 32) + warp) * WARP_KEYS;
+    long long ahead = -1;
+    if (next_page >= 0 && next_page < p.num_pages) ahead = ((long long)next_page * p.kv_heads + g) * p.page_tokens + next_key % p.page_tokens;
+    else if (next_page != NO_PAGE) atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
 #pragma unroll
     for (int idx = lane; idx < WARP_KEYS * KCHUNKS; idx += 32) {
       const int row = idx / KCHUNKS, c = idx % KCHUNKS;
@@ -893,8 +903,8 @@ multimap_attention_mma_kernel(const MultiMapParams p) {
 //
 // Bound by the caches' way from memory once a tile's instructions are few: 64 requests over 3,000 to 6,000 keys of 4 heads of 128 + 128,
 // capped scores (590 MB):
-// 199 us with the keys as columns and 64-key tiles that a CTA's warps copy together, 167 with a warp's own copies, 145 so (4.1 TB/s); one
-// map of 64 172 and 115, two maps of 64 268 and 150, 8 requests over 3,000 to 6,000 keys 54 and 42.  A warp alone takes 1.1 us a tile.
+// 199 us with the keys as columns and 64-key tiles that a CTA's warps copy together, 126 so (4.7 TB/s); one map of 64 172 and 101, two maps
+// of 64 268 and 136, 8 requests over 3,000 to 6,000 keys 54 and 36.  A warp alone takes 1 us a tile, of latencies behind one another.
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
   uint32_t d;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
@@ -941,32 +951,29 @@ multimap_rows8_kernel(const MultiMapParams p) {
       }
   }
 
-  // The next 16 keys to copy: `ahead` is where the first one's rows lie, of all lanes (`whole`: they follow one another), or lane l holds
-  // where key l's rows lie, -1 if no row sees it.
+  // The next 16 keys to copy: key `next_key` of every lane in page `next_page` (`whole`: the rows follow one another), or lane l's key l;
+  // NO_PAGE: no row sees it.  Looked up a tile ahead and looked at when it is copied, so that nothing waits for the block table.
+  constexpr int NO_PAGE = -0x7fffffff;
   const bool runs = p.page_tokens % WARP_KEYS == 0;
-  long long ahead = -1;
+  const int page_shift = (p.page_tokens & (p.page_tokens - 1)) == 0 ? __ffs(p.page_tokens) - 1 : -1;
+  auto page_of = [&](int key) { return page_shift >= 0 ? key >> page_shift : key / p.page_tokens; };
+  int next_key = 0, next_page = NO_PAGE;
   bool whole = false;
-  auto row_of = [&](int key) -> long long {
-    const int page = table[key / p.page_tokens];
-    if (page >= 0 && page < p.num_pages) return ((long long)page * p.kv_heads + g) * p.page_tokens + key % p.page_tokens;
-    atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
-    return -1;
-  };
   auto look_ahead = [&](int i) {
-    ahead = -1;
-    whole = false;
+    next_page = NO_PAGE;
     if (i >= list_tiles) return;
     const int key = key_of(i);
-    if (runs && key + WARP_KEYS - 1 <= max_limit && (key >= min_lo || key + WARP_KEYS <= p.mask_keep)) {
-      ahead = row_of(key);
-      whole = true;                                    // a page that is not there: -1 in every lane
-    } else if (lane < WARP_KEYS && key + lane <= max_limit && (key + lane >= min_lo || key + lane < p.mask_keep)) {
-      ahead = row_of(key + lane);
-    }
+    whole = runs && key + WARP_KEYS - 1 <= max_limit && (key >= min_lo || key + WARP_KEYS <= p.mask_keep);
+    next_key = whole ? key : key + lane;
+    if (whole || (lane < WARP_KEYS && next_key <= max_limit && (next_key >= min_lo || next_key < p.mask_keep)))
+      next_page = table[page_of(next_key)];
   };
   auto copy_keys = [&](int stage) {
     __nv_bfloat16* sk = stages + stage * STAGE;
     __nv_bfloat16* sv = sk + WARP_KEYS * KSTRIDE;
+    long long ahead = -1;                              // where the rows of this lane's key lie
+    if (next_page >= 0 && next_page < p.num_pages) ahead = ((long long)next_page * p.kv_heads + g) * p.page_tokens + (next_key - page_of(next_key) * p.page_tokens);
+    else if (next_page != NO_PAGE) atomicOr(p.status, SPROUT_STATUS_BAD_PAGE);
     if (whole && ahead >= 0) {
       const __nv_bfloat16* ks = p.k_cache + ahead * KW + lane * 8;
       const __nv_bfloat16* vs = p.v_cache + ahead * VDIM + lane * 8;
