@@ -1765,8 +1765,28 @@ def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: in
 
 # ---------------------------------------------------------------------------------- recurrences with a decay made from the input
 
-SCAN_CHUNK = 64             # tokens of a chunk of the gated scan
+SCAN_CHUNK = 64             # tokens of a chunk of the gated scan that is walked token by token
 SCAN_CHUNKED_FROM = 128     # a step whose longest portion has at least this many tokens walks chunks side by side
+# The same where chunks are walked 16 tokens at a time on tensor cores.  On the device they pay from 33 tokens on (16 heads of 128 x 128, a
+# layer: 64 tokens 101 us walked whole, 63 in chunks, 100 tokens 140 and 71), but launched one by one their three more kernels take the
+# host 25 us (the same layers 100 and 123 us, 138 and 123).
+SCAN_MMA_CHUNKED_FROM = 96
+
+
+@functools.lru_cache(maxsize=4096)
+def scan_mma_chunk(tokens: int, requests: int, longest: int, blocks: int, sms: int) -> int:
+    """Tokens of a chunk where chunks are walked 16 tokens at a time, with ``blocks`` blocks a chunk: the least of rounds of blocks (two an
+    SM) x steps of 16 tokens, 9.2 us each in both walks, 2 us a round, and 0.65 us a chunk of the longest portion for the carry.  Measured at 4, 8 and
+    16 heads of 128 x 128 over 14 steps of 130 to 2,500 tokens it is within 3 % of the best of these sizes.  A layer, 64 tokens a chunk
+    and so: 3 portions of 2,500 tokens 299 and 278 us, 1 of 2,048 238 and 227, of 400 114 and 94, 8 heads 92 and 68."""
+    best, least = SCAN_CHUNK, None
+    for chunk in (16, 32, 48, 64, 80, 96, 112, 128, 144, 160, 192):
+        grid = -(-(2 * tokens + (requests - 1) * chunk) // (2 * chunk)) * blocks       # half a chunk of every request but one is empty
+        rounds = -(-grid // (2 * sms))
+        cost = rounds * (9.2 * (chunk // 16) + 2.0) + 0.65 * -(-longest // chunk)
+        if least is None or cost < least:
+            best, least = chunk, cost
+    return best
 
 
 def _scan_view(t, name: str, width: int, dtype):
@@ -1793,7 +1813,8 @@ def gated_scan(q, k, v, z, bias, ctx, state, out, heads: int, groups: int, dim: 
     column v_cols is fed the constant 1 as a value (the columns after it 0): that column of the state is then the sum of the
     decayed c k, and that column of the output its product with q_scale q, a normaliser.
     out float32 [tokens, heads * vdim].  A step whose longest portion has ``SCAN_CHUNKED_FROM`` tokens or more cuts the
-    portions into chunks of ``SCAN_CHUNK`` tokens that are walked side by side (``SPROUT_GATED_SCAN=whole`` keeps one walk
+    portions into chunks of ``SCAN_CHUNK`` tokens (bfloat16 and key sizes 64 and 128 with decays per channel or head: from
+    ``SCAN_MMA_CHUNKED_FROM`` tokens, of ``scan_mma_chunk``) that are walked side by side (``SPROUT_GATED_SCAN=whole`` keeps one walk
     per request): scratch for every token's decay and every chunk's sums."""
     tokens, dtype = v.shape[0], v.dtype
     v_cols = v.shape[1] // heads if ones_col else vdim
@@ -1828,9 +1849,14 @@ def gated_scan(q, k, v, z, bias, ctx, state, out, heads: int, groups: int, dim: 
     global LAUNCHES
     requests = state.slots.numel()
     da = dc = sums = prods = None
-    max_chunks = 0
-    if getattr(ctx, "max_q_len", 1) >= SCAN_CHUNKED_FROM and os.environ.get("SPROUT_GATED_SCAN", "chunks") != "whole":
-        max_chunks = tokens // SCAN_CHUNK + requests
+    max_chunks, chunk = 0, SCAN_CHUNK
+    longest = getattr(ctx, "max_q_len", 1)
+    mma = dtype == torch.bfloat16 and dim in (64, 128) and floor is None and bonus is None and v_cols % 8 == 0 \
+        and (q_stride | k_stride | v_stride) % 8 == 0 and (q_ptr | k_ptr | v_ptr) % 16 == 0
+    if longest >= (SCAN_MMA_CHUNKED_FROM if mma else SCAN_CHUNKED_FROM) and os.environ.get("SPROUT_GATED_SCAN", "chunks") != "whole":
+        if mma:
+            chunk = scan_mma_chunk(tokens, requests, longest, heads * (1 if vdim <= 64 else -(-vdim // 128)), sm_count(v.device))
+        max_chunks = tokens // chunk + requests
         if given is None:
             da = torch.empty(tokens * (heads if per_head else heads * dim), dtype=torch.float32, device=v.device)
             dc = torch.empty(tokens * heads, dtype=torch.float32, device=v.device) if per_head else None
@@ -1844,7 +1870,7 @@ def gated_scan(q, k, v, z, bias, ctx, state, out, heads: int, groups: int, dim: 
          _ptr(bonus, "bonus", torch.float32, True), 1.0 / float(tau), float(q_scale), 2 if given is not None else 3 if floor is not None else 4 if bonus is not None else 1 if per_head else 0, state.slots.numel(), heads, groups, dim, vdim,
          _ptr(ctx.q_start, "q_start", torch.int32), _ptr(state.slots, "state_slots", torch.int32),
          _ptr(buffer, "state", torch.float32), buffer.shape[0], _ptr(out, "out", torch.float32),
-         _ptr(status, "status", torch.int32), tokens, SCAN_CHUNK, max_chunks, _ptr(da, "decays", torch.float32, True),
+         _ptr(status, "status", torch.int32), tokens, chunk, max_chunks, _ptr(da, "decays", torch.float32, True),
          _ptr(dc, "steps", torch.float32, True), _ptr(sums, "sums", torch.float32, True), _ptr(prods, "products", torch.float32, True),
          v_cols, 1 if ones_col else 0, 1 if q_silu else 0, _stream())
 

@@ -359,3 +359,16 @@ def test_linear_plan_covers_the_matrix_and_fits(ctas):
         qkv, o = kernels.small_batch_plan("linear", 8, 1152, 896), kernels.small_batch_plan("linear", 8, 896, 896)
         assert (qkv["row_groups"], qkv["k_splits"], qkv["max_tiles"], qkv["max_ksteps"]) == (9, 16, 8, 4)
         assert (o["row_groups"], o["k_splits"], o["max_tiles"], o["max_ksteps"]) == (7, 21, 8, 3)
+
+
+def test_scan_chunk_fills_the_device_in_few_steps():
+    """Chunks of the gated scan: multiples of 16 tokens, short while the device has room for the blocks, one round of blocks where that
+    takes no more steps, the longest for portions that no size fits."""
+    from sprout_lm_b200.kernels import scan_mma_chunk
+    assert scan_mma_chunk(130, 1, 130, 16, 148) == 16 and scan_mma_chunk(400, 1, 400, 16, 148) == 32
+    assert scan_mma_chunk(2048, 1, 2048, 16, 148) == 128 and scan_mma_chunk(2500, 3, 1000, 16, 148) == 160
+    for tokens in (33, 500, 5000, 200000):
+        for blocks in (1, 8, 64):
+            chunk = scan_mma_chunk(tokens, 1, tokens, blocks, 148)
+            assert chunk % 16 == 0 and 16 <= chunk <= 192
+    assert scan_mma_chunk(200000, 1, 200000, 64, 148) == 192
