@@ -347,8 +347,10 @@ int sprout_experts_product_tc(const void* rows, const int* offsets, const int* o
   CUtensorMap map_w;
   RowMaps maps_x;
   if (weight_map(w, experts, N, K, gated, &map_w)) return 1;
-  for (int b = 0; b < ROW_MAPS; b++)
-    if (tensor_map(rows, entries, K, K, 8 << b, &maps_x.box[b])) return 1;
+  for (int b = 0; b < ROW_MAPS; b++) {
+    if (b > 0 && (8 << b) >= entries) maps_x.box[b] = maps_x.box[b - 1];       // no tile has so many rows: not used
+    else if (tensor_map(rows, entries, K, K, 8 << b, &maps_x.box[b])) return 1;
+  }
   if (unit < 0) return launch_experts<KIND_DOWN>(map_w, maps_x, p, work, stream);
   if (unit == sprout_experts::UNIT_CLAMPED) return launch_experts<KIND_CLAMPED>(map_w, maps_x, p, work, stream);
   if (unit == sprout_experts::UNIT_SILU) return launch_experts<KIND_SILU>(map_w, maps_x, p, work, stream);

@@ -107,6 +107,7 @@ _SIGNATURES = {
     "sprout_latent_rotate": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_latent_unfolded_attention": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P],
     "sprout_moe_tc_supported": [_I, _I, _I, _I, _I, _I],
+    "sprout_moe_routed": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
 }
 
 _lock = threading.Lock()
@@ -1731,6 +1732,41 @@ def _experts_route(entries: int, experts: int, top: int, width: int, ff: int, h_
     if not lib.sprout_moe_mma_supported(width, ff, h_stride):
         return "plain"
     return "tcgen05" if width * ff >= least and lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
+
+
+def moe_routed(h, router, correction, counts, offsets, w_gate_up, w_down, experts: int, top: int, scale: float, limit: float, alpha: float,
+               unit=None, weight_on_input: bool = False, groups=None, renormalize: bool = True, extra_out=None, sigmoid: bool = False, status=None):
+    """``moe_route``, ``moe_arrange`` and ``moe_experts`` of bfloat16 rows on tcgen05 in one call (a layer of a small step is bound by the
+    host): (ids, weights, place_of, rows) for ``moe_combine``, or None where these sizes take other kernels."""
+    global LAUNCHES
+    T, width = h.shape
+    entries, ff = T * top, w_down.shape[2]
+    if h.dtype != torch.bfloat16 or h.stride(1) != 1 or status is None or os.environ.get("SPROUT_MOE", "mma") != "mma" \
+            or _experts_route(entries, experts, top, width, ff, h.stride(0), EXPERTS_TC_ELEMENTS) != "tcgen05" \
+            or (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16:
+        return None
+    extra = 0 if extra_out is None else extra_out.shape[1]
+    outputs = router.shape[0] - extra
+    group_count, group_keep = (int(groups[0]), int(groups[1])) if groups else (1, 1)
+    code = _unit_code(unit, limit)
+    if (extra and (extra_out.dtype != torch.float32 or not extra_out.is_contiguous() or extra_out.shape[0] != T)) or not router.is_contiguous() \
+            or router.shape[1] != width or (correction is not None and correction.numel() != outputs) or counts.numel() < max(experts, 1) \
+            or offsets.numel() < experts + 1 or tuple(w_gate_up.shape) != (experts, ff if code == 1 else 2 * ff, width) \
+            or tuple(w_down.shape) != (experts, width, ff) or not w_gate_up.is_contiguous() or not w_down.is_contiguous():
+        raise KernelError("moe_routed: shapes do not fit")
+    device = h.device
+    ids, order, place_of = torch.empty((3, T, top), dtype=torch.int32, device=device).unbind(0)
+    weights = torch.empty((T, top), dtype=torch.float32, device=device)
+    act = torch.empty((entries, ff), dtype=h.dtype, device=device)
+    rows = torch.empty((entries, width), dtype=torch.float32, device=device)       # the gathered rows' place too: read before these are written
+    _run("sprout_moe_routed", _ptr(h, "h"), h.stride(0), _ptr(router, "router", torch.float32), _ptr(correction, "correction", torch.float32, True),
+         ids.data_ptr(), weights.data_ptr(), _ptr(counts, "counts", torch.int32), _ptr(offsets, "offsets", torch.int32), order.data_ptr(),
+         place_of.data_ptr(), _ptr(w_gate_up, "w_gate_up", torch.bfloat16), _ptr(w_down, "w_down", torch.bfloat16), act.data_ptr(),
+         rows.data_ptr(), T, width, outputs, experts, top, float(scale), extra, _ptr(extra_out, "extra_out", torch.float32, True),
+         group_count, group_keep, 1 if renormalize else 0, 1 if sigmoid else 0, ff, code, 1 if weight_on_input else 0, float(limit), float(alpha),
+         _ptr(status, "status", torch.int32), _stream())
+    LAUNCHES += 4               # five kernels behind one call
+    return ids, weights, place_of, rows
 
 
 def moe_experts(h, order, offsets, w_gate_up, w_down, act, rows_out, experts: int, top: int, limit: float, alpha: float, unit=None,

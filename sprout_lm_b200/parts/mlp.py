@@ -347,16 +347,12 @@ class RoutedExperts(Part):
         self.counts = torch.zeros(max(self.experts, 1), dtype=torch.int32, device=device)   # left zeroed by every step
         self.offsets = torch.zeros(self.experts + 1, dtype=torch.int32, device=device)
 
-    def forward(self, h, x, ctx=None):
+    def _routed_by_steps(self, h, scale, routing):
         tokens, device = h.shape[0], h.device
         entries = tokens * self.top
         ids = torch.empty((tokens, self.top), dtype=torch.int32, device=device)
         weights = torch.empty((tokens, self.top), dtype=torch.float32, device=device)
-        gate_logits = torch.empty((tokens, 1), dtype=torch.float32, device=device) if self.shared_gate else None
-        # a factor on the output goes onto the weights, unless they go into the experts
-        scale = self.scale if self.weight_on_input else self.scale * self.out_scale
-        kernels.moe_route(h, self.router, self.correction, ids, weights, self.counts, self.experts, self.top, scale,
-                          groups=self.groups, renormalize=self.renormalize, extra_out=gate_logits, sigmoid=self.sigmoid)
+        kernels.moe_route(h, self.router, self.correction, ids, weights, self.counts, self.experts, self.top, scale, **routing)
         place_of = torch.empty(entries, dtype=torch.int32, device=device)
         rows = None
         if self.experts:
@@ -368,6 +364,18 @@ class RoutedExperts(Part):
                                 self.expert_limit, self.alpha, unit=self.expert_kind, row_weights=weights if self.weight_on_input else None, status=self.runtime.status)
         else:
             place_of.fill_(-1)
+        return ids, weights, place_of, rows
+
+    def forward(self, h, x, ctx=None):
+        tokens, device = h.shape[0], h.device
+        gate_logits = torch.empty((tokens, 1), dtype=torch.float32, device=device) if self.shared_gate else None
+        # a factor on the output goes onto the weights, unless they go into the experts
+        scale = self.scale if self.weight_on_input else self.scale * self.out_scale
+        routing = dict(groups=self.groups, renormalize=self.renormalize, extra_out=gate_logits, sigmoid=self.sigmoid)
+        routed = kernels.moe_routed(h, self.router, self.correction, self.counts, self.offsets, self.w_gate_up, self.w_down, self.experts, self.top,
+                                    scale, self.expert_limit, self.alpha, unit=self.expert_kind, weight_on_input=self.weight_on_input,
+                                    status=self.runtime.status, **routing) if self.experts else None
+        ids, weights, place_of, rows = routed if routed is not None else self._routed_by_steps(h, scale, routing)
         if self.shared is not None and self.shared_gate and self.plain:
             self.shared.forward(h, x, row_logits=gate_logits)
         elif self.shared is not None and self.shared_gate:
