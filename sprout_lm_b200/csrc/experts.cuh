@@ -21,6 +21,6 @@ __device__ __forceinline__ float glu(int unit, float g, float u, float limit, fl
 // One of the experts' products on tcgen05 in CTA pairs (experts_tcgen05.cu): rows [entries, K] bfloat16 arranged by expert (`offsets`
 // [experts + 1]), w [experts, matrix rows, K].  GLU or gelu units (`unit` >= 0): out bfloat16 [entries, N], the matrix has 2 N rows
 // (gate rows, then up rows) or for UNIT_PLAIN N; `row_weights` (of entry order[row]) multiply the products before the activation.
-// `unit` -1: out float32 [entries, N], the products as they are.
-int sprout_experts_product_tc(const void* rows, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
+// `unit` -1: out float32 [entries, N], the products as they are.  `offsets` null: one expert that has every row.
+int sprout_experts_product_tc(const void* rows, int row_stride, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
                               int K, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream);

@@ -49,8 +49,8 @@ struct RowMaps { CUtensorMap box[ROW_MAPS]; };
 
 struct ExpertsParams {
   void* out;                       // [entries, N]: bfloat16, or float32 for KIND_DOWN
-  int N, K, experts;
-  const int* offsets; const int* order;
+  int N, K, experts, entries;
+  const int* offsets; const int* order;        // null: one expert with all entries
   const float* row_weights;        // of entry order[row], or null: multiply the products before the activation
   float limit, alpha;
   int* status;
@@ -101,7 +101,8 @@ experts_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   if (warp == 0) {
     int before = 0;
     for (int e0 = 0; e0 < p.experts; e0 += 32) {
-      const int e = e0 + lane, begin = e < p.experts ? p.offsets[e] : 0, end = e < p.experts ? p.offsets[e + 1] : 0;
+      const int e = e0 + lane;
+      const int begin = p.offsets && e < p.experts ? p.offsets[e] : 0, end = e >= p.experts ? 0 : p.offsets ? p.offsets[e + 1] : p.entries;
       const int own = tiles_of(end - begin);
       int sum = own;
 #pragma unroll
@@ -335,21 +336,22 @@ int launch_experts(const CUtensorMap& map_w, const RowMaps& maps_x, const Expert
 
 }  // namespace
 
-int sprout_experts_product_tc(const void* rows, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
+int sprout_experts_product_tc(const void* rows, int row_stride, const int* offsets, const int* order, const void* w, void* out, int entries, int experts, int N,
                               int K, int unit, const float* row_weights, float limit, float alpha, int* status, cudaStream_t stream) {
   const bool gated = unit == sprout_experts::UNIT_CLAMPED || unit == sprout_experts::UNIT_SILU;
-  SPROUT_REQUIRE(rows && offsets && order && w && out && status && entries > 0 && experts > 0, "experts_product: bad arguments");
+  SPROUT_REQUIRE(rows && w && out && status && entries > 0 && experts > 0 && (offsets ? (order != nullptr) : (experts == 1 && !row_weights)),
+                 "experts_product: bad arguments");
   SPROUT_REQUIRE(N % 8 == 0 && K % 8 == 0 && experts <= MAX_EXPERTS, "experts_product: sizes in multiples of 8, up to 2,048 experts (N=%d K=%d, %d experts)", N, K, experts);
   const int features = gated ? BLOCK_M : 2 * BLOCK_M;                  // of a pair's tile
   const long long work = ((long long)entries / MAX_N + experts) * ((N + features - 1) / features);        // at most, whatever the routing
   SPROUT_REQUIRE((long long)experts * N * 2 <= 0x7fffffffLL && work <= 0x7fffffffLL, "experts_product: too many rows");
-  const ExpertsParams p{out, N, K, experts, offsets, order, row_weights, limit, alpha, status};
+  const ExpertsParams p{out, N, K, experts, entries, offsets, order, row_weights, limit, alpha, status};
   CUtensorMap map_w;
   RowMaps maps_x;
   if (weight_map(w, experts, N, K, gated, &map_w)) return 1;
   for (int b = 0; b < ROW_MAPS; b++) {
     if (b > 0 && (8 << b) >= entries) maps_x.box[b] = maps_x.box[b - 1];       // no tile has so many rows: not used
-    else if (tensor_map(rows, entries, K, K, 8 << b, &maps_x.box[b])) return 1;
+    else if (tensor_map(rows, entries, K, row_stride, 8 << b, &maps_x.box[b])) return 1;
   }
   if (unit < 0) return launch_experts<KIND_DOWN>(map_w, maps_x, p, work, stream);
   if (unit == sprout_experts::UNIT_CLAMPED) return launch_experts<KIND_CLAMPED>(map_w, maps_x, p, work, stream);

@@ -790,9 +790,9 @@ SPROUT_API int sprout_moe_experts_tc(const void* h, int h_stride, const int* ord
   sprout_launch(moe_gather_kernel, dim3(entries), dim3(256), 0, stream, (const __nv_bfloat16*)h, h_stride, order, offsets, experts, top, width,
                 (__nv_bfloat16*)gathered);
   if (int code = sprout_check_launch("moe_gather")) return code;
-  if (int code = sprout_experts_product_tc(gathered, offsets, order, w_gate_up, act, entries, experts, ff, width, unit, row_weights, limit, alpha, status, stream))
+  if (int code = sprout_experts_product_tc(gathered, width, offsets, order, w_gate_up, act, entries, experts, ff, width, unit, row_weights, limit, alpha, status, stream))
     return code;
-  return sprout_experts_product_tc(act, offsets, order, w_down, rows_out, entries, experts, width, ff, -1, nullptr, 0.f, 0.f, status, stream);
+  return sprout_experts_product_tc(act, ff, offsets, order, w_down, rows_out, entries, experts, width, ff, -1, nullptr, 0.f, 0.f, status, stream);
 }
 
 // sprout_moe_route, sprout_moe_arrange and sprout_moe_experts_tc behind one call, for bfloat16 rows of sizes that the last takes;
@@ -810,6 +810,14 @@ SPROUT_API int sprout_moe_routed(const void* h, int h_stride, const float* route
   // the gathered rows lie where the down product, which runs once they have been read, writes its results
   return sprout_moe_experts_tc(h, h_stride, order, offsets, w_gate_up, w_down, rows_out, act, rows_out, entries, experts, top, width, ff, unit,
                                weight_rows ? weights : nullptr, limit, alpha, status, stream);
+}
+
+// out [tokens, ff] bfloat16 = the clamped gated unit of h w^T, w [2 ff, width] with the gate rows first.
+SPROUT_API int sprout_clamped_glu_product(const void* h, int h_stride, const void* w, void* out, int tokens, int ff, int width, float limit, float alpha,
+                                          int* status, cudaStream_t stream) {
+  SPROUT_REQUIRE(h && w && out && status && tokens > 0 && ff > 0 && width > 0 && h_stride >= width && h_stride % 8 == 0, "clamped_glu_product: bad arguments");
+  SPROUT_REQUIRE((((uintptr_t)h | (uintptr_t)w | (uintptr_t)out) & 15) == 0, "clamped_glu_product: buffers must start on 16-byte boundaries");
+  return sprout_experts_product_tc(h, h_stride, nullptr, nullptr, w, out, tokens, 1, ff, width, UNIT_CLAMPED, nullptr, limit, alpha, status, stream);
 }
 
 // act [entries, ff] bfloat16 = glu(W_gate a, W_up a); rows_out [entries, width] float32 = W_down act, over the arranged rows.

@@ -108,6 +108,7 @@ _SIGNATURES = {
     "sprout_latent_unfolded_attention": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P],
     "sprout_moe_tc_supported": [_I, _I, _I, _I, _I, _I],
     "sprout_moe_routed": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
+    "sprout_clamped_glu_product": [_P, _I, _P, _P, _I, _I, _I, _F, _F, _P, _P],
 }
 
 _lock = threading.Lock()
@@ -1319,6 +1320,27 @@ def relu2(z, out):
     if not z.is_contiguous() or not out.is_contiguous() or z.shape != out.shape or z.dtype != out.dtype:
         raise KernelError("relu2: z and out must be contiguous and alike")
     _run("sprout_relu2", _ptr(z, "z"), _ptr(out, "out"), _dtype_code(z.dtype), z.numel(), _stream())
+
+
+# Tiles (256 tokens x 128 units) from which a clamped gated unit's product has its activation in the epilogue: the kernel's pairs of CTAs
+# leave SMs idle below (the unit with its down product, activation in a kernel of its own and so: 2,048 tokens of 2,048 over 2,048 62 and
+# 56 us, 512 tokens 30 and 34; 400 of 4,096 over 1,024 32 and 28; 1,024 of 1,024 over 1,024 24 and 28)
+GLU_PRODUCT_TILES = 64
+
+
+def clamped_glu_product(h, gate_up, out, limit: float, alpha: float, status) -> bool:
+    """out = glu_clamped(h gate_up^T) in one kernel, gate_up [2 ff, hidden] with the gate rows first: the routed experts' product with one
+    expert that has every row.  False, and nothing done, where the sizes or the addresses are not the kernel's or it does not pay."""
+    tokens, hidden = h.shape
+    ff = out.shape[1]
+    if h.dtype != torch.bfloat16 or -(-tokens // 256) * -(-ff // 128) < GLU_PRODUCT_TILES or ff < 256 or hidden < 512 or (hidden | ff | h.stride(0)) % 8 or h.stride(1) != 1 \
+            or (h.data_ptr() | gate_up.data_ptr() | out.data_ptr()) % 16:
+        return False
+    if tuple(gate_up.shape) != (2 * ff, hidden) or out.shape[0] != tokens or not gate_up.is_contiguous() or not out.is_contiguous():
+        raise KernelError("clamped_glu_product: shapes do not fit")
+    _run("sprout_clamped_glu_product", _ptr(h, "h"), h.stride(0), _ptr(gate_up, "gate_up", torch.bfloat16), _ptr(out, "out", torch.bfloat16), tokens, ff,
+         hidden, float(limit), float(alpha), _ptr(status, "status", torch.int32), _stream())
+    return True
 
 
 def glu_clamped(gate_up, out, limit: float, alpha: float):

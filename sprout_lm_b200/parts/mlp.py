@@ -140,15 +140,15 @@ class ClampedGLU:
 
     def __init__(self, gate, up, down, limit: float, alpha: float, source: WeightSource):
         status = source.runtime.status
-        self.limit, self.alpha = float(limit), float(alpha)
+        self.limit, self.alpha, self.status = float(limit), float(alpha), status
         self.ff = gate.shape[0]
         self.gate_up = Linear(source.to_device_matrix(torch.cat([gate, up], dim=0)), None, status, any_inner_size=True)
         self.down = Linear(source.to_device_matrix(down), None, status, any_inner_size=True)
 
     def forward(self, h, x):
-        gate_up = self.gate_up.forward(h)
         act = torch.empty((h.shape[0], self.ff), dtype=h.dtype, device=h.device)
-        kernels.glu_clamped(gate_up, act, self.limit, self.alpha)
+        if not kernels.clamped_glu_product(h, self.gate_up.weight, act, self.limit, self.alpha, self.status):
+            kernels.glu_clamped(self.gate_up.forward(h), act, self.limit, self.alpha)
         self.down.forward(act, residual=x)
 
 

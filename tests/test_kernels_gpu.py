@@ -1291,6 +1291,24 @@ def test_experts_on_tcgen05(status, monkeypatch, unit, counts, width, ff, weight
         assert (tc - plain).abs().max() <= 2 ** -6 * plain.abs().max()
 
 
+@pytest.mark.parametrize("tokens,hidden,ff,stride", [(1, 512, 256, 512), (257, 520, 328, 1040), (700, 1032, 1040, 1032)])
+def test_clamped_glu_product(status, monkeypatch, tokens, hidden, ff, stride):
+    """A gated unit's product with the activation in its epilogue against the product and the activation's kernel, rows side by side or apart."""
+    from sprout_lm_b200 import kernels
+    g = torch.Generator().manual_seed(tokens)
+    h = torch.randn(tokens, stride, generator=g).to(torch.bfloat16).to(DEV)[:, :hidden]
+    w = (torch.randn(2 * ff, hidden, generator=g) * 2.0 * hidden ** -0.5).to(torch.bfloat16).to(DEV)
+    got, want = (torch.zeros(tokens, ff, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    monkeypatch.setattr(kernels, "GLU_PRODUCT_TILES", 0)             # the kernel under test, whether it pays at these sizes or not
+    assert kernels.clamped_glu_product(h, w, got, 2.0, 1.702, status) and int(status.item()) == 0
+    gate_up = torch.empty(tokens, 2 * ff, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_bf16(h, w, gate_up, status)
+    kernels.glu_clamped(gate_up, want, 2.0, 1.702)
+    # a product on the edge of a bfloat16 rounding moves its activation by 2^-8 of itself
+    error = got.float() - want.float()
+    assert error.norm() <= 2 ** -9 * want.float().norm() and error.abs().max() <= 2 ** -6 * want.float().abs().max()
+
+
 @pytest.mark.parametrize("unit", ["clamped_glu", "plain"])
 def test_experts_tiles_of_every_width(status, monkeypatch, unit):
     """Rows of an expert in one tile of 16 to 256 columns, in two and more of equal size, features and K that no tile divides."""
