@@ -1,7 +1,7 @@
 // out[m, n] = sum_k A[m, k] * W[n, k] (+ bias[n]) (+ residual[m, n]) on CUDA cores with
 // float32 fused multiply-adds: the matrix product of the true 32-bit path (no tensor cores,
 // no reduced-precision mode), and a plain reference for the tensor-core kernels.  Each output
-// element is one sum in ascending k, or two or four such sums over equal shares of K added in their order; how many follows from the
+// element is one sum in ascending k, or two to eight such sums over equal shares of K added in their order; how many follows from the
 // matrix alone (`split_of`), so its value does not depend on how many rows the call has, on where a row sits among them, or on the
 // tile that a call's sizes pick.
 //
@@ -278,7 +278,7 @@ int launch_tile(const TA* A, const TW* W, const float* bias, const float* residu
 
 // The tile for a call's sizes, measured in float32.  Few rows are a stream of weights: rows of 128 bytes a
 // k-block and no more sums than rows.  Between: 64 x 64, so that small matrices still put a CTA on most SMs.  From eight CTAs an SM on
-// (shares counted), 128 x 64 with 8 x 8 sums a thread reads less shared memory a multiply-add (2,048 rows of 9,728 x 896: 745 us = 48
+// (shares counted; from sixteen where there are eight shares), 128 x 64 with 8 x 8 sums a thread reads less shared memory a multiply-add (2,048 rows of 9,728 x 896: 745 us = 48
 // TFLOP/s; 64 x 64 802, 128 x 128 761 us).
 template <int SPLIT, bool VEC, typename TA, typename TW, typename TO>
 int launch_sizes(const TA* A, const TW* W, const float* bias, const float* residual, TO* out, int M, int N, int K, int lda, int ldo,
@@ -286,7 +286,7 @@ int launch_sizes(const TA* A, const TW* W, const float* bias, const float* resid
   if (M <= 8) return launch_tile<8, 128, 32, 2, 4, SPLIT, VEC>(A, W, bias, residual, out, M, N, K, lda, ldo, stream);
   if (M <= 16) return launch_tile<16, 128, 32, 4, 4, SPLIT, VEC>(A, W, bias, residual, out, M, N, K, lda, ldo, stream);
   const long long tiles = (long long)((M + 127) / 128) * ((N + 63) / 64) * SPLIT;
-  if (tiles >= 8 * sprout_sm_count()) return launch_tile<128, 64, 16, 8, 8, SPLIT, VEC>(A, W, bias, residual, out, M, N, K, lda, ldo, stream);
+  if (tiles >= (SPLIT > 4 ? 16 : 8) * sprout_sm_count()) return launch_tile<128, 64, 16, 8, 8, SPLIT, VEC>(A, W, bias, residual, out, M, N, K, lda, ldo, stream);
   return launch_tile<64, 64, 16, 8, 4, SPLIT, VEC>(A, W, bias, residual, out, M, N, K, lda, ldo, stream);
 }
 
@@ -294,10 +294,11 @@ int launch_sizes(const TA* A, const TW* W, const float* bias, const float* resid
 // have too few tiles for the device (M x 896 x 4,864 in one, two, four shares: 1 row 135, 73, 33 us; 64 rows 203, 113, 54; 512 rows 203,
 // 152, 153; 2,048 rows 712, 468, 413; M x 1,152 x 896: 64 rows 39, 24, 13, 2,048 rows 138, 104, 106).  Wide ones fill it by their columns
 // from some hundred rows on (M x 9,728 x 896: 64 rows 60, 46, 36; 512 rows 230, 211, 213; 2,048 rows 752, 745, 804), and a vocabulary's
-// from one (1 x 151,936 x 896: 136, 160, 165).
+// from one (1 x 151,936 x 896: 136, 160, 165).  Eight shares from a K of 4,096 on (M x 896 x 4,864, four and eight: 1 row
+// 35, 19, 64 rows 55, 35, 512 rows 151, 119, 2,048 rows 415, 411; M x 2,048 x 2,048: 64 rows 33, 26, but 512 rows 114, 119).
 int split_of(int N, int K) {
   if (K < 256 || N > 65536) return 1;
-  return N <= 4096 ? 4 : 2;
+  return N > 4096 ? 2 : K < 4096 ? 4 : 8;
 }
 
 template <typename TA, typename TW, typename TO>
@@ -310,6 +311,7 @@ int launch(const void* A, const void* W, const float* bias, const float* residua
     return vec ? launch_sizes<SPLIT, true>((const TA*)A, (const TW*)W, bias, residual, (TO*)out, M, N, K, lda, ldo, stream)
                : launch_sizes<SPLIT, false>((const TA*)A, (const TW*)W, bias, residual, (TO*)out, M, N, K, lda, ldo, stream);
   };
+  if (split == 8) return sizes(std::integral_constant<int, 8>());
   if (split == 4) return sizes(std::integral_constant<int, 4>());
   if (split == 2) return sizes(std::integral_constant<int, 2>());
   return sizes(std::integral_constant<int, 1>());

@@ -304,6 +304,12 @@ def test_gemm_simple_shares_of_k(M, N, K):
         assert torch.equal(x, out + 2.0) and (wide[:, :lead] == 2.0).all() and (wide[:, lead + N:] == 2.0).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 70, 4097), (17, 900, 4100), (64, 1030, 4864), (130, 66, 8190)])
+def test_gemm_simple_eight_shares_of_k(M, N, K):
+    """K shared by the eight CTAs of a cluster (from 4,096 on, up to 4,096 columns), the last shares short or empty."""
+    test_gemm_simple_shares_of_k(M, N, K)
+
+
 @pytest.mark.parametrize("orientation", [0, 1, 2, 3, 4])
 @pytest.mark.parametrize("M,N,K", SHAPES)
 def test_gemm_bf16_tensor_cores(status, M, N, K, orientation):
