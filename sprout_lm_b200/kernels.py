@@ -1584,10 +1584,11 @@ def moe_combine(y, h, ids, weights, place_of, rows, top: int, factor: float = 1.
          _ptr(rows, "rows", torch.float32, True), T, width, top, _stream())
 
 
+@functools.lru_cache(maxsize=4096)
 def multimap_key_split(requests: int, kv_heads: int, group: int, max_q_len: int, planned_keys: int, sms: int | None = None) -> int:
     """Into how many CTAs a step of single tokens divides a request's 64-key tiles; 1 for steps with longer portions.  At least enough to
     give every SM a CTA, at most 8 and the tiles there are; with 12 tiles or more a share, as many as the SMs hold beside one another
-    (three each), or four where the undivided launch fills more than half of those places but its lengths leave the SMs uneven (64
+    (three each), or four where the undivided launch fills between half and all of those places but its lengths leave the SMs uneven (64
     tiles and more).  Heads of 128 + 128: 96 CTAs of up to 47 tiles 46 us in two shares, 40 in four; 256 of up to 94 tiles 140 us
     undivided, 142 in two, 128 in four; 256 of up to 32 tiles 57 us undivided, 60 in four."""
     if max_q_len * group > 16:
@@ -1597,7 +1598,7 @@ def multimap_key_split(requests: int, kv_heads: int, group: int, max_q_len: int,
     sms = sms or sm_count()
     least = min(8, tiles, -(-sms // ctas))
     places = 3 * sms
-    wide = places // ctas if 2 * ctas <= places else 4 if tiles >= 64 else 1
+    wide = places // ctas if 2 * ctas <= places else 4 if tiles >= 64 and ctas <= places else 1
     return max(1, least, min(8, wide, tiles // 12))
 
 
