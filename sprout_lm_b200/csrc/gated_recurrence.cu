@@ -722,7 +722,7 @@ gated_group_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate
 // The same for parts of up to 256 elements in multiples of 4 whose rows start on 16 bytes: the lanes of a warp share PARTS parts of a row
 // (32 / LANES of them, LANES = part / VEC rounded up to a power of two), VEC elements a lane in 16-byte accesses, the part in registers
 // between its sum and its scaling, no block-wide barrier.  Bound by memory: 2,500 rows of 16 parts of 128: 45 us as a block of 128
-// threads per part, 19 us so.
+// threads per part, 19 us with 4 elements a lane placed by 64-bit divisions, 13 us so.
 template <typename TG, int VEC>
 __global__ void __launch_bounds__(256)
 gated_group_norm_warp_kernel(const float* __restrict__ o, const TG* __restrict__ gate, int gate_stride, const float* __restrict__ weight,

@@ -39,8 +39,8 @@ namespace {
 // threads of a router block: 32 warps, so that the router's rows are walked by as many warps as the SM holds (a block's time is
 // the latency of its rounds over the outputs: 33 outputs are 2 rounds of 32 warps, 5 of 8)
 // Steps of many tokens over enough outputs: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four
-// products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so, 25 us with registers
-// for two blocks of 9 warps an SM).
+// products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so; with registers for
+// one and for two blocks of 9 warps an SM, cold caches, 44 and 29.5 us).
 constexpr int ROUTE_THREADS = 1024;
 
 // A block takes ROUTE_TOKENS tokens (8 in steps of many tokens, 1 in steps of few, where blocks are scarce; a token's

@@ -284,7 +284,7 @@ def test_gemm_simple_tiles(M, N, K):
 
 @pytest.mark.parametrize("M,N,K", [(8, 129, 256), (16, 65, 300), (17, 200, 4099), (130, 4097, 257), (64, 4096, 1000), (1153, 63, 260), (700, 2048, 256)])
 def test_gemm_simple_shares_of_k(M, N, K):
-    """K shared by a cluster's CTAs (in four up to 4,096 columns, in two beyond), at ragged ends of rows, columns and shares, on and off 16-byte rows:
+    """K shared by a cluster's CTAs (in four or eight up to 4,096 columns, in two beyond), at ragged ends of rows, columns and shares, on and off 16-byte rows:
     a row's bits depend neither on the rows beside it nor on the tile; strided output, bias and residual."""
     from sprout_lm_b200 import kernels
     a, w, bias = rand(M, K), rand(N, K, seed=1), rand(N, seed=2)
