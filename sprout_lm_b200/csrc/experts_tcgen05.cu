@@ -13,8 +13,9 @@
 // accumulators alternate: a tile's epilogue runs under the next one's products.  Persistent: a pair walks the tiles with the stride of
 // the grid, an expert's row tiles of the same features side by side, so that the second finds the weights in L2.
 //
-// 32 experts of 1,024 over 2,048 wide rows, both products: 2,048 tokens of 4 experts each 133 us with the rows on M, 110 so (70 us the
-// gated one, which reads 300 MB and keeps the tensor cores busy for half of that time); 64 tokens 105 and 76 us (402 MB, 5.3 TB/s).
+// 32 experts of 1,024 over 2,048 wide rows, top 4, the whole layer: 2,048 tokens 303 us with the rows on M, 272 so, 64 tokens 156 and 121.
+// Both products and the gather 134 and 95 us (cold caches): for 2,048 tokens the gated one takes 70 us, reads 300 MB and keeps the tensor
+// cores busy for half of that time; for 64 tokens 402 MB pass at 4.2 TB/s with the launches' ends.
 //
 // Waits are bounded as in the dense products.
 #include <cuda.h>
