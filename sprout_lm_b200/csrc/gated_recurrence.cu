@@ -719,8 +719,8 @@ gated_group_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate
   }
 }
 
-// The same for parts of up to 256 elements in multiples of 4 whose rows start on 16 bytes: the lanes of a warp share PARTS parts of a row
-// (32 / LANES of them, LANES = part / VEC rounded up to a power of two), VEC elements a lane in 16-byte accesses, the part in registers
+// The same for parts that a warp's lanes hold (up to 128 elements in multiples of 4, up to 256 in multiples of 8) whose rows start on 16
+// bytes: the lanes of a warp share PARTS parts of a row (32 / LANES of them, LANES = part / VEC rounded up to a power of two), VEC elements a lane in 16-byte accesses, the part in registers
 // between its sum and its scaling, no block-wide barrier.  Bound by memory: 2,500 rows of 16 parts of 128: 45 us as a block of 128
 // threads per part, 19 us with 4 elements a lane placed by 64-bit divisions, 13 us so.
 template <typename TG, int VEC>
@@ -803,7 +803,7 @@ int launch_group_norm(const float* o, const void* gate, int gate_stride, const f
     int lanes_log2 = 0;
     while ((vec << lanes_log2) < part) lanes_log2++;
     const long long parts = (long long)rows * groups, blocks = ((parts << lanes_log2) + 255) / 256;
-    if (part % vec == 0 && parts <= 0x7fffffffLL) {
+    if (part % vec == 0 && lanes_log2 <= 5 && parts <= 0x7fffffffLL) {        // a part is one warp's: 132 to 252 in fours that are not eights are not
       SPROUT_REQUIRE(blocks <= 0x7fffffffLL, "gated_group_norm: too many rows");
       if (vec == 8)
         sprout_launch(gated_group_norm_warp_kernel<TG, 8>, dim3((unsigned)blocks), dim3(256), 0, stream, o, (const TG*)gate, gate_stride, weight,

@@ -1396,7 +1396,11 @@ def test_latent_attention_unfolded(monkeypatch, window, sink, interleaved, dim, 
     # from 1,024 parts on a group of lanes has a part, below a block
     (1023, 4, 1, 4, None, False, True), (1025, 4, 1, 4, None, False, True), (171, 64, 6, 64, torch.float32, True, True),
     (343, 100, 3, 300, torch.bfloat16, False, False), (114, 128, 9, 128, torch.bfloat16, True, False), (205, 136, 5, 680, torch.float32, False, True),
-    (513, 256, 2, 256, torch.bfloat16, False, True)])
+    (513, 256, 2, 256, torch.bfloat16, False, True),
+    # around the sizes at which a lane takes eight elements, and beyond what a warp's lanes hold in fours
+    *[(rows, part, groups, part * (groups if wide else 1), gate, first, silu) for rows, groups in ((343, 3), (340, 3), (1024, 1))
+      for part, wide, gate, first, silu in ((60, True, None, False, True), (68, False, torch.bfloat16, False, True), (124, True, torch.float32, True, False),
+                                            (132, False, None, False, True), (132, True, torch.bfloat16, True, True), (252, True, torch.bfloat16, False, False))]])
 def test_gated_group_norm_lanes(rows, part, groups, period, gate_dtype, gate_first, silu):
     """A part per group of lanes: the smallest and largest parts, lanes without elements, a last warp that is not full, every kind of gate."""
     from sprout_lm_b200 import kernels
