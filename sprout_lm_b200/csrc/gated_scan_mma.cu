@@ -14,6 +14,12 @@
 // it has the layout of the A operand of o^T = S^T q^T, so it is split into terms without leaving the registers.  The vectors of the next
 // 16 tokens come by cp.async while these are worked on.
 //
+// Infinities and NaN: the terms of an infinity are not one (infinity - infinity), and the tensor cores multiply the triangle's zeros with
+// the values of tokens that an output does not see.  Either way what comes out is NaN, never a wrong number, and only in the value columns
+// of such a value or state, or in all columns from a token on.  So such columns' 16 tokens are walked again in turn (`walk`), which gives
+// the outputs that are not finite and the state; the outputs that are finite stay as they came.  A value reaches its own column from its
+// own token on, as in the walk token by token.  Looking for them costs 2,500 tokens of three requests 8 of 263 us (the layer).
+//
 // Bound by the issue of instructions (some 300 products and 1,700 others a warp and 16 tokens) at eight warps an SM; walking token by
 // token, every element of S took a packed multiply and multiply-add a token.  2,500 tokens of three requests, 16 heads of 128 x 128: the
 // sums' walk 106 us there and 29 here, the outputs' 243 and 105, the layer 565 and 295; the outputs' error against 64 bits 1.5e-7 in
@@ -98,6 +104,7 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
         const int col = wcol + 16 * m + g + 8 * (e >> 1), d = 8 * n + c2 + (e & 1);
         S[m][n][e] = OUT && col < p.vdim ? from[(size_t)d * p.vdim + col] : 0.f;
       }
+  unsigned walked_before = 0;                                  // SUMS: columns that have been walked in turn
   float prod0 = 1.f, prod1 = 1.f;                              // SUMS: the chunk's decays of two channels (threads of the keys)
 
   auto fetch = [&](int t0, int stage) {
@@ -164,11 +171,13 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
       a0 = t < n_tokens ? a.x : 1.f;
       a1 = t < n_tokens ? a.y : 1.f;
     };
+    bool k_bad = false;                                        // a key's term or a decay that is not finite
     // ---- the terms of k_j P(j, 16) and q_i P(0, i): two channels a thread, half of the threads (a quarter each at 64) for either
     constexpr int HALF = DIM / 2;
     if (tid < HALF) {
       const int d = 2 * tid;
       float s0 = 1.f, s1 = 1.f;
+      __nv_bfloat162 most = __floats2bfloat162_rn(0.f, 0.f);   // NaN once a term is not finite
 #pragma unroll
       for (int t = STEP - 1; t >= 0; t--) {
         float x0, x1, a0, a1;
@@ -177,6 +186,7 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
         const float factor = PER_HEAD ? a_in[STEP + t] : 1.f;
         uint32_t high, mid, low;
         split3(x0 * factor * s0, x1 * factor * s1, high, mid, low);
+        most = __hfma2(*(const __nv_bfloat162*)&high, __floats2bfloat162_rn(0.f, 0.f), most);
         uint8_t* to = smem + L::OFF_KS + t * L::ROW + d * 2;
         *(uint32_t*)to = high;
         *(uint32_t*)(to + STEP * L::ROW) = mid;
@@ -184,6 +194,7 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
         s0 *= a0;
         s1 *= a1;
       }
+      k_bad = fmaf(s0, 0.f, fmaf(s1, 0.f, __low2float(most) + __high2float(most))) != 0.f;
       *(float2*)(total + d) = make_float2(s0, s1);
       prod0 *= s0;
       prod1 *= s1;
@@ -252,13 +263,81 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
         }
       }
     }
-    __syncthreads();
+    k_bad = __syncthreads_or(k_bad);
     // ---- tensor cores
     const uint8_t* own_values = v_in + (warp * WC) * 2;
     uint32_t v[MT][4];                                         // v^T: rows value columns, columns tokens
 #pragma unroll
     for (int m = 0; m < MT; m++)
       ldmatrix_x4_trans(v[m], own_values + ((lane & 7) + ((lane >> 4) & 1) * 8) * L::V_ROW + (16 * m + ((lane >> 3) & 1) * 8) * 2);
+    // one bit for every column of the thread (16 m + g, + 8), the same in the four lanes that share it: walk this column in turn
+    unsigned walked = k_bad ? (1u << 2 * MT) - 1 : 0;
+    auto votes = [&](bool yes) { return (__ballot_sync(0xffffffffu, yes) >> (lane & 28) & 15u) != 0; };
+    if (!OUT) {                                                // values that are not finite; a column once walked stays so
+      uint32_t seen[MT][2], any = 0;
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+          seen[m][half] = ((v[m][half] & 0x7f807f80u) + 0x00800080u) | ((v[m][half + 2] & 0x7f807f80u) + 0x00800080u);
+          any |= seen[m][half];
+        }
+      if (__any_sync(0xffffffffu, any & 0x80008000u)) {
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+          for (int half = 0; half < 2; half++) walked |= (unsigned)votes(seen[m][half] & 0x80008000u) << (2 * m + half);
+      }
+      walked |= walked_before;
+      walked_before = walked;
+    }
+    // the 16 tokens in turn for the columns in `walked`: the state, and of the outputs those that are not finite
+    auto walk = [&](float (&o)[MT][2][4]) {
+#pragma unroll 1
+      for (int t = 0; t < n_tokens; t++) {
+        float value[MT][2], part[MT][2];
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            value[m][half] = __bfloat162float(*(const __nv_bfloat16*)(own_values + t * L::V_ROW + (16 * m + 8 * half + g) * 2));
+            part[m][half] = 0.f;
+          }
+        const float factor = PER_HEAD ? a_in[STEP + t] : 1.f;
+#pragma unroll
+        for (int n = 0; n < 2 * KT; n++) {
+          float k[2], a[2], q[2] = {0.f, 0.f};
+          two(k_in + t * DIM + 8 * n + c2, k[0], k[1]);
+          decay2(t, 8 * n + c2, a[0], a[1]);
+          if (OUT) two(q_in + t * DIM + 8 * n + c2, q[0], q[1]);
+#pragma unroll
+          for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const int half = e >> 1, x = e & 1;
+              if (walked >> (2 * m + half) & 1) S[m][n][e] = fmaf(a[x], S[m][n][e], k[x] * factor * value[m][half]);
+              if (OUT) part[m][half] = fmaf(p.q_scale * q[x], S[m][n][e], part[m][half]);
+            }
+        }
+        if (OUT) {
+#pragma unroll
+          for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+              float sum = part[m][half] + __shfl_xor_sync(0xffffffffu, part[m][half], 1);
+              sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+              sum = fmaf(skip, value[m][half], sum);
+#pragma unroll
+              for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int x = 0; x < 2; x++) {
+                  float& at = o[m][n][2 * half + x];
+                  if (8 * n + c2 + x == t && (walked >> (2 * m + half) & 1) && !isfinite(at)) at = sum;
+                }
+            }
+        }
+      }
+    };
     const int nt_row = (lane & 7) + ((lane >> 4) & 1) * 8, nt_col = ((lane >> 3) & 1) * 8;
     if (OUT) {
       float o[MT][2][4], small[MT][2][4];                      // o^T: rows value columns, columns tokens (8 n + c2, + 1); the lesser terms' part
@@ -309,6 +388,27 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
 #pragma unroll
           for (int e = 0; e < 4; e++) o[m][n][e] += c[e] + small[m][n][e];
         }
+      float probe = 0.f;                                       // NaN if an output is not finite: as all of a column's are if its state or a value is not
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) probe = fmaf(o[m][n][e], 0.f, probe);
+      if (__any_sync(0xffffffffu, probe != 0.f)) {
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            float of_column = 0.f;
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+              for (int x = 0; x < 2; x++) of_column = fmaf(o[m][n][2 * half + x], 0.f, of_column);
+            walked |= (unsigned)votes(of_column != 0.f) << (2 * m + half);
+          }
+      }
+      if (__any_sync(0xffffffffu, walked)) walk(o);
 #pragma unroll
       for (int m = 0; m < MT; m++)
 #pragma unroll
@@ -319,6 +419,9 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
             if (t < n_tokens && col < p.vdim) p.out[((size_t)(t0 + t) * p.heads + h) * p.vdim + col] = o[m][n][e];
           }
       if (last_chunk ? false : t0 + STEP >= last) break;       // the state after the chunk is the next one's, made by the carry
+    } else if (__any_sync(0xffffffffu, walked)) {
+      float none[MT][2][4];
+      walk(none);
     }
 #pragma unroll
     for (int kt = 0; kt < KT; kt++) {
@@ -336,7 +439,8 @@ scan_mma_kernel(const ScanParams<__nv_bfloat16> p) {
           mma_bf16(c, v[m], k[0][2 * n], k[0][2 * n + 1]);
           const float2 d = n == 0 ? d0 : d1;
 #pragma unroll
-          for (int e = 0; e < 4; e++) S[m][2 * kt + n][e] = fmaf(S[m][2 * kt + n][e], e & 1 ? d.y : d.x, c[e]);
+          for (int e = 0; e < 4; e++)
+            if (!(walked >> (2 * m + (e >> 1)) & 1)) S[m][2 * kt + n][e] = fmaf(S[m][2 * kt + n][e], e & 1 ? d.y : d.x, c[e]);
         }
     }
   }

@@ -1574,6 +1574,83 @@ def test_gated_scan_16_tokens_at_a_time(status, form, strength, dim, vdim, ones)
         assert np.abs(got - expected).max() <= 2e-5 * max(1.0, np.abs(expected).max())
 
 
+@pytest.mark.parametrize("what,value", [("q", math.inf), ("k", math.inf), ("k", math.nan), ("v", -math.inf), ("v", math.nan), ("decay", math.nan),
+                                        ("state", math.inf), ("state", math.nan)])
+@pytest.mark.parametrize("form,dim,vdim", [("channel", 64, 72), ("channel", 128, 136), ("head", 128, 64), ("given", 64, 40)])
+def test_gated_scan_values_that_are_not_finite(status, monkeypatch, form, dim, vdim, what, value):
+    """An infinity or a NaN at the start, in the middle and at the end of 16 tokens, of a chunk and of a portion, through the walk on tensor cores: infinities and
+    NaN come where the recurrence in turn (float64) has them; outputs before its 16 tokens, other columns (of a value or a state) and other requests keep their
+    bits, outputs before it among its 16 tokens their value."""
+    from types import SimpleNamespace
+    from sprout_lm_b200 import kernels
+    monkeypatch.setattr(kernels, "scan_mma_chunk", lambda *a, **k: 48)
+    heads, lengths, slots = 2, [17, 145, 66], [2, 0, 3]
+    g = torch.Generator().manual_seed(dim + vdim)
+    T, begin = sum(lengths), lengths[0]
+    make = lambda *shape: torch.randn(*shape, generator=g).to(torch.bfloat16)
+    clean = dict(q=make(T, dim), k=make(T, dim), v=make(T, heads * vdim), state=torch.randn(4, heads, dim, vdim, generator=g))
+    # weak decays: over a chunk their product stays a float32, so that an infinite state stays one
+    clean["decay"] = torch.rand(T, heads, generator=g) ** 0.1 if form == "given" else torch.randn(T, heads * (dim if form == "channel" else 1), generator=g)
+    bias, factor, skip = torch.linspace(-1.0, 1.0, clean["decay"].shape[1]), torch.rand(T, heads, generator=g) + 0.5, torch.tensor([-0.5, 1.0])
+    f64 = lambda t: t.double().numpy()
+
+    def run(x):
+        x = {name: t.to(DEV) for name, t in x.items()}
+        more = dict(given=(x["decay"], factor.to(DEV))) if form == "given" else dict(per_head=True, a_log=torch.full((heads,), math.log(0.1), device=DEV)) if form == "head" \
+            else dict(tau=10.0)
+        ctx = SimpleNamespace(q_start=torch.tensor(np.cumsum([0] + lengths), dtype=torch.int32, device=DEV), max_q_len=max(lengths))
+        state = SimpleNamespace(buffer=x["state"], slots=torch.tensor(slots, dtype=torch.int32, device=DEV))
+        out = torch.full((T, heads * vdim), 7.0, device=DEV)
+        z = (None, None) if form == "given" else (x["decay"], bias.to(DEV))
+        kernels.gated_scan(x["q"], x["k"], x["v"], *z, ctx, state, out, heads, 1, dim, vdim, status, q_scale=0.5, skip=skip.to(DEV), **more)
+        assert int(status.item()) == 0
+        return out.cpu().view(T, heads, vdim), state.buffer.cpu()
+
+    before, state_before = run(clean)
+    for at in (0, 15, 24, 47, 48, 100, 144):
+        x = {name: t.clone() for name, t in clean.items()}
+        t = begin + at
+        column = at % vdim
+        if what == "state":
+            x["state"][slots[1], 1, dim // 2, column] = value
+            t = begin
+        elif what == "v":
+            x["v"][t, vdim + column] = value
+        else:
+            x[what][t, -1] = value
+        got, state = run(x)
+        with np.errstate(all="ignore"):
+            z = f64(x["decay"]) + (0.0 if form == "given" else f64(bias))
+            if form == "given":
+                decay, weight = np.repeat(z[:, :, None], dim, axis=2), f64(factor)
+            elif form == "head":
+                weight = np.logaddexp(0.0, z)
+                decay = np.repeat(np.exp(-0.1 * weight)[:, :, None], dim, axis=2)
+            else:
+                decay, weight = (1.0 / (1.0 + np.exp(-z.reshape(T, heads, dim)))) ** 0.1, np.ones((T, heads))
+            want, want_state = np.zeros((T, heads, vdim)), f64(x["state"]).copy()
+            of_heads = lambda name, part: np.repeat(f64(x[name][part])[:, None], heads, axis=1)
+            first = 0
+            for n, slot in zip(lengths, slots):
+                part = slice(first, first + n)
+                want[part] = scan_oracle(form, of_heads("q", part) * 0.5, of_heads("k", part), f64(x["v"][part]).reshape(n, heads, vdim), decay[part], weight[part], None,
+                                         want_state[slot])
+                first += n
+            want += f64(skip)[:, None] * f64(x["v"]).reshape(T, heads, vdim)
+        assert not np.isfinite(want).all()
+        for result, expected in ((f64(got), want), (f64(state), want_state)):
+            finite = np.isfinite(expected)
+            assert (np.isnan(result) == np.isnan(expected)).all() and (result[np.isinf(expected)] == expected[np.isinf(expected)]).all()
+            # as the walk over finite values, see above
+            assert np.abs(result[finite] - expected[finite]).max() <= 2e-5 * max(1.0, np.abs(expected[finite]).max())
+        for part in (slice(0, begin + (t - begin) // 16 * 16), slice(begin + lengths[1], T)):
+            assert torch.equal(got[part], before[part])
+        if what in ("v", "state"):
+            keep = torch.ones(heads, vdim, dtype=torch.bool)
+            keep[1, column] = False
+            assert torch.equal(got[:, keep], before[:, keep]) and torch.equal(state.transpose(1, 2)[:, :, keep], state_before.transpose(1, 2)[:, :, keep])
+
+
 @pytest.mark.parametrize("form", ["channel", "head", "floor", "bonus"])
 @pytest.mark.parametrize("dim,vdim", [(16, 24), (64, 40), (128, 64), (256, 20), (40, 12)])
 def test_float32_scan_keeps_its_bits_beside_a_long_portion(status, form, dim, vdim):
