@@ -1315,6 +1315,35 @@ def test_clamped_glu_product(status, monkeypatch, tokens, hidden, ff, stride):
     assert error.norm() <= 2 ** -9 * want.float().norm() and error.abs().max() <= 2 ** -6 * want.float().abs().max()
 
 
+@pytest.mark.parametrize("unit", ["clamped_glu", "silu_glu", "dense"])
+def test_gated_units_of_exact_products(status, monkeypatch, unit):
+    """The same activation in every kernel, bit for bit, where the products are exact (a matrix of ones and zeros picks them), for gates whose exponential is
+    nothing, everything and nearly too large for float32."""
+    from sprout_lm_b200 import kernels
+    tokens, ff = 600, 256
+    h = torch.cat([torch.linspace(-92.0, 30.0, tokens * ff).view(tokens, ff), torch.linspace(-9.0, 9.0, tokens * ff).view(ff, tokens).T], 1).to(torch.bfloat16).to(DEV)
+    w = torch.eye(2 * ff, dtype=torch.bfloat16, device=DEV)
+    if unit == "dense":
+        monkeypatch.setattr(kernels, "GLU_PRODUCT_TILES", 0)
+        got, want = (torch.zeros(tokens, ff, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        assert kernels.clamped_glu_product(h, w, got, 7.0, 1.0, status)
+        kernels.glu_clamped(h, want, 7.0, 1.0)
+        results = [got, want]
+    else:
+        order, offsets = torch.arange(tokens, dtype=torch.int32, device=DEV), torch.tensor([0, tokens], dtype=torch.int32, device=DEV)
+        down, results = torch.zeros(1, 2 * ff, ff, dtype=torch.bfloat16, device=DEV), []
+        monkeypatch.setattr(kernels, "EXPERTS_TC_ELEMENTS", 0)
+        for choice in ("mma", "mma_sync", "plain"):
+            monkeypatch.setenv("SPROUT_MOE", choice)
+            act = torch.zeros(tokens, ff, dtype=torch.bfloat16, device=DEV)
+            kernels.moe_experts(h, order, offsets, w[None], down, act, torch.zeros(tokens, 2 * ff, device=DEV), 1, 1, 7.0 if unit == "clamped_glu" else 0.0, 1.0,
+                                unit=unit, status=status)
+            results.append(act)
+    assert int(status.item()) == 0
+    for other in results[1:]:
+        assert torch.equal(results[0].view(torch.int16), other.view(torch.int16))
+
+
 @pytest.mark.parametrize("unit", ["clamped_glu", "plain"])
 def test_experts_tiles_of_every_width(status, monkeypatch, unit):
     """Rows of an expert in one tile of 16 to 256 columns, in two and more of equal size, features and K that no tile divides."""
