@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 import os
 import threading
 from ctypes import c_float, c_int, c_void_p
@@ -1832,17 +1833,53 @@ SCAN_CHUNKED_FROM = 128     # a step whose longest portion has at least this man
 SCAN_MMA_CHUNKED_FROM = 96
 
 
+SCAN_SCRATCH = 64 << 20     # bytes of chunks' states within which chunks may be shorter than SCAN_CHUNK
+
+
+def scan_mma_pays(requests: int, longest: int, heads: int, dim: int, vdim: int, sms: int) -> bool:
+    """Whether a step goes in chunks where they are walked 16 tokens at a time.  Portions under ``SCAN_CHUNKED_FROM`` of small states keep one
+    walk each when there are blocks of them for every SM, three at least (heads of 64 x 64, portions of up to 96 tokens: 64 of 8 heads 102 us whole and
+    114 in chunks, 128 ragged ones of 16 heads 238 and 295; 32 of 16 heads 105 and 110, but 16 of them 82 and 55)."""
+    if dim <= 64 and vdim <= 64 and longest < SCAN_CHUNKED_FROM and requests * heads >= 3 * sms:
+        return False
+    return longest >= SCAN_MMA_CHUNKED_FROM
+
+
 @functools.lru_cache(maxsize=4096)
-def scan_mma_chunk(tokens: int, requests: int, longest: int, blocks: int, sms: int) -> int:
-    """Tokens of a chunk where chunks are walked 16 tokens at a time, with ``blocks`` blocks a chunk: the least of rounds of blocks (two an
-    SM) x steps of 16 tokens, 9.2 us each in both walks, 2 us a round, and 0.65 us a chunk of the longest portion for the carry.  Measured at 4, 8 and
-    16 heads of 128 x 128 over 14 steps of 130 to 2,500 tokens it is within 3 % of the best of these sizes.  A layer, 64 tokens a chunk
-    and so: 3 portions of 2,500 tokens 299 and 278 us, 1 of 2,048 238 and 227, of 400 114 and 94, 8 heads 92 and 68."""
+def scan_mma_chunk(tokens: int, requests: int, longest: int, blocks: int, sms: int, state_bytes: int | None = None) -> int:
+    """Tokens of a chunk where chunks are walked 16 tokens at a time, with ``blocks`` blocks a chunk (two an SM) and ``state_bytes`` of state a
+    chunk: the least of three times, in us.  The outputs' walk takes 6 a step of 16 tokens: rounds of blocks x steps, or, since portions differ and
+    rounds overlap, all steps over the places and 0.6 of a block after them.  The sums' walk takes 4, over all chunks but every request's
+    last, and 0.5 a chunk of the longest portion for the carry.  The states are read by the outputs' walk and, of the chunks with sums, written, carried and
+    written, at 8.1 TB/s (caches take part).  Of the portions only their number, sum and longest are known (a replayed step may have
+    others): 0.43 of a chunk of every request but one is taken for empty; of portions under ``SCAN_CHUNKED_FROM``, taken for spread evenly up to the
+    longest, those beyond a chunk leave sums; chunks of the longest portion leave none.  No size
+    under ``SCAN_CHUNK`` whose states take more than ``SCAN_SCRATCH``.
+
+    Measured at 16 to 192 tokens a chunk over six layers (4 and 16 heads of 128 x 128, 8 and 16 of 64 x 64, 32 of 64 x 128, 16 of 128 x
+    256) and 57 steps of 1 to 128 portions and 96 to 13,000 tokens: 3 % (geometric mean) above the best of these sizes, at most 1.5 x (3 portions of
+    1,000, 16 heads of 64 x 64: 106 and 70 us).  128 ragged portions of up to 96 tokens of 32 heads of 64 x 128: 2,755 us in chunks of 16, which are fewest
+    steps, 841 in chunks of 96, 806 walked whole; 64 of 100 of 16 heads of 128 x 128 1,042, 420 and 1,255."""
+    places = 2 * sms
+    state_bytes = blocks * (128 * 128 * 4) if state_bytes is None else state_bytes
+
+    def walk(chunks, steps, all_steps):
+        rounds = -(-chunks * blocks // places)
+        return rounds * steps if rounds <= 1 else min(rounds * steps, all_steps * blocks / places + 0.6 * steps)
+
     best, least = SCAN_CHUNK, None
     for chunk in (16, 32, 48, 64, 80, 96, 112, 128, 144, 160, 192):
-        grid = -(-(2 * tokens + (requests - 1) * chunk) // (2 * chunk)) * blocks       # half a chunk of every request but one is empty
-        rounds = -(-grid // (2 * sms))
-        cost = rounds * (9.2 * (chunk // 16) + 2.0) + 0.65 * -(-longest // chunk)
+        if chunk < SCAN_CHUNK and (tokens // chunk + requests) * state_bytes > SCAN_SCRATCH:
+            continue
+        inner, steps = 0, -(-min(chunk, longest) // 16)              # chunks with sums; steps of a chunk
+        if chunk < longest:
+            inner = max(0, math.ceil(tokens / chunk + 0.43 * (requests - 1)) - requests)
+            if longest < SCAN_CHUNKED_FROM:
+                inner = max(inner, math.ceil(min(requests * (1 - chunk / longest), (tokens - requests) / chunk)))
+        chunks = requests + inner
+        cost = 6 * walk(chunks, steps, tokens / 16 + requests / 2) + (chunks + 3 * inner) * state_bytes / 8.1e6
+        if inner > 0:
+            cost += 4 * walk(inner, steps, inner * steps) + 0.5 * -(-longest // chunk)
         if least is None or cost < least:
             best, least = chunk, cost
     return best
@@ -1912,9 +1949,10 @@ def gated_scan(q, k, v, z, bias, ctx, state, out, heads: int, groups: int, dim: 
     longest = getattr(ctx, "max_q_len", 1)
     mma = dtype == torch.bfloat16 and dim in (64, 128) and floor is None and bonus is None and v_cols % 8 == 0 \
         and (q_stride | k_stride | v_stride) % 8 == 0 and (q_ptr | k_ptr | v_ptr) % 16 == 0
-    if longest >= (SCAN_MMA_CHUNKED_FROM if mma else SCAN_CHUNKED_FROM) and os.environ.get("SPROUT_GATED_SCAN", "chunks") != "whole":
+    sms = sm_count(v.device)
+    if (scan_mma_pays(requests, longest, heads, dim, vdim, sms) if mma else longest >= SCAN_CHUNKED_FROM) and os.environ.get("SPROUT_GATED_SCAN", "chunks") != "whole":
         if mma:
-            chunk = scan_mma_chunk(tokens, requests, longest, heads * (1 if vdim <= 64 else -(-vdim // 128)), sm_count(v.device))
+            chunk = scan_mma_chunk(tokens, requests, longest, heads * (1 if vdim <= 64 else -(-vdim // 128)), sms, heads * dim * vdim * 4)
         max_chunks = tokens // chunk + requests
         if given is None:
             da = torch.empty(tokens * (heads if per_head else heads * dim), dtype=torch.float32, device=v.device)

@@ -372,3 +372,21 @@ def test_scan_chunk_fills_the_device_in_few_steps():
             chunk = scan_mma_chunk(tokens, 1, tokens, blocks, 148)
             assert chunk % 16 == 0 and 16 <= chunk <= 192
     assert scan_mma_chunk(200000, 1, 200000, 64, 148) == 192
+
+
+def test_scan_chunk_counts_the_states_it_moves():
+    """Many portions: the scratch stays within what chunks of 64 take or 64 MB, and a chunk is not a fraction of the portions when the blocks fill the
+    device many times over; many short portions of small states are walked whole."""
+    from sprout_lm_b200.kernels import SCAN_SCRATCH, scan_mma_chunk, scan_mma_pays
+    for state in (1 << 18, 1 << 20, 1 << 21):
+        for requests in (1, 2, 8, 32, 64, 128):
+            for longest in (96, 100, 128, 200, 2048):
+                for tokens in (requests + longest - 1, requests * (longest + 1) // 2 + longest, requests * longest):
+                    chunk = scan_mma_chunk(tokens, requests, longest, state >> 16, 148, state)
+                    assert chunk % 16 == 0 and 16 <= chunk <= 192
+                    assert (tokens // chunk + requests) * state <= max(SCAN_SCRATCH, (tokens // 64 + requests) * state)
+    assert (2048 // scan_mma_chunk(2048, 32, 128, 16, 148, 1 << 20) + 32) << 20 <= SCAN_SCRATCH
+    for requests in (32, 64, 128):
+        assert scan_mma_chunk(requests * 100, requests, 100, 16, 148, 1 << 20) in (112, 128)
+    assert scan_mma_pays(1, 96, 16, 128, 128, 148) and scan_mma_pays(128, 127, 16, 128, 128, 148) and not scan_mma_pays(1, 95, 16, 128, 128, 148)
+    assert not scan_mma_pays(128, 127, 16, 64, 64, 148) and scan_mma_pays(128, 128, 16, 64, 64, 148) and scan_mma_pays(16, 96, 16, 64, 64, 148)
