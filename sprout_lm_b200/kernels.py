@@ -1586,21 +1586,37 @@ def moe_combine(y, h, ids, weights, place_of, rows, top: int, factor: float = 1.
 
 
 @functools.lru_cache(maxsize=4096)
-def multimap_key_split(requests: int, kv_heads: int, group: int, max_q_len: int, planned_keys: int, sms: int | None = None) -> int:
-    """Into how many CTAs a step of single tokens divides a request's 64-key tiles; 1 for steps with longer portions.  At least enough to
-    give every SM a CTA, at most 8 and the tiles there are; with 12 tiles or more a share, as many as the SMs hold beside one another
-    (three each), or four where the undivided launch fills between half and all of those places but its lengths leave the SMs uneven (64
-    tiles and more).  Heads of 128 + 128: 96 CTAs of up to 47 tiles 46 us in two shares, 40 in four; 256 of up to 94 tiles 140 us
-    undivided, 142 in two, 128 in four; 256 of up to 32 tiles 57 us undivided, 60 in four."""
+def multimap_key_split(requests: int, kv_heads: int, group: int, max_q_len: int, planned_keys: int, sms: int | None = None, maps: int = 1,
+                       dim: int = 128, vdim: int = 128) -> int:
+    """Into how many CTAs, 8 at most, a step of single tokens divides a request's 64-key tiles; 1 for steps with longer portions.  The least of,
+    in us: a tile's time (1.12 of latencies, or what the CTAs beside one another read at 8.7 TB/s) x a CTA's tiles, rounds of CTAs counted with
+    a weight of 1/8 and, since lengths differ, the work over all places (half of it, as contexts are shorter than the longest) and 0.6 of a
+    CTA after them with the rest; 2.1 for every CTA an SM starts; 5.2 for a merge.  An SM holds as many CTAs as their shared memory lets it, at
+    most 6.  A CTA's tiles count as a fraction, so that a growing context meets each number of shares once: captured steps are told apart by it.
+
+    Measured with 1 to 8 shares over eight kernels, 32 to 512 CTAs and contexts of 300 to 6,000 keys (1,000 launches): 2 % (geometric mean)
+    above the best, at most 1.2 x; 0.94 of the time of shares by the places alone (three an SM, four shares from 64 tiles on while 222 to 444 CTAs), 0.90
+    of that of a CTA for every SM, at most 1.15 x (heads of 64 + 64, 380 CTAs of 94 tiles, equal lengths: 99 us undivided, 114 in two).  Heads of
+    128 + 128, lengths from half to all of 6,000 keys, one and four shares: 256 CTAs 122 and 109, 300 139 and 124, 380 161 and 150, 440 186 and 177, 512 228 and 204 us."""
     if max_q_len * group > 16:
         return 1
-    tiles = max(1, -(-planned_keys // 64))
-    ctas = max(1, requests * kv_heads)
+    tiles, ctas = max(1, -(-planned_keys // 64)), max(1, requests * kv_heads)
     sms = sms or sm_count()
-    least = min(8, tiles, -(-sms // ctas))
-    places = 3 * sms
-    wide = places // ctas if 2 * ctas <= places else 4 if tiles >= 64 and ctas <= places else 1
-    return max(1, least, min(8, wide, tiles // 12))
+    if max_q_len * group <= 8:                  # the CTA's shared memory: its warps' stages, or their results at the end
+        shared = max(256 * (maps * dim + vdim + 16), 16 * (8 * maps * (2 + vdim) + vdim))
+    else:
+        shared = max(288 * (maps * dim + 8) + 256 * (vdim + 8), 512 * maps * (vdim // 2 + 4))
+    held = max(1, min(6, (227 << 10) // (shared + 1024)))
+    best, least = 1, None
+    for shares in range(1, min(8, tiles) + 1):
+        share, beside = tiles / shares, min(held, ctas * shares / sms)
+        tile = max(1.12, 128 * (maps * dim + vdim) * beside * sms / 8.7e6)
+        rounds = -(-ctas * shares // (held * sms)) * share
+        uneven = max(share, 0.5 * ctas * tiles / (held * sms) + 0.6 * share)
+        cost = (rounds / 8 + uneven * 7 / 8) * tile + 2.1 * ctas * shares / sms + (5.2 if shares > 1 else 0.0)
+        if least is None or cost < least:
+            best, least = shares, cost
+    return best
 
 
 def visible_keys(mask, context: int) -> int:
@@ -1671,7 +1687,7 @@ def multimap_attention(q, cache, ctx, out, heads: int, kv_heads: int, maps: int,
         ksplit = 1
         if max_q_len * group <= 16:                # single tokens; other steps do not divide a request's keys here
             planned = int(getattr(ctx, "planned_context", 0) or getattr(ctx, "max_context", 0) or 0)
-            ksplit = multimap_key_split(requests, kv_heads, group, max_q_len, visible_keys(mask, planned)) if planned else 1
+            ksplit = multimap_key_split(requests, kv_heads, group, max_q_len, visible_keys(mask, planned), None, maps, dim, vdim) if planned else 1
         mask_kind, mask_size, mask_keep = _mask_code(mask)
         gate_ptr, gate_stride, gate_elements = _gate_args(gate, q.shape[0], heads, vdim, q.dtype, "multimap_attention")
         turn_cos, turn_sin, turned = _turn_args(turn, vdim, "multimap_attention")

@@ -121,7 +121,7 @@ class MultiMapAttention(Part):
     def decode_plan(self, requests: int, max_keys: int, planned_context: int, page_tokens: int):
         """Into how many CTAs a step of one token per request divides a request's keys: it follows the contexts' length."""
         return kernels.multimap_key_split(requests, self.kv_heads, self.heads // self.kv_heads, 1,
-                                          kernels.visible_keys(self.mask, planned_context))
+                                          kernels.visible_keys(self.mask, planned_context), None, self.maps, self.dim, self.value_dim)
 
     def tensor_decls(self):
         n = self.names

@@ -390,3 +390,20 @@ def test_scan_chunk_counts_the_states_it_moves():
         assert scan_mma_chunk(requests * 100, requests, 100, 16, 148, 1 << 20) in (112, 128)
     assert scan_mma_pays(1, 96, 16, 128, 128, 148) and scan_mma_pays(128, 127, 16, 128, 128, 148) and not scan_mma_pays(1, 95, 16, 128, 128, 148)
     assert not scan_mma_pays(128, 127, 16, 64, 64, 148) and scan_mma_pays(128, 128, 16, 64, 64, 148) and scan_mma_pays(16, 96, 16, 64, 64, 148)
+
+
+def test_key_shares_follow_the_places_of_the_kernel():
+    """Shares of a single-token step's keys: enough for the SMs of a small step, few for short contexts, each number once as a
+    context grows (a captured step is kept for each), by what an SM holds of the kernel, none for steps with longer portions."""
+    from sprout_lm_b200.kernels import multimap_key_split
+
+    def shares(ctas, keys, maps=1, dim=128, vdim=128, group=4):
+        return multimap_key_split(ctas, 1, group, 1, keys, 148, maps, dim, vdim)
+    assert multimap_key_split(64, 4, 4, 5, 6000, 148) == 1 and shares(64, 1) == 1 and shares(1, 6000) == 8
+    assert [shares(ctas, 6000) for ctas in (56, 96, 148, 256, 300, 380, 440, 512)] == [6, 3, 6, 5, 4, 4, 4, 4]
+    for sizes in (dict(), dict(dim=64, vdim=64), dict(maps=2, dim=64), dict(maps=2), dict(dim=64, vdim=64, group=16)):
+        for ctas in (1, 8, 32, 96, 148, 222, 256, 300, 380, 440, 444, 445, 512):
+            row = [shares(ctas, 64 * tiles, **sizes) for tiles in range(1, 130)]
+            changes = [n for n, before in zip(row[1:], row) if n != before]
+            assert all(1 <= n <= min(8, tiles) for tiles, n in enumerate(row, 1))
+            assert row[0] == 1 and len(set(changes)) == len(changes) <= 7
