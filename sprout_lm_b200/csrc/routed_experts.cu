@@ -40,16 +40,16 @@ namespace {
 // the latency of its rounds over the outputs: 33 outputs are 2 rounds of 32 warps, 5 of 8)
 // Steps of many tokens over enough outputs: fewer warps, each with four outputs, so that a warp's shared-memory reads serve four
 // products (bfloat16, 2,048 tokens of 2,048 over 36 outputs: 62 us with an output a warp and 32 warps, 39 us so; with registers for
-// one and for two blocks of 9 warps an SM, cold caches, 44 and 29.5 us).
-constexpr int ROUTE_THREADS = 1024;
+// one and for two blocks of 9 warps an SM, cold caches, 44 and 29.5 us).  Up to 10 warps leave 96 registers a thread to two blocks.
+constexpr int ROUTE_THREADS = 1024, ROUTE_SIDE_BY_SIDE = 320, ROUTE_FOURS = 512;      // four outputs a warp: blocks of up to 10 warps (two an SM) and up to 16
 
 // A block takes ROUTE_TOKENS tokens (8 in steps of many tokens, 1 in steps of few, where blocks are scarce; a token's
 // sums are the same in all forms): its warps share the router's outputs (warp w of 32 takes outputs w, w + 32, ...; of 8 to 16 warps four
 // neighbouring outputs at a time) and apply every weight they load to all the block's tokens; a lane sums its own elements in ascending order (four neighbours of every 128 where the rows
 // are multiples of four, else every 32nd), the lanes are added in a fixed order, so a token's
 // scores do not depend on the tokens beside it.  Warp t then takes token t's softmax and choices.
-template <typename T, int ROUTE_TOKENS, int ROUTE_OUTPUTS>
-__global__ void __launch_bounds__(ROUTE_OUTPUTS > 1 ? 512 : ROUTE_THREADS) __maxnreg__(ROUTE_OUTPUTS > 1 ? 104 : 64)
+template <typename T, int ROUTE_TOKENS, int ROUTE_OUTPUTS, int THREADS = ROUTE_THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == ROUTE_SIDE_BY_SIDE ? 2 : 1)
 moe_route_kernel(const T* __restrict__ h, int h_stride, const float* __restrict__ router, const float* __restrict__ correction,
                  int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int tokens, int width,
                  int softmax_outputs, int experts, int top, float scale, int extra, float* __restrict__ extra_out,
@@ -689,10 +689,12 @@ SPROUT_API int sprout_moe_route(const void* h, int h_stride, int dtype, const fl
   if (!prepared) {
     cudaFuncSetAttribute(moe_route_kernel<float, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(moe_route_kernel<float, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_route_kernel<float, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<float, 8, 4, ROUTE_SIDE_BY_SIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<float, 8, 4, ROUTE_FOURS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 4, ROUTE_SIDE_BY_SIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 8, 4, ROUTE_FOURS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     prepared = true;
   }
   dim3 grid((tokens + per_block - 1) / per_block);
@@ -702,13 +704,15 @@ SPROUT_API int sprout_moe_route(const void* h, int h_stride, int dtype, const fl
   const bool four = per_block > 1 && width % 4 == 0 && rows_of_router >= (dtype == SPROUT_BF16 ? 16 : 64);
   const int warps = (rows_of_router + 3) / 4;
   const dim3 threads(!four ? ROUTE_THREADS : 32 * (warps < 8 ? 8 : warps > 16 ? 16 : warps));
-#define ROUTE(T, N, U)                                                                                                 \
-  sprout_launch(moe_route_kernel<T, N, U>, grid, threads, smem, stream, (const T*)h, h_stride, router, correction, ids, \
+  const bool side_by_side = threads.x <= ROUTE_SIDE_BY_SIDE;
+#define ROUTE(T, N, ...)                                                                                               \
+  sprout_launch(moe_route_kernel<T, N, __VA_ARGS__>, grid, threads, smem, stream, (const T*)h, h_stride, router, correction, ids, \
                 weights, counts, tokens, width, outputs, experts, top, scale, extra, extra_out, group_count, group_keep, renormalize, sigmoid_scores)
   if (dtype == SPROUT_F32) {
-    if (per_block == 1) ROUTE(float, 1, 1); else if (four) ROUTE(float, 8, 4); else ROUTE(float, 8, 1);
+    if (per_block == 1) ROUTE(float, 1, 1); else if (!four) ROUTE(float, 8, 1); else if (side_by_side) ROUTE(float, 8, 4, ROUTE_SIDE_BY_SIDE); else ROUTE(float, 8, 4, ROUTE_FOURS);
   } else if (dtype == SPROUT_BF16) {
-    if (per_block == 1) ROUTE(__nv_bfloat16, 1, 1); else if (four) ROUTE(__nv_bfloat16, 8, 4); else ROUTE(__nv_bfloat16, 8, 1);
+    if (per_block == 1) ROUTE(__nv_bfloat16, 1, 1); else if (!four) ROUTE(__nv_bfloat16, 8, 1);
+    else if (side_by_side) ROUTE(__nv_bfloat16, 8, 4, ROUTE_SIDE_BY_SIDE); else ROUTE(__nv_bfloat16, 8, 4, ROUTE_FOURS);
   } else {
     return sprout_fail("moe_route: unknown dtype %d", dtype);
   }
