@@ -11,8 +11,8 @@
 // TMEM allocation, warps 2-9 run the epilogue (two per 32-lane quarter of tensor memory).
 //
 // Two orientations share the pipeline:
-//   tokens on M (prefill): D rows are tokens, D columns output features; BN = 256 where that
-//       tiles N exactly (less operand traffic from L2), else 128.
+//   tokens on M (prefill): D rows are tokens, D columns output features; single CTAs or pairs and
+//       BN = 128..256 by a cost, for any N (`pick_token_tiles`).
 //   weights on M (decode, "swap"): D rows are output features, D columns tokens in tiles of
 //       BN = 16..256.  A decode step streams every weight once and the 128-row tensor-core tile
 //       is filled by weight rows instead of by a handful of tokens.
@@ -578,14 +578,16 @@ int launch(const CUtensorMap& rows_map, const CUtensorMap& cols_map, const CUten
 // before: 4,001 x 3,088 x 2,048 43.3 us and 36.3 now, 2,500 x 8,224 x 2,048 69.7 and 57.2, 300 x 3,072 x 1,024 9.9 and 5.8,
 // 2,048 x 3,072 x 2,048 24.2 and 20.9.
 struct TokenTiles { bool pair; int width, split; };
-TokenTiles pick_token_tiles(long long M, long long N, int total_kb, int group_rows, bool reduce, bool swiglu) {
+// `only_pairs`: among the pairs' forms, but for groups of features that none of them divides.
+TokenTiles pick_token_tiles(long long M, long long N, int total_kb, int group_rows, bool reduce, bool swiglu, bool only_pairs) {
   struct Form { bool pair; int width, ends, block; };
   const Form forms[] = {{false, 128, 3900, 230}, {false, 192, 4500, 327}, {false, 224, 5700, 350}, {false, 256, 5300, 375},
                         {true, 192, 5900, 277}, {true, 224, 6100, 320}, {true, 256, 6000, 337}};
   TokenTiles best{false, 128, 1};
+  if (group_rows && group_rows % 192 && group_rows % 224 && group_rows % 256) only_pairs = false;
   long long best_cost = -1;
   for (const Form& f : forms) {
-    if (group_rows && group_rows % f.width) continue;
+    if ((group_rows && group_rows % f.width) || (only_pairs && !f.pair)) continue;
     if (swiglu && f.width % 128) continue;               // the two warps of a quarter would not have equal shares
     const long long rows = f.pair ? 2 * BLOCK_M : BLOCK_M, slots = f.pair ? sm_count() / 2 : sm_count();
     for (int split = 1; split <= (reduce && !f.pair ? 4 : 1); split++) {
@@ -605,8 +607,8 @@ TokenTiles pick_token_tiles(long long M, long long N, int total_kb, int group_ro
 // A [M, K] bf16 row stride lda; W [N, K] bf16 contiguous; out [M, N] row stride ldo, bf16 or
 // float32.  residual != 0: out is float32 and the product is added to it.  orientation: 0 picks
 // by M (weight rows on the MMA's M axis up to 256 tokens, up to 64 with the SwiGLU epilogue, tokens on M beyond), 1 forces tokens
-// on M (128 x 128 tiles, or 256 x 256 tiles of CTA pairs where N is a multiple of 256), 2 weights
-// on M (tokens in tiles of 16..256), 3 tokens on M with single CTAs only, 4 with CTA pairs only.
+// on M (tiles as `pick_token_tiles` has them, as 0 does beyond those tokens), 2 weights on M (tokens in tiles of 16..256), 3 tokens on M
+// in single CTAs' 128 x 128 tiles, 4 in the tiles that the pick has among CTA pairs'.
 // split_k > 1 (weights on M, residual, at most 256 tokens) divides K among CTAs and adds with
 // atomics.
 // residual == 2: the SwiGLU epilogue (no bias; out is bfloat16 [M, N/2]; N a multiple of 16); residual == 3: the same with
@@ -639,12 +641,11 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
   // weights past few tokens (up to 256 tokens; with split K where the epilogue adds).  The SwiGLU
   // epilogue cannot split K, so its 128-row weight tiles leave SMs idle while the token tiles grow:
   // measured at the 0.5B / 7B / 14B gate/up shapes, weights on M wins up to 64 tokens, tokens on M
-  // with single CTAs from 65 to 128 (9.7 against 12.5 us at 128 tokens of the 0.5B shape), CTA
-  // pairs beyond (12.7 against 18.1 us at 256).
+  // beyond (9.7 against 12.5 us at 128 tokens of the 0.5B shape, 12.7 against 18.1 us at 256).
   // Between 33 and 64 tokens the SwiGLU product goes tokens on M as well when its 128-row weight tiles
   // would leave more than two SMs in five idle (the 0.5B shape: 76 tiles, 9.2 against 9.8 us).
   const bool few_weight_tiles = swiglu && M > 32 && 5LL * ((N + BLOCK_M - 1) / BLOCK_M) < 3LL * sm_count();
-  const bool swap = orientation == 2 || (orientation == 0 && M <= (swiglu ? 64 : 256) && !few_weight_tiles);    // 1: tokens on M in CTA pairs, 3: single CTAs
+  const bool swap = orientation == 2 || (orientation == 0 && M <= (swiglu ? 64 : 256) && !few_weight_tiles);
   if (split_k < 1) split_k = 1;
   SPROUT_REQUIRE(split_k == 1 || (swap && residual && M <= 256), "gemm_bf16: split_k needs weights-on-M with a residual output and at most 256 tokens "
                  "(with tokens on M the kernel splits K by itself where that pays)");
@@ -679,12 +680,8 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
   // Tokens on M.  The residual epilogue goes through the TMA unit where the output's rows allow a
   // tensor map; its additions are atomic in L2, so a tile's K range may then be split among CTAs.
   const bool reduce = p.epilogue == EPI_RESIDUAL && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
-  TokenTiles tiles{orientation == 4, 128, 1};
-  if (orientation == 4) {
-    if (N % 256 == 0 && (groups == 1 || group_rows % 256 == 0)) tiles.width = 256;
-  } else if (orientation != 3) {
-    tiles = pick_token_tiles(M, N, total_kb, groups > 1 ? group_rows : 0, reduce, swiglu);
-  }
+  TokenTiles tiles{false, 128, 1};
+  if (orientation != 3) tiles = pick_token_tiles(M, N, total_kb, groups > 1 ? group_rows : 0, reduce, swiglu, orientation == 4);
   const bool pair = tiles.pair;
   const int bn = tiles.width;
   split_k = tiles.split;
@@ -703,8 +700,7 @@ SPROUT_API int sprout_gemm_bf16(const void* A, const void* W, const float* bias,
     switch (bn) {
       case 256: return launch_pair<256>(map_a, map_w, map_out, p, (int)work, stream);
       case 224: return launch_pair<224>(map_a, map_w, map_out, p, (int)work, stream);
-      case 192: return launch_pair<192>(map_a, map_w, map_out, p, (int)work, stream);
-      default: return launch_pair<128>(map_a, map_w, map_out, p, (int)work, stream);
+      default: return launch_pair<192>(map_a, map_w, map_out, p, (int)work, stream);
     }
   }
   switch (bn) {

@@ -399,8 +399,8 @@ def gemm_bf16(a, weight, out, status, bias=None, residual=None, orientation=0, s
     """out = a @ weight.T (+ bias) (+ residual) on the tcgen05 tensor cores; a and weight bfloat16.
 
     ``residual`` must be ``out`` itself (float32): the product is added in place.  orientation 0
-    lets the kernel choose (weight rows on the MMA's M axis for up to 128 tokens), 1 forces
-    tokens on M, 2 weights on M.  ``split_k`` > 1 divides K among CTAs (weights on M with a
+    lets the kernel choose (weight rows on the MMA's M axis for up to 256 tokens, 64 with ``swiglu``), 1 forces
+    tokens on M, 2 weights on M, 3 tokens on M in single CTAs' 128 x 128 tiles, 4 in CTA pairs' tiles.  ``split_k`` > 1 divides K among CTAs (weights on M with a
     residual only; the partial sums are added with atomics).  ``swiglu``: weight rows interleave
     gate and up in blocks of 8 and ``out`` is bfloat16 [M, N/2] = act(gate) * up, act = ``gate_activation``: "silu" or
     "gelu_tanh" (the tanh form of gelu).  ``groups`` > 1: a is [M, groups * K], and output features [g * group_rows,
