@@ -95,8 +95,10 @@ constexpr int SCAN_THREADS = 128, SCAN_MAX_TOKENS = 8;
 // gated_scan_mma.cu where their rows allow it, in the same three launches around the same carry.  Other sizes and rows off 16-byte boundaries keep a
 // number at a time: pairs without the wide fetches cost 12 % (four heads of 96 x 96), and with two slices or one, 4 % (8 x 512, 16 x 64).
 // Each element of S sees S <- fma(a, S, (c k) v) once per token in the tokens' order.  An output's sum over the rows has one order in
-// the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn, so a bfloat16 request of one
-// chunk may differ in the last bits of a 32-bit sum by whether another portion of the step is long.
+// the 32-bit path, whatever the cutting and the batch; with PAIRS it is added in pairs, without in turn.  A bfloat16 request's last bits
+// depend on the whole step: whether its portions are walked whole or in chunks and, in gated_scan_mma.cu, on the chunks' length, which
+// follows from the step's tokens, number of portions and longest portion and from the SMs (a replayed step keeps that of the step it was
+// recorded for).
 //
 // Long portions are cut into chunks of `p.chunk` tokens so that more blocks than (request, head, columns) have work, in
 // three launches: SCAN_CHUNK_SUMS walks every chunk but a request's last from a zero state and leaves the chunk's own

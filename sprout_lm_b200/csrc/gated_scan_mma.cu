@@ -21,9 +21,10 @@
 // own token on, as in the walk token by token.  Looking for them costs 2,500 tokens of three requests 8 of 263 us (the layer).
 //
 // Bound by the issue of instructions (some 300 products and 1,700 others a warp and 16 tokens) at eight warps an SM; walking token by
-// token, every element of S took a packed multiply and multiply-add a token.  2,500 tokens of three requests, 16 heads of 128 x 128: the
-// sums' walk 106 us there and 29 here, the outputs' 243 and 105, the layer 565 and 295; the outputs' error against 64 bits 1.5e-7 in
-// both, the states' 1.4e-7 and 1.3e-7.
+// token, every element of S took a packed multiply and multiply-add a token.  2,500 tokens of three requests, 16 heads of 128 x 128: in
+// chunks of 64 the sums' walk 106 us there and 29 here, the outputs' 243 and 105; in the chunks of 160 that `kernels.scan_mma_chunk` gives
+// them, cold caches, 28 and 99, the layer 262 (565 token by token); the outputs' error against 64 bits 1.5e-7 in both, the states' 1.4e-7
+// and 1.3e-7.
 #include "attention_bf16.cuh"
 #include "gated_scan.cuh"
 

@@ -1925,8 +1925,8 @@ def gated_scan(q, k, v, z, bias, ctx, state, out, heads: int, groups: int, dim: 
     column v_cols is fed the constant 1 as a value (the columns after it 0): that column of the state is then the sum of the
     decayed c k, and that column of the output its product with q_scale q, a normaliser.
     out float32 [tokens, heads * vdim].  A step whose longest portion has ``SCAN_CHUNKED_FROM`` tokens or more cuts the
-    portions into chunks of ``SCAN_CHUNK`` tokens (bfloat16 and key sizes 64 and 128 with decays per channel or head: from
-    ``SCAN_MMA_CHUNKED_FROM`` tokens, of ``scan_mma_chunk``) that are walked side by side (``SPROUT_GATED_SCAN=whole`` keeps one walk
+    portions into chunks of ``SCAN_CHUNK`` tokens (bfloat16 and key sizes 64 and 128 with decays per channel or head: where
+    ``scan_mma_pays`` says so, of ``scan_mma_chunk``) that are walked side by side (``SPROUT_GATED_SCAN=whole`` keeps one walk
     per request): scratch for every token's decay and every chunk's sums."""
     tokens, dtype = v.shape[0], v.dtype
     v_cols = v.shape[1] // heads if ones_col else vdim

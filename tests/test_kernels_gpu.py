@@ -1603,6 +1603,15 @@ def test_gated_scan_16_tokens_at_a_time(status, form, strength, dim, vdim, ones)
         assert np.abs(got - expected).max() <= 2e-5 * max(1.0, np.abs(expected).max())
 
 
+@pytest.mark.parametrize("chunk", [48, 192])
+@pytest.mark.parametrize("form,dim,vdim,ones", [("channel", 128, 136, False), ("head", 64, 72, False), ("given", 128, 130, True)])
+def test_gated_scan_16_tokens_at_a_time_in_chunks(status, monkeypatch, chunk, form, dim, vdim, ones):
+    """The same in chunks of several steps of 16 tokens, portions that end within one, and in one chunk a portion (the rule takes one step a chunk there)."""
+    from sprout_lm_b200 import kernels
+    monkeypatch.setattr(kernels, "scan_mma_chunk", lambda *a, **k: chunk)
+    test_gated_scan_16_tokens_at_a_time(status, form, 1.0, dim, vdim, ones)
+
+
 @pytest.mark.parametrize("what,value", [("q", math.inf), ("k", math.inf), ("k", math.nan), ("v", -math.inf), ("v", math.nan), ("decay", math.nan),
                                         ("state", math.inf), ("state", math.nan)])
 @pytest.mark.parametrize("form,dim,vdim", [("channel", 64, 72), ("channel", 128, 136), ("head", 128, 64), ("given", 64, 40)])
