@@ -799,18 +799,26 @@ SPROUT_API int sprout_moe_experts_tc(const void* h, int h_stride, const int* ord
   return sprout_experts_product_tc(act, ff, offsets, order, w_down, rows_out, entries, experts, width, ff, -1, nullptr, 0.f, 0.f, status, stream);
 }
 
-// sprout_moe_route, sprout_moe_arrange and sprout_moe_experts_tc behind one call, for bfloat16 rows of sizes that the last takes;
-// `weight_rows`: the places' weights multiply the experts' first products.
+// sprout_moe_route, sprout_moe_arrange and sprout_moe_experts_tc (`on_tc`) or sprout_moe_experts_mma behind one call, for bfloat16 rows of
+// sizes that the last takes; `weight_rows`: the places' weights multiply the experts' first products.
+SPROUT_API int sprout_moe_experts_mma(const void* h, int h_stride, const int* order, const int* offsets, const void* w_gate_up,
+                                      const void* w_down, void* act, float* rows_out, int entries, int experts, int top,
+                                      int width, int ff, int unit, const float* row_weights, float limit, float alpha,
+                                      cudaStream_t stream);
+
 SPROUT_API int sprout_moe_routed(const void* h, int h_stride, const float* router, const float* correction, int* ids, float* weights, int* counts,
                                  int* offsets, int* order, int* place_of, const void* w_gate_up, const void* w_down, void* act, float* rows_out,
                                  int tokens, int width, int outputs, int experts, int top, float scale, int extra, float* extra_out,
                                  int group_count, int group_keep, int renormalize, int sigmoid_scores, int ff, int unit, int weight_rows, float limit,
-                                 float alpha, int* status, cudaStream_t stream) {
+                                 float alpha, int on_tc, int* status, cudaStream_t stream) {
   SPROUT_REQUIRE((long long)tokens * top <= 0x7fffffffLL, "moe_routed: too many entries");
   const int entries = tokens * top;
   if (int code = sprout_moe_route(h, h_stride, SPROUT_BF16, router, correction, ids, weights, counts, tokens, width, outputs, experts, top, scale, extra,
                                   extra_out, group_count, group_keep, renormalize, sigmoid_scores, stream)) return code;
   if (int code = sprout_moe_arrange(ids, counts, offsets, order, place_of, entries, experts, stream)) return code;
+  if (!on_tc)
+    return sprout_moe_experts_mma(h, h_stride, order, offsets, w_gate_up, w_down, act, rows_out, entries, experts, top, width, ff, unit,
+                                  weight_rows ? weights : nullptr, limit, alpha, stream);
   // the gathered rows lie where the down product, which runs once they have been read, writes its results
   return sprout_moe_experts_tc(h, h_stride, order, offsets, w_gate_up, w_down, rows_out, act, rows_out, entries, experts, top, width, ff, unit,
                                weight_rows ? weights : nullptr, limit, alpha, status, stream);

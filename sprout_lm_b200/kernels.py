@@ -108,7 +108,7 @@ _SIGNATURES = {
     "sprout_latent_rotate": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "sprout_latent_unfolded_attention": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P],
     "sprout_moe_tc_supported": [_I, _I, _I, _I, _I, _I],
-    "sprout_moe_routed": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
+    "sprout_moe_routed": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _P],
     "sprout_clamped_glu_product": [_P, _I, _P, _P, _I, _I, _I, _F, _F, _P, _P],
 }
 
@@ -1760,7 +1760,9 @@ def decay_attention(rows, ctx, state, decay, out, heads: int, dim: int, vdim: in
 
 
 # Elements of an expert's matrix from which its products run on tcgen05 (16 experts of 512 over 512, 256 tokens: 38 us on mma.sync, 28 us
-# on tcgen05; 8 of 256 over 512: 28 and 26 us, but 512 tokens 28 and 34)
+# on tcgen05; 8 of 256 over 512: 28 and 26 us, but 512 tokens 28 and 34), in steps whose entries read 4.5 times as many: with fewer the
+# three launches' ways in and out are longer than the few-token kernel's two (8 experts of 512 over 512, top 2, gated, the products: 1
+# token 9.9 and 13.4 us, 2 10.3 and 13.3, 4 13.3 and 13.9, 7 15.9 and 14.2; 16 of 264 over 1,000 12.3 and 16.0, 13.8 and 15.8, 18.3 and 15.9)
 EXPERTS_TC_ELEMENTS = 1 << 18
 
 
@@ -1771,19 +1773,20 @@ def _experts_route(entries: int, experts: int, top: int, width: int, ff: int, h_
     lib = load_library()
     if not lib.sprout_moe_mma_supported(width, ff, h_stride):
         return "plain"
-    return "tcgen05" if width * ff >= least and lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
+    return "tcgen05" if width * ff >= least and 2 * entries * width * ff > 9 * least and lib.sprout_moe_tc_supported(entries, experts, top, width, ff, h_stride) else "mma_sync"
 
 
 def moe_routed(h, router, correction, counts, offsets, w_gate_up, w_down, experts: int, top: int, scale: float, limit: float, alpha: float,
                unit=None, weight_on_input: bool = False, groups=None, renormalize: bool = True, extra_out=None, sigmoid: bool = False, status=None):
-    """``moe_route``, ``moe_arrange`` and ``moe_experts`` of bfloat16 rows on tcgen05 in one call (a layer of a small step is bound by the
+    """``moe_route``, ``moe_arrange`` and ``moe_experts`` of bfloat16 rows on tensor cores in one call (a layer of a small step is bound by the
     host): (ids, weights, place_of, rows) for ``moe_combine``, or None where these sizes take other kernels."""
     global LAUNCHES
     T, width = h.shape
     entries, ff = T * top, w_down.shape[2]
-    if h.dtype != torch.bfloat16 or h.stride(1) != 1 or status is None or os.environ.get("SPROUT_MOE", "mma") != "mma" \
-            or _experts_route(entries, experts, top, width, ff, h.stride(0), EXPERTS_TC_ELEMENTS) != "tcgen05" \
-            or (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16:
+    if h.dtype != torch.bfloat16 or h.stride(1) != 1 or status is None or os.environ.get("SPROUT_MOE", "mma") != "mma":
+        return None
+    route = _experts_route(entries, experts, top, width, ff, h.stride(0), EXPERTS_TC_ELEMENTS)
+    if route == "plain" or width * ff < EXPERTS_TC_ELEMENTS or (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16:
         return None
     extra = 0 if extra_out is None else extra_out.shape[1]
     outputs = router.shape[0] - extra
@@ -1804,8 +1807,8 @@ def moe_routed(h, router, correction, counts, offsets, w_gate_up, w_down, expert
          place_of.data_ptr(), _ptr(w_gate_up, "w_gate_up", torch.bfloat16), _ptr(w_down, "w_down", torch.bfloat16), act.data_ptr(),
          rows.data_ptr(), T, width, outputs, experts, top, float(scale), extra, _ptr(extra_out, "extra_out", torch.float32, True),
          group_count, group_keep, 1 if renormalize else 0, 1 if sigmoid else 0, ff, code, 1 if weight_on_input else 0, float(limit), float(alpha),
-         _ptr(status, "status", torch.int32), _stream())
-    LAUNCHES += 4               # five kernels behind one call
+         1 if route == "tcgen05" else 0, _ptr(status, "status", torch.int32), _stream())
+    LAUNCHES += 4 if route == "tcgen05" else 3          # five kernels behind one call, or four
     return ids, weights, place_of, rows
 
 

@@ -407,3 +407,16 @@ def test_key_shares_follow_the_places_of_the_kernel():
             changes = [n for n, before in zip(row[1:], row) if n != before]
             assert all(1 <= n <= min(8, tiles) for tiles, n in enumerate(row, 1))
             assert row[0] == 1 and len(set(changes)) == len(changes) <= 7
+
+
+def test_few_entries_of_small_experts_keep_the_few_token_kernel():
+    """The experts' products go to tcgen05 from matrices of 256 x 1,024 on, but not where a step's entries read less than its launches take."""
+    from sprout_lm_b200.kernels import EXPERTS_TC_ELEMENTS, _experts_route
+
+    def route(tokens, experts, top, width, ff):
+        return _experts_route(tokens * top, experts, top, width, ff, width, EXPERTS_TC_ELEMENTS)
+    assert [route(n, 8, 2, 512, 512) for n in (1, 2, 4, 2048)] == ["mma_sync", "mma_sync", "tcgen05", "tcgen05"]
+    assert [route(n, 16, 2, 1000, 264) for n in (1, 2, 4)] == ["mma_sync", "mma_sync", "tcgen05"]
+    assert [route(n, 4, 1, 1024, 1024) for n in (1, 2)] == ["mma_sync", "tcgen05"]
+    assert route(1, 32, 4, 2048, 1024) == route(1, 16, 4, 1024, 512) == "tcgen05"
+    assert route(100, 8, 2, 512, 256) == "mma_sync" and route(100, 8, 2, 516, 512) == "plain"

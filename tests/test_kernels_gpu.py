@@ -1344,6 +1344,28 @@ def test_gated_units_of_exact_products(status, monkeypatch, unit):
         assert torch.equal(results[0].view(torch.int16), other.view(torch.int16))
 
 
+@pytest.mark.parametrize("tokens,weighted", [(1, False), (2, True), (3, False), (40, True)])
+def test_routed_in_one_call(status, tokens, weighted):
+    """Router, arrangement and products behind one call (a few tokens on the few-token kernel, more on tcgen05) give what they give one after another, bit for bit."""
+    from sprout_lm_b200 import kernels
+    experts, top, width, ff = 8, 2, 512, 512
+    g = torch.Generator().manual_seed(tokens)
+    make = lambda *shape: (torch.randn(*shape, generator=g) * shape[-1] ** -0.5).to(torch.bfloat16).to(DEV)
+    h, w_up, w_down, router = make(tokens, width), make(experts, 2 * ff, width), make(experts, width, ff), torch.randn(experts, width, generator=g).to(DEV)
+    counts, offsets = torch.zeros(experts, dtype=torch.int32, device=DEV), torch.zeros(experts + 1, dtype=torch.int32, device=DEV)
+    got_ids, got_weights, got_place, got_rows = kernels.moe_routed(h, router, None, counts, offsets, w_up, w_down, experts, top, 1.5, 7.0, 1.7,
+                                                                   unit="clamped_glu", weight_on_input=weighted, status=status)
+    ids, weights = torch.zeros(tokens, top, dtype=torch.int32, device=DEV), torch.zeros(tokens, top, device=DEV)
+    order, place = (torch.zeros(tokens * top, dtype=torch.int32, device=DEV) for _ in range(2))
+    kernels.moe_route(h, router, None, ids, weights, counts, experts, top, 1.5)
+    kernels.moe_arrange(ids, counts, offsets, order, place, experts)
+    act, rows = torch.empty(tokens * top, ff, dtype=torch.bfloat16, device=DEV), torch.empty(tokens * top, width, device=DEV)
+    kernels.moe_experts(h, order, offsets, w_up, w_down, act, rows, experts, top, 7.0, 1.7, unit="clamped_glu", row_weights=weights if weighted else None, status=status)
+    assert torch.equal(got_ids, ids) and torch.equal(got_weights, weights) and int(status.item()) == 0
+    # entries of an expert may lie in another order: an entry's row is compared
+    assert torch.equal(got_rows[got_place.flatten().long()], rows[place.long()])
+
+
 @pytest.mark.parametrize("unit", ["clamped_glu", "plain"])
 def test_experts_tiles_of_every_width(status, monkeypatch, unit):
     """Rows of an expert in one tile of 16 to 256 columns, in two and more of equal size, features and K that no tile divides."""
