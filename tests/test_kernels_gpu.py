@@ -1372,7 +1372,7 @@ def test_experts_tiles_of_every_width(status, monkeypatch, unit):
     test_experts_on_tcgen05(status, monkeypatch, unit, [15, 16, 31, 33, 240, 241, 255, 513, 0, 783, 4353], 648, 328, False)
 
 
-@pytest.mark.parametrize("experts,entries", [(1, 1), (5, 1025), (33, 8193), (1025, 9000), (2048, 700)])
+@pytest.mark.parametrize("experts,entries", [(1, 1), (5, 1025), (32, 9000), (33, 8193), (1025, 9000), (2048, 700)])
 def test_entries_arranged_by_expert(experts, entries):
     """Offsets from the counts, every entry once within its expert, identity experts without a place, the counts left zeroed."""
     from sprout_lm_b200 import kernels
