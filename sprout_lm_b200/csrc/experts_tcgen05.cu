@@ -14,7 +14,7 @@
 // the grid, an expert's row tiles of the same features side by side, so that the second finds the weights in L2.
 //
 // 32 experts of 1,024 over 2,048 wide rows, top 4, the whole layer when the matrices moved to M: 2,048 tokens 303 -> 272 us, 64 tokens 156 ->
-// 121 (with the router, the arrangement and the calls as they are now 255 and 118).  Both products and the gather 134 and 95 us (cold caches): for 2,048 tokens the gated one takes 70 us, reads 300 MB and keeps the tensor
+// 121 (with the router, the arrangement and the calls as they are now 246 and 117).  Both products and the gather 134 and 95 us (cold caches): for 2,048 tokens the gated one takes 70 us, reads 300 MB and keeps the tensor
 // cores busy for half of that time; for 64 tokens 402 MB pass at 4.2 TB/s with the launches' ends.
 //
 // Waits are bounded as in the dense products.
@@ -33,10 +33,40 @@ constexpr int TABLE_BYTES = (2 * (MAX_EXPERTS + 1) * 4 + 15) / 16 * 16;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TABLE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
 constexpr int ROW_MAPS = 5;                            // boxes of 8, 16, 32, 64 and 128 rows
 
-// The unit is part of the kernel: as a question to every activation it kept them from running side by side.  The activations are those of the
-// other kernels (experts.cuh) with their IEEE quotients: `__fdividef` took the layer of 2,048 tokens from 255 to 245 us, but it is 2 units in
-// the last place off, and 0 where the exponential is above 2^126.
+// The unit is part of the kernel: as a question to every activation it kept them from running side by side.
 enum Kind : int { KIND_CLAMPED = 0, KIND_SILU = 1, KIND_GELU = 2, KIND_DOWN = 3 };
+
+// 1 / x and g / x for x of 1 to infinity (1 + exp), rounded as IEEE has it: from an approximate reciprocal r, r + r (1 - x r) and
+// q + r (g - x q), each remainder in one fused multiply-add (Newton's iteration; its last rounding: P. W. Markstein, IBM J. Res. Develop. 34,
+// 1990).  The operators are right for any operand and branch for that, and eight activations no longer run side by side: 2,048 tokens of
+// 2,048 over 2,048, the clamped unit's product 49 us with them, 31 so.  Compared with the operators: 1 / x over every x up to 2^126, g / x
+// over every bfloat16 g.  Above 2^126 (a sigmoid under 2^-126) 1 / x may be off by the last bit of its denormal.
+__device__ __forceinline__ float scaled_reciprocal(float x, float& scaled, float& scale) {
+  scale = x > 0x1p100f ? 0x1p-64f : 1.0f;                // keeps the reciprocal normal
+  scaled = x * scale;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(scaled));
+  r = fmaf(r, fmaf(-scaled, r, 1.0f), r);
+  return x == INFINITY ? 0.f : r;
+}
+__device__ __forceinline__ float reciprocal_of(float x) {
+  float scaled, scale;
+  return scaled_reciprocal(x, scaled, scale) * scale;
+}
+__device__ __forceinline__ float quotient_of(float g, float x) {
+  float scaled, scale;
+  const float r = scaled_reciprocal(x, scaled, scale), q = g * r, rest = fmaf(-scaled, q, g);
+  return (fabsf(rest) > 0.f ? fmaf(rest, r, q) : q) * scale;       // nothing left, or no number left (infinities): q as it is
+}
+
+// The gated units as the other kernels compute them (experts.cuh).
+template <int KIND>
+__device__ __forceinline__ float gated_unit(float g, float u, float limit, float alpha) {
+  if (KIND == KIND_SILU) return quotient_of(g, 1.0f + expf(-g)) * u;
+  g = fminf(g, limit);
+  u = fminf(fmaxf(u, -limit), limit);
+  return g * reciprocal_of(1.0f + expf(-alpha * g)) * (u + 1.0f);
+}
 
 struct RowMaps { CUtensorMap box[ROW_MAPS]; };
 
@@ -222,7 +252,7 @@ experts_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             // rounded to bfloat16 before the activation, as separate products would leave them
             const float g = __bfloat162float(__float2bfloat16_rn((upper ? other : mine) * weight[j]));
             const float u = __bfloat162float(__float2bfloat16_rn((upper ? mine : other) * weight[j]));
-            v[j] = sprout_experts::glu(KIND == KIND_SILU ? sprout_experts::UNIT_SILU : sprout_experts::UNIT_CLAMPED, g, u, p.limit, p.alpha);
+            v[j] = gated_unit<KIND>(g, u, p.limit, p.alpha);
           }
           __nv_bfloat16* out = (__nv_bfloat16*)p.out + (size_t)(t.row0 + c + upper) * p.N + feature;
           const int left = feature < p.N ? t.rows - c - upper : 0;

@@ -1321,7 +1321,10 @@ def test_gated_units_of_exact_products(status, monkeypatch, unit):
     nothing, everything and nearly too large for float32."""
     from sprout_lm_b200 import kernels
     tokens, ff = 600, 256
-    h = torch.cat([torch.linspace(-92.0, 30.0, tokens * ff).view(tokens, ff), torch.linspace(-9.0, 9.0, tokens * ff).view(ff, tokens).T], 1).to(torch.bfloat16).to(DEV)
+    h = torch.cat([torch.linspace(-92.0, 30.0, tokens * ff).view(tokens, ff), torch.linspace(-9.0, 9.0, tokens * ff).view(ff, tokens).T], 1)
+    special = torch.tensor([0.0, 1e-38, -1e-38, 3e38, -3e38, -89.0, -300.0])
+    h[0, :len(special)] = special
+    h = h.to(torch.bfloat16).to(DEV)
     w = torch.eye(2 * ff, dtype=torch.bfloat16, device=DEV)
     if unit == "dense":
         monkeypatch.setattr(kernels, "GLU_PRODUCT_TILES", 0)
