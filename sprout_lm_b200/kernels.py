@@ -1589,31 +1589,34 @@ def moe_combine(y, h, ids, weights, place_of, rows, top: int, factor: float = 1.
 def multimap_key_split(requests: int, kv_heads: int, group: int, max_q_len: int, planned_keys: int, sms: int | None = None, maps: int = 1,
                        dim: int = 128, vdim: int = 128) -> int:
     """Into how many CTAs, 8 at most, a step of single tokens divides a request's 64-key tiles; 1 for steps with longer portions.  The least of,
-    in us: a tile's time (1.12 of latencies, or what the CTAs beside one another read at 8.7 TB/s) x a CTA's tiles, rounds of CTAs counted with
-    a weight of 1/8 and, since lengths differ, the work over all places (half of it, as contexts are shorter than the longest) and 0.6 of a
-    CTA after them with the rest; 2.1 for every CTA an SM starts; 5.2 for a merge.  An SM holds as many CTAs as their shared memory lets it, at
-    most 6.  A CTA's tiles count as a fraction, so that a growing context meets each number of shares once: captured steps are told apart by it.
+    in us: a tile's time (latencies of 0.8 and 0.45 for every 256 elements of a key and its value, 0.15 more with 16 rows, or what the CTAs beside
+    one another read at 8 TB/s) x a CTA's tiles, rounds of CTAs counted with a weight of 1/5 and, since lengths differ, the work over
+    all places (0.6 of it, as contexts are shorter than the longest) and 0.3 of a CTA after them with the rest; 1.75 for every CTA an SM
+    starts; a merge of 3 to 6.  An SM holds as many CTAs as their shared memory lets it, at most 6.  Beyond 8 tiles a CTA's tiles count as a fraction,
+    so that a growing context changes the number of shares seldom: captured steps are told apart by it.
 
-    Measured with 1 to 8 shares over eight kernels, 32 to 512 CTAs and contexts of 300 to 6,000 keys (1,000 launches): 2 % (geometric mean)
-    above the best, at most 1.2 x; 0.94 of the time of shares by the places alone (three an SM, four shares from 64 tiles on while 222 to 444 CTAs), 0.90
-    of that of a CTA for every SM, at most 1.15 x (heads of 64 + 64, 380 CTAs of 94 tiles, equal lengths: 99 us undivided, 114 in two).  Heads of
+    Measured with 1 to 8 shares over 16 kernels, 1 to 512 CTAs and contexts of 100 to 6,000 keys (1,950 launches): 1.5 % (geometric mean)
+    above the best, at most 1.25 x; 0.94 of the time of shares by the places alone (three an SM, four shares from 64 tiles on while 222 to 444 CTAs), at
+    most 1.12 x; 0.91 of that of a CTA for every SM, at most 1.17 x.  Heads of
     128 + 128, lengths from half to all of 6,000 keys, one and four shares: 256 CTAs 122 and 109, 300 139 and 124, 380 161 and 150, 440 186 and 177, 512 228 and 204 us."""
     if max_q_len * group > 16:
         return 1
     tiles, ctas = max(1, -(-planned_keys // 64)), max(1, requests * kv_heads)
     sms = sms or sm_count()
-    if max_q_len * group <= 8:                  # the CTA's shared memory: its warps' stages, or their results at the end
-        shared = max(256 * (maps * dim + vdim + 16), 16 * (8 * maps * (2 + vdim) + vdim))
-    else:
+    sixteen, elements = max_q_len * group > 8, maps * dim + vdim
+    if sixteen:                                 # the CTA's shared memory: its keys, or its warps' results at the end
         shared = max(288 * (maps * dim + 8) + 256 * (vdim + 8), 512 * maps * (vdim // 2 + 4))
+    else:
+        shared = max(256 * (elements + 16), 16 * (8 * maps * (2 + vdim) + vdim))
     held = max(1, min(6, (227 << 10) // (shared + 1024)))
+    latency, merge = 0.8 + 0.45 * elements / 256 + 0.15 * sixteen, 6.0 * min(1.0, 0.5 + ctas / sms)
     best, least = 1, None
     for shares in range(1, min(8, tiles) + 1):
-        share, beside = tiles / shares, min(held, ctas * shares / sms)
-        tile = max(1.12, 128 * (maps * dim + vdim) * beside * sms / 8.7e6)
+        share, beside = tiles / shares if tiles > 8 else -(-tiles // shares), min(held, ctas * shares / sms)
+        tile = max(latency, 128 * elements * beside * sms / 8e6)
         rounds = -(-ctas * shares // (held * sms)) * share
-        uneven = max(share, 0.5 * ctas * tiles / (held * sms) + 0.6 * share)
-        cost = (rounds / 8 + uneven * 7 / 8) * tile + 2.1 * ctas * shares / sms + (5.2 if shares > 1 else 0.0)
+        uneven = max(share, 0.6 * ctas * tiles / (held * sms) + 0.3 * share)
+        cost = (0.2 * rounds + 0.8 * uneven) * tile + 1.75 * ctas * shares / sms + (merge if shares > 1 else 0.0)
         if least is None or cost < least:
             best, least = shares, cost
     return best

